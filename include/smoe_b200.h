@@ -221,6 +221,13 @@ int smoe_quant_iso32(const void* x_bf16, int64_t rows, int64_t cols, void* q, vo
  * (sonicmoe/quack_utils/blockscaled_fp8_gemm.py:3765-3856): a weight [N,K] is kept once, K-major for the forward
  * GEMM (row_isa) and read MN-major by smoe_gemm_varlen_m_bt for the activation gradient (col_isa). */
 
+/* Expert weights, both orientations from one read: W bf16 [E,N,K] -> q e4m3 [E,N,K] quantised 1x32 along K + ISA scales
+ * for (E*N, K), and q_t e4m3 [E,K,N] quantised 1x32 along N + ISA scales for (K,N) per expert (E consecutive blocks of
+ * K/128 * N/128 * 512 bytes).  A (payload, scales) pair may be null: that orientation is not written.  Replaces the
+ * per-weight caches of sonicmoe/quack_utils/blockscaled_fp8_gemm.py:4243-4315,4363-4406.  N % 128 == 0, K % 128 == 0. */
+int smoe_quant_weight(const void* w_bf16, int64_t E, int64_t N, int64_t K, void* q, void* row_isa, void* q_t,
+                      void* col_isa, void* stream);
+
 /* dst[b][c][r] = src[b][r][c] over a batch of [rows, cols] byte matrices (rows, cols multiples of 64, batch <=
  * 65535).  Makes the transient K-major copy of an ISO32 weight for a GEMM that cannot read it MN-major (the
  * reference does the same for w2 in its backward, sonicmoe/functional/__init__.py:2160). */

@@ -143,43 +143,63 @@ def _base_of(w: torch.Tensor) -> torch.Tensor:
     return w._base if w._base is not None else w
 
 
+def _weight_cache_get(w, base, kind):
+    """(payload, scales) of a cached FP8 copy that is still current, else None."""
+    hit = _WEIGHT_CACHE.get((w.data_ptr(), tuple(w.shape), tuple(w.stride()), kind, w.device.index))
+    # address + version are not enough: a freed weight's address is handed out again by the caching allocator,
+    # with a fresh version counter that can coincide - the entry also remembers WHICH tensor it was made from
+    if hit is not None and hit[0] == base._version and hit[3]() is base:
+        return hit[1], hit[2]
+    return None
+
+
+def _weight_cache_put(w, base, kind, q, sf):
+    if len(_WEIGHT_CACHE) >= _WEIGHT_CACHE_MAX:
+        _WEIGHT_CACHE.pop(next(iter(_WEIGHT_CACHE)))
+    _WEIGHT_CACHE[(w.data_ptr(), tuple(w.shape), tuple(w.stride()), kind, w.device.index)] = (
+        base._version, q, sf, weakref.ref(base))
+
+
+def _bf16_weight(w):
+    src = w.detach()
+    return (src if src.dtype == torch.bfloat16 else src.to(torch.bfloat16)).contiguous()
+
+
 def weight_fp8(w: torch.Tensor, transposed: bool):
     """w [E,N,K] bf16 -> (e4m3 bytes [E,N,K], ISA scales) or, transposed, the same for w^T [E,K,N].
     Replaces precompute_weight_fp8_warmup / the per-weight caches
     (sonicmoe/quack_utils/blockscaled_fp8_gemm.py:299-345,4363-4406)."""
     base = _base_of(w)
-    key = (w.data_ptr(), tuple(w.shape), tuple(w.stride()), transposed, w.device.index)
-    ver = base._version
-    hit = _WEIGHT_CACHE.get(key)
-    # address + version are not enough: a freed weight's address is handed out again by the caching allocator,
-    # with a fresh version counter that can coincide - the entry also remembers WHICH tensor it was made from
-    if hit is not None and hit[0] == ver and hit[3]() is base:
-        return hit[1], hit[2]
+    hit = _weight_cache_get(w, base, transposed)
+    if hit is not None:
+        return hit
     with torch.no_grad():
-        src = w.detach()
-        if src.dtype != torch.bfloat16:
-            src = src.to(torch.bfloat16)
-        src = src.contiguous()
+        src = _bf16_weight(w)
         E, N, K = src.shape
-        if transposed and N % 128 == 0 and K % 128 == 0:
-            # W^T quantised row-wise (1x32 along N) is W quantised column-wise (32 consecutive rows of W) with the
-            # bytes written transposed: the column quantizer reads W as it lies and no transposed bf16 copy is made
-            # (the reference reads each weight once for both orientations, blockscaled_fp8_gemm.py:4243-4315)
-            q = torch.empty(E, K, N, dtype=torch.uint8, device=src.device)
-            per = ops.isa_bytes(K, N)
-            sf = torch.empty(E * per, dtype=torch.uint8, device=src.device)
-            for e in range(E):
-                ops.quant_cols_t(src[e], None, N, out=(q[e], sf[e * per:(e + 1) * per]))
+        if N % 128 == 0 and K % 128 == 0:
+            q, sf = ops.quant_weight(src, rows=not transposed, cols=transposed)[2 * transposed:2 * transposed + 2]
         else:
             if transposed:
                 src = src.transpose(1, 2).contiguous()
                 E, N, K = src.shape
             q, _, sf = ops.quant_rows(src.view(E * N, K), raw=False, isa=True)
             q = q.view(E, N, K)
-    if len(_WEIGHT_CACHE) >= _WEIGHT_CACHE_MAX:
-        _WEIGHT_CACHE.pop(next(iter(_WEIGHT_CACHE)))
-    _WEIGHT_CACHE[key] = (ver, q, sf, weakref.ref(base))
+    _weight_cache_put(w, base, transposed, q, sf)
     return q, sf
+
+
+def _weight_fp8_both(w: torch.Tensor):
+    """Fill both orientations of `weight_fp8`; when both are due, W is read once for the two of them (as the reference
+    does, blockscaled_fp8_gemm.py:4243-4315)."""
+    base = _base_of(w)
+    if w.shape[1] % 128 or w.shape[2] % 128 or any(_weight_cache_get(w, base, t) is not None for t in (False, True)):
+        weight_fp8(w, False)
+        weight_fp8(w, True)
+        return
+    with torch.no_grad():
+        q, sf, q_t, sf_t = ops.quant_weight(_bf16_weight(w))
+    _weight_cache_put(w, base, False, q, sf)
+    _weight_cache_put(w, base, True, q_t, sf_t)
 
 
 def _iso32_ok(w: torch.Tensor) -> bool:
@@ -192,16 +212,11 @@ def weight_fp8_iso32(w: torch.Tensor):
     one, so half the FP8 weight memory of the two 1x32 copies (the reference's ISO32 weight cache,
     sonicmoe/quack_utils/blockscaled_fp8_gemm.py:3765-3856; coarser scales: one per 1024 values instead of 32)."""
     base = _base_of(w)
-    key = (w.data_ptr(), tuple(w.shape), tuple(w.stride()), "iso32", w.device.index)
-    ver = base._version
-    hit = _WEIGHT_CACHE.get(key)
-    if hit is not None and hit[0] == ver and hit[3]() is base:
-        return hit[1], hit[2][0], hit[2][1]
+    hit = _weight_cache_get(w, base, "iso32")
+    if hit is not None:
+        return hit[0], hit[1][0], hit[1][1]
     with torch.no_grad():
-        src = w.detach()
-        if src.dtype != torch.bfloat16:
-            src = src.to(torch.bfloat16)
-        src = src.contiguous()
+        src = _bf16_weight(w)
         E, N, K = src.shape
         q = torch.empty(E, N, K, dtype=torch.uint8, device=src.device)
         per_r, per_c = ops.isa_bytes(N, K), ops.isa_bytes(K, N)
@@ -209,9 +224,7 @@ def weight_fp8_iso32(w: torch.Tensor):
         col_sf = torch.empty(E * per_c, dtype=torch.uint8, device=src.device)
         for e in range(E):
             ops.quant_iso32(src[e], out=(q[e], row_sf[e * per_r:(e + 1) * per_r], col_sf[e * per_c:(e + 1) * per_c]))
-    if len(_WEIGHT_CACHE) >= _WEIGHT_CACHE_MAX:
-        _WEIGHT_CACHE.pop(next(iter(_WEIGHT_CACHE)))
-    _WEIGHT_CACHE[key] = (ver, q, (row_sf, col_sf), weakref.ref(base))
+    _weight_cache_put(w, base, "iso32", q, (row_sf, col_sf))
     return q, row_sf, col_sf
 
 
@@ -283,8 +296,7 @@ def precompute_weight_fp8(w1: torch.Tensor, w2: torch.Tensor, iso32_weight: bool
         if iso and _iso32_ok(w):
             weight_fp8_iso32(w)
         else:
-            weight_fp8(w, False)
-            weight_fp8(w, True)
+            _weight_fp8_both(w)
 
 
 def clear_weight_cache():

@@ -425,6 +425,20 @@ def quant_iso32(x, transposed_payload=True, out=None):
 
 
 @_timed
+def quant_weight(w, rows=True, cols=True):
+    """bf16 [E,N,K] (N, K multiples of 128) -> (q e4m3 [E,N,K] with 1x32 groups along K, ISA scales of (E*N, K), q_t e4m3
+    [E,K,N] with 1x32 groups along N, ISA scales of (K,N) per expert); an orientation switched off is None."""
+    _cuda(w)
+    assert w.dtype == torch.bfloat16 and w.dim() == 3
+    E, N, K = w.shape
+    e = lambda *shape: torch.empty(*shape, dtype=_U8, device=w.device)
+    q, ri = (e(E, N, K), e(isa_bytes(E * N, K))) if rows else (None, None)
+    q_t, ci = (e(E, K, N), e(E * isa_bytes(K, N))) if cols else (None, None)
+    check(lib.smoe_quant_weight(_p(w), E, N, K, _p(q), _p(ri), _p(q_t), _p(ci), _stream()), "quant_weight")
+    return q, ri, q_t, ci
+
+
+@_timed
 def transpose_u8(src):
     """u8 [B, R, C] -> u8 [B, C, R] (R, C multiples of 64)."""
     _cuda(src)

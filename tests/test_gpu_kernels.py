@@ -806,3 +806,23 @@ def test_two_weight_gradients_in_one_launch_give_the_bits_of_two_launches(ops):
             assert torch.equal(o1, r1) and torch.equal(o2, r2), (a_rows_tk, accumulate)
             if not accumulate:
                 assert bool((o1[1] == 0).all()) and bool((o2[1] == 0).all())      # the empty expert
+
+
+@pytest.mark.parametrize("E,N,K", [(1, 128, 128), (3, 256, 128), (2, 384, 512), (5, 128, 640)])
+def test_quant_weight_both_orientations_from_one_read(ops, E, N, K):
+    """Bytes and scales of the row quantizer over W and over W^T, in one pass or one orientation at a time."""
+    g = torch.Generator().manual_seed(E + N + K)
+    w = (torch.randn(E, N, K, generator=g) * torch.exp(2 * torch.randn(E, N, 1, generator=g))).to(torch.bfloat16)
+    w[0, :32] = 0                                        # all-zero groups in both directions
+    w[-1, 5, 7], w[-1, 6, 7] = 1.75 * 2.0 ** 40, 2.0 ** -126          # scale carry threshold, smallest normal
+    wd = w.to(DEV)
+    q, ri, q_t, ci = ops.quant_weight(wd)
+    torch.cuda.synchronize()
+    for got, isa, src, rows, cols in ((q, ri, w, N, K), (q_t, ci, w.transpose(1, 2).contiguous(), K, N)):
+        o_q, o_sc = Q.row_quant(src.view(E * rows, cols).float())
+        assert torch.equal(got.view(E * rows, cols).cpu(), o_q)
+        assert torch.equal(isa.cpu(), Q.pack_isa(o_sc, E * rows, cols))
+    only_q, only_ri, none_q, none_i = ops.quant_weight(wd, cols=False)
+    assert none_q is None and none_i is None and torch.equal(only_q, q) and torch.equal(only_ri, ri)
+    none_q, none_i, only_qt, only_ci = ops.quant_weight(wd, rows=False)
+    assert none_q is None and none_i is None and torch.equal(only_qt, q_t) and torch.equal(only_ci, ci)
