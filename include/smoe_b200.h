@@ -311,6 +311,13 @@ int smoe_gemm_wgrad_mn(const void* a_fp8, const void* a_sf, const void* b_fp8, c
                        float* c, int64_t M, int64_t N, int64_t TKp, int64_t E, int accumulate, int layout,
                        int32_t* status, void* stream);
 
+/* The same product rounded once to bf16 on its way out (c bf16 [E,M,N], overwritten): the gradient of a bf16 parameter
+ * without an f32 main_grad.  Operand layouts as in smoe_gemm_wgrad_mn; with A = the column-quantised dout and B = y1s it
+ * yields dw2 in the parameter's own [E,H,I] order.  M % 256 == 0, N % 256 == 0, E <= 256. */
+int smoe_gemm_wgrad_bf16(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int32_t* efo,
+                         void* c_bf16, int64_t M, int64_t N, int64_t TKp, int64_t E, int layout, int32_t* status,
+                         void* stream);
+
 /* Two such products in ONE launch: c1[e] (+)= A1_e^T B1_e (M1 x N) and c2[e] (+)= A2_e^T B2_e (M2 x N) over the same
  * expert segments - in the layer dw1 (A = dz, B = x) and dw2 (A = y1s, B = dout).  Run one after the other their
  * tile counts (768 and 384 at the reference shape, on 74 CTA pairs) leave a partly filled last wave each; together

@@ -57,6 +57,14 @@ static int make_tmap(CUtensorMap* m, CUtensorMapDataType dt, int esize, const vo
   return r == CUDA_SUCCESS ? SMOE_OK : SMOE_ERR_TMAP;
 }
 
+// Output of a weight gradient, [E, rows, N] in boxes of 32 rows x 64 bytes (f32, or bf16 with GemmParams::out_bf16).
+static int make_tmap_dw(CUtensorMap* m, const GemmParams& p) {
+  return p.out_bf16 ? make_tmap(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.c, (uint64_t)p.E * p.rows, p.N, 32, 32,
+                                CU_TENSOR_MAP_SWIZZLE_64B)
+                    : make_tmap(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.c, (uint64_t)p.E * p.rows, p.N, 16, 32,
+                                CU_TENSOR_MAP_SWIZZLE_64B);
+}
+
 static int g_force_bn = 0;
 static int g_skip_store = 0;
 static int g_force_v1 = 0;
@@ -183,8 +191,7 @@ static int run3(const void* a, int64_t a_rows, int64_t a_cols, const void* b, in
   if (rc) return rc;
   int64_t pair_tiles;
   if (MODE == WGRAD) {
-    rc = make_tmap(&tc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.c, (uint64_t)p.E * p.rows, p.N, 16, 32,
-                   CU_TENSOR_MAP_SWIZZLE_64B);
+    rc = make_tmap_dw(&tc, p);
     pair_tiles = (int64_t)p.E * (p.rows / 256) * (p.N / kBN3);
   } else {
     rc = make_tmap(&tc, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.c, p.rows, p.N, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
@@ -304,8 +311,7 @@ static int run(const void* a, int64_t a_rows, int64_t a_cols, const void* b, int
         rc = make_tmap(&om.c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.c, p.rows, p.N, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
         om.c2 = om.c;
       } else if (MODE == WGRAD) {
-        rc = make_tmap(&om.c, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.c, (uint64_t)p.E * p.rows, p.N, 16, 32,
-                       CU_TENSOR_MAP_SWIZZLE_64B);
+        rc = make_tmap_dw(&om.c, p);
         om.c2 = om.c;
       } else if (MODE == DGATEDQ) {
         rc = make_tmap(&om.c, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.dz, p.rows, 2 * (uint64_t)p.N, 64, 32,
@@ -502,6 +508,25 @@ int smoe_gemm_wgrad_mn(const void* a_fp8, const void* a_sf, const void* b_fp8, c
   p.efo = efo; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)b_sf;
   p.sfa_ktiles = (int)(TKp / 128); p.sfb_ktiles = (int)(TKp / 128);
   p.c = c; p.accumulate = accumulate; p.status = status; p.debug_skip_store = g_skip_store;
+  p.a_mn = layout & 1; p.b_mn = (layout >> 1) & 1;
+  return run<WGRAD>(a_fp8, p.a_mn ? TKp : M, p.a_mn ? M : TKp, b_fp8, p.b_mn ? TKp : N, p.b_mn ? N : TKp, p,
+                    (int)(E * (M / 128) * (N / 128)), (cudaStream_t)stream);
+}
+
+int smoe_gemm_wgrad_bf16(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,
+                         void* c_bf16, int64_t M, int64_t N, int64_t TKp, int64_t E, int layout, int* status,
+                         void* stream) {
+  if (M <= 0 || N <= 0 || M % 256 || N % 256 || TKp < 0 || TKp % 128 || E <= 0 || E > kMaxExperts2 || (layout & ~3))
+    return SMOE_ERR_SHAPE;
+  if (g_force_v1 || g_force_bn == 128 || g_force_bn == 192) return SMOE_ERR_SHAPE;      // the tests' tile forcing
+  if (c_bf16 == nullptr) return SMOE_ERR_ARG;
+  if (TKp == 0)
+    return cudaMemsetAsync(c_bf16, 0, (size_t)E * M * N * 2, (cudaStream_t)stream) == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  GemmParams p{};
+  p.rows = (int)M; p.N = (int)N; p.K = (int)TKp; p.E = (int)E;
+  p.efo = efo; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)b_sf;
+  p.sfa_ktiles = (int)(TKp / 128); p.sfb_ktiles = (int)(TKp / 128);
+  p.c = c_bf16; p.out_bf16 = 1; p.status = status; p.debug_skip_store = g_skip_store;
   p.a_mn = layout & 1; p.b_mn = (layout >> 1) & 1;
   return run<WGRAD>(a_fp8, p.a_mn ? TKp : M, p.a_mn ? M : TKp, b_fp8, p.b_mn ? TKp : N, p.b_mn ? N : TKp, p,
                     (int)(E * (M / 128) * (N / 128)), (cudaStream_t)stream);

@@ -43,6 +43,7 @@ struct GemmParams {
   int rows2;            // WGRAD, 256x384 kernel: output rows per expert of a SECOND product run by the same launch
   void* c2;             //   (same N, K range and operand layouts; own A, B, scales and f32 [E,rows2,N] output); 0: none
   int accumulate;       // WGRAD: add into c instead of overwriting
+  int out_bf16;         // WGRAD (two-CTA kernels): c is bf16 [E,rows,N], rounded once from the f32 accumulator; no accumulate
   int a_mn, b_mn;       // WGRAD (two-CTA kernel): operand stored [TKp, M] / [TKp, N] (MN-major) instead of transposed
   uint8_t* z_fp8;       // GATED out / DGATED in: [TKp, N_z] e4m3
   uint8_t* z_sc;        // raw ue8m0 [TKp, N_z/32]

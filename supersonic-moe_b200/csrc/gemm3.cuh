@@ -391,7 +391,11 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const size_t grow = (size_t)t.m0 + row_in_tile;
       long long es[6] = {0, 0, 0, 0, 0, 0};
       if (t.nkt == 0) {
-        if (MODE == WGRAD && !p.accumulate) {
+        if (MODE == WGRAD && p.out_bf16) {
+          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.c) +
+                                                ((size_t)t.e * p.rows + grow) * p.N + t.n0 + grp * (BN / 2));
+          for (int i = 0; i < BN / 16; ++i) dst[i] = make_uint4(0, 0, 0, 0);
+        } else if (MODE == WGRAD && !p.accumulate) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(t.prob ? p.c2 : p.c) +
@@ -486,6 +490,23 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster_relaxed(tempty0 + 8 * h);
           if (!drain) continue;
+          if (p.out_bf16) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+              const uint32_t sb = stg + buf * 2048;
+              if (lane == 0) bulk_wait_group_read<S::EPI_BUFS - 1>();
+              __syncwarp();
+              stage_bf16_32(sb, lane, acc[c]);
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                tma_store_2d(&tmap_c, sb, t.n0 + h * HN + grp * CPW + c * 32, t.e * p.rows + t.m0 + q * 32);
+                bulk_commit_group();
+              }
+              buf ^= 1;
+            }
+            continue;
+          }
 #pragma unroll
           for (int c = 0; c < 2 * NC; ++c) {
             const uint32_t sb = stg + buf * 2048;

@@ -559,13 +559,17 @@ class _UpProjection(torch.autograd.Function):
             else:                # column scales; payload [TKp, H] or transposed, whichever the GEMM runs fastest on
                 xc, x_sf, xc_rows = _col_operand(x, x_gather_idx, TKp, efo[-1:], E, N2, H)
             mg, base = _grad_target(w1, (E, N2, H))
-            out = mg if mg is not None else torch.empty(E, N2, H, dtype=torch.float32, device=dz_q.device)
+            in_bf16 = mg is None and w1.dtype == torch.bfloat16 and _mn_wgrad_ok(E, N2, H)
+            if not in_bf16:
+                out = mg if mg is not None else torch.empty(E, N2, H, dtype=torch.float32, device=dz_q.device)
             # a row-major dz payload (32x32-block scales) doubles as the MN-major weight-gradient operand
             if paired is not None and not xc_rows:
                 ops.gemm_wgrad_pair(dz_q, dz_csf, xc, x_sf, mg, paired["a_op"], paired["sf_a"], paired["b_op"],
                                     paired["sf_b"], paired["mg"], efo, True, True)
                 _after_accumulate(paired["base"])
                 paired = None
+            elif in_bf16:        # no f32 gradient exists: the epilogue rounds to the parameter's type
+                dw1 = ops.gemm_wgrad_bf16(dz_q if dz_t is None else dz_t, dz_csf, xc, x_sf, efo, E, dz_t is None, xc_rows)
             else:
                 if paired is not None:
                     deferred_dw2()
@@ -574,7 +578,7 @@ class _UpProjection(torch.autograd.Function):
                        mg is not None)
             if mg is not None:
                 _after_accumulate(base)
-            else:
+            elif not in_bf16:
                 dw1 = out.to(w1.dtype)
             del xc, x_sf
         del dz_q, dz_rsf, dz_t, dz_csf
@@ -739,6 +743,9 @@ class _DownProjection(torch.autograd.Function):
             elif mg is not None:
                 _wgrad(a_op, y1s_sf, a_rows, b_op, dout_sf, b_rows, efo, mg, True)
                 _after_accumulate(base)
+            elif w2.dtype == torch.bfloat16 and _mn_wgrad_ok(E, H, I):
+                # operands exchanged: the product leaves as bf16 [E,H,I], the layout of the parameter itself
+                dw2 = ops.gemm_wgrad_bf16(b_op, dout_sf, a_op, y1s_sf, efo, E, b_rows, a_rows)
             else:
                 out = torch.empty(E, I, H, dtype=torch.float32, device=s.device)
                 _wgrad(a_op, y1s_sf, a_rows, b_op, dout_sf, b_rows, efo, out, False)

@@ -582,6 +582,20 @@ def gemm_wgrad_mn(a, a_sf, b, b_sf, efo, out, accumulate, a_rowmajor_tk, b_rowma
 
 
 @_timed
+def gemm_wgrad_bf16(a, a_sf, b, b_sf, efo, E, a_rowmajor_tk, b_rowmajor_tk):
+    """Weight gradient rounded to bf16 in the GEMM's epilogue -> bf16 [E,M,N]; operands as in `gemm_wgrad_mn`."""
+    _cuda(a, a_sf, b, b_sf, efo)
+    TKp, M = a.shape if a_rowmajor_tk else a.shape[::-1]
+    N = b.shape[1] if b_rowmajor_tk else b.shape[0]
+    assert tuple(b.shape) == ((TKp, N) if b_rowmajor_tk else (N, TKp))
+    out = torch.empty(E, M, N, dtype=torch.bfloat16, device=a.device)
+    layout = (1 if a_rowmajor_tk else 0) | (2 if b_rowmajor_tk else 0)
+    check(lib.smoe_gemm_wgrad_bf16(_p(a), _p(a_sf), _p(b), _p(b_sf), _p(efo), _p(out), M, N, TKp, E, layout,
+                                   _p(status_word(a.device)), _stream()), "gemm_wgrad_bf16")
+    return out
+
+
+@_timed
 def gemm_wgrad_pair(a1, a1_sf, b1, b1_sf, out1, a2, a2_sf, b2, b2_sf, out2, efo, accumulate, a_rowmajor_tk):
     """Two weight gradients in one launch (256 x 384 kernel): out1 [E,M1,N] (+)= A1^T B1 and out2 [E,M2,N] (+)= A2^T B2
     over the same expert segments.  A operands u8 [TKp, M] (a_rowmajor_tk) or [M, TKp]; B operands u8 [N, TKp];

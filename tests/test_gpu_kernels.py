@@ -826,3 +826,25 @@ def test_quant_weight_both_orientations_from_one_read(ops, E, N, K):
     assert none_q is None and none_i is None and torch.equal(only_q, q) and torch.equal(only_ri, ri)
     none_q, none_i, only_qt, only_ci = ops.quant_weight(wd, rows=False)
     assert none_q is None and none_i is None and torch.equal(only_qt, q_t) and torch.equal(only_ci, ci)
+
+
+@pytest.mark.parametrize("layout", [0, 1, 2, 3])
+@pytest.mark.parametrize("M,N,tiles", [(256, 256, [1, 0, 2, 1]), (512, 768, [3, 2, 0, 0, 4, 1, 1, 2]), (256, 384 * 4, [9, 0, 5])])
+def test_gemm_wgrad_bf16_is_the_rounded_f32_product(ops, layout, M, N, tiles):
+    """Same kernel, same sums, one rounding: bit for bit the f32 result converted to bf16; empty experts are zero."""
+    g = torch.Generator().manual_seed(M + N + layout)
+    E = len(tiles)
+    efo = make_efo(tiles)
+    TKp = int(efo[-1]) + 128
+    a_q, a_sc = rand_fp8((M, TKp), g)
+    b_q, b_sc = rand_fp8((N, TKp), g)
+    a_sf, b_sf = Q.pack_isa(a_sc, M, TKp).to(DEV), Q.pack_isa(b_sc, N, TKp).to(DEV)
+    a_in = a_q.to(DEV).t().contiguous() if layout & 1 else a_q.to(DEV)
+    b_in = b_q.to(DEV).t().contiguous() if layout & 2 else b_q.to(DEV)
+    want = torch.full((E, M, N), 7.0, device=DEV)
+    ops.gemm_wgrad_mn(a_in, a_sf, b_in, b_sf, efo.to(DEV), want, False, bool(layout & 1), bool(layout & 2))
+    got = ops.gemm_wgrad_bf16(a_in, a_sf, b_in, b_sf, efo.to(DEV), E, bool(layout & 1), bool(layout & 2))
+    torch.cuda.synchronize()
+    ops.check_status(DEV)
+    assert torch.equal(got, want.to(torch.bfloat16))
+    assert all((got[e] == 0).all() for e in range(E) if tiles[e] == 0)
