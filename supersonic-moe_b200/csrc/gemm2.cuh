@@ -255,6 +255,32 @@ __device__ __forceinline__ PairTile pair_tile(int tile, int rank, const GemmPara
   return t;
 }
 
+// s_pairs[e] = row pairs (256 rows) of the experts before e, s_pairs[E] = all of them; one warp, eight experts a lane
+__device__ __forceinline__ void prefix_row_pairs(const int* s_efo, int* s_pairs, int E, int lane) {
+  constexpr int PER = (kMaxExperts2 + 31) / 32;
+  int v[PER], sum = 0;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = lane * PER + i;
+    v[i] = e < E ? ((s_efo[e + 1] - s_efo[e]) / BM + 1) >> 1 : 0;
+    sum += v[i];
+  }
+  int inc = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, inc, d);
+    if (lane >= d) inc += y;
+  }
+  int run = inc - sum;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = lane * PER + i;
+    if (e <= E) s_pairs[e] = run;
+    run += v[i];
+  }
+  if (lane == 31 && E == 32 * PER) s_pairs[E] = run;
+}
+
 template <int BN, int MODE, bool CPG = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((Gemm2Smem<BN, MODE, CPG>::THREADS), 1)
 gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -289,13 +315,8 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   for (int i = threadIdx.x; i <= p.E; i += blockDim.x) s_efo[i] = p.efo[i];
   __syncthreads();
+  if (warp == 2) prefix_row_pairs(s_efo, s_pairs, p.E, lane);
   if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int e = 0; e < p.E; ++e) {
-      s_pairs[e] = acc;
-      acc += ((s_efo[e + 1] - s_efo[e]) / BM + 1) >> 1;
-    }
-    s_pairs[p.E] = acc;
     for (int s = 0; s < S::STAGES; ++s) {
       mbar_init(bar_full + 8 * s, S::FULL_ARRIVALS);   // leader's: its producer arms it, both CTAs' copies credit it
       mbar_init(bar_empty + 8 * s, 1);       // one commit arrival per use, in each CTA
@@ -360,6 +381,12 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const int b_row = (b_mn_plain ? n0 : b_base) + rank * (BN / 2);
       const int b_k0 = b_mn_plain ? te * p.K : 0;
       const int a_row = valid ? m0 : 0;
+      // an expert with an odd number of row tiles: the pair's second half is a phantom, whose A rows need not be
+      // fetched (whatever its ring slots hold only reaches accumulator rows that nobody stores)
+      const bool phantom = MODE != WGRAD && !GATHER && !CPG &&
+                           __shfl_sync(0xffffffffu, m0 + (rank ? 0 : BM) >= s_efo[te + 1], 0);
+      const uint32_t tx_bytes = S::TX_BYTES - (phantom ? S::A_BYTES : 0);
+      const bool load_a = !(phantom && rank == 1);
       for (int kt = kt0; kt < kt0 + nkt; ++kt) {
         ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * stage, phase ^ 1));
         if (!ok) break;
@@ -371,9 +398,9 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         } else {
           ++dbg_filled;
           if (elect_one()) {
-            if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, S::TX_BYTES);
+            if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, tx_bytes);
             if (a_mn) tma_load_2d_pair(a_dst, &tmap_a, full, m0, kt * BK);
-            else if (!GATHER && !CPG) tma_load_2d_pair(a_dst, &tmap_a, full, kt * BK, a_row);
+            else if (!GATHER && !CPG && load_a) tma_load_2d_pair(a_dst, &tmap_a, full, kt * BK, a_row);
             if (b_mn) tma_load_2d_pair(b_dst, &tmap_b, full, b_row, b_k0 + kt * BK);
             else tma_load_2d_pair(b_dst, &tmap_b, full, kt * BK, b_row);
             const int kp = kt + p.l2_prefetch;

@@ -92,13 +92,8 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   for (int i = threadIdx.x; i <= p.E; i += blockDim.x) s_efo[i] = p.efo[i];
   __syncthreads();
+  if (warp == 2) prefix_row_pairs(s_efo, s_pairs, p.E, lane);
   if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int e = 0; e < p.E; ++e) {
-      s_pairs[e] = acc;
-      acc += ((s_efo[e + 1] - s_efo[e]) / BM + 1) >> 1;
-    }
-    s_pairs[p.E] = acc;
     for (int s = 0; s < S::STAGES; ++s) {
       mbar_init(bar_full + 8 * s, 1);        // leader's: its own producer arms it; both CTAs' copies credit it
       mbar_init(bar_empty + 8 * s, 1);       // one commit arrival per use, in each CTA
@@ -158,6 +153,9 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const int b_base = (MODE == WGRAD) ? n0 : te * p.N + n0;
       const int b_row = b_base + rank * (HN / 2);        // this CTA's 96 rows of half 0; half 1 lies HN rows further
       const int a_row = valid ? m0 : 0;
+      // the phantom half of an odd last row pair: its A rows are not fetched (see gemm2_mxf8_kernel)
+      const bool phantom = MODE != WGRAD && __shfl_sync(0xffffffffu, m0 + (rank ? 0 : BM) >= s_efo[te + 1], 0);
+      const uint32_t tx_bytes = S::TX_BYTES - (phantom ? S::A_BYTES : 0);
       const bool second_prob = MODE == WGRAD && __shfl_sync(0xffffffffu, tl.prob, 0) != 0;
       const CUtensorMap* ta = second_prob ? &second.a : &tmap_a;
       const CUtensorMap* tb = second_prob ? &second.b : &tmap_b;
@@ -172,9 +170,9 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         } else {
           ++dbg_filled;
           if (elect_one()) {
-            if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, S::TX_BYTES);
+            if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, tx_bytes);
             if (a_mn) tma_load_2d_pair(a_dst, ta, full, m0, kt * BK);
-            else tma_load_2d_pair(a_dst, ta, full, kt * BK, a_row);
+            else if (!(phantom && rank == 1)) tma_load_2d_pair(a_dst, ta, full, kt * BK, a_row);
             tma_load_2d_pair(b_dst, tb, full, kt * BK, b_row);
             tma_load_2d_pair(b_dst + S::BH_BYTES, tb, full, kt * BK, b_row + HN);
           }
