@@ -168,7 +168,8 @@ int smoe_quant_dual_gather(const void* x_bf16, const int32_t* idx, const int32_t
 
 /* Same result in scatter form: every token row of x [T,K] is read and quantised once and written to each
  * expert-sorted position it occupies, s_rev[naept[t] .. naept[t+1]); pad rows (s_scatter_idx[row] >= naept[T]) are
- * zero-filled (the gather form copies token 0 there; either way they are multiplied by a zero score downstream).
+ * zero-filled (the gather form copies token 0 there; either way they are multiplied by a zero score downstream), or
+ * left as they are when s_scatter_idx is null (enough where no backward follows).
  * K % 128 == 0, K <= 16384. */
 int smoe_quant_rows_scatter(const void* x_bf16, int64_t T, int64_t K, const int32_t* naept, const int32_t* s_rev,
                             const int32_t* s_scatter_idx, const int32_t* valid_rows, int64_t rows, void* q,
@@ -242,6 +243,13 @@ int smoe_transpose_u8(const void* src, int64_t batch, int64_t rows, int64_t cols
 int smoe_gemm_varlen_m(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int32_t* efo,
                        void* c_bf16, int64_t rows, int64_t N, int64_t K, int64_t E, int32_t* status, void* stream);
 
+/* The same, not storing what only padding would receive: where s_scatter_idx (may be null: as above) says that 32
+ * consecutive rows are all padding (s_scatter_idx[row] >= *real_tk), their rows of c are left untouched.  The combine reads
+ * real rows only. */
+int smoe_gemm_varlen_m_live(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,
+                            const int* s_scatter_idx, const int* real_tk, void* c_bf16, int64_t rows, int64_t N, int64_t K,
+                            int64_t E, int* status, void* stream);
+
 /* The same product with B stored [E,K,N] (N contiguous, "MN-major"): B[e] is read as it lies in a weight kept once
  * for both orientations; b_sf = ISA scales for (E*N, K) as above.  Replaces the zero-copy `.permute(0,2,1)` view the
  * reference hands its GEMM in ISO32 mode (sonicmoe/quack_utils/blockscaled_fp8_gemm.py:3822-3840).  256-column
@@ -262,6 +270,12 @@ int smoe_gemm_varlen_m_bt(const void* a_fp8, const void* a_sf, const void* b_kn_
 int smoe_gemm_gated(const void* x_fp8, int64_t T, const int32_t* a_idx, const void* a_sf, const void* w1_fp8,
                     const void* w1_sf, const int32_t* efo, void* z_fp8, void* z_scales, void* y1_fp8, void* y1_sf,
                     int64_t rows, int64_t N, int64_t K, int64_t E, int32_t* status, void* stream);
+
+/* smoe_gemm_gated where no backward follows: z is not written, nor y1 rows of 32-row groups of nothing but padding
+ * (s_scatter_idx[row] >= *real_tk); pad rows of x may hold anything.  Expert-sorted x [rows,K]; E <= 256. */
+int smoe_gemm_gated_infer(const void* x_sorted_fp8, const void* a_sf, const void* w1_fp8, const void* w1_sf, const int* efo,
+                          const int* s_scatter_idx, const int* real_tk, void* y1_fp8, void* y1_sf, int64_t rows, int64_t N,
+                          int64_t K, int64_t E, int* status, void* stream);
 
 /* Backward of the activation: D = dout[a_idx] . W2T[e]^T (N = I, K = H) and, against the saved e4m3 z,
  * dz (bf16 [rows,2N]), y1s = s*y (bf16 [rows,N]) and per-column-tile partial sums of ds ([partials, rows] f32).

@@ -325,16 +325,18 @@ static int run(const void* a, int64_t a_rows, int64_t a_cols, const void* b, int
           rc = make_tmap(&om.c2, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.y1s, p.rows, p.N, 32, 32,
                          CU_TENSOR_MAP_SWIZZLE_64B);
       } else {  // GATED: z e4m3 [rows, N] in 32 x 64 boxes, y1 e4m3 [rows, N/2] in 32 x 32 boxes
-        rc = make_tmap(&om.c, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.z_fp8, p.rows, p.N, 64, 32, CU_TENSOR_MAP_SWIZZLE_64B);
-        if (!rc)
-          rc = make_tmap(&om.c2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.y1_fp8, p.rows, p.N / 2, 32, 32,
-                         CU_TENSOR_MAP_SWIZZLE_32B);
+        rc = make_tmap(&om.c2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.y1_fp8, p.rows, p.N / 2, 32, 32,
+                       CU_TENSOR_MAP_SWIZZLE_32B);
+        om.c = om.c2;                                   // without z the map is never used
+        if (!rc && p.z_fp8 != nullptr)
+          rc = make_tmap(&om.c, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.z_fp8, p.rows, p.N, 64, 32, CU_TENSOR_MAP_SWIZZLE_64B);
       }
       if (rc) return rc;
       om.c3 = om.c;
       return run2<MODE>(a, a_rows, a_cols, b, b_rows, b_cols, p, om, bn2, sfa_tiles, sfb_tiles, stream);
     }
   }
+  if (MODE == GATED && p.z_fp8 == nullptr) return SMOE_ERR_SHAPE;       // z may be left out in the two-CTA kernel only
   if (MODE == DGATEDQ) return SMOE_ERR_SHAPE;     // fused-quantizer epilogue exists in the two-CTA kernel only
   if ((MODE == WGRAD || MODE == PLAIN) && (p.a_mn || p.b_mn)) return SMOE_ERR_SHAPE;   // so do MN-major operands
   constexpr int M1 = (MODE == DGATEDQ) ? DGATED : MODE;
@@ -379,16 +381,24 @@ int smoe_internal_gemm_knobs(int bn) {
   return SMOE_OK;
 }
 
-int smoe_gemm_varlen_m(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,
-                       void* c_bf16, int64_t rows, int64_t N, int64_t K, int64_t E, int* status, void* stream) {
+int smoe_gemm_varlen_m_live(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,
+                            const int* s_scatter_idx, const int* real_tk, void* c_bf16, int64_t rows, int64_t N, int64_t K,
+                            int64_t E, int* status, void* stream) {
   if (rows < 0 || rows % 128 || N % 128 || K % 128 || E <= 0) return SMOE_ERR_SHAPE;
   if (rows == 0) return SMOE_OK;                  // no routed rows (an expert-parallel rank may receive none)
+  if (s_scatter_idx != nullptr && real_tk == nullptr) return SMOE_ERR_ARG;
   GemmParams p{};
   p.rows = (int)rows; p.N = (int)N; p.K = (int)K; p.E = (int)E;
   p.efo = efo; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)b_sf;
   p.sfa_ktiles = (int)(K / 128); p.sfb_ktiles = (int)(K / 128);
+  p.s_scatter = s_scatter_idx; p.real_tk = real_tk;
   p.c = c_bf16; p.status = status; p.debug_skip_store = g_skip_store;
   return run<PLAIN>(a_fp8, rows, K, b_fp8, E * N, K, p, (int)((rows / 128) * (N / 128)), (cudaStream_t)stream);
+}
+
+int smoe_gemm_varlen_m(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,
+                       void* c_bf16, int64_t rows, int64_t N, int64_t K, int64_t E, int* status, void* stream) {
+  return smoe_gemm_varlen_m_live(a_fp8, a_sf, b_fp8, b_sf, efo, nullptr, nullptr, c_bf16, rows, N, K, E, status, stream);
 }
 
 int smoe_gemm_varlen_m_bt(const void* a_fp8, const void* a_sf, const void* b_kn_fp8, const void* b_sf, const int* efo,
@@ -417,6 +427,21 @@ int smoe_gemm_gated(const void* x_fp8, int64_t T, const int* a_idx, const void* 
   p.z_fp8 = (uint8_t*)z_fp8; p.z_sc = (uint8_t*)z_scales; p.y1_fp8 = (uint8_t*)y1_fp8; p.y1_sf = (uint8_t*)y1_sf;
   p.status = status; p.debug_skip_store = g_skip_store;
   return run<GATED>(x_fp8, T, K, w1_fp8, E * N, K, p, (int)((rows / 128) * (N / 128)), (cudaStream_t)stream);
+}
+
+int smoe_gemm_gated_infer(const void* x_sorted_fp8, const void* a_sf, const void* w1_fp8, const void* w1_sf, const int* efo,
+                          const int* s_scatter_idx, const int* real_tk, void* y1_fp8, void* y1_sf, int64_t rows, int64_t N,
+                          int64_t K, int64_t E, int* status, void* stream) {
+  if (rows < 0 || rows % 128 || N % 256 || K % 128 || E <= 0 || E > kMaxExperts2 || g_force_v1) return SMOE_ERR_SHAPE;
+  if (rows == 0) return SMOE_OK;
+  if (s_scatter_idx == nullptr || real_tk == nullptr) return SMOE_ERR_ARG;
+  GemmParams p{};
+  p.rows = (int)rows; p.N = (int)N; p.K = (int)K; p.E = (int)E;
+  p.efo = efo; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)w1_sf;
+  p.sfa_ktiles = (int)(K / 128); p.sfb_ktiles = (int)(K / 128);
+  p.y1_fp8 = (uint8_t*)y1_fp8; p.y1_sf = (uint8_t*)y1_sf; p.s_scatter = s_scatter_idx; p.real_tk = real_tk;
+  p.status = status; p.debug_skip_store = g_skip_store;
+  return run<GATED>(x_sorted_fp8, rows, K, w1_fp8, E * N, K, p, (int)((rows / 128) * (N / 128)), (cudaStream_t)stream);
 }
 
 int64_t smoe_gemm_dgated_partials(int64_t N);

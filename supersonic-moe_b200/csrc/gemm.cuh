@@ -57,6 +57,8 @@ struct GemmParams {
   uint8_t* dz_col_sf;   // DGATEDQ out: ISA scales of dz^T as a (2N, TKp) operand
   uint8_t* y1s_col_sf;  // DGATEDQ out: ISA scales of y1s^T as a (N, TKp) operand (1x32 along TKp)
   int* status;          // device status word: 0 ok, else first failure code
+  const int* s_scatter; // PLAIN / GATED, may be null: row r is padding where s_scatter[r] >= *real_tk; 32-row slabs of
+  const int* real_tk;   // nothing but padding are then not stored (the two-CTA kernels)
   int debug_skip_store; // timing experiments only: drain TMEM but skip the global stores
   int dbg_stage_cut;    // timing experiments only: use this many fewer ring stages
   int l2_prefetch;      // K tiles ahead of the shared-memory ring at which operand tiles are prefetched into L2 (0 = off)

@@ -281,6 +281,13 @@ __device__ __forceinline__ void prefix_row_pairs(const int* s_efo, int* s_pairs,
   if (lane == 31 && E == 32 * PER) s_pairs[E] = run;
 }
 
+// Whether a warp's 32 rows starting at `row` hold anything to store.  The padding of an expert's segment lies at its end,
+// so a slab whose first row is padding is all padding.  A decode step of 64 tokens over 128 experts has four real rows in
+// each 128-row tile: three of a tile's four slabs are left out.
+__device__ __forceinline__ bool slab_live(const GemmParams& p, const PairTile& t, int row) {
+  return t.valid && (p.s_scatter == nullptr || p.s_scatter[row] < *p.real_tk);
+}
+
 template <int BN, int MODE, bool CPG = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((Gemm2Smem<BN, MODE, CPG>::THREADS), 1)
 gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -651,6 +658,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         sc = *reinterpret_cast<const uint16_t*>(p.z_sc + grow * (Nz / 32) + (2 * c_base) / 32);
         s_row = p.s[grow];
       }
+      const bool live = (MODE == PLAIN || MODE == GATED) && slab_live(p, t, t.m0 + q * 32);
       if (lane == 0) ok = mbar_wait(bar_tfull + 8 * as, aphase);
       ok = __shfl_sync(0xffffffff, ok, 0);
       if (!ok) break;
@@ -689,7 +697,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           const uint32_t sb = stg;                 // one 2 KB staging buffer per warp
           if (lane == 0) bulk_wait_group_read<0>();
           __syncwarp();
-          if (t.valid) {
+          if (live) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
               st_shared_v4(sb + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4), pk[c][4 * j], pk[c][4 * j + 1],
@@ -779,7 +787,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
 #pragma unroll
         for (int ci = 0; ci < PER; ++ci) {
-          if (ci >= nch) break;
+          if (ci >= nch || !live) break;
           const int zc = t.n0 + (ch0 + ci) * 64;           // first z column of the chunk
           float y[32];
           uint32_t zs = 0;
@@ -794,14 +802,15 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               tmem_ld_wait();
             }
             const uint32_t* r = DRAIN ? &acc[DRAIN ? (ci * 2 + h) * 32 : 0] : rl;
-            float amax = 0.f;
-#pragma unroll
-            for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(__uint_as_float(r[i])));
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               const float g = __uint_as_float(r[2 * i]), u = __uint_as_float(r[2 * i + 1]);
               y[h * 16 + i] = bf16_rne((g * fast_sigmoid(g)) * u);
             }
+            if (p.z_fp8 == nullptr) continue;              // no backward will read z
+            float amax = 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(__uint_as_float(r[i])));
             const int e = e8m0_of(fmaxf(amax, 1e-4f));
             const float qs = qscale_of(e);
             zs |= (uint32_t)e << (8 * h);
@@ -833,13 +842,13 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
           fence_proxy_async_smem();
           __syncwarp();
-          if (t.valid && !(p.debug_skip_store & 1)) {
+          if (!(p.debug_skip_store & 1)) {
             if (lane == 0) {
-              tma_store_2d(&tmap_c, stg, zc, t.m0 + q * 32);                 // z e4m3 [rows, 2I]
+              if (p.z_fp8 != nullptr) tma_store_2d(&tmap_c, stg, zc, t.m0 + q * 32);     // z e4m3 [rows, 2I]
               tma_store_2d(&tmap_c2, stg + 2048, zc / 2, t.m0 + q * 32);     // y1 e4m3 [rows, I]
               bulk_commit_group();
             }
-            *reinterpret_cast<uint16_t*>(p.z_sc + grow * (Nz / 32) + zc / 32) = (uint16_t)zs;
+            if (p.z_fp8 != nullptr) *reinterpret_cast<uint16_t*>(p.z_sc + grow * (Nz / 32) + zc / 32) = (uint16_t)zs;
             const int g = zc / 64;
             p.y1_sf[((grow / 128) * (size_t)(Ny / 128) + g / 4) * 512 + (grow % 32) * 16 + ((grow % 128) / 32) * 4 +
                     (g % 4)] = (uint8_t)e;

@@ -405,6 +405,7 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         continue;
       }
       if (MODE == PLAIN) {
+        const bool live = slab_live(p, t, t.m0 + q * 32);
         // both halves are drained (bf16-packed) before anything is stored, so that neither accumulator waits
         // for the other one's stores
         uint32_t pk[2][NC][16];
@@ -447,7 +448,7 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           for (int i = 0; i < 6; ++i) etrace[8 * etrace_n + i] = es[i];
         }
         ++etrace_n;
-        if (t.valid && !(p.debug_skip_store & 8)) {
+        if (live && !(p.debug_skip_store & 8)) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
 #pragma unroll

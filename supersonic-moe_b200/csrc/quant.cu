@@ -606,13 +606,15 @@ int smoe_quant_rows_scatter(const void* x_bf16, int64_t T, int64_t K, const int3
                             void* isa_scales, void* stream) {
   if (T < 0 || rows < 0 || K <= 0 || K % 128 || K > 16384) return SMOE_ERR_SHAPE;
   if (rows == 0) return SMOE_OK;      // nothing routed: not an error, and the (empty) buffers may be null
-  if (!naept || !s_rev || !s_scatter_idx || !isa_scales) return SMOE_ERR_ARG;
+  if (!naept || !s_rev || !isa_scales) return SMOE_ERR_ARG;
   if (((uintptr_t)x_bf16 & 15) || ((uintptr_t)q & 15)) return SMOE_ERR_ALIGN;
   const int row_bytes = (int)((K + 4 * (K / 128) + 15) & ~(int64_t)15);
   const int warps = row_bytes * 8 <= 48 * 1024 ? 8 : (row_bytes * 4 <= 48 * 1024 ? 4 : 2);
   const int token_blocks = (int)((T + warps - 1) / warps);
   int pad_blocks = (int)((rows + 63) / 64);
   if (pad_blocks > 296) pad_blocks = 296;
+  if (!s_scatter_idx) pad_blocks = 0;               // pad rows stay as they are
+  if (token_blocks + pad_blocks == 0) return SMOE_OK;
   quant_rows_scatter_kernel<<<token_blocks + pad_blocks, warps * 32, (size_t)warps * row_bytes,
                               (cudaStream_t)stream>>>((const uint4*)x_bf16, T, (int)K, naept, s_rev, s_scatter_idx,
                                                       valid_rows, rows, (uint4*)q, (uint8_t*)isa_scales, token_blocks);

@@ -239,10 +239,10 @@ def _weight_operand(w: torch.Tensor, transposed: bool, iso32: bool):
     return q, sf, False
 
 
-def _gemm_plain(a_q, a_sf, b_q, b_sf, stored_kn, efo):
+def _gemm_plain(a_q, a_sf, b_q, b_sf, stored_kn, efo, s_scatter_idx=None, naept=None):
     """rows grouped by expert x B[e]^T -> bf16.  `stored_kn`: B lies [E, K, N] (see `_weight_operand`)."""
     if not stored_kn:
-        return ops.gemm_varlen_m(a_q, a_sf, b_q, b_sf, efo)
+        return ops.gemm_varlen_m(a_q, a_sf, b_q, b_sf, efo, s_scatter_idx, naept)
     E, K, N = b_q.shape
     if N % 256 == 0 and E <= 256:
         return ops.gemm_varlen_m_bt(a_q, a_sf, b_q, b_sf, efo)
@@ -446,11 +446,12 @@ class _UpProjection(torch.autograd.Function):
         return super().apply(x, w1, b1, expert_frequency_offset, total_expert_freq, K, stream_id, x_gather_idx,
                              s_scatter_idx, s_reverse_scatter_idx, num_activated_expert_per_token_offset,
                              is_varlen_K, activation_type, is_inference_mode_enabled,
-                             use_low_precision_postact_buffer, prequant_activation_payload, fp8_config)
+                             use_low_precision_postact_buffer, prequant_activation_payload, fp8_config,
+                             torch.is_grad_enabled())
 
     @staticmethod
     def forward(ctx, x, w1, b1, efo, TKp, K, stream_id, x_gather_idx, s_scatter_idx, s_rev, naept, is_varlen_K,
-                activation_type, is_inference, low_precision_postact, prequant_payload, fp8_config):
+                activation_type, is_inference, low_precision_postact, prequant_payload, fp8_config, grad_mode):
         ctx.set_materialize_grads(False)   # an unused output must not be handed a zero-filled [TKp, I] gradient
         _require_fp8()
         act = activation_code(activation_type)
@@ -477,6 +478,8 @@ class _UpProjection(torch.autograd.Function):
         elif USE_TMA_GATHER and act == 0:
             x_q, x_raw, _ = ops.quant_rows(x.contiguous(), raw=True)
         iso32, stagewise = _modes(fp8_config)
+        # no graph is recorded, so no backward will read z (nor finite values in the pad rows of x)
+        no_z = not grad_mode and act == 0 and gated_out is None and E <= 256
         w1_q, w1_sf, _ = _weight_operand(w1, False, iso32)
         if USE_TMA_GATHER and act == 0:
             a_sf = packed_sf if packed_sf is not None else ops.gather_scales_isa(x_raw, x_gather_idx, TKp, H)
@@ -489,8 +492,13 @@ class _UpProjection(torch.autograd.Function):
             elif x_q is not None:
                 xg_q, a_sf = ops.scatter_rows_fp8(x_q, x_raw, naept, s_rev, s_scatter_idx, TKp, efo[-1:])
             else:      # quantise straight into expert-sorted order
-                xg_q, a_sf = ops.quant_rows_scatter(x.contiguous(), naept, s_rev, s_scatter_idx, TKp, efo[-1:])
-            z_q, z_sc, y1_q, y1_sf = _up_projection(xg_q, a_sf, w1_q, w1_sf, efo, TKp, act, out=gated_out)
+                xg_q, a_sf = ops.quant_rows_scatter(x.contiguous(), naept, s_rev, None if no_z else s_scatter_idx, TKp,
+                                                    efo[-1:])
+            if no_z:
+                z_q = z_sc = None
+                y1_q, y1_sf = ops.gemm_gated_infer(xg_q, a_sf, w1_q, w1_sf, efo, s_scatter_idx, naept)
+            else:
+                z_q, z_sc, y1_q, y1_sf = _up_projection(xg_q, a_sf, w1_q, w1_sf, efo, TKp, act, out=gated_out)
             del xg_q
         _log_stage_memory(stagewise, "forward: after up-projection")
         out_buf, ctx.dx_buf = _take_placement()
@@ -511,7 +519,7 @@ class _UpProjection(torch.autograd.Function):
         ctx.x_is_fp8 = prequant_payload is not None
         ctx.x_dtype = x.dtype
         ctx.save_for_backward(x if prequant_payload is None else x_q, x_raw if prequant_payload is not None else None,
-                              w1, efo, x_gather_idx, s_rev, naept)
+                              w1, efo, x_gather_idx, s_rev, naept, s_scatter_idx)
         y1 = _placeholder(x, (TKp, N2 // 2))
         z = _placeholder(x, (TKp, N2))
         _handoff_put(z, link)
@@ -520,7 +528,7 @@ class _UpProjection(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, _dy1, _dz):
-        x, x_raw, w1, efo, x_gather_idx, s_rev, naept = ctx.saved_tensors
+        x, x_raw, w1, efo, x_gather_idx, s_rev, naept, s_scatter_idx = ctx.saved_tensors
         link = ctx.link
         dz_q, dz_rsf, dz_t, dz_csf = link.pop("dz")
         E, N2, H = w1.shape
@@ -531,7 +539,7 @@ class _UpProjection(torch.autograd.Function):
         dx = None
         if ctx.needs_input_grad[0]:
             w1t_q, w1t_sf, kn = _weight_operand(w1, True, link.get("iso32", False))
-            dx_exp = _gemm_plain(dz_q, dz_rsf, w1t_q, w1t_sf, kn, efo)
+            dx_exp = _gemm_plain(dz_q, dz_rsf, w1t_q, w1t_sf, kn, efo, s_scatter_idx, naept)
             del w1t_q, w1t_sf
             buf = ctx.dx_buf if (ctx.dx_buf is not None and ctx.x_dtype == torch.bfloat16) else None
             dx = ops.combine(dx_exp, s_rev, naept, None, ctx.T, out=buf)
@@ -584,7 +592,7 @@ class _UpProjection(torch.autograd.Function):
         del dz_q, dz_rsf, dz_t, dz_csf
         _log_stage_memory(link.get("stagewise", False), "backward: after dw1")
         ops.post_status(x.device)      # last kernels of the layer's backward: let the next call see their status
-        return (dx, dw1) + (None,) * 15
+        return (dx, dw1) + (None,) * 16
 
 
 def _recompute_z(args):
@@ -629,7 +637,7 @@ class _DownProjection(torch.autograd.Function):
         link = _handoff_take(z)
         y1_q, y1_sf = link.pop("y1")
         w2_q, w2_sf, _ = _weight_operand(w2, False, link.get("iso32", False))
-        y2 = ops.gemm_varlen_m(y1_q, y1_sf, w2_q, w2_sf, efo)
+        y2 = ops.gemm_varlen_m(y1_q, y1_sf, w2_q, w2_sf, efo, s_scatter_idx, naept)
         del y1_q, y1_sf
         o = ops.combine(y2, s_rev, naept, topk_scores, int(T), out=link.pop("out_buf", None))
         del y2

@@ -321,7 +321,7 @@ def quant_dual_gather(x, idx, rows, valid_rows=None, with_rows=True):
 @_timed
 def quant_rows_scatter(x, naept, s_rev, s_scatter_idx, rows, valid_rows=None):
     """bf16 [T,K] -> (e4m3 rows in expert-sorted order [rows,K], ISA scales of (rows,K)); each token is
-    quantised once and written to all its positions; pad rows are zero."""
+    quantised once and written to all its positions; pad rows are zero, or (s_scatter_idx None) left as they are."""
     _cuda(x, naept, s_rev, s_scatter_idx, valid_rows)
     assert x.dtype == torch.bfloat16 and x.ndim == 2
     T, K = x.shape
@@ -451,14 +451,16 @@ def transpose_u8(src):
 
 # ---------------------------------------------------------------- GEMMs
 @_timed
-def gemm_varlen_m(a_q, a_sf, b_q, b_sf, efo):
-    """a_q u8 [rows,K], b_q u8 [E,N,K] -> bf16 [rows,N]."""
-    _cuda(a_q, a_sf, b_q, b_sf, efo)
+def gemm_varlen_m(a_q, a_sf, b_q, b_sf, efo, s_scatter_idx=None, naept=None):
+    """a_q u8 [rows,K], b_q u8 [E,N,K] -> bf16 [rows,N].  With s_scatter_idx and naept, groups of 32 rows that are all
+    padding are not written."""
+    _cuda(a_q, a_sf, b_q, b_sf, efo, s_scatter_idx, naept)
     rows, K = a_q.shape
     E, N, _ = b_q.shape
     c = torch.empty(rows, N, dtype=torch.bfloat16, device=a_q.device)
-    check(lib.smoe_gemm_varlen_m(_p(a_q), _p(a_sf), _p(b_q), _p(b_sf), _p(efo), _p(c), rows, N, K, E,
-                                 _p(status_word(a_q.device)), _stream()), "gemm_varlen_m")
+    real_tk = None if s_scatter_idx is None else naept.data_ptr() + 4 * (naept.numel() - 1)
+    check(lib.smoe_gemm_varlen_m_live(_p(a_q), _p(a_sf), _p(b_q), _p(b_sf), _p(efo), _p(s_scatter_idx), real_tk, _p(c),
+                                      rows, N, K, E, _p(status_word(a_q.device)), _stream()), "gemm_varlen_m")
     return c
 
 
@@ -502,6 +504,21 @@ def gemm_gated(x_q, a_idx, a_sf, w1_q, w1_sf, efo, rows, out=None):
     check(lib.smoe_gemm_gated(_p(x_q), T, _p(a_idx), _p(a_sf), _p(w1_q), _p(w1_sf), _p(efo), _p(z_q), _p(z_sc),
                               _p(y1_q), _p(y1_sf), rows, N, K, E, _p(status_word(dev)), _stream()), "gemm_gated")
     return z_q, z_sc, y1_q, y1_sf
+
+
+@_timed
+def gemm_gated_infer(x_q, a_sf, w1_q, w1_sf, efo, s_scatter_idx, naept):
+    """`gemm_gated` on expert-sorted x where no backward follows -> (y1_q [rows,I], y1_sf); z is not kept and pad rows hold
+    whatever they held."""
+    _cuda(x_q, a_sf, w1_q, w1_sf, efo, s_scatter_idx, naept)
+    rows, K = x_q.shape
+    E, N, _ = w1_q.shape
+    y1_q = torch.empty(rows, N // 2, dtype=_U8, device=x_q.device)
+    y1_sf = torch.empty(isa_bytes(rows, N // 2), dtype=_U8, device=x_q.device)
+    check(lib.smoe_gemm_gated_infer(_p(x_q), _p(a_sf), _p(w1_q), _p(w1_sf), _p(efo), _p(s_scatter_idx),
+                                    naept.data_ptr() + 4 * (naept.numel() - 1), _p(y1_q), _p(y1_sf), rows, N, K, E,
+                                    _p(status_word(x_q.device)), _stream()), "gemm_gated_infer")
+    return y1_q, y1_sf
 
 
 @_timed

@@ -87,6 +87,29 @@ def oracle_dense(x, dy, w1, w2, wr, K, logits):
     return r
 
 
+@pytest.mark.parametrize("T,H,I,E,K", [(1, 256, 128, 8, 2), (64, 384, 256, 64, 4), (300, 768, 384, 5, 3), (513, 512, 256, 3, 3)])
+def test_forward_without_a_graph_gives_the_same_bits(sm, T, H, I, E, K):
+    """Under no_grad z is not written, pad rows are neither cleared nor stored, phantom tile halves not fetched: the output
+    is that of the training forward bit for bit, whatever the buffers held before (NaN here)."""
+    x, _, w1, w2, wr, _ = make_layer(T, H, I, E, K, T)
+    moe = sm.MoE(E, K, H, I, sm.ActivationType.SWIGLU, add_bias=False, std=0.02).to(DEV).to(torch.bfloat16)
+    with torch.no_grad():
+        moe.router.weight.copy_(wr)
+        moe.c_fc.weight.copy_(w1)
+        moe.c_proj.weight.copy_(w2)
+    xd = x.to(DEV)
+    want, _ = moe(xd, use_fp8=True)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    poison = [torch.full((n,), 255, dtype=torch.uint8, device=DEV) for n in (1 << 24, 1 << 23, 1 << 22, 1 << 20, 1 << 18)]
+    del poison                                       # the allocator hands these bytes out again
+    with torch.no_grad():
+        got, _ = moe(xd, is_inference_mode=True, use_fp8=True)
+    torch.cuda.synchronize()
+    sm.ops.check_status(DEV)
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("T,H,I,E,K,seed", [(256, 256, 128, 8, 2, 0), (1024, 512, 256, 16, 4, 1),
                                              (512, 1024, 384, 8, 8, 2)])
 def test_moe_module_fwd_bwd_vs_fp32_oracle(sm, T, H, I, E, K, seed):
