@@ -124,6 +124,12 @@ __device__ __forceinline__ void tc_cp_sf_pair(uint32_t dst_tmem, uint64_t src_de
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
+__device__ __forceinline__ void st_shared_u16(uint32_t addr, uint16_t v) {
+  asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
+}
+__device__ __forceinline__ void ld_shared_v4(uint32_t addr, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(addr) : "memory");
+}
 // one lane's 32 f32 columns -> its 64-byte bf16 row of a 32-row staging tile in the 64-byte TMA swizzle
 __device__ __forceinline__ void stage_bf16_32(uint32_t stg, int lane, const uint32_t (&a)[32]) {
 #pragma unroll
@@ -144,11 +150,62 @@ __device__ __forceinline__ float fast_sigmoid(float x) {
   return r;
 }
 
+// pairs of f32 in one instruction (round to nearest, as the scalar forms)
+struct F2 {
+  uint64_t v;
+};
+__device__ __forceinline__ F2 f2(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+// fast_sigmoid of a pair
+__device__ __forceinline__ F2 f2_sigmoid(F2 x) {
+  const float2 t = f2_get(x * f2(-1.4426950408889634f, -1.4426950408889634f));
+  float e0, e1, r0, r1;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(t.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(t.y));
+  const float2 d = f2_get(f2(e0, e1) + f2(1.0f, 1.0f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(d.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d.y));
+  return f2(r0, r1);
+}
+
 // element-wise max of two bf16 pairs
 __device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
   uint32_t r;
   asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
+}
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+// four bf16 values, already scaled, -> four e4m3 bytes
+__device__ __forceinline__ uint32_t pack_e4m3x4_bf16(uint32_t a, uint32_t b) {
+  return pack_e4m3x4(__uint_as_float(a << 16), __uint_as_float(a & 0xFFFF0000u), __uint_as_float(b << 16),
+                     __uint_as_float(b & 0xFFFF0000u));
 }
 // max |x| over the warp, delivered to every lane
 __device__ __forceinline__ float warp_max_abs(float x) {
@@ -860,6 +917,11 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         // per column and 32 rows - and leave as e4m3 in row-major order.  A 32x32-block scale serves dz both as
         // the activation-gradient operand (scales along 2I) and as the weight-gradient operand (scales along
         // TKp, fed MN-major), so one copy of the payload is enough.  Each warp works on its own.
+        // Issue slots of the epilogue warps bound the tile, not the MMAs: a profile counted 1500 instructions per warp and
+        // 32-column chunk at 0.43 issued a cycle, 21 k cycles a tile for 9.2 k cycles of MMAs (H=3072).  So the f32
+        // arithmetic runs on pairs, maxima and power-of-two scalings on bf16 pairs, the column scales travel through shared
+        // memory, and the wait for the staging tile comes as late as it can: 316 -> 296 us at T=8192, H=3072, I=1536,
+        // E=K=8, 1333 -> 1232 us at H=I=4096.  (Twelve epilogue warps of 64 columns instead of eight of 96: 309 us.)
         // a ragged last column tile (N not a multiple of BN): chunks at or beyond column N hold products with
         // rows of the next expert's weights (or TMA zero fill) and are skipped whole (N is a multiple of 32)
         if (t.valid && c_base < p.N && !(p.debug_skip_store & 2)) {
@@ -868,7 +930,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           const int row_grp = (t.m0 + q * 32) >> 5;      // 32-row group index along TKp
           const int kt_rows = p.rows >> 7;               // K tiles of the weight-gradient operands
           constexpr int NCH = COLS_PER_WARP / 32;
-          float ds_acc = 0.f;
+          F2 ds2 = f2(0.f, 0.f);                         // even and odd columns
 #pragma unroll 1
           for (int c = 0; c < NCH; ++c) {
             const int dcol = c_base + c * 32;            // first D / y1s column of the chunk
@@ -890,8 +952,6 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             const float sc0 = __int_as_float((int)(sc & 0xFF) << 23);
             const float sc1 = __int_as_float((int)(sc >> 8) << 23);
             tmem_ld_wait();
-            if (lane == 0) bulk_wait_group_read<0>();    // the previous chunk's stores have read the staging
-            __syncwarp();
             const uint32_t* zw = reinterpret_cast<const uint32_t*>(zb);
             uint32_t Y[16];                              // y1s of this lane's row, bf16 pairs of adjacent columns
             uint32_t e_blk = 0;
@@ -900,41 +960,42 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               // 16 D columns -> 32 dz columns = one 32x32 scale block; dz stays packed in bf16 pairs until its
               // block maximum is known
               uint32_t P[16];
-              float amax = 0.f;
+              uint32_t amax2 = 0;
               const float scale = b ? sc1 : sc0;
 #pragma unroll
               for (int i2 = 0; i2 < 8; ++i2) {
-                float yq[2];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                  const int pi = b * 16 + 2 * i2 + h;
-                  const uint32_t pair = (zw[pi >> 1] >> (16 * (pi & 1))) & 0xFFFF;
-                  const float2 gu = e4m3x2_to_f32(pair);
-                  const float g = gu.x * scale, u = gu.y * scale;
-                  const float D = __uint_as_float(b ? r1[2 * i2 + h] : r0[2 * i2 + h]);
-                  const float dout = s * D;
-                  const float sig = fast_sigmoid(g);
-                  const float silu = g * sig;
-                  const float sd = silu * dout;
-                  const float yv = silu * u;
-                  ds_acc = fmaf(yv, D, ds_acc);
-                  const uint32_t dzp = pack_bf16x2(((sig - silu * sig) * dout + sd) * u, sd);   // rounds to bf16
-                  P[2 * i2 + h] = dzp;
-                  yq[h] = s * yv;
-                  amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(dzp << 16)), fabsf(__uint_as_float(dzp & 0xFFFF0000u))));
-                }
-                Y[b * 8 + i2] = pack_bf16x2(yq[0], yq[1]);
+                // two D columns at a time, every product and sum on pairs
+                const uint32_t zz = zw[b * 8 + i2];
+                const float2 p0 = e4m3x2_to_f32(zz & 0xFFFF), p1 = e4m3x2_to_f32(zz >> 16);      // (g, u) of each
+                const F2 sc2 = f2(scale, scale);
+                const F2 g = f2(p0.x, p1.x) * sc2, u = f2(p0.y, p1.y) * sc2;
+                const F2 D = f2(__uint_as_float(b ? r1[2 * i2] : r0[2 * i2]), __uint_as_float(b ? r1[2 * i2 + 1] : r0[2 * i2 + 1]));
+                const F2 dout = f2(s, s) * D;
+                const F2 sig = f2_sigmoid(g);
+                const F2 silu = g * sig;
+                const F2 sd = silu * dout;
+                const F2 yv = silu * u;
+                ds2 = f2_fma(yv, D, ds2);
+                const F2 dsig = f2_fma(silu, sig * f2(-1.0f, -1.0f), sig);                       // sig - silu * sig
+                const float2 dg = f2_get(f2_fma(dsig, dout, sd) * u), sdp = f2_get(sd), y = f2_get(f2(s, s) * yv);
+                P[2 * i2] = pack_bf16x2(dg.x, sdp.x);                                            // rounds to bf16
+                P[2 * i2 + 1] = pack_bf16x2(dg.y, sdp.y);
+                amax2 = max_bf16x2(amax2, max_bf16x2(P[2 * i2] & 0x7FFF7FFFu, P[2 * i2 + 1] & 0x7FFF7FFFu));
+                Y[b * 8 + i2] = pack_bf16x2(y.x, y.y);
               }
               uint32_t w[8];
-              const int e = e8m0_of(warp_max_abs(amax));
-              const float qs = qscale_of(e);
+              const int e = e8m0_of(warp_max_abs(fmaxf(__uint_as_float(amax2 << 16), __uint_as_float(amax2 & 0xFFFF0000u))));
+              // the scale is a power of two: multiplying the bf16 pair by it is exact wherever e4m3 keeps a bit of it
+              const uint32_t qs2 = __byte_perm(__float_as_uint(qscale_of(e)), 0, 0x3232);
               e_blk |= (uint32_t)e << (8 * b);
 #pragma unroll
-              for (int i = 0; i < 8; ++i)
-                w[i] = pack_e4m3x4(__uint_as_float(P[2 * i] << 16) * qs, __uint_as_float(P[2 * i] & 0xFFFF0000u) * qs,
-                                   __uint_as_float(P[2 * i + 1] << 16) * qs,
-                                   __uint_as_float(P[2 * i + 1] & 0xFFFF0000u) * qs);
-              // this half's 32 dz bytes of the row go to the staging tile right away
+              for (int i = 0; i < 8; ++i) w[i] = pack_e4m3x4_bf16(mul_bf16x2(P[2 * i], qs2), mul_bf16x2(P[2 * i + 1], qs2));
+              // this half's 32 dz bytes of the row go to the staging tile right away, once the previous chunk's stores
+              // have read it (asked only now: their latency lies under the arithmetic above)
+              if (b == 0) {
+                if (lane == 0) bulk_wait_group_read<0>();
+                __syncwarp();
+              }
 #pragma unroll
               for (int j = 0; j < 2; ++j)
                 st_shared_v4(stg + lane * 64 + (((2 * b + j) ^ ((lane >> 1) & 3)) << 4), w[4 * j], w[4 * j + 1],
@@ -958,18 +1019,17 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             }
             A[0] = max_bf16x2(A[0], __shfl_xor_sync(0xffffffff, A[0], 1));
             const int e_mine = e8m0_of(__uint_as_float((lane & 1) ? (A[0] & 0xFFFF0000u) : (A[0] << 16)));
-            const float qs_mine = qscale_of(e_mine);
+            // every lane needs all 32 column scales, as bf16 pairs: through the y1s staging tile (its last store has been
+            // read), four broadcast loads instead of 32 shuffles
+            st_shared_u16(stg + 2048 + 2 * lane, (uint16_t)(__float_as_uint(qscale_of(e_mine)) >> 16));
+            __syncwarp();
+            uint32_t qy[16];
 #pragma unroll
-            for (int i4 = 0; i4 < 8; ++i4) {
-              float qv[4];
+            for (int j = 0; j < 4; ++j) ld_shared_v4(stg + 2048 + 16 * j, qy[4 * j], qy[4 * j + 1], qy[4 * j + 2], qy[4 * j + 3]);
+            __syncwarp();                                // the tile is about to receive the payload
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const int cc = 4 * i4 + j;
-                const float yv = __uint_as_float((cc & 1) ? (Y[cc >> 1] & 0xFFFF0000u) : (Y[cc >> 1] << 16));
-                qv[j] = yv * __shfl_sync(0xffffffff, qs_mine, cc);
-              }
-              wy[i4] = pack_e4m3x4(qv[0], qv[1], qv[2], qv[3]);
-            }
+            for (int i = 0; i < 8; ++i)
+              wy[i] = pack_e4m3x4_bf16(mul_bf16x2(Y[2 * i], qy[2 * i]), mul_bf16x2(Y[2 * i + 1], qy[2 * i + 1]));
 #pragma unroll
             for (int j = 0; j < 2; ++j)
               st_shared_v4(stg + 2048 + lane * 32 + ((j ^ ((lane >> 2) & 1)) << 4), wy[4 * j], wy[4 * j + 1],
@@ -1000,7 +1060,8 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             for (int i = 0; i < 4; ++i) zb[i] = zn[i];
             sc = scn;
           }
-          p.ds_partial[(size_t)((t.n0 / BN) * S::COL_GROUPS + half) * p.rows + grow] = ds_acc;
+          const float2 ds_eo = f2_get(ds2);
+          p.ds_partial[(size_t)((t.n0 / BN) * S::COL_GROUPS + half) * p.rows + grow] = ds_eo.x + ds_eo.y;
         }
       } else {  // DGATED
         // this warp: D columns [c_base, c_base + BN/2) of I in chunks of 32 -> dz 64 bf16 (128-byte rows,
