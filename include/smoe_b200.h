@@ -396,6 +396,36 @@ int smoe_topk_softmax(const float* logits, int64_t T, int64_t E, int64_t K, floa
 int smoe_topk_softmax_bwd(const float* scores, const int32_t* idx, const float* dscores, int64_t T, int64_t E, int64_t K,
                           float* dlogits, void* stream);
 
+/* A whole layer pass in one call: routing metadata, quantizers, GEMMs and combine of the SwiGLU layer, launched back to back
+ * on `stream` by the entry points above, intermediates in two caller-supplied arenas (256-byte aligned).  Layers so small
+ * that their kernels finish before a caller that makes the calls one by one has issued them.  E <= 256, H % 128 == 0,
+ * I % 128 == 0, TKp_alloc % 128 == 0 (sizes as smoe_topk_metadata takes them). */
+enum { SMOE_DW_NONE = 0, SMOE_DW_ACCUMULATE = 1, SMOE_DW_STORE = 2, SMOE_DW_BF16 = 3 };
+typedef struct {
+  int64_t T, H, I, E, K, TK_alloc, TKp_alloc;
+  int32_t lane_order, pad_mode;
+  int32_t keep_z;              /* forward: a backward will follow; backward: must be what the forward was given, and set */
+  int32_t dw1_mode, dw2_mode;  /* SMOE_DW_*: f32 [E,2I,H] / [E,I,H] added to or overwritten, or bf16 [E,2I,H] / [E,H,I] */
+  int32_t reserved;
+  const void* x;               /* bf16 [T,H] */
+  const void* dout;            /* backward: bf16 [T,H] */
+  const int32_t* idx;          /* forward: [T,K] */
+  const float* probs;          /* forward: [T,K] */
+  const void *w1, *w1_sf;      /* forward: W1 [E,2I,H]; backward: W1^T [E,H,2I] */
+  const void *w2, *w2_sf;      /* forward: W2 [E,H,I]; backward: W2^T [E,I,H] */
+  void* out;                   /* forward: bf16 o [T,H]; backward: bf16 dx [T,H] or null */
+  float* ds;                   /* backward: gradient of probs [T,K], or null */
+  void *dw1, *dw2;
+  int32_t* counts;             /* forward: tokens per expert [E] */
+  void *saved, *scratch;       /* smoe_layer_bytes(args, 0); (args, 1) in the forward, (args, 2) in the backward */
+  int32_t* status;
+  int32_t* host_word;          /* pinned mirror of *status, posted at the end (not while capturing); may be null */
+} smoe_layer_args;
+/* Bytes of an arena: which = 0 saved, 1 forward scratch, 2 backward scratch; -1 for sizes that are not taken. */
+int64_t smoe_layer_bytes(const smoe_layer_args* args, int which);
+int smoe_layer_forward(const smoe_layer_args* args, void* stream);
+int smoe_layer_backward(const smoe_layer_args* args, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -14,6 +14,17 @@ LIB_PATH = os.path.join(_HERE, "libsmoe_b200.so")
 
 _P, _I, _L = c_void_p, c_int, c_int64
 
+
+class LayerArgs(ctypes.Structure):
+    """smoe_layer_args"""
+    _fields_ = ([(n, c_int64) for n in ("T", "H", "I", "E", "K", "TK_alloc", "TKp_alloc")]
+                + [(n, ctypes.c_int32) for n in ("lane_order", "pad_mode", "keep_z", "dw1_mode", "dw2_mode", "reserved")]
+                + [(n, c_void_p) for n in ("x", "dout", "idx", "probs", "w1", "w1_sf", "w2", "w2_sf", "out", "ds", "dw1",
+                                           "dw2", "counts", "saved", "scratch", "status", "host_word")])
+
+
+DW_NONE, DW_ACCUMULATE, DW_STORE, DW_BF16 = 0, 1, 2, 3
+
 # name -> (restype, argtypes); mirrors include/smoe_b200.h one to one
 SIGNATURES = {
     "smoe_count_cumsum": (_I, [_P, _I, _L, _L, _P, _P, _P]),
@@ -61,6 +72,9 @@ SIGNATURES = {
     "smoe_gather_scores": (_I, [_P, _P, _L, _P, _P]),
     "smoe_ds_finalize": (_I, [_P, _L, _L, _P, _L, _P, _P, _P, _P, _P]),
     "smoe_status_post": (_I, [_P, _P, _P]),
+    "smoe_layer_bytes": (_L, [ctypes.POINTER(LayerArgs), _I]),
+    "smoe_layer_forward": (_I, [ctypes.POINTER(LayerArgs), _P]),
+    "smoe_layer_backward": (_I, [ctypes.POINTER(LayerArgs), _P]),
     "smoe_topk_softmax": (_I, [_P, _L, _L, _L, _P, _P, _P]),
     "smoe_topk_softmax_bwd": (_I, [_P, _P, _P, _L, _L, _L, _P, _P]),
 }

@@ -25,7 +25,7 @@ from contextlib import contextmanager
 import torch
 import torch.nn.functional as F
 
-from .. import ops
+from .. import _lib, ops
 from ..config import get_active_config
 from ..enums import ActivationType, activation_code, require_swiglu
 
@@ -789,6 +789,126 @@ class _DownProjection(torch.autograd.Function):
 
 
 # ----------------------------------------------------------------------------
+# small layers: the same launches from one native call per pass
+# ----------------------------------------------------------------------------
+# Bytes of scratch up to which a layer takes the one-call path (csrc/layer.cu).  All intermediates of a pass are alive at
+# once there, where the step-by-step path frees each after its last reader, so the peak grows by at most the bound.  It lies
+# where the kernels begin to outlast the host: a forward + backward of T=1024, H=3072, I=1536, E=K=8 (200 MB) is 0.53 ms of
+# kernels and took 0.73 ms step by step (0.56 in one call), T=8192 is 2.7 ms of kernels for 0.72 ms of Python.
+_ONE_CALL_BYTES = 256 << 20
+
+
+def _one_call_args(x, idx, w1, w2, E, K, TK, TKp, act, fp8_config):
+    """LayerArgs of a layer that the one-call path takes, else None."""
+    cfg = fp8_config if fp8_config is not None else get_active_config()
+    if (act != 0 or ops._recorder is not None or _PLACEMENT or USE_TMA_GATHER or not FUSE_DGATED_QUANT or not _DEFER_DW2
+            or not _PAIR_WGRADS or x.dtype != torch.bfloat16 or x.dim() != 2 or not x.is_cuda or not x.is_contiguous()
+            or x.data_ptr() % 16 or any(_modes(fp8_config)) or (cfg is not None and cfg.resolve_recompute_z())):
+        return None
+    T, H = x.shape
+    I = w2.shape[2]
+    if (T == 0 or E > 256 or H % 128 or I % 128 or TKp % 128 or tuple(w1.shape) != (E, 2 * I, H) or tuple(w2.shape) != (E, H, I)
+            or TKp * (5 * H + 4 * I if torch.is_grad_enabled() else 3 * H + I) > _ONE_CALL_BYTES):
+        return None
+    a = _lib.LayerArgs(T, H, I, E, K, TK, TKp)
+    a.x = x.data_ptr()
+    a.status, a.host_word = ops.status_pointers(x.device)
+    return a
+
+
+def _u8(n, device):
+    return torch.empty(n, dtype=torch.uint8, device=device)
+
+
+class _OneCallLayer(torch.autograd.Function):
+    """Forward and backward of the expert compute (metadata to combine; see csrc/layer.cu).  `scores` [T,K] receives the
+    router gradient; `idx` / `probs` are what the metadata is made from."""
+
+    @staticmethod
+    def forward(ctx, x, w1, w2, scores, idx, probs, args, lane_order, pad_mode, grad_mode):
+        ctx.set_materialize_grads(False)
+        _require_fp8()
+        dev = x.device
+        w1_q, w1_sf = weight_fp8(w1, False)
+        w2_q, w2_sf = weight_fp8(w2, False)
+        out = torch.empty_like(x)
+        counts = torch.empty(args.E, dtype=torch.int32, device=dev)
+        args.lane_order, args.pad_mode, args.keep_z = lane_order, pad_mode, int(grad_mode)
+        saved = _u8(_lib.lib.smoe_layer_bytes(args, 0), dev)
+        scratch = _u8(_lib.lib.smoe_layer_bytes(args, 1), dev)
+        args.idx, args.probs = idx.data_ptr(), probs.data_ptr()
+        args.w1, args.w1_sf, args.w2, args.w2_sf = w1_q.data_ptr(), w1_sf.data_ptr(), w2_q.data_ptr(), w2_sf.data_ptr()
+        args.out, args.counts, args.saved, args.scratch = (out.data_ptr(), counts.data_ptr(), saved.data_ptr(),
+                                                           scratch.data_ptr())
+        _lib.check(_lib.lib.smoe_layer_forward(args, ops._stream()), "layer_forward")
+        if grad_mode:
+            ctx.sizes = (args.T, args.H, args.I, args.E, args.K, args.TK_alloc, args.TKp_alloc)
+            ctx.save_for_backward(x, w1, w2, saved)
+        ctx.mark_non_differentiable(counts)
+        return out, counts
+
+    @staticmethod
+    def backward(ctx, dout, _dcounts):
+        if dout is None:
+            return (None,) * 10
+        x, w1, w2, saved = ctx.saved_tensors
+        need_x, need_w1, need_w2, need_s = ctx.needs_input_grad[:4]
+        dev = x.device
+        if dout.dtype != torch.bfloat16:
+            dout = dout.to(torch.bfloat16)
+        dout = dout.contiguous()
+        if dout.data_ptr() % 16:
+            dout = dout.clone()
+        a = _lib.LayerArgs(*ctx.sizes)
+        T, H, I, E = a.T, a.H, a.I, a.E
+        a.keep_z = 1
+        a.status, a.host_word = ops.status_pointers(dev)
+        a.x, a.dout, a.saved = x.data_ptr(), dout.data_ptr(), saved.data_ptr()
+        w2t_q, w2t_sf = weight_fp8(w2, True)
+        a.w2, a.w2_sf = w2t_q.data_ptr(), w2t_sf.data_ptr()
+        dx = dw1 = dw2 = ds = mg1 = mg2 = None
+        if need_x:
+            w1t_q, w1t_sf = weight_fp8(w1, True)
+            a.w1, a.w1_sf = w1t_q.data_ptr(), w1t_sf.data_ptr()
+            dx = torch.empty_like(x)
+            a.out = dx.data_ptr()
+            _RESULT_READY.pop(a.out, None)       # an event noted for an earlier tensor at this address says nothing here
+        if need_s:
+            ds = torch.empty(T, a.K, dtype=torch.float32, device=dev)
+            a.ds = ds.data_ptr()
+        if need_w2:
+            mg2, base2 = _grad_target(w2, (E, I, H))
+            if mg2 is not None:
+                a.dw2_mode, a.dw2 = _lib.DW_ACCUMULATE, mg2.data_ptr()
+            elif w2.dtype == torch.bfloat16 and _mn_wgrad_ok(E, H, I):
+                dw2 = torch.empty(E, H, I, dtype=torch.bfloat16, device=dev)
+                a.dw2_mode, a.dw2 = _lib.DW_BF16, dw2.data_ptr()
+            else:
+                dw2 = torch.empty(E, I, H, dtype=torch.float32, device=dev)
+                a.dw2_mode, a.dw2 = _lib.DW_STORE, dw2.data_ptr()
+        if need_w1:
+            mg1, base1 = _grad_target(w1, (E, 2 * I, H))
+            if mg1 is not None:
+                a.dw1_mode, a.dw1 = _lib.DW_ACCUMULATE, mg1.data_ptr()
+            else:
+                bf16 = w1.dtype == torch.bfloat16 and _mn_wgrad_ok(E, 2 * I, H)
+                dw1 = torch.empty(E, 2 * I, H, dtype=torch.bfloat16 if bf16 else torch.float32, device=dev)
+                a.dw1_mode, a.dw1 = _lib.DW_BF16 if bf16 else _lib.DW_STORE, dw1.data_ptr()
+        scratch = _u8(_lib.lib.smoe_layer_bytes(a, 2), dev)
+        a.scratch = scratch.data_ptr()
+        _lib.check(_lib.lib.smoe_layer_backward(a, ops._stream()), "layer_backward")
+        if mg2 is not None:
+            _after_accumulate(base2)
+        elif a.dw2_mode == _lib.DW_STORE:
+            dw2 = dw2.transpose(1, 2).to(w2.dtype)
+        if mg1 is not None:
+            _after_accumulate(base1)
+        elif a.dw1_mode == _lib.DW_STORE:
+            dw1 = dw1.to(w1.dtype)
+        return (dx, dw1, dw2, ds) + (None,) * 6
+
+
+# ----------------------------------------------------------------------------
 # router: top-k on logits, softmax over the K selected (forward.py:217-236,
 # backward.py:572-641)
 # ----------------------------------------------------------------------------
@@ -826,7 +946,13 @@ def moe_TC_softmax_topk_layer(x, router_w, w1, b1, w2, b2, K, stream_id, activat
     w1_e, w2_e = _expert_major(w1), _expert_major(w2)
     logits = F.linear(x, router_w)
     scores, idx = _TopKSoftmax.apply(logits.float(), K)
-    md = ops.topk_metadata(idx, scores.detach(), E, 128, TK_alloc=T * K, lane_order=1, pad_mode=1)
+    TK = T * K
+    args = (_one_call_args(x, idx, w1_e, w2_e, E, K, TK, -(-TK // 128) * 128 + E * 128, activation_code(activation_type), None)
+            if b1 is None and b2 is None and K <= _MAX_PAIRS_PER_TOKEN else None)
+    if args is not None:
+        o, counts = _OneCallLayer.apply(x, w1_e, w2_e, scores, idx, scores.detach(), args, 1, 1, torch.is_grad_enabled())
+        return o, logits, counts
+    md = ops.topk_metadata(idx, scores.detach(), E, 128, TK_alloc=TK, lane_order=1, pad_mode=1)
     y1, z = _UpProjection.apply(x, w1_e, b1, md["efo"], md["TKp_alloc"], K, stream_id, md["x_gather_idx"],
                                 md["s_scatter_idx"], md["s_reverse_scatter_idx"], md["naept"], False,
                                 activation_type, is_inference_mode_enabled)

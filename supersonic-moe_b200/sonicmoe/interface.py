@@ -7,8 +7,8 @@ import torch
 
 from . import ops
 from .enums import ActivationType, activation_code
-from .functional import (_DownProjection, _UpProjection, attach_preallocated_gated_outputs, enable_fp8,
-                         place_results)
+from .functional import (_DownProjection, _OneCallLayer, _one_call_args, _UpProjection,
+                         attach_preallocated_gated_outputs, enable_fp8, place_results)
 
 
 def scale_bytes(fp8_scale: torch.Tensor, H: int) -> torch.Tensor:
@@ -62,7 +62,18 @@ def run_sonic_moe(hidden_states, topk_indices, topk_scores, K, E, w1, w2, fp8=Fa
         counts = tokens_per_expert.tolist() if isinstance(tokens_per_expert, torch.Tensor) else list(tokens_per_expert)
         TK = int(sum(counts))
         TKp = int(sum(-(-c // 128) * 128 for c in counts if c > 0))
-    md = ops.topk_metadata(idx.contiguous(), probs.contiguous(), E, 128, TK, TKp)
+    idx, probs = idx.contiguous(), probs.contiguous()
+    if fp8_scale is None and out is None and dx_out is None and fp8_combine_grad_handle is None \
+            and idx.ndim == 2 and idx.shape == probs.shape and idx.shape[1] <= 16 and idx.is_cuda and probs.is_cuda:
+        TK1 = TK if TK is not None else N * min(idx.shape[1], E)
+        TKp1 = TKp if TKp is not None else -(-TK1 // 128) * 128 + E * 128
+        args = _one_call_args(hidden_states, idx, w1, w2, E, idx.shape[1], TK1, TKp1, activation_code(activation_type),
+                              fp8_config)
+        if args is not None:
+            with enable_fp8(True):
+                return _OneCallLayer.apply(hidden_states, w1, w2, topk_scores, idx, probs, args, 0, 0,
+                                           torch.is_grad_enabled())[0]
+    md = ops.topk_metadata(idx, probs, E, 128, TK, TKp)
     stream_id = torch.cuda.current_stream().cuda_stream
     payload = None
     if fp8_scale is not None:

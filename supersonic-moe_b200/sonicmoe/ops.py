@@ -110,6 +110,15 @@ def post_status(device):
     check(lib.smoe_status_post(_p(status_word(device)), host.data_ptr(), _stream()), "status_post")
 
 
+def status_pointers(device):
+    """(device address of the status word, host address of its pinned mirror)."""
+    key = _dev_index(device)
+    host = _posted.get(key)
+    if host is None:
+        host = _posted[key] = torch.zeros(1, dtype=_I32).pin_memory()
+    return status_word(key).data_ptr(), host.data_ptr()
+
+
 def poll_status(device):
     """Look at the host mirror of the status word; raise on a recorded failure.  Never waits."""
     if torch.device(device).type != "cuda":

@@ -87,6 +87,40 @@ def oracle_dense(x, dy, w1, w2, wr, K, logits):
     return r
 
 
+@pytest.mark.parametrize("grads", ["main_grad", "bf16", "f32_weights", "w2_only", "no_scores"])
+@pytest.mark.parametrize("T,H,I,E,K", [(1, 256, 128, 8, 2), (130, 768, 256, 6, 3), (257, 512, 256, 4, 4), (64, 384, 128, 40, 8)])
+def test_one_call_layer_gives_the_bits_of_the_step_by_step_path(sm, monkeypatch, T, H, I, E, K, grads):
+    """csrc/layer.cu makes the calls of the autograd Functions: outputs and every gradient are the same bits, also with
+    masked slots, exact sizing, and only some of the inputs wanting gradients."""
+    x, dy, w1, w2, _, _ = make_layer(T, H, I, E, K, T + H)
+    g = torch.Generator().manual_seed(E)
+    idx = torch.rand(T, E, generator=g).topk(K, dim=-1).indices.to(torch.int32)
+    idx[torch.rand(T, K, generator=g) < 0.3] = -1
+    probs = torch.rand(T, K, generator=g)
+    counts = torch.bincount(idx[idx >= 0].long(), minlength=E)
+
+    def run(limit, **kw):
+        monkeypatch.setattr(sm.functional, "_ONE_CALL_BYTES", limit)
+        dt = torch.float32 if grads == "f32_weights" else torch.bfloat16
+        a = [t.to(DEV, copy=True) for t in (x, w1.to(dt), w2.to(dt), probs)]
+        for t, want in zip(a, (grads != "w2_only", grads != "w2_only", True, grads not in ("w2_only", "no_scores"))):
+            t.requires_grad_(want)
+        if grads == "main_grad":
+            a[1].main_grad = torch.full((E, 2 * I, H), 0.5, device=DEV)
+            a[2].main_grad = torch.full((E, I, H), 0.25, device=DEV)
+        out = sm.run_sonic_moe(a[0], idx.to(DEV), a[3], K, E, a[1], a[2], fp8=True, **kw)
+        out.backward(dy.to(DEV))
+        torch.cuda.synchronize()
+        sm.ops.check_status(DEV)
+        return [out.detach()] + [t.grad for t in a] + [getattr(t, "main_grad", None) for t in a[1:3]]
+
+    for kw in ({}, {"tokens_per_expert": counts}):
+        for i, (got, want) in enumerate(zip(run(1 << 40, **kw), run(0, **kw))):
+            assert (got is None) == (want is None), i
+            if want is not None:
+                assert got.dtype == want.dtype and torch.equal(got, want), i
+
+
 @pytest.mark.parametrize("T,H,I,E,K", [(1, 256, 128, 8, 2), (64, 384, 256, 64, 4), (300, 768, 384, 5, 3), (513, 512, 256, 3, 3)])
 def test_forward_without_a_graph_gives_the_same_bits(sm, T, H, I, E, K):
     """Under no_grad z is not written, pad rows are neither cleared nor stored, phantom tile halves not fetched: the output
