@@ -426,6 +426,22 @@ int64_t smoe_layer_bytes(const smoe_layer_args* args, int which);
 int smoe_layer_forward(const smoe_layer_args* args, void* stream);
 int smoe_layer_backward(const smoe_layer_args* args, void* stream);
 
+/* The two above on logits / dlogits of either type: bf16 != 0 takes them as the router's bf16 GEMM leaves them. */
+int smoe_router_topk(const void* logits, int bf16, int64_t T, int64_t E, int64_t K, float* scores, int32_t* idx,
+                     void* stream);
+int smoe_router_topk_bwd(const float* scores, const int32_t* idx, const float* dscores, int64_t T, int64_t E, int64_t K,
+                         void* dlogits, int bf16, void* stream);
+
+/* Switch auxiliary loss E * sum_e (acc_e / max(|acc|_1, eps)) (freq_e / max(|freq|_1, eps)), acc = sum over the T rows of
+ * softmax(logits), eps = 1e-12, and grad[e] = d loss / d acc_e (both f32); the second call turns grad and the incoming
+ * scalar gradient *dloss into dlogits (type of the logits).  Replaces _compute_switch_loss (sonicmoe/moe.py:640-662) and
+ * its backward.  E <= 1024; workspace: smoe_switch_loss_workspace(E) bytes. */
+int64_t smoe_switch_loss_workspace(int64_t E);
+int smoe_switch_loss(const void* logits, int bf16, const int32_t* freq, int64_t T, int64_t E, float* loss, float* grad,
+                     void* workspace, void* stream);
+int smoe_switch_loss_bwd(const void* logits, int bf16, const float* grad, const float* dloss, int64_t T, int64_t E,
+                         void* dlogits, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -79,13 +79,19 @@ __global__ void ds_finalize_kernel(const float* __restrict__ part, int partials,
 // fewer than K finite logits still gets K distinct, in-range indices: once the
 // finite ones are used up, the lowest not-yet-selected index is taken with a
 // score of exactly zero (all K scores are zero when nothing in the row is finite).
+// Bound by instruction issue (K passes over a lane's PER slots), so PER is the smallest power of two that holds E / 32
+// experts: with 32 slots for every E, T=4096, E=32, K=8 took 20 us.  Logits are f32, or bf16 as the router's GEMM left
+// them.
+__device__ __forceinline__ float logit_of(const float* p, size_t i) { return p[i]; }
+__device__ __forceinline__ float logit_of(const __nv_bfloat16* p, size_t i) { return __bfloat162float(p[i]); }
+
+template <int PER, typename L>
 __global__ void __launch_bounds__(256)
-topk_softmax_kernel(const float* __restrict__ logits, int64_t T, int E, int K, float* __restrict__ scores,
+topk_softmax_kernel(const L* __restrict__ logits, int64_t T, int E, int K, float* __restrict__ scores,
                     int* __restrict__ idx) {
   const int lane = threadIdx.x & 31;
   const int64_t row = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= T) return;
-  constexpr int PER = 32;  // up to 1024 experts
   float v[PER];
   const int per = (E + 31) / 32;
   uint32_t open = 0;       // bit i: this lane's i-th expert exists and has not been selected yet
@@ -93,7 +99,7 @@ topk_softmax_kernel(const float* __restrict__ logits, int64_t T, int E, int K, f
   for (int i = 0; i < PER; ++i) {
     const int e = i * 32 + lane;
     const bool in = (i < per && e < E);
-    const float x = in ? logits[row * E + e] : -INFINITY;
+    const float x = in ? logit_of(logits, row * E + e) : -INFINITY;
     v[i] = (x != x) ? -INFINITY : x;
     if (in) open |= 1u << i;
   }
@@ -130,13 +136,17 @@ topk_softmax_kernel(const float* __restrict__ logits, int64_t T, int E, int K, f
   }
 }
 
+__device__ __forceinline__ void store_grad(float* p, size_t i, float v) { p[i] = v; }
+__device__ __forceinline__ void store_grad(__nv_bfloat16* p, size_t i, float v) { p[i] = __float2bfloat16_rn(v); }
+
+template <typename L>
 __global__ void __launch_bounds__(256)
 topk_softmax_bwd_kernel(const float* __restrict__ scores, const int* __restrict__ idx, const float* __restrict__ ds,
-                        int64_t T, int E, int K, float* __restrict__ dlogits) {
+                        int64_t T, int E, int K, L* __restrict__ dlogits) {
   const int lane = threadIdx.x & 31;
   const int64_t row = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= T) return;
-  for (int e = lane; e < E; e += 32) dlogits[row * E + e] = 0.f;
+  for (int e = lane; e < E; e += 32) store_grad(dlogits, row * E + e, 0.f);
   __syncwarp();
   const float s = lane < K ? scores[row * K + lane] : 0.f;
   const float g = lane < K ? ds[row * K + lane] : 0.f;
@@ -145,7 +155,127 @@ topk_softmax_bwd_kernel(const float* __restrict__ scores, const int* __restrict_
   for (int d = 16; d > 0; d >>= 1) dot += __shfl_xor_sync(0xffffffff, dot, d);
   if (lane < K) {
     const int e = idx[row * K + lane];
-    if (e >= 0 && e < E) dlogits[row * E + e] = s * (g - dot);     // an out-of-range index is ignored, never written
+    if (e >= 0 && e < E) store_grad(dlogits, row * E + e, s * (g - dot));     // an out-of-range index is ignored, never written
+  }
+}
+
+// ---- switch auxiliary loss: E * sum_e (acc_e / |acc|_1) (f_e / |f|_1), acc_e = sum_t softmax(logits_t)_e ----------------
+// Written out as tensor operations it is some 35 launches of 2 us per forward + backward, each with its gap.  Three kernels
+// instead: per-block sums of the softmax rows, their reduction with the loss, and the gradient.  All sums in f32 in a fixed
+// order.  A lane owns the experts lane, lane + 32, ...; a warp walks rows.
+constexpr int kAuxBlocks = 148, kAuxWarps = 8;
+constexpr float kAuxEps = 1e-12f;      // torch.nn.functional.normalize's lower bound of a norm
+
+// softmax of one row into v (0 beyond E)
+template <int PER, typename L>
+__device__ __forceinline__ void softmax_row(const L* __restrict__ logits, size_t row, int E, int lane, float (&v)[PER]) {
+  float m = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = i * 32 + lane;
+    v[i] = e < E ? logit_of(logits, row * E + e) : -INFINITY;
+    m = fmaxf(m, v[i]);
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffff, m, d));
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    v[i] = i * 32 + lane < E ? expf(v[i] - m) : 0.f;
+    sum += v[i];
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffff, sum, d);
+  const float inv = 1.0f / sum;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) v[i] *= inv;
+}
+
+template <int PER, typename L>
+__global__ void __launch_bounds__(32 * kAuxWarps)
+switch_loss_sums_kernel(const L* __restrict__ logits, int64_t T, int E, float* __restrict__ part /* [blocks, E] */) {
+  __shared__ float s_acc[kAuxWarps][PER * 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float acc[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) acc[i] = 0.f;
+  for (int64_t row = (int64_t)blockIdx.x * kAuxWarps + warp; row < T; row += (int64_t)gridDim.x * kAuxWarps) {
+    float v[PER];
+    softmax_row<PER>(logits, row, E, lane, v);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) acc[i] += v[i];
+  }
+#pragma unroll
+  for (int i = 0; i < PER; ++i) s_acc[warp][i * 32 + lane] = acc[i];
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    float a = 0.f;
+    for (int w = 0; w < kAuxWarps; ++w) a += s_acc[w][e];
+    part[(size_t)blockIdx.x * E + e] = a;
+  }
+}
+
+// sum over a block of 256 threads, in a fixed order, to every thread
+__device__ __forceinline__ float block_sum(float x, float* s_red) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffff, x, d);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = x;
+  __syncthreads();
+  float a = 0.f;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) a += s_red[w];
+  return a;
+}
+
+// loss, and grad[e] = d loss / d acc_e
+__global__ void __launch_bounds__(256)
+switch_loss_finish_kernel(const float* __restrict__ part, int blocks, const int* __restrict__ freq, int E,
+                          float* __restrict__ loss, float* __restrict__ grad) {
+  __shared__ float s_acc[1024], s_red[8];
+  float na = 0.f, nf = 0.f;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    float a = 0.f;
+    for (int b = 0; b < blocks; ++b) a += part[(size_t)b * E + e];
+    s_acc[e] = a;
+    na += fabsf(a);
+    nf += fabsf((float)freq[e]);
+  }
+  na = block_sum(na, s_red);
+  nf = fmaxf(block_sum(nf, s_red), kAuxEps);
+  const bool clamped = na < kAuxEps;
+  na = fmaxf(na, kAuxEps);
+  float dot = 0.f;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) dot += (s_acc[e] / na) * ((float)freq[e] / nf);
+  dot = block_sum(dot, s_red);
+  if (threadIdx.x == 0) *loss = (float)E * dot;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    const float sign = s_acc[e] > 0.f ? 1.f : (s_acc[e] < 0.f ? -1.f : 0.f);
+    grad[e] = (float)E * ((float)freq[e] / nf - (clamped ? 0.f : sign * dot)) / na;
+  }
+}
+
+template <int PER, typename L>
+__global__ void __launch_bounds__(256)
+switch_loss_bwd_kernel(const L* __restrict__ logits, int64_t T, int E, const float* __restrict__ grad,
+                       const float* __restrict__ dloss, L* __restrict__ dlogits) {
+  const int lane = threadIdx.x & 31;
+  const int64_t row = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= T) return;
+  float v[PER], g[PER], dot = 0.f;
+  softmax_row<PER>(logits, row, E, lane, v);
+  const float d = *dloss;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = i * 32 + lane;
+    g[i] = e < E ? d * grad[e] : 0.f;
+    dot = fmaf(v[i], g[i], dot);
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) dot += __shfl_xor_sync(0xffffffff, dot, s);
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = i * 32 + lane;
+    if (e < E) store_grad(dlogits, row * E + e, v[i] * (g[i] - dot));
   }
 }
 
@@ -194,21 +324,96 @@ int smoe_status_post(const int32_t* status, int32_t* pinned_host_word, void* str
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 
-int smoe_topk_softmax(const float* logits, int64_t T, int64_t E, int64_t K, float* scores, int32_t* idx,
-                      void* stream) {
+#define SMOE_ROUTER_PER(E, F) \
+  ((E) <= 32 ? F(1) : (E) <= 64 ? F(2) : (E) <= 128 ? F(4) : (E) <= 256 ? F(8) : F(32))
+
+int smoe_router_topk(const void* logits, int bf16, int64_t T, int64_t E, int64_t K, float* scores, int32_t* idx,
+                     void* stream) {
   if (T < 0 || E <= 0 || E > 1024 || K <= 0 || K > 32 || K > E) return SMOE_ERR_SHAPE;
   if (T == 0) return SMOE_OK;
-  topk_softmax_kernel<<<(unsigned)((T + 7) / 8), 256, 0, (cudaStream_t)stream>>>(logits, T, (int)E, (int)K, scores,
-                                                                                 idx);
+  const unsigned grid = (unsigned)((T + 7) / 8);
+  if (bf16) {
+#define SMOE_F(P) topk_softmax_kernel<P, __nv_bfloat16>
+    auto kern = SMOE_ROUTER_PER(E, SMOE_F);
+#undef SMOE_F
+    kern<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, T, (int)E, (int)K, scores, idx);
+  } else {
+#define SMOE_F(P) topk_softmax_kernel<P, float>
+    auto kern = SMOE_ROUTER_PER(E, SMOE_F);
+#undef SMOE_F
+    kern<<<grid, 256, 0, (cudaStream_t)stream>>>((const float*)logits, T, (int)E, (int)K, scores, idx);
+  }
+  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+}
+
+int smoe_topk_softmax(const float* logits, int64_t T, int64_t E, int64_t K, float* scores, int32_t* idx,
+                      void* stream) {
+  return smoe_router_topk(logits, 0, T, E, K, scores, idx, stream);
+}
+
+int smoe_router_topk_bwd(const float* scores, const int32_t* idx, const float* dscores, int64_t T, int64_t E, int64_t K,
+                         void* dlogits, int bf16, void* stream) {
+  if (T < 0 || E <= 0 || K <= 0 || K > 32) return SMOE_ERR_SHAPE;
+  if (T == 0) return SMOE_OK;
+  const unsigned grid = (unsigned)((T + 7) / 8);
+  if (bf16)
+    topk_softmax_bwd_kernel<__nv_bfloat16><<<grid, 256, 0, (cudaStream_t)stream>>>(scores, idx, dscores, T, (int)E, (int)K,
+                                                                    (__nv_bfloat16*)dlogits);
+  else
+    topk_softmax_bwd_kernel<float><<<grid, 256, 0, (cudaStream_t)stream>>>(scores, idx, dscores, T, (int)E, (int)K,
+                                                                    (float*)dlogits);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 
 int smoe_topk_softmax_bwd(const float* scores, const int32_t* idx, const float* dscores, int64_t T, int64_t E,
                           int64_t K, float* dlogits, void* stream) {
-  if (T < 0 || E <= 0 || K <= 0 || K > 32) return SMOE_ERR_SHAPE;
+  return smoe_router_topk_bwd(scores, idx, dscores, T, E, K, dlogits, 0, stream);
+}
+
+int64_t smoe_switch_loss_workspace(int64_t E) { return E > 0 ? kAuxBlocks * E * (int64_t)sizeof(float) : 0; }
+
+int smoe_switch_loss(const void* logits, int bf16, const int32_t* freq, int64_t T, int64_t E, float* loss, float* grad,
+                     void* workspace, void* stream) {
+  if (T < 0 || E <= 0 || E > 1024) return SMOE_ERR_SHAPE;
+  if ((T > 0 && !logits) || !freq || !loss || !grad || !workspace) return SMOE_ERR_ARG;
+  int64_t blocks = (T + kAuxWarps - 1) / kAuxWarps;
+  if (blocks > kAuxBlocks) blocks = kAuxBlocks;
+  float* part = (float*)workspace;
+  if (blocks > 0) {
+    if (bf16) {
+#define SMOE_F(P) switch_loss_sums_kernel<P, __nv_bfloat16>
+      auto kern = SMOE_ROUTER_PER(E, SMOE_F);
+#undef SMOE_F
+      kern<<<(unsigned)blocks, 32 * kAuxWarps, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, T, (int)E, part);
+    } else {
+#define SMOE_F(P) switch_loss_sums_kernel<P, float>
+      auto kern = SMOE_ROUTER_PER(E, SMOE_F);
+#undef SMOE_F
+      kern<<<(unsigned)blocks, 32 * kAuxWarps, 0, (cudaStream_t)stream>>>((const float*)logits, T, (int)E, part);
+    }
+  }
+  switch_loss_finish_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(part, (int)blocks, freq, (int)E, loss, grad);
+  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+}
+
+int smoe_switch_loss_bwd(const void* logits, int bf16, const float* grad, const float* dloss, int64_t T, int64_t E,
+                         void* dlogits, void* stream) {
+  if (T < 0 || E <= 0 || E > 1024) return SMOE_ERR_SHAPE;
   if (T == 0) return SMOE_OK;
-  topk_softmax_bwd_kernel<<<(unsigned)((T + 7) / 8), 256, 0, (cudaStream_t)stream>>>(scores, idx, dscores, T, (int)E,
-                                                                                     (int)K, dlogits);
+  if (!logits || !grad || !dloss || !dlogits) return SMOE_ERR_ARG;
+  const unsigned grid = (unsigned)((T + 7) / 8);
+  if (bf16) {
+#define SMOE_F(P) switch_loss_bwd_kernel<P, __nv_bfloat16>
+    auto kern = SMOE_ROUTER_PER(E, SMOE_F);
+#undef SMOE_F
+    kern<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, T, (int)E, grad, dloss,
+                                                 (__nv_bfloat16*)dlogits);
+  } else {
+#define SMOE_F(P) switch_loss_bwd_kernel<P, float>
+    auto kern = SMOE_ROUTER_PER(E, SMOE_F);
+#undef SMOE_F
+    kern<<<grid, 256, 0, (cudaStream_t)stream>>>((const float*)logits, T, (int)E, grad, dloss, (float*)dlogits);
+  }
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 

@@ -77,6 +77,11 @@ SIGNATURES = {
     "smoe_layer_backward": (_I, [ctypes.POINTER(LayerArgs), _P]),
     "smoe_topk_softmax": (_I, [_P, _L, _L, _L, _P, _P, _P]),
     "smoe_topk_softmax_bwd": (_I, [_P, _P, _P, _L, _L, _L, _P, _P]),
+    "smoe_router_topk": (_I, [_P, _I, _L, _L, _L, _P, _P, _P]),
+    "smoe_router_topk_bwd": (_I, [_P, _P, _P, _L, _L, _L, _P, _I, _P]),
+    "smoe_switch_loss_workspace": (_L, [_L]),
+    "smoe_switch_loss": (_I, [_P, _I, _P, _L, _L, _P, _P, _P, _P]),
+    "smoe_switch_loss_bwd": (_I, [_P, _I, _P, _P, _L, _L, _P, _P]),
 }
 
 # exported for the library's own tests and timing experiments only (csrc/smoe_internal.h); not product ABI

@@ -917,14 +917,34 @@ class _TopKSoftmax(torch.autograd.Function):
     def forward(ctx, logits, K):
         scores, idx = ops.topk_softmax(logits.contiguous(), int(K))
         ctx.save_for_backward(scores, idx)
-        ctx.E = logits.shape[1]
+        ctx.E, ctx.dtype = logits.shape[1], logits.dtype
         ctx.mark_non_differentiable(idx)
         return scores, idx
 
     @staticmethod
     def backward(ctx, dscores, _didx):
         scores, idx = ctx.saved_tensors
-        return ops.topk_softmax_bwd(scores, idx, dscores.contiguous().float(), ctx.E), None
+        return ops.topk_softmax_bwd(scores, idx, dscores.contiguous().float(), ctx.E, ctx.dtype), None
+
+
+class _SwitchLoss(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, logits, expert_frequency):
+        logits = logits.contiguous()
+        loss, grad = ops.switch_loss(logits, expert_frequency.contiguous())
+        ctx.save_for_backward(logits, grad)
+        return loss
+
+    @staticmethod
+    def backward(ctx, dloss):
+        logits, grad = ctx.saved_tensors
+        return ops.switch_loss_bwd(logits, grad, dloss.float().contiguous()), None
+
+
+def switch_loss(logits: torch.Tensor, expert_frequency: torch.Tensor) -> torch.Tensor:
+    """Switch auxiliary loss of router logits [T,E] and tokens per expert [E]: the expression of
+    `MoE._compute_switch_loss` in three kernels."""
+    return _SwitchLoss.apply(logits, expert_frequency)
 
 
 def _expert_major(w: torch.Tensor) -> torch.Tensor:
@@ -945,7 +965,7 @@ def moe_TC_softmax_topk_layer(x, router_w, w1, b1, w2, b2, K, stream_id, activat
     E = router_w.shape[0]
     w1_e, w2_e = _expert_major(w1), _expert_major(w2)
     logits = F.linear(x, router_w)
-    scores, idx = _TopKSoftmax.apply(logits.float(), K)
+    scores, idx = _TopKSoftmax.apply(logits if logits.dtype == torch.bfloat16 else logits.float(), K)
     TK = T * K
     args = (_one_call_args(x, idx, w1_e, w2_e, E, K, TK, -(-TK // 128) * 128 + E * 128, activation_code(activation_type), None)
             if b1 is None and b2 is None and K <= _MAX_PAIRS_PER_TOKEN else None)

@@ -12,7 +12,7 @@ import torch.nn.functional as F
 
 from .config import SonicMoEConfig
 from .enums import ActivationType, KernelBackendMoE, is_glu
-from .functional import enable_fp8, moe_TC_softmax_topk_layer
+from .functional import enable_fp8, moe_TC_softmax_topk_layer, switch_loss
 
 
 class Experts(nn.Module):
@@ -75,6 +75,9 @@ class MoE(nn.Module):
         hidden_states = hidden_states.view(original_shape)
         if is_inference_mode:
             aux_loss = None
+        elif (type(self)._compute_switch_loss is MoE._compute_switch_loss and self.num_experts <= 1024
+              and router_logits.dtype in (torch.float32, torch.bfloat16)):
+            aux_loss = switch_loss(router_logits, expert_frequency)
         else:
             aux_loss = self._compute_switch_loss(
                 logits=router_logits, probs=F.softmax(router_logits, dim=-1, dtype=torch.float32),

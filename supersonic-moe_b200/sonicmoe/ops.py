@@ -712,19 +712,47 @@ def ds_finalize(ds_partial, s_rev, TK, real_tk=None, src_idx=None, scatter_numel
 
 @_timed
 def topk_softmax(logits, K):
+    """Top-K of each row of f32 or bf16 logits [T,E] and the softmax over the K selected -> (scores f32 [T,K], idx [T,K])."""
     _cuda(logits)
-    assert logits.dtype == torch.float32 and logits.ndim == 2
+    assert logits.dtype in (torch.float32, torch.bfloat16) and logits.ndim == 2
     T, E = logits.shape
     scores = torch.empty(T, K, dtype=torch.float32, device=logits.device)
     idx = torch.empty(T, K, dtype=_I32, device=logits.device)
-    check(lib.smoe_topk_softmax(_p(logits), T, E, K, _p(scores), _p(idx), _stream()), "topk_softmax")
+    check(lib.smoe_router_topk(_p(logits), int(logits.dtype == torch.bfloat16), T, E, K, _p(scores), _p(idx), _stream()),
+          "topk_softmax")
     return scores, idx
 
 
 @_timed
-def topk_softmax_bwd(scores, idx, dscores, E):
+def topk_softmax_bwd(scores, idx, dscores, E, dtype=torch.float32):
     _cuda(scores, idx, dscores)
     T, K = scores.shape
-    out = torch.empty(T, E, dtype=torch.float32, device=scores.device)
-    check(lib.smoe_topk_softmax_bwd(_p(scores), _p(idx), _p(dscores), T, E, K, _p(out), _stream()), "topk_softmax_bwd")
+    out = torch.empty(T, E, dtype=dtype, device=scores.device)
+    check(lib.smoe_router_topk_bwd(_p(scores), _p(idx), _p(dscores), T, E, K, _p(out), int(dtype == torch.bfloat16),
+                                   _stream()), "topk_softmax_bwd")
+    return out
+
+
+@_timed
+def switch_loss(logits, freq):
+    """f32 or bf16 logits [T,E], tokens per expert i32 [E] -> (loss f32 scalar, its gradient f32 [E] with respect to the
+    column sums of softmax(logits))."""
+    _cuda(logits, freq)
+    assert logits.dtype in (torch.float32, torch.bfloat16) and freq.dtype == _I32
+    T, E = logits.shape
+    loss = torch.empty((), dtype=torch.float32, device=logits.device)
+    grad = torch.empty(E, dtype=torch.float32, device=logits.device)
+    ws = torch.empty(lib.smoe_switch_loss_workspace(E), dtype=_U8, device=logits.device)
+    check(lib.smoe_switch_loss(_p(logits), int(logits.dtype == torch.bfloat16), _p(freq), T, E, _p(loss), _p(grad), _p(ws),
+                               _stream()), "switch_loss")
+    return loss, grad
+
+
+@_timed
+def switch_loss_bwd(logits, grad, dloss):
+    _cuda(logits, grad, dloss)
+    T, E = logits.shape
+    out = torch.empty_like(logits)
+    check(lib.smoe_switch_loss_bwd(_p(logits), int(logits.dtype == torch.bfloat16), _p(grad), _p(dloss), T, E, _p(out),
+                                   _stream()), "switch_loss_bwd")
     return out

@@ -237,6 +237,34 @@ def test_topk_softmax_fwd_bwd(ops, T, E, K):
     torch.testing.assert_close(dl.cpu(), OM.router_backward(s.cpu(), ri, dsc, E), rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("T,E", [(1, 1), (9, 31), (64, 32), (65, 33), (300, 64), (301, 65), (64, 128), (33, 129), (40, 257), (17, 1024)])
+def test_router_kernels_on_bf16_logits(ops, T, E):
+    """bf16 logits go in as they are: the scores, indices and (rounded) gradients of the same values in f32, at the edges
+    of the kernels' expert slots; the auxiliary loss and its gradient against the tensor expression in f64."""
+    import torch.nn.functional as F
+    from sonicmoe.functional import switch_loss
+    g = torch.Generator().manual_seed(T + E)
+    K = min(E, 8)
+    logits = (2 * torch.randn(T, E, generator=g)).to(torch.bfloat16).to(DEV)
+    s, i = ops.topk_softmax(logits, K)
+    s32, i32 = ops.topk_softmax(logits.float(), K)
+    assert torch.equal(s, s32) and torch.equal(i, i32)
+    rs, ri = OM.router_topk_softmax(logits.float().cpu(), K)
+    assert torch.equal(i.cpu(), ri) and torch.allclose(s.cpu(), rs, rtol=1e-5, atol=1e-7)
+    ds = torch.randn(T, K, generator=g).to(DEV)
+    assert torch.equal(ops.topk_softmax_bwd(s, i, ds, E, torch.bfloat16), ops.topk_softmax_bwd(s, i, ds, E).to(torch.bfloat16))
+    freq = torch.randint(0, 50, (E,), generator=g, dtype=torch.int32).to(DEV)
+    for dt, tol in ((torch.bfloat16, 2 ** -8), (torch.float32, 1e-5)):        # one rounding of the result
+        x = logits.to(dt, copy=True).requires_grad_(True)
+        loss = switch_loss(x, freq)
+        loss.backward(torch.tensor(0.3, device=DEV))
+        x64 = logits.double().requires_grad_(True)
+        ref = E * (F.normalize(torch.softmax(x64, -1).sum(0), p=1, dim=0) * F.normalize(freq.double(), p=1, dim=0)).sum()
+        ref.backward(torch.tensor(0.3, device=DEV, dtype=torch.float64))
+        assert x.grad.dtype == dt and abs(float(loss.detach()) - float(ref.detach())) <= 1e-5 * abs(float(ref.detach())) + 1e-7
+        assert (x.grad.double() - x64.grad).norm() <= tol * x64.grad.norm() + 1e-7, (dt, E)
+
+
 def test_topk_softmax_rows_with_fewer_than_k_finite_logits(ops):
     """-inf-masked and NaN logits: the K indices stay distinct and in range (the finite ones first, then the lowest
     unused index with a score of exactly zero), the scores of the finite picks are their softmax, and the backward
