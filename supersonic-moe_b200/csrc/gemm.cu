@@ -57,12 +57,13 @@ static int make_tmap(CUtensorMap* m, CUtensorMapDataType dt, int esize, const vo
   return r == CUDA_SUCCESS ? SMOE_OK : SMOE_ERR_TMAP;
 }
 
-// Output of a weight gradient, [E, rows, N] in boxes of 32 rows x 64 bytes (f32, or bf16 with GemmParams::out_bf16).
-static int make_tmap_dw(CUtensorMap* m, const GemmParams& p) {
-  return p.out_bf16 ? make_tmap(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.c, (uint64_t)p.E * p.rows, p.N, 32, 32,
-                                CU_TENSOR_MAP_SWIZZLE_64B)
-                    : make_tmap(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.c, (uint64_t)p.E * p.rows, p.N, 16, 32,
-                                CU_TENSOR_MAP_SWIZZLE_64B);
+// Output of a weight gradient, [E, rows, N] in boxes of 32 rows: 64 bytes wide (f32, or bf16 with GemmParams::out_bf16),
+// or 128 bytes where the products are added to what is there.
+static int make_tmap_dw(CUtensorMap* m, const GemmParams& p, void* c, uint64_t rows) {
+  if (p.out_bf16)
+    return make_tmap(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c, (uint64_t)p.E * rows, p.N, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+  return make_tmap(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, (uint64_t)p.E * rows, p.N, p.accumulate ? 32 : 16, 32,
+                   p.accumulate ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 static int g_force_bn = 0;
@@ -136,6 +137,8 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   if (pairs <= 0) return SMOE_OK;
   GemmParams q = p;
   q.dbg_stage_cut = g_stage_cut;
+  if (MODE == WGRAD && p.accumulate && !p.out_bf16)
+    q.stages_lent = (S::EPI_WARPS * 4096 + S::STAGE_BYTES - 1) / S::STAGE_BYTES;
   q.l2_prefetch = g_l2_prefetch >= 0 ? g_l2_prefetch : kDefaultL2Prefetch;
   kern<<<(unsigned)(2 * pairs), S::THREADS, S::TOTAL, stream>>>(ta, tb, tsa, tsb, om.c, om.c2, om.c3, q);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
@@ -191,7 +194,7 @@ static int run3(const void* a, int64_t a_rows, int64_t a_cols, const void* b, in
   if (rc) return rc;
   int64_t pair_tiles;
   if (MODE == WGRAD) {
-    rc = make_tmap_dw(&tc, p);
+    rc = make_tmap_dw(&tc, p, p.c, p.rows);
     pair_tiles = (int64_t)p.E * (p.rows / 256) * (p.N / kBN3);
   } else {
     rc = make_tmap(&tc, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.c, p.rows, p.N, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
@@ -223,10 +226,8 @@ static int run3_wgrad_pair(const void* a1, const void* b1, GemmParams& p, const 
                           CU_TENSOR_MAP_SWIZZLE_NONE);
   if (!rc) rc = make_tmap(&sm.sfb, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, sfb2, sfb_tiles, 128, 128, kSfGroup2,
                           CU_TENSOR_MAP_SWIZZLE_NONE);
-  if (!rc) rc = make_tmap(&tc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.c, (uint64_t)p.E * M1, p.N, 16, 32,
-                          CU_TENSOR_MAP_SWIZZLE_64B);
-  if (!rc) rc = make_tmap(&sm.c, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.c2, (uint64_t)p.E * M2, p.N, 16, 32,
-                          CU_TENSOR_MAP_SWIZZLE_64B);
+  if (!rc) rc = make_tmap_dw(&tc, p, p.c, M1);
+  if (!rc) rc = make_tmap_dw(&sm.c, p, p.c2, M2);
   if (rc) return rc;
   const int64_t pair_tiles = (int64_t)p.E * ((M1 + M2) / 256) * (p.N / kBN3);
   return launch3<WGRAD>(ta, tb, tsa, tsb, tc, p, pair_tiles, stream, &sm);
@@ -311,7 +312,7 @@ static int run(const void* a, int64_t a_rows, int64_t a_cols, const void* b, int
         rc = make_tmap(&om.c, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.c, p.rows, p.N, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
         om.c2 = om.c;
       } else if (MODE == WGRAD) {
-        rc = make_tmap_dw(&om.c, p);
+        rc = make_tmap_dw(&om.c, p, p.c, p.rows);
         om.c2 = om.c;
       } else if (MODE == DGATEDQ) {
         rc = make_tmap(&om.c, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.dz, p.rows, 2 * (uint64_t)p.N, 64, 32,

@@ -59,6 +59,7 @@ struct GemmParams {
   int* status;          // device status word: 0 ok, else first failure code
   const int* s_scatter; // PLAIN / GATED, may be null: row r is padding where s_scatter[r] >= *real_tk; 32-row slabs of
   const int* real_tk;   // nothing but padding are then not stored (the two-CTA kernels)
+  int stages_lent;      // two-CTA WGRAD into an existing f32 gradient: ring stages that hold its staging tiles instead
   int debug_skip_store; // timing experiments only: drain TMEM but skip the global stores
   int dbg_stage_cut;    // timing experiments only: use this many fewer ring stages
   int l2_prefetch;      // K tiles ahead of the shared-memory ring at which operand tiles are prefetched into L2 (0 = off)

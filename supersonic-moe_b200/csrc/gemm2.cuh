@@ -141,6 +141,12 @@ __device__ __forceinline__ void stage_bf16_32(uint32_t stg, int lane, const uint
     st_shared_v4(stg + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4), w[0], w[1], w[2], w[3]);
   }
 }
+// one lane's 32 f32 columns -> its 128-byte row of a 32-row staging tile in the 128-byte TMA swizzle
+__device__ __forceinline__ void stage_f32_32(uint32_t stg, int lane, const uint32_t (&a)[32]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    st_shared_v4(stg + lane * 128 + ((j ^ (lane & 7)) << 4), a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
+}
 // sigmoid with two MUFU ops (ex2 + rcp); relative error ~1e-7, far below the
 // bf16 / e4m3 resolution of everything it feeds
 __device__ __forceinline__ float fast_sigmoid(float x) {
@@ -411,7 +417,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const uint32_t sf_base = smem_u32(sfring);
   const int n_col_tiles = (p.N + BN - 1) / BN;
   const int n_total = (MODE == WGRAD) ? p.E * (p.rows / (2 * BM)) * n_col_tiles : s_pairs[p.E] * n_col_tiles;
-  const int nst = S::STAGES - p.dbg_stage_cut;       // ring stages in use (all of them outside timing experiments)
+  const int nst = S::STAGES - p.dbg_stage_cut - p.stages_lent;       // ring stages in use
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
@@ -795,6 +801,26 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               bulk_commit_group();
             }
           }
+        } else if (p.accumulate) {
+          // Reduce-adds in whole 128-byte lines (32 columns), from 4 KB staging tiles in the ring stages lent for them; the
+          // L2 merges a 64-byte piece no cheaper than a line (E=128, M=768, N=2048: 400 -> 366 us; M=1536: 755 -> 729).
+          // What bounds the rest is read-modify-write traffic in tile order: reading the old values with the epilogue's
+          // own loads instead took 920 us, more staging tiles (two or three a warp) 760 and 834 us, fetching the tile
+          // towards L2 ahead of time 800 us.
+          const uint32_t sb = smem_base + nst * S::STAGE_BYTES + (warp - 2) * 4096;
+          const int crow = t.e * p.rows + t.m0 + q * 32;
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            if (lane == 0) bulk_wait_group_read<0>();
+            __syncwarp();
+            stage_f32_32(sb, lane, acc[c]);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_reduce_add_2d(&tmap_c, sb, c_base + c * 32, crow);
+              bulk_commit_group();
+            }
+          }
         } else
 #pragma unroll
         for (int c = 0; c < 2 * NC; ++c) {
@@ -810,8 +836,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           __syncwarp();
           if (lane == 0) {
             const int crow = t.e * p.rows + t.m0 + q * 32;
-            if (p.accumulate) tma_reduce_add_2d(&tmap_c, sb, c_base + c * 16, crow);
-            else tma_store_2d(&tmap_c, sb, c_base + c * 16, crow);
+            tma_store_2d(&tmap_c, sb, c_base + c * 16, crow);
             bulk_commit_group();
           }
         }

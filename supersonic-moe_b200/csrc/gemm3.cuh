@@ -506,6 +506,22 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             }
             continue;
           }
+          if (p.accumulate) {                   // whole 128-byte lines, both staging buffers as one (see gemm2.cuh)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+              if (lane == 0) bulk_wait_group_read<0>();
+              __syncwarp();
+              stage_f32_32(stg, lane, acc[c]);
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                tma_reduce_add_2d(t.prob ? &second.c : &tmap_c, stg, t.n0 + h * HN + grp * CPW + c * 32,
+                                  t.e * (t.prob ? p.rows2 : p.rows) + t.m0 + q * 32);
+                bulk_commit_group();
+              }
+            }
+            continue;
+          }
 #pragma unroll
           for (int c = 0; c < 2 * NC; ++c) {
             const uint32_t sb = stg + buf * 2048;
@@ -522,8 +538,7 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               const int crow = t.e * (t.prob ? p.rows2 : p.rows) + t.m0 + q * 32;
               const int ccol = t.n0 + h * HN + grp * CPW + c * 16;
               const CUtensorMap* tc = t.prob ? &second.c : &tmap_c;
-              if (p.accumulate) tma_reduce_add_2d(tc, sb, ccol, crow);
-              else tma_store_2d(tc, sb, ccol, crow);
+              tma_store_2d(tc, sb, ccol, crow);
               bulk_commit_group();
             }
             buf ^= 1;

@@ -580,6 +580,36 @@ def test_quant_dual_gather_matches_single_direction_kernels(ops, T, K, rows, val
     assert torch.equal(q_col[:valid].cpu(), o_q) and torch.equal(got[:, :valid // 32], o_sc)
 
 
+@pytest.mark.parametrize("bn,M,N,layout", [(0, 256, 768, 0), (0, 512, 256, 3), (256, 256, 768, 1), (192, 512, 384, 0), (128, 256, 384, 0)])
+def test_wgrad_accumulation_is_one_f32_addition(ops, bn, M, N, layout):
+    """Every tile form adds its product to the old gradient exactly once: old + (the product an overwriting call stores), to
+    the bit, for experts of one to nine row tiles, none, and after an empty one."""
+    from sonicmoe._lib import lib
+    g = torch.Generator().manual_seed(M + N + bn)
+    tiles = [1, 0, 9, 2, 1]
+    efo = make_efo(tiles).to(DEV)
+    TKp, E = int(efo[-1]), len(tiles)
+    a_q, a_sc = rand_fp8((M, TKp), g)
+    b_q, b_sc = rand_fp8((N, TKp), g)
+    a_sf, b_sf = Q.pack_isa(a_sc, M, TKp).to(DEV), Q.pack_isa(b_sc, N, TKp).to(DEV)
+    a = (a_q.t() if layout & 1 else a_q).contiguous().to(DEV)
+    b = (b_q.t() if layout & 2 else b_q).contiguous().to(DEV)
+    old = torch.randn(E, M, N, generator=g).to(DEV)
+    out, fresh = old.clone(), torch.full_like(old, 7.0)
+    lib.smoe_internal_gemm_knobs(bn)
+    try:
+        for dst, acc in ((out, True), (fresh, False)):
+            if layout:
+                ops.gemm_wgrad_mn(a, a_sf, b, b_sf, efo, dst, acc, bool(layout & 1), bool(layout & 2))
+            else:
+                ops.gemm_wgrad(a, a_sf, b, b_sf, efo, dst, accumulate=acc)
+        torch.cuda.synchronize()
+        ops.check_status(DEV)
+    finally:
+        lib.smoe_internal_gemm_knobs(0)
+    assert torch.equal(out, old + fresh)
+
+
 @pytest.mark.parametrize("layout", [1, 2, 3])
 @pytest.mark.parametrize("M,N,tiles", [(256, 256, [1, 0, 2, 1]), (512, 768, [3, 2, 0, 0, 4, 1, 1, 2]), (768, 256, [2, 1, 3])])
 def test_gemm_wgrad_mn_major_operands(ops, layout, M, N, tiles):
