@@ -61,6 +61,19 @@ def test_topk_metadata_bit_exact(ops, N, K, E, p_mask, skew, lane_order, pad_mod
         assert torch.equal(got[k].cpu(), ref[k]), k
 
 
+@pytest.mark.parametrize("K", [1, 3, 5, 9, 16])
+@pytest.mark.parametrize("N", [31, 33, 290])
+@pytest.mark.parametrize("lane_order", [0, 1])
+def test_topk_metadata_slot_counts_between_powers_of_two(ops, K, N, lane_order):
+    """The scatter runs a unit of 32 rows on 1 to 16 warps: every width, full and partial units, masked slots."""
+    idx, probs = make_routing(N, K, 20, 0.3, seed=N + K)
+    got = ops.topk_metadata(idx.to(DEV), probs.to(DEV), 20, 128, lane_order=lane_order)
+    ref = R.topk_metadata(idx, probs, 20, 128, TK_alloc=got["TK_alloc"], TKp_alloc=got["TKp_alloc"],
+                          lane_order=["expert", "slot"][lane_order])
+    for k in MD_KEYS:
+        assert torch.equal(got[k].cpu(), ref[k]), k
+
+
 def test_topk_metadata_alignment_one(ops):
     idx, probs = make_routing(500, 4, 16, 0.1, seed=9)
     got = ops.topk_metadata(idx.to(DEV), probs.to(DEV), 16, 1)
