@@ -84,11 +84,11 @@ quant_rows_kernel(const uint4* __restrict__ x, int64_t M, int K, uint2* __restri
       const int g = col >> 5;
       if (in && (lane & 15) == 0) {
         const uint32_t word = (uint32_t)e | (b1 << 8) | (b2 << 16) | (b3 << 24);
-        if (g + 3 < groups) {
+        if (g + 3 < groups && (groups & 3) == 0) {       // rows of scales start on words
           if (raw) *reinterpret_cast<uint32_t*>(raw + row * groups + g) = word;
           if (isa) *reinterpret_cast<uint32_t*>(isa + isa_offset(row, g, k_tiles)) = word;
         } else {
-          for (int j = 0; g + j < groups; ++j) {
+          for (int j = 0; j < 4 && g + j < groups; ++j) {
             const uint8_t b = (uint8_t)(word >> (8 * j));
             if (raw) raw[row * groups + g + j] = b;
             if (isa) isa[isa_offset(row, g + j, k_tiles)] = b;
