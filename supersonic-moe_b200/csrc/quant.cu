@@ -421,6 +421,12 @@ quant_cols_kernel(const void* __restrict__ src_, const uint8_t* __restrict__ src
 // Measured at E=128, H=2048, I=768 (604 M weights, 2.45 GB, one launch per weight): 421 us = 5.8 TB/s, 0.89 of a plain
 // copy; one launch per expert for the transposed copy and a second read for the row copy took 3719 us (host-bound: 256
 // launches; their kernels alone 1345 us).
+__device__ __forceinline__ uint32_t q_max_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+
 constexpr int QW_TILE = 128, QW_PITCH = QW_TILE + 8;      // bf16 elements; 272 bytes: 16-byte aligned rows
 
 template <bool ROW, bool COL>
@@ -509,6 +515,177 @@ quant_weight_kernel(const __nv_bfloat16* __restrict__ w, int N, int K, uint8_t* 
   }
 }
 
+// ------------------------------------------------------------------ columns of gathered rows
+// Column-quantised operands of the weight gradients: row r of the operand is source row idx[r] (or r), one scale per column
+// and 32 rows.  FP8: the source is e4m3 with raw row-wise 1x32 scales, dequantised (exact in bf16) first.
+// A warp quantises 32 rows x 64 columns by itself: a lane holds eight consecutive rows of eight columns in registers and two
+// shuffles complete a column's maximum.  There is no barrier: every form that had one (64 columns staged in bf16, the
+// kernel above; 128 x 128 tiles whose bytes cross shared memory, with and without the next tile prefetched) took 86-96 us at
+// T=8192, H=3072, K=E=8 (201 MB out), 65 us of it with neither loads nor stores: the warps waited for one another.
+
+// Eight rows of this lane's eight columns, as bf16 pairs of adjacent columns
+template <bool FP8>
+__device__ __forceinline__ void qc_load(const void* __restrict__ src, const uint8_t* __restrict__ src_scales,
+                                        const int (&srow)[8], int dim, int col, uint4 (&v)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const size_t at = (size_t)srow[i] * dim + col;
+    if (FP8) {
+      const uint2 b = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(src) + at));
+      v[i] = make_uint4(b.x, b.y, __ldg(src_scales + (size_t)srow[i] * (dim >> 5) + (col >> 5)), 0);
+    } else {
+      v[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(src) + at));
+    }
+  }
+}
+// Dequantises (FP8) and scales: qs[j] of column j of the eight; returns the scale bytes of columns 2 * sub and 2 * sub + 1
+template <bool FP8>
+__device__ __forceinline__ uint32_t qc_scales(uint4 (&v)[8], int sub, float (&qs)[8]) {
+  if (FP8) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float sc = __int_as_float((int)v[i].z << 23);
+      const uint32_t w[2] = {v[i].x, v[i].y};
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t h2;
+        asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"((uint16_t)(w[j >> 1] >> (16 * (j & 1)))));
+        const float lo = __half2float(__ushort_as_half((unsigned short)(h2 & 0xFFFF))) * sc;
+        const float hi = __half2float(__ushort_as_half((unsigned short)(h2 >> 16))) * sc;
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[j]) : "f"(hi), "f"(lo));
+      }
+      v[i] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+  uint32_t e_pair = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t w = j == 0 ? v[i].x : j == 1 ? v[i].y : j == 2 ? v[i].z : v[i].w;
+      m = q_max_bf16x2(m, w & 0x7FFF7FFFu);
+    }
+    m = q_max_bf16x2(m, __shfl_xor_sync(0xffffffff, m, 8));
+    m = q_max_bf16x2(m, __shfl_xor_sync(0xffffffff, m, 16));
+    const int e0 = q_e8m0_of(__uint_as_float(m << 16)), e1 = q_e8m0_of(__uint_as_float(m & 0xFFFF0000u));
+    qs[2 * j] = q_scale_of(e0);
+    qs[2 * j + 1] = q_scale_of(e1);
+    if (sub == j) e_pair = (uint32_t)e0 | ((uint32_t)e1 << 8);
+  }
+  return e_pair;
+}
+
+// q [rows, dim], read MN-major by the weight-gradient GEMM.  A block is four 32-row groups x 128 columns, column tiles
+// fastest.  T=8192, H=3072, K=E=8: 86.0 -> 71.7 us; T=16384, H=2048, K=8, E=128 (285 MB out): 125 -> 102 us, against a warp
+// per 32 x 256 slab, whose 255 registers left four warps an SM.
+constexpr int QC_TILES = 4;      // row tiles of a block, one after the other
+
+__global__ void __launch_bounds__(256, 4)
+quant_cols_rows_kernel(const void* __restrict__ src, const int* __restrict__ idx, const int* __restrict__ valid_rows,
+                       int64_t rows, int dim, uint8_t* __restrict__ q, uint8_t* __restrict__ col_isa) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane >> 3;
+  const int ct = blockIdx.x % (dim >> 7), rt0 = blockIdx.x / (dim >> 7) * QC_TILES;
+  const int grp = warp >> 1;                                          // 32-row group of the 128-row tile
+  const int col = ct * 128 + (warp & 1) * 64 + (lane & 7) * 8;        // this lane's columns [col, col + 8)
+  const int row0 = grp * 32 + sub * 8;                                // and rows of a tile [row0, row0 + 8)
+  const int rt_end = min(rt0 + QC_TILES, (int)(rows >> 7));
+  int srow[8];                                                        // their source rows, one tile ahead
+#pragma unroll
+  for (int i = 0; i < 8; ++i) srow[i] = idx ? idx[(int64_t)rt0 * 128 + row0 + i] : rt0 * 128 + row0 + i;
+  const int64_t n_valid = valid_rows != nullptr ? min((int64_t)*valid_rows, rows) : rows;
+  for (int rt = rt0; rt < rt_end; ++rt) {
+    const int64_t r0 = (int64_t)rt * 128;
+    if (r0 + 32 * grp >= n_valid) return;                             // over-allocated tail: no GEMM reads it
+    uint4 v[8];
+    qc_load<false>(src, nullptr, srow, dim, col, v);
+    if (rt + 1 < rt_end) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) srow[i] = idx ? idx[r0 + 128 + row0 + i] : (int)r0 + 128 + row0 + i;
+    }
+    float qs[8];
+    const uint32_t e_pair = qc_scales<false>(v, sub, qs);
+    uint8_t* dst = q + (size_t)(r0 + row0) * dim + col;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float f[8];
+      bf16x8_to_f32(v[i], f);
+      *reinterpret_cast<uint2*>(dst + (size_t)i * dim) =
+          make_uint2(q_pack4(f[0] * qs[0], f[1] * qs[1], f[2] * qs[2], f[3] * qs[3]),
+                     q_pack4(f[4] * qs[4], f[5] * qs[5], f[6] * qs[6], f[7] * qs[7]));
+    }
+    const int cc = (col + 2 * sub) & 127;                             // ISA tile of (column tile, row tile)
+    uint8_t* isa = col_isa + ((size_t)ct * (size_t)(rows >> 7) + rt) * 512 + (cc >> 5) * 4 + grp;
+    isa[(cc & 31) * 16] = (uint8_t)e_pair;
+    isa[((cc & 31) + 1) * 16] = (uint8_t)(e_pair >> 8);
+  }
+}
+
+// q [dim, rows]: the reduction dimension contiguous.  A warp walks the four 32-row groups of a 128-row tile, gathers the bytes
+// of its 64 columns in 8 KB of shared memory of its own and then stores them as whole 128-byte lines (32-byte pieces
+// straight from the registers: 96 us).  Same sizes as above: 96 -> 85 and 137 -> 117 us.  (Writes alone bound it: plain stores
+// of 201 MB take 55 us.)
+constexpr int QT_WARPS = 4;
+
+template <bool FP8>
+__global__ void __launch_bounds__(32 * QT_WARPS, 6)
+quant_cols_t_kernel(const void* __restrict__ src, const uint8_t* __restrict__ src_scales, const int* __restrict__ idx,
+                    const int* __restrict__ valid_rows, int64_t rows, int dim, uint8_t* __restrict__ q_t,
+                    uint8_t* __restrict__ col_isa) {
+  __shared__ __align__(16) uint8_t s_bytes[QT_WARPS][64 * 128];       // [column][row], 8-byte chunks swizzled
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l8 = lane & 7, sub = lane >> 3;
+  const int64_t r0 = (int64_t)blockIdx.x * 128;
+  const int c0 = (blockIdx.y * QT_WARPS + warp) * 64;                 // this warp's columns [c0, c0 + 64)
+  if (c0 >= dim) return;
+  const int col = c0 + l8 * 8;
+  int srow[8];                                                        // source rows of a group, one group ahead
+#pragma unroll
+  for (int i = 0; i < 8; ++i) srow[i] = idx ? idx[r0 + sub * 8 + i] : (int)r0 + sub * 8 + i;
+  if (valid_rows != nullptr && r0 >= *valid_rows) return;             // over-allocated tail: no GEMM reads it
+  uint8_t* s = s_bytes[warp];
+  const int swz = (l8 & 3) << 2;                                      // chunk c of a column lies at slot c ^ swz
+  uint32_t sc0 = 0, sc1 = 0;                                          // four scale bytes of columns 2 * sub, 2 * sub + 1
+#pragma unroll 1
+  for (int g = 0; g < 4; ++g) {
+    uint4 v[8];
+    qc_load<FP8>(src, src_scales, srow, dim, col, v);
+    if (g < 3) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int64_t r = r0 + (g + 1) * 32 + sub * 8 + i;
+        srow[i] = idx ? idx[r] : (int)r;
+      }
+    }
+    float qs[8];
+    const uint32_t e_pair = qc_scales<FP8>(v, sub, qs);
+    sc0 |= (e_pair & 0xFF) << (8 * g);
+    sc1 |= (e_pair >> 8) << (8 * g);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float f[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t w = (j >> 1) == 0 ? v[i].x : (j >> 1) == 1 ? v[i].y : (j >> 1) == 2 ? v[i].z : v[i].w;
+        f[i] = __uint_as_float((j & 1) ? (w & 0xFFFF0000u) : (w << 16)) * qs[j];
+      }
+      *reinterpret_cast<uint2*>(s + (l8 * 8 + j) * 128 + (((g * 4 + sub) ^ swz) << 3)) =
+          make_uint2(q_pack4(f[0], f[1], f[2], f[3]), q_pack4(f[4], f[5], f[6], f[7]));
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int p = 0; p < 16; ++p) {
+    const int c = p * 4 + sub;
+    const uint4 o = *reinterpret_cast<const uint4*>(s + c * 128 + ((l8 ^ (((c >> 3) & 3) << 1)) << 4));
+    *reinterpret_cast<uint4*>(q_t + (size_t)(c0 + c) * rows + r0 + l8 * 16) = o;
+  }
+  const int cc = (col + 2 * sub) & 127;                               // ISA tile of (column tile, row tile)
+  uint8_t* isa = col_isa + ((size_t)(col >> 7) * (size_t)(rows >> 7) + blockIdx.x) * 512 + (cc >> 5) * 4;
+  *reinterpret_cast<uint32_t*>(isa + (cc & 31) * 16) = sc0;
+  *reinterpret_cast<uint32_t*>(isa + ((cc & 31) + 1) * 16) = sc1;
+}
+
 }  // namespace smoe
 
 using namespace smoe;
@@ -518,7 +695,6 @@ using namespace smoe;
 // loads in flight).  Column scales (one per column and 32 rows) need no communication at all, row scales
 // (one per row and 32 columns) two shuffles per row.  Both payloads leave row-major: the column-scaled one is a
 // weight-gradient operand read MN-major by the tensor core, so no transposed copy is written.
-template <bool WITH_ROWS>
 __global__ void __launch_bounds__(128)
 quant_dual_kernel(const uint4* __restrict__ x, const int* __restrict__ idx, const int* __restrict__ valid_rows,
                   int64_t rows, int K, uint2* __restrict__ q_row, uint8_t* __restrict__ row_isa,
@@ -554,17 +730,15 @@ quant_dual_kernel(const uint4* __restrict__ x, const int* __restrict__ idx, cons
       cam[j] = fmaxf(cam[j], fabsf(f[j]));
       ram = fmaxf(ram, fabsf(f[j]));
     }
-    if (WITH_ROWS) {
-      ram = fmaxf(ram, __shfl_xor_sync(0xffffffff, ram, 1));
-      ram = fmaxf(ram, __shfl_xor_sync(0xffffffff, ram, 2));
-      const int e = q_e8m0_of(ram);
-      const float qs = q_scale_of(e);
-      uint2 o;
-      o.x = q_pack4(f[0] * qs, f[1] * qs, f[2] * qs, f[3] * qs);
-      o.y = q_pack4(f[4] * qs, f[5] * qs, f[6] * qs, f[7] * qs);
-      q_row[((r0 + r) * K + col0) >> 3] = o;
-      if ((lane & 3) == 0) row_isa[isa_offset((size_t)(r0 + r), (size_t)(col0 >> 5), row_kt)] = (uint8_t)e;
-    }
+    ram = fmaxf(ram, __shfl_xor_sync(0xffffffff, ram, 1));
+    ram = fmaxf(ram, __shfl_xor_sync(0xffffffff, ram, 2));
+    const int e = q_e8m0_of(ram);
+    const float qs = q_scale_of(e);
+    uint2 o;
+    o.x = q_pack4(f[0] * qs, f[1] * qs, f[2] * qs, f[3] * qs);
+    o.y = q_pack4(f[4] * qs, f[5] * qs, f[6] * qs, f[7] * qs);
+    q_row[((r0 + r) * K + col0) >> 3] = o;
+    if ((lane & 3) == 0) row_isa[isa_offset((size_t)(r0 + r), (size_t)(col0 >> 5), row_kt)] = (uint8_t)e;
   }
   float qs[8];
 #pragma unroll
@@ -584,6 +758,12 @@ quant_dual_kernel(const uint4* __restrict__ x, const int* __restrict__ idx, cons
   }
 }
 
+
+// The barrier-free form of the transposed column quantizer (every dim a GEMM takes; at dim = 3072 96 -> 85 us, see there).
+// Half a scale tile more, or buffers off the 16-byte boundary of its accesses, go to the kernel that stages 64 columns.
+static bool whole_tiles(int64_t dim, const void* src, const void* q, const void* isa) {
+  return dim % 128 == 0 && (((uintptr_t)src | (uintptr_t)q | (uintptr_t)isa) & 15) == 0;
+}
 
 extern "C" {
 
@@ -660,6 +840,12 @@ int smoe_quant_cols_t(const void* src_bf16, const int32_t* idx, const int32_t* v
                       void* q_t, void* isa, void* stream) {
   if (rows < 0 || rows % 128 || dim <= 0 || dim % 64) return SMOE_ERR_SHAPE;
   if (rows == 0) return SMOE_OK;
+  if (whole_tiles(dim, src_bf16, q_t, isa)) {
+    quant_cols_t_kernel<false><<<dim3((unsigned)(rows / 128), (unsigned)((dim + 255) / 256)), 32 * QT_WARPS, 0,
+                                 (cudaStream_t)stream>>>(src_bf16, nullptr, idx, valid_rows, rows, (int)dim, (uint8_t*)q_t,
+                                                         (uint8_t*)isa);
+    return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  }
   dim3 grid((unsigned)(rows / CT_ROWS), (unsigned)(dim / CT_COLS));
   quant_cols_kernel<false, false><<<grid, 256, 0, (cudaStream_t)stream>>>(
       src_bf16, nullptr, idx, rows, (int)dim, (uint8_t*)q_t, (uint8_t*)isa, nullptr, nullptr, valid_rows);
@@ -671,6 +857,12 @@ int smoe_requant_cols_t(const void* src_fp8, const void* src_scales, const int32
   if (rows < 0 || rows % 128 || dim <= 0 || dim % 64) return SMOE_ERR_SHAPE;
   if (rows == 0) return SMOE_OK;      // nothing routed: not an error, and the (empty) buffers may be null
   if (!src_scales) return SMOE_ERR_ARG;
+  if (whole_tiles(dim, src_fp8, q_t, isa)) {
+    quant_cols_t_kernel<true><<<dim3((unsigned)(rows / 128), (unsigned)((dim + 255) / 256)), 32 * QT_WARPS, 0,
+                                (cudaStream_t)stream>>>(src_fp8, (const uint8_t*)src_scales, idx, valid_rows, rows, (int)dim,
+                                                        (uint8_t*)q_t, (uint8_t*)isa);
+    return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  }
   dim3 grid((unsigned)(rows / CT_ROWS), (unsigned)(dim / CT_COLS));
   quant_cols_kernel<false, true><<<grid, 256, 0, (cudaStream_t)stream>>>(
       src_fp8, (const uint8_t*)src_scales, idx, rows, (int)dim, (uint8_t*)q_t, (uint8_t*)isa, nullptr, nullptr,
@@ -721,15 +913,17 @@ int smoe_quant_dual_gather(const void* x_bf16, const int32_t* idx, const int32_t
   if (rows < 0 || rows % 128 || K <= 0 || K % 256) return SMOE_ERR_SHAPE;
   if (rows == 0) return SMOE_OK;      // nothing routed: not an error, and the (empty) buffers may be null
   if (!q_col || !col_isa || ((q_row == nullptr) != (row_isa == nullptr))) return SMOE_ERR_ARG;
-  const int64_t tasks = (rows / 32) * (K / 256);
-  const unsigned blocks = (unsigned)((tasks + 3) / 4);
-  if (q_row)
-    quant_dual_kernel<true><<<blocks, 128, 0, (cudaStream_t)stream>>>(
+  if (((uintptr_t)x_bf16 & 15) || ((uintptr_t)q_col & 7) || ((uintptr_t)q_row & 7)) return SMOE_ERR_ALIGN;
+  if (q_row) {
+    const int64_t tasks = (rows / 32) * (K / 256);
+    quant_dual_kernel<<<(unsigned)((tasks + 3) / 4), 128, 0, (cudaStream_t)stream>>>(
         (const uint4*)x_bf16, idx, valid_rows, rows, (int)K, (uint2*)q_row, (uint8_t*)row_isa, (uint2*)q_col,
         (uint8_t*)col_isa);
-  else
-    quant_dual_kernel<false><<<blocks, 128, 0, (cudaStream_t)stream>>>(
-        (const uint4*)x_bf16, idx, valid_rows, rows, (int)K, nullptr, nullptr, (uint2*)q_col, (uint8_t*)col_isa);
+  } else {
+    const int64_t blocks = (K / 128) * ((rows / 128 + QC_TILES - 1) / QC_TILES);
+    quant_cols_rows_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(x_bf16, idx, valid_rows, rows, (int)K,
+                                                                               (uint8_t*)q_col, (uint8_t*)col_isa);
+  }
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 

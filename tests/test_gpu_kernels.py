@@ -567,6 +567,33 @@ def test_gemm_wgrad(ops, bn, M, N, tiles):
         torch.testing.assert_close(out[e], init[e].to(DEV) + ref, rtol=1e-4, atol=1e-2 * ref.abs().max().item() + 1e-6)
 
 
+@pytest.mark.parametrize("form", ["transposed", "fp8", "rows"])
+@pytest.mark.parametrize("T,dim,rows,valid", [(40, 256, 384, 384), (300, 768, 256, 160), (9, 512, 128, 32), (130, 192, 256, 256), (70, 256, 256, 0)])
+def test_column_quantizer_tiles(ops, form, T, dim, rows, valid):
+    """Column scales of gathered rows against the oracle: adversarial magnitudes, a last tile that is partly beyond
+    *valid_rows (32-row groups of the row-major form, whole tiles of the others), half a column tile, nothing valid."""
+    if form == "rows" and dim % 256:
+        pytest.skip("the row-major form takes multiples of 256")
+    g = torch.Generator().manual_seed(T + dim)
+    x = adversarial_rows(max(T, 8), dim, T)
+    idx = torch.randint(0, x.shape[0], (rows,), generator=g, dtype=torch.int32)
+    vr = torch.tensor([valid], dtype=torch.int32, device=DEV)
+    src = x
+    if form == "fp8":
+        q, raw, _ = ops.quant_rows(x.to(DEV), raw=True)
+        src = deq(q.cpu(), raw.cpu()).to(torch.bfloat16)
+        got, isa = ops.requant_cols_t(q, raw, idx.to(DEV), rows, vr)
+    elif form == "transposed":
+        got, isa = ops.quant_cols_t(x.to(DEV), idx.to(DEV), rows, valid_rows=vr)
+    else:
+        _, _, got, isa = ops.quant_dual_gather(x.to(DEV), idx.to(DEV), rows, vr, with_rows=False)
+    torch.cuda.synchronize()
+    o_q, o_sc = Q.col_quant(src[idx.long()].float())
+    got = got.cpu() if form == "rows" else got.t().cpu()
+    assert torch.equal(got[:valid], o_q[:valid])
+    assert torch.equal(Q.unpack_isa(isa.cpu(), dim, rows)[:, :valid // 32], o_sc[:, :valid // 32])
+
+
 @pytest.mark.parametrize("T,K,rows,valid", [(64, 256, 256, 256), (300, 768, 1024, 896), (128, 512, 384, 128)])
 def test_quant_dual_gather_matches_single_direction_kernels(ops, T, K, rows, valid):
     """One pass over gathered rows = the bytes of quant_rows_gather (row-wise) and quant_cols_t (column-wise)."""
