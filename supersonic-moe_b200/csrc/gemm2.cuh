@@ -1087,6 +1087,9 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
           const float2 ds_eo = f2_get(ds2);
           p.ds_partial[(size_t)((t.n0 / BN) * S::COL_GROUPS + half) * p.rows + grow] = ds_eo.x + ds_eo.y;
+        } else if (t.valid && c_base >= p.N) {
+          // a column group wholly beyond a ragged N: its partial sum is one of those added up
+          p.ds_partial[(size_t)((t.n0 / BN) * S::COL_GROUPS + half) * p.rows + grow] = 0.f;
         }
       } else {  // DGATED
         // this warp: D columns [c_base, c_base + BN/2) of I in chunks of 32 -> dz 64 bf16 (128-byte rows,

@@ -570,7 +570,7 @@ def gemm_dgated_fused(dg_q, a_sf, w2t_q, w2t_sf, efo, z_q, z_sc, s, rows, a_idx=
     dz_rsf = torch.empty(isa_bytes(rows, 2 * N), dtype=_U8, device=dev)
     dz_csf = torch.empty(isa_bytes(2 * N, rows), dtype=_U8, device=dev)
     y1s_sf = torch.empty(isa_bytes(N, rows), dtype=_U8, device=dev)
-    dsp = torch.zeros(parts, rows, dtype=torch.float32, device=dev)
+    dsp = torch.empty(parts, rows, dtype=torch.float32, device=dev)      # every partial of a row below efo[E] is written
     if a_idx is not None:
         check(lib.smoe_gemm_dgated_fused_gather(_p(dg_q), dg_q.shape[0], _p(a_idx), _p(a_sf), _p(w2t_q), _p(w2t_sf),
                                                 _p(efo), _p(z_q), _p(z_sc), _p(s), _p(dz_q), _p(dz_rsf), _p(dz_csf),

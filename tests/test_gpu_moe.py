@@ -88,7 +88,8 @@ def oracle_dense(x, dy, w1, w2, wr, K, logits):
 
 
 @pytest.mark.parametrize("grads", ["main_grad", "bf16", "f32_weights", "w2_only", "no_scores"])
-@pytest.mark.parametrize("T,H,I,E,K", [(1, 256, 128, 8, 2), (130, 768, 256, 6, 3), (257, 512, 256, 4, 4), (64, 384, 128, 40, 8)])
+@pytest.mark.parametrize("T,H,I,E,K", [(1, 256, 128, 8, 2), (130, 768, 256, 6, 3), (257, 512, 256, 4, 4), (64, 384, 128, 40, 8),
+                                       (40, 256, 4096, 3, 2)])
 def test_one_call_layer_gives_the_bits_of_the_step_by_step_path(sm, monkeypatch, T, H, I, E, K, grads):
     """csrc/layer.cu makes the calls of the autograd Functions: outputs and every gradient are the same bits, also with
     masked slots, exact sizing, and only some of the inputs wanting gradients."""
@@ -108,6 +109,10 @@ def test_one_call_layer_gives_the_bits_of_the_step_by_step_path(sm, monkeypatch,
         if grads == "main_grad":
             a[1].main_grad = torch.full((E, 2 * I, H), 0.5, device=DEV)
             a[2].main_grad = torch.full((E, I, H), 0.25, device=DEV)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        dirt = [torch.full((1 << n,), 255, dtype=torch.uint8, device=DEV) for n in range(27, 15, -1)]
+        del dirt                                     # scratch starts as NaN on either path
         out = sm.run_sonic_moe(a[0], idx.to(DEV), a[3], K, E, a[1], a[2], fp8=True, **kw)
         out.backward(dy.to(DEV))
         torch.cuda.synchronize()
