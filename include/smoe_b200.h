@@ -370,6 +370,10 @@ int smoe_glu_bwd(const void* d_bf16, const void* z_fp8, const void* z_scales, co
 int smoe_combine(const void* y_bf16, const int32_t* s_rev, const int32_t* naept, const float* scores, void* out_bf16,
                  int64_t T, int64_t H, void* stream);
 
+/* The same, and - with pinned_host_word, see smoe_status_post - the status word stored there by the same kernel. */
+int smoe_combine_post(const void* y_bf16, const int32_t* s_rev, const int32_t* naept, const float* scores, void* out_bf16,
+                      int64_t T, int64_t H, const int32_t* status, int32_t* pinned_host_word, void* stream);
+
 /* s[p] = scores[s_scatter_idx[p]] for p < rows (replaces the score gather of
  * sonicmoe/functional/__init__.py:2105). */
 int smoe_gather_scores(const float* scores, const int32_t* s_scatter_idx, int64_t rows, float* s, void* stream);

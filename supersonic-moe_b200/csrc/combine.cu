@@ -25,11 +25,14 @@ __device__ __forceinline__ uint32_t cvt_bf16x2(float lo, float hi) {
 }
 
 // One block per token; a thread owns 8 consecutive columns (16-byte accesses).
-// Lanes of the token are added in ascending order.
+// Lanes of the token are added in ascending order.  Being the last kernel of a forward pass, it may also leave the status word
+// where the host looks for it (`host_word`, null: not): a kernel of its own for that one store costs a launch, 3 us and a gap.
 __global__ void __launch_bounds__(512)
 combine_kernel(const uint4* __restrict__ y, const int* __restrict__ s_rev, const int* __restrict__ naept,
-               const float* __restrict__ scores, uint4* __restrict__ out, int H8) {
+               const float* __restrict__ scores, uint4* __restrict__ out, int H8, const int* __restrict__ status,
+               volatile int* host_word) {
   const int64_t t = blockIdx.x;
+  if (host_word != nullptr && t == 0 && threadIdx.x == 0) *host_word = *status;
   const int beg = naept[t], end = naept[t + 1];
   for (int c = threadIdx.x; c < H8; c += blockDim.x) {
     float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -289,17 +292,22 @@ using namespace smoe;
 
 extern "C" {
 
-int smoe_combine(const void* y_bf16, const int32_t* s_rev, const int32_t* naept, const float* scores, void* out_bf16,
-                 int64_t T, int64_t H, void* stream) {
+int smoe_combine_post(const void* y_bf16, const int32_t* s_rev, const int32_t* naept, const float* scores, void* out_bf16,
+                      int64_t T, int64_t H, const int32_t* status, int32_t* pinned_host_word, void* stream) {
   if (T < 0 || H <= 0 || H % 8) return SMOE_ERR_SHAPE;
   if (((uintptr_t)y_bf16 & 15) || ((uintptr_t)out_bf16 & 15)) return SMOE_ERR_ALIGN;
+  if (pinned_host_word && !status) return SMOE_ERR_ARG;
   if (T == 0) return SMOE_OK;
   const int H8 = (int)(H / 8);
-  int threads = H8 >= 512 ? 512 : ((H8 + 31) / 32) * 32;
-  if (H8 > 256 && H8 < 512) threads = ((H8 + 31) / 32) * 32;
+  const int threads = H8 >= 512 ? 512 : ((H8 + 31) / 32) * 32;
   combine_kernel<<<(unsigned)T, threads, 0, (cudaStream_t)stream>>>((const uint4*)y_bf16, s_rev, naept, scores,
-                                                                    (uint4*)out_bf16, H8);
+                                                                    (uint4*)out_bf16, H8, status, pinned_host_word);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+}
+
+int smoe_combine(const void* y_bf16, const int32_t* s_rev, const int32_t* naept, const float* scores, void* out_bf16,
+                 int64_t T, int64_t H, void* stream) {
+  return smoe_combine_post(y_bf16, s_rev, naept, scores, out_bf16, T, H, nullptr, nullptr, stream);
 }
 
 int smoe_gather_scores(const float* scores, const int32_t* s_scatter_idx, int64_t rows, float* s, void* stream) {

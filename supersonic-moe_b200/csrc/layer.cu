@@ -118,11 +118,14 @@ static int check_args(const smoe_layer_args* a) {
   return SMOE_OK;
 }
 
-static int post_status(const smoe_layer_args& a, void* stream) {
+// the host word to post to, or null while a graph is captured
+static int host_word(const smoe_layer_args& a, void* stream, int32_t** word) {
+  *word = nullptr;
   if (!a.host_word) return SMOE_OK;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing((cudaStream_t)stream, &cap) != cudaSuccess) return SMOE_ERR_LAUNCH;
-  return cap == cudaStreamCaptureStatusNone ? smoe_status_post(a.status, a.host_word, stream) : SMOE_OK;
+  if (cap == cudaStreamCaptureStatusNone) *word = a.host_word;
+  return SMOE_OK;
 }
 
 #define SMOE_TRY(call)          \
@@ -181,8 +184,9 @@ int smoe_layer_forward(const smoe_layer_args* args, void* stream) {
                                    H, E, a.status, stream));
   SMOE_TRY(smoe_gemm_varlen_m_live(sc.y1, sc.y1_sf, a.w2, a.w2_sf, sv.efo, sv.s_scatter, real_tk, sc.y2, R, H, I, E, a.status,
                                    stream));
-  SMOE_TRY(smoe_combine(sc.y2, sv.s_rev, sv.naept, sv.scores, a.out, a.T, H, stream));
-  return post_status(a, stream);
+  int32_t* word;
+  SMOE_TRY(host_word(a, stream, &word));
+  return smoe_combine_post(sc.y2, sv.s_rev, sv.naept, sv.scores, a.out, a.T, H, a.status, word, stream);
 }
 
 int smoe_layer_backward(const smoe_layer_args* args, void* stream) {
@@ -242,7 +246,9 @@ int smoe_layer_backward(const smoe_layer_args* args, void* stream) {
       SMOE_TRY(wgrad(b.fused ? b.dz : b.dz_t, b.dz_csf, b.fused, b.xc, b.xc_sf, xc_rows, sv.efo, a.dw1, 2 * I, H, R, E,
                      a.dw1_mode, a.status, stream));
   }
-  return post_status(a, stream);
+  int32_t* word;
+  SMOE_TRY(host_word(a, stream, &word));
+  return word ? smoe_status_post(a.status, word, stream) : SMOE_OK;
 }
 
 }  // extern "C"

@@ -69,6 +69,7 @@ SIGNATURES = {
     "smoe_glu_fwd": (_I, [_P, _L, _L, _I, _P, _P, _P, _P, _P]),
     "smoe_glu_bwd": (_I, [_P, _P, _P, _P, _L, _L, _I, _P, _P, _P, _P]),
     "smoe_combine": (_I, [_P, _P, _P, _P, _P, _L, _L, _P]),
+    "smoe_combine_post": (_I, [_P, _P, _P, _P, _P, _L, _L, _P, _P, _P]),
     "smoe_gather_scores": (_I, [_P, _P, _L, _P, _P]),
     "smoe_ds_finalize": (_I, [_P, _L, _L, _P, _L, _P, _P, _P, _P, _P]),
     "smoe_status_post": (_I, [_P, _P, _P]),
