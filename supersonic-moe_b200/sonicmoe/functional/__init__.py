@@ -930,20 +930,28 @@ class _TopKSoftmax(torch.autograd.Function):
 class _SwitchLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, expert_frequency):
-        logits = logits.contiguous()
-        loss, grad = ops.switch_loss(logits, expert_frequency.contiguous())
-        ctx.save_for_backward(logits, grad)
+        loss, grad = ops.switch_loss(logits.contiguous(), expert_frequency.contiguous())
+        ctx.save_for_backward(logits, grad, expert_frequency)
         return loss
 
     @staticmethod
     def backward(ctx, dloss):
-        logits, grad = ctx.saved_tensors
-        return ops.switch_loss_bwd(logits, grad, dloss.float().contiguous()), None
+        logits, grad, expert_frequency = ctx.saved_tensors
+        if torch.is_grad_enabled():          # create_graph: a gradient that can itself be differentiated
+            return torch.autograd.grad(switch_loss_expression(logits, expert_frequency), logits, dloss, create_graph=True)[0], None
+        return ops.switch_loss_bwd(logits.contiguous(), grad, dloss.float().contiguous()), None
+
+
+def switch_loss_expression(logits, expert_frequency, probs=None):
+    """E * sum_e normalize1(sum_t softmax(logits))_e * normalize1(expert_frequency)_e as tensor operations."""
+    E = logits.size(-1)
+    probs = F.softmax(logits, dim=-1, dtype=torch.float32) if probs is None else probs
+    return E * (F.normalize(probs.view(-1, E).sum(0), p=1, dim=0)
+                * F.normalize(expert_frequency.float(), p=1, dim=0)).sum()
 
 
 def switch_loss(logits: torch.Tensor, expert_frequency: torch.Tensor) -> torch.Tensor:
-    """Switch auxiliary loss of router logits [T,E] and tokens per expert [E]: the expression of
-    `MoE._compute_switch_loss` in three kernels."""
+    """Switch auxiliary loss of router logits [T,E] and tokens per expert [E]: `switch_loss_expression` in three kernels."""
     return _SwitchLoss.apply(logits, expert_frequency)
 
 

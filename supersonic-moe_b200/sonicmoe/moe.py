@@ -12,7 +12,7 @@ import torch.nn.functional as F
 
 from .config import SonicMoEConfig
 from .enums import ActivationType, KernelBackendMoE, is_glu
-from .functional import enable_fp8, moe_TC_softmax_topk_layer, switch_loss
+from .functional import enable_fp8, moe_TC_softmax_topk_layer, switch_loss, switch_loss_expression
 
 
 class Experts(nn.Module):
@@ -75,7 +75,7 @@ class MoE(nn.Module):
         hidden_states = hidden_states.view(original_shape)
         if is_inference_mode:
             aux_loss = None
-        elif (type(self)._compute_switch_loss is MoE._compute_switch_loss and self.num_experts <= 1024
+        elif (getattr(self._compute_switch_loss, "__func__", None) is MoE._compute_switch_loss and self.num_experts <= 1024
               and router_logits.dtype in (torch.float32, torch.bfloat16)):
             aux_loss = switch_loss(router_logits, expert_frequency)
         else:
@@ -85,9 +85,4 @@ class MoE(nn.Module):
         return hidden_states, aux_loss
 
     def _compute_switch_loss(self, logits, probs, expert_frequency):
-        logits = logits.view(-1, logits.size(-1))
-        probs = probs.view(-1, probs.size(-1))
-        num_experts = logits.size(1)
-        acc_probs = probs.sum(0)
-        expert_frequency = expert_frequency.float()
-        return num_experts * (F.normalize(acc_probs, p=1, dim=0) * F.normalize(expert_frequency, p=1, dim=0)).sum()
+        return switch_loss_expression(logits.view(-1, logits.size(-1)), expert_frequency, probs)

@@ -278,6 +278,19 @@ def test_router_kernels_on_bf16_logits(ops, T, E):
         assert (x.grad.double() - x64.grad).norm() <= tol * x64.grad.norm() + 1e-7, (dt, E)
 
 
+def test_switch_loss_differentiates_twice(ops):
+    from sonicmoe.functional import switch_loss, switch_loss_expression
+    g = torch.Generator().manual_seed(3)
+    freq = torch.randint(0, 50, (40,), generator=g, dtype=torch.int32).to(DEV)
+    x0 = torch.randn(70, 40, generator=g).to(DEV)
+    second = []
+    for f in (switch_loss, switch_loss_expression):
+        x = x0.clone().requires_grad_(True)
+        d, = torch.autograd.grad(f(x, freq), x, create_graph=True)
+        second.append(torch.autograd.grad((d * d).sum(), x)[0])
+    assert torch.allclose(*second, rtol=1e-4, atol=1e-9) and second[0].abs().max() > 0
+
+
 def test_topk_softmax_rows_with_fewer_than_k_finite_logits(ops):
     """-inf-masked and NaN logits: the K indices stay distinct and in range (the finite ones first, then the lowest
     unused index with a score of exactly zero), the scores of the finite picks are their softmax, and the backward
