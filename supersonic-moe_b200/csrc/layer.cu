@@ -198,7 +198,9 @@ int smoe_layer_backward(const smoe_layer_args* args, void* stream) {
   const int64_t R = a.TKp_alloc, H = a.H, I = a.I, E = a.E;
   const int32_t *rows = sv.efo + E, *real_tk = sv.naept + a.T;
   const bool dw1 = a.dw1_mode != SMOE_DW_NONE, dw2 = a.dw2_mode != SMOE_DW_NONE;
-  const bool dc_rows = b.fused && !wide_ok(E, I, H);
+  // dout's column-quantised copy: transposed where dw2 joins the 256 x 384 kernel, else left as rows (13 us cheaper to make
+  // at T=8192, H=3072, K=8; the 256 x 256 kernel reads either in the same time)
+  const bool dc_rows = b.fused && (!wide_ok(E, I, H) || a.dw2_mode == SMOE_DW_BF16);
   SMOE_TRY(smoe_gather_scores(sv.scores, sv.s_scatter, R, b.s, stream));
   SMOE_TRY(smoe_quant_rows_scatter(a.dout, a.T, H, sv.naept, sv.s_rev, sv.s_scatter, rows, R, b.dg, b.dg_sf, stream));
   if (b.fused && dw2) SMOE_TRY(column_operand(a.dout, sv, rows, R, H, dc_rows, b.dc, b.dc_sf, stream));

@@ -113,10 +113,12 @@ def _wide_wgrad_ok(E: int, M: int, N: int) -> bool:
     return E <= 256 and M % 256 == 0 and N % 384 == 0
 
 
-def _col_operand(src, idx, TKp, valid_rows, E, M, N):
+def _col_operand(src, idx, TKp, valid_rows, E, M, N, narrow=False):
     """Column-quantised (1x32 along the routed rows) B operand of a weight-gradient GEMM from bf16 `src` rows
-    gathered by `idx`: (payload, ISA scales for (N, TKp), payload_is_rows_major)."""
-    if _mn_wgrad_ok(E, M, N) and not _wide_wgrad_ok(E, M, N):
+    gathered by `idx`: (payload, ISA scales for (N, TKp), payload_is_rows_major).  `narrow`: the 256 x 256 kernel will
+    read it, which takes either layout in the same time; left as rows it is cheaper to make (72 against 85 us at T=8192,
+    H=3072, K=8)."""
+    if _mn_wgrad_ok(E, M, N) and (narrow or not _wide_wgrad_ok(E, M, N)):
         _, _, q, sf = ops.quant_dual_gather(src, idx, TKp, valid_rows, with_rows=False)
         return q, sf, True
     q_t, sf = ops.quant_cols_t(src, idx, TKp, valid_rows=valid_rows)
@@ -679,6 +681,9 @@ class _DownProjection(torch.autograd.Function):
         # memory-lean order: the column-quantised copy of dout is made after GemmDGated has run and z and the
         # gathered dout rows are freed, and dw2 runs (and frees its operands) before dx_expanded is allocated
         early_cols = not stagewise
+        # no main_grad, bf16 parameter: dw2 leaves the 256 x 256 kernel in the parameter's layout, with exchanged operands
+        dw2_bf16 = (getattr(_base_of(w2), "main_grad", None) is None and w2.dtype == torch.bfloat16
+                    and _mn_wgrad_ok(E, H, I))
         w2t_q, w2t_sf, kn = _weight_operand(w2, True, link.get("iso32", False))
         if kn:
             # GemmDGated reads B K-major only (its 192-column slices are no MN-major swizzle atoms): a transient
@@ -687,7 +692,7 @@ class _DownProjection(torch.autograd.Function):
         if USE_TMA_GATHER and act == 0:
             a_sf = ops.gather_scales_isa(dout_raw, x_gather_idx, TKp, H)
             if early_cols and dout is not None and ctx.needs_input_grad[2] and _mn_wgrad_ok(E, I, H):
-                dout_c, dout_sf, dout_c_rows = _col_operand(dout, x_gather_idx, TKp, efo[-1:], E, I, H)
+                dout_c, dout_sf, dout_c_rows = _col_operand(dout, x_gather_idx, TKp, efo[-1:], E, I, H, dw2_bf16)
             if FUSE_DGATED_QUANT and _mn_wgrad_ok(E, I, H):
                 dz_q, dz_rsf, dz_csf, y1s_q, y1s_sf, dsp = ops.gemm_dgated_fused(
                     dout_q, a_sf, w2t_q, w2t_sf, efo, z_q, z_sc, s, TKp, a_idx=x_gather_idx)
@@ -703,7 +708,7 @@ class _DownProjection(torch.autograd.Function):
                 # in a second, gathered pass (93 us); the one-pass dual kernel measured 209 us there
                 dg_q, a_sf = ops.quant_rows_scatter(dout, naept, s_rev, s_scatter_idx, TKp, efo[-1:])
                 if early_cols and ctx.needs_input_grad[2] and _mn_wgrad_ok(E, I, H):
-                    dout_c, dout_sf, dout_c_rows = _col_operand(dout, x_gather_idx, TKp, efo[-1:], E, I, H)
+                    dout_c, dout_sf, dout_c_rows = _col_operand(dout, x_gather_idx, TKp, efo[-1:], E, I, H, dw2_bf16)
             if act != 0:
                 # ReGLU / GEGLU: D from a plain GEMM, then the stand-alone activation-gradient kernel; dz / y1s in bf16
                 # take the separate quantizers below
@@ -731,7 +736,7 @@ class _DownProjection(torch.autograd.Function):
                 if dout is None:
                     dout_t, dout_sf = ops.requant_cols_t(dout_q, dout_raw, x_gather_idx, TKp, efo[-1:])
                 elif _mn_wgrad_ok(E, I, H):
-                    dout_c, dout_sf, dout_c_rows = _col_operand(dout, x_gather_idx, TKp, efo[-1:], E, I, H)
+                    dout_c, dout_sf, dout_c_rows = _col_operand(dout, x_gather_idx, TKp, efo[-1:], E, I, H, dw2_bf16)
                 else:
                     dout_t, dout_sf = ops.quant_cols_t(dout, x_gather_idx, TKp, valid_rows=efo[-1:])
             mg, base = _grad_target(w2, (E, I, H))
