@@ -955,7 +955,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           const int row_grp = (t.m0 + q * 32) >> 5;      // 32-row group index along TKp
           const int kt_rows = p.rows >> 7;               // K tiles of the weight-gradient operands
           constexpr int NCH = COLS_PER_WARP / 32;
-          F2 ds2 = f2(0.f, 0.f);                         // even and odd columns
+          float ds_acc = 0.f;                            // one chain in column order, as GemmDGated without quantizers adds
 #pragma unroll 1
           for (int c = 0; c < NCH; ++c) {
             const int dcol = c_base + c * 32;            // first D / y1s column of the chunk
@@ -1000,7 +1000,8 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 const F2 silu = g * sig;
                 const F2 sd = silu * dout;
                 const F2 yv = silu * u;
-                ds2 = f2_fma(yv, D, ds2);
+                const float2 yvp = f2_get(yv), Dp = f2_get(D);
+                ds_acc = fmaf(yvp.y, Dp.y, fmaf(yvp.x, Dp.x, ds_acc));
                 const F2 dsig = f2_fma(silu, sig * f2(-1.0f, -1.0f), sig);                       // sig - silu * sig
                 const float2 dg = f2_get(f2_fma(dsig, dout, sd) * u), sdp = f2_get(sd), y = f2_get(f2(s, s) * yv);
                 P[2 * i2] = pack_bf16x2(dg.x, sdp.x);                                            // rounds to bf16
@@ -1085,8 +1086,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             for (int i = 0; i < 4; ++i) zb[i] = zn[i];
             sc = scn;
           }
-          const float2 ds_eo = f2_get(ds2);
-          p.ds_partial[(size_t)((t.n0 / BN) * S::COL_GROUPS + half) * p.rows + grow] = ds_eo.x + ds_eo.y;
+          p.ds_partial[(size_t)((t.n0 / BN) * S::COL_GROUPS + half) * p.rows + grow] = ds_acc;
         } else if (t.valid && c_base >= p.N) {
           // a column group wholly beyond a ragged N: its partial sum is one of those added up
           p.ds_partial[(size_t)((t.n0 / BN) * S::COL_GROUPS + half) * p.rows + grow] = 0.f;

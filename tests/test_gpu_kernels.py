@@ -748,6 +748,31 @@ def test_gemm_dgated_fused_quantizers_match_separate_kernels(ops, T, H, I, tiles
     assert torch.equal(g_out[5].sum(0)[:n], f_dsp.sum(0)[:n])
 
 
+@pytest.mark.parametrize("T,H,I,tiles,bn", [(300, 256, 128, [1, 2, 0, 1], 128), (1000, 512, 768, [3, 1, 2], 0),
+                                            (600, 256, 2048, [2, 1, 3], 128)])
+def test_gemm_dgated_ds_partials_keep_one_order_of_addition(ops, T, H, I, tiles, bn):
+    """Where both kernels run column tiles of one width, the fused one adds a row's ds partials in the order of the other:
+    the same bits.  (A router rounds what follows from ds to bf16, where another order shows.)"""
+    from sonicmoe._lib import lib
+    g, E, efo, rows, dout, _, a_idx = gated_inputs(T, H, I, tiles, 23)
+    wq, ws = Q.row_quant((torch.randn(E, I, H, generator=g) * 0.05).to(torch.bfloat16).reshape(E * I, H))
+    zq, zs = Q.row_quant(torch.randn(rows, 2 * I, generator=g), amax_floor=1e-4)
+    dq, dsc = Q.row_quant(dout)
+    args = (Q.gather_scales_to_isa(dsc, a_idx, H).to(DEV), wq.reshape(E, I, H).to(DEV), Q.pack_isa(ws, E * I, H).to(DEV),
+            efo.to(DEV), zq.to(DEV), zs.to(DEV), torch.rand(rows, generator=g).to(DEV), rows)
+    a_in = dq[a_idx.long()].contiguous().to(DEV)
+    lib.smoe_internal_gemm_knobs(bn)
+    try:
+        want = ops.gemm_dgated(a_in, None, *args)[2]
+        got = ops.gemm_dgated_fused(a_in, *args)[5]
+        torch.cuda.synchronize()
+        ops.check_status(DEV)
+    finally:
+        lib.smoe_internal_gemm_knobs(0)
+    n = int(efo[-1])
+    assert got.shape == want.shape and torch.equal(got[:, :n], want[:, :n])
+
+
 @pytest.mark.parametrize("T,K,E,world", [(333, 4, 16, 4), (1000, 8, 8, 8), (64, 2, 6, 2)])
 def test_ep_dispatch_plan_from_metadata_kernels_matches_torch_construction(ops, T, K, E, world):
     """The plan built with the routing-metadata kernels (destination ranks as experts) equals the device-agnostic
