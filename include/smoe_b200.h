@@ -54,8 +54,10 @@ int64_t smoe_topk_metadata_workspace(int64_t N, int64_t E);
  *               1 = by top-k slot (dense path, functional/triton_kernels/__init__.py:66-155)
  *   pad_mode:   0 = pad rows scatter to real_TK (kernel.cu:611-650),
  *               1 = i-th pad row scatters to real_TK + i (functional/__init__.py:226-234)
- *   TK_alloc / TKp_alloc smaller than what idx really holds (buffers sized from stale per-expert counts): the rows
- *   that do not fit are dropped and efo is clamped to TKp_alloc - nothing is written outside the buffers. */
+ *   TK_alloc / TKp_alloc smaller than what idx really holds (buffers sized from stale per-expert counts): nothing is
+ *   written outside the buffers, and the metadata describes a smaller problem that fits them.  Entries whose expert-sorted
+ *   position does not fit count as masked; of the rest the first TK_alloc, token-major, stay; naept ends at their number, efo is
+ *   clamped to TKp_alloc, and every row without an entry is a pad row scattering to naept[N].  counts stay those of idx. */
 int smoe_topk_metadata(const int32_t* idx, const float* probs, int64_t N, int64_t K, int64_t E, int64_t alignment,
                        int64_t TK_alloc, int64_t TKp_alloc, int lane_order, int pad_mode, int32_t* efo,
                        int32_t* x_gather_idx, int32_t* s_scatter_idx, int32_t* s_reverse_scatter_idx, int32_t* naept,

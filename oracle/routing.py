@@ -55,6 +55,10 @@ def topk_metadata(idx: torch.Tensor, probs: torch.Tensor, E: int, alignment: int
     position of (t,k) is naept[t] + (#valid slots before k) - equal to the flat
     index t*K+k when every slot is valid (the dense Triton path).
 
+    TK_alloc / TKp_alloc too small for what idx holds: entries whose expert-sorted position does not fit count as
+    masked, of the rest the first TK_alloc (token-major) stay, and every row without a published entry is a pad row
+    that scatters to the number of published entries (whatever pad_mode says).
+
     pad_mode "sentinel": pad rows' s_scatter_idx = real_TK (kernel.cu:611-650);
     "virtual": the i-th pad row (ascending position) gets real_TK + i
     (functional/__init__.py:226-234).
@@ -73,8 +77,14 @@ def topk_metadata(idx: torch.Tensor, probs: torch.Tensor, E: int, alignment: int
     real_TKp = int(efo[-1])
     TK = real_TK if TK_alloc is None else TK_alloc
     TKp = real_TKp if TKp_alloc is None else TKp_alloc
-    assert TK >= real_TK and TKp >= real_TKp
-
+    limit = TKp // alignment * alignment
+    cut = TK < real_TK or limit < real_TKp
+    if cut:
+        # (row, slot) -> rank among the rows of its expert; what lies at or beyond the limit is masked
+        for e in range(E):
+            t_e, k_e = np.nonzero(valid & (idx_np == e))
+            drop = efo[e] + np.arange(len(t_e)) >= limit
+            valid[t_e[drop], k_e[drop]] = False
     naept = np.zeros(N + 1, dtype=np.int64)
     naept[1:] = np.cumsum(valid.sum(axis=1))
 
@@ -93,9 +103,17 @@ def topk_metadata(idx: torch.Tensor, probs: torch.Tensor, E: int, alignment: int
     t_s, k_s, e_s = t_ids[order], k_ids[order], e_ids[order]
     base = np.zeros(E, dtype=np.int64)
     base[1:] = np.cumsum(counts)[:-1]
-    local = np.arange(real_TK) - base[e_s]
+    if cut:
+        base[1:] = np.cumsum(np.bincount(e_s, minlength=E))[:-1]
+    local = np.arange(len(e_s)) - base[e_s]
     pos = efo[e_s] + local                        # padded expert-sorted position
     tm = naept[t_s] + rank[t_s, k_s]              # token-major position
+    if cut:
+        real_TK = min(int(naept[-1]), max(TK, 0))
+        naept = np.minimum(naept, real_TK)
+        keep = tm < real_TK
+        t_s, k_s, pos, tm = t_s[keep], k_s[keep], pos[keep], tm[keep]
+        efo = np.minimum(efo, limit)
 
     x_gather = np.zeros(TKp, dtype=np.int32)
     s_scatter = np.full(TKp, real_TK, dtype=np.int32)
@@ -107,7 +125,7 @@ def topk_metadata(idx: torch.Tensor, probs: torch.Tensor, E: int, alignment: int
     s_rev[tm] = pos
     scores[tm] = pr_np[t_s, k_s]
     src[tm] = t_s * K + k_s
-    if pad_mode == "virtual":
+    if pad_mode == "virtual" and not cut:
         is_real = np.zeros(TKp, dtype=bool)
         is_real[pos] = True
         pads = np.nonzero(~is_real)[0]

@@ -93,7 +93,7 @@ unit_masks_kernel(const int* __restrict__ idx, int N, int K, int E, uint32_t* __
 // block  E     : unit_base[u] = exclusive scan of unit_valid; naept[N] = total
 __global__ void __launch_bounds__(kRtThreads)
 scan_kernel(const uint32_t* __restrict__ mask, const int* __restrict__ unit_valid, int units, int E, int N,
-            int* __restrict__ unit_off, int* __restrict__ counts, int* __restrict__ unit_base,
+            int TK_alloc, int* __restrict__ unit_off, int* __restrict__ counts, int* __restrict__ unit_base,
             int* __restrict__ naept) {
   __shared__ int s_warp[33];
   const int e = blockIdx.x;
@@ -105,7 +105,7 @@ scan_kernel(const uint32_t* __restrict__ mask, const int* __restrict__ unit_vali
   } else {
     const int total = block_excl_scan(
         units, [&](int u) { return unit_valid[u]; }, [&](int u, int ex) { unit_base[u] = ex; }, s_warp);
-    if (threadIdx.x == 0) naept[N] = total;
+    if (threadIdx.x == 0) naept[N] = min(total, TK_alloc);
   }
 }
 
@@ -137,12 +137,24 @@ scatter_fill_kernel(const int* __restrict__ idx, const float* __restrict__ probs
     s_base[E] = tot_u;
   }
   __syncthreads();
-  // published offsets never point past the allocation (they can only exceed it when the caller sized the buffers
-  // from counts that do not match idx): the GEMMs that walk efo then stay inside the buffers too
+  // Published offsets never point past the allocation (they can only exceed it when the caller sized the buffers from counts
+  // that do not match idx), and neither does anything that a reader of this metadata follows.  Such a pass is `cut`: an entry
+  // whose expert-sorted position lies at or beyond `limit` counts as if its slot were masked - expert e keeps its first
+  // clamp(limit - s_efo[e]) rows, so the token-major base of a unit is the sum of what its experts keep of the units before -
+  // and of what is left the first TK_alloc entries stay; the row of a later one becomes a pad row (it lies among the last rows
+  // of its expert: token-major order is ascending there).  naept, s_rev, s_scatter and the scores then agree with each other.
+  const int limit = TKp_alloc / alignment * alignment;
   if (blockIdx.x == 0)
-    for (int e = threadIdx.x; e <= E; e += blockDim.x) efo_out[e] = min(s_efo[e], TKp_alloc / alignment * alignment);
-  const int real_TK = tot_u;        // == naept[N]
+    for (int e = threadIdx.x; e <= E; e += blockDim.x) efo_out[e] = min(s_efo[e], limit);
   const int real_TKp = tot_p;
+  const bool cut = tot_p > limit || tot_u > TK_alloc;
+  int real_TK = tot_u;              // entries that are published, naept[N]
+  if (cut) {
+    const int fit = block_excl_scan(
+        E, [&](int e) { return max(min(counts[e], limit - s_efo[e]), 0); }, [](int, int) {}, s_warp);
+    real_TK = min(fit, TK_alloc);
+    if (blockIdx.x == 0 && threadIdx.x == 0) naept[N] = real_TK;
+  }
 
   // ---- scatter: one thread per (row, slot) ----
   // A unit of 32 rows is KP warps (KP: slots a row, rounded up to a power of two), slots fastest: the loads of indices and
@@ -158,13 +170,25 @@ scatter_fill_kernel(const int* __restrict__ idx, const float* __restrict__ probs
     const bool in = row < N && k < K;
     int e = in ? idx[(size_t)row * K + k] : -1;
     if (e < 0 || e >= E) e = -1;
+    int pos = 0;
+    if (e >= 0) {
+      const uint32_t m = mask[(size_t)unit * E + e];
+      pos = s_efo[e] + unit_off[(size_t)unit * E + e] + __popc(m & ((1u << r) - 1u));
+      if (pos >= limit) e = -1;
+    }
     const uint32_t ball = __ballot_sync(0xffffffffu, e >= 0);
     if (lane == 0) s_warp[warp] = __popc(ball);
     __syncthreads();
-    int tm_base = unit * 32 < N ? unit_base[unit] : 0;
+    int tm_base = 0;
+    if (unit * 32 < N) {
+      if (!cut) tm_base = unit_base[unit];
+      else
+        for (int j = 0; j < E; ++j) tm_base += max(min(unit_off[(size_t)unit * E + j], limit - s_efo[j]), 0);
+    }
     for (int w = warp - warp % KP; w < warp; ++w) tm_base += s_warp[w];
     const int row_base = tm_base + __popc(ball & ((1u << (rw * KP)) - 1u));        // rw * KP <= 31
-    if (row < N && k == 0) naept[row] = row_base;
+    const int cap = cut ? real_TK : TK_alloc;
+    if (row < N && k == 0) naept[row] = min(row_base, cap);
     int rank = 0;
     if (lane_order == 0) {
 #pragma unroll
@@ -176,20 +200,15 @@ scatter_fill_kernel(const int* __restrict__ idx, const float* __restrict__ probs
       rank = __popc(ball & ((1u << lane) - 1u)) - __popc(ball & ((1u << (rw * KP)) - 1u));
     }
     if (e >= 0) {
-      const uint32_t m = mask[(size_t)unit * E + e];
-      const int pos = s_efo[e] + unit_off[(size_t)unit * E + e] + __popc(m & ((1u << r) - 1u));
       const int tm = row_base + rank;
-      // buffers sized from a caller's (possibly stale) per-expert counts may be too small for what the indices really
-      // hold: the excess is dropped, never written past the allocation
-      if (pos < TKp_alloc) {
-        x_gather[pos] = row;
-        s_scatter[pos] = tm;
-      }
-      if (tm < TK_alloc) {
-        s_rev[tm] = pos < TKp_alloc ? pos : 0;
+      const bool kept = tm < cap;
+      x_gather[pos] = kept ? row : 0;
+      s_scatter[pos] = kept ? tm : real_TK;
+      if (kept) {
+        s_rev[tm] = pos;
         src_idx[tm] = row * K + k;
+        if (tm < TKp_alloc) scores[tm] = probs[(size_t)row * K + k];
       }
-      if (tm < TKp_alloc) scores[tm] = probs[(size_t)row * K + k];
     }
   }
 
@@ -199,7 +218,12 @@ scatter_fill_kernel(const int* __restrict__ idx, const float* __restrict__ probs
   for (int pos = gtid; pos < TKp_alloc; pos += nthreads) {
     if (pos >= real_TKp) {
       x_gather[pos] = 0;
-      s_scatter[pos] = pad_mode == 0 ? real_TK : pos;   // virtual numbering continues through the tail
+      s_scatter[pos] = pad_mode == 0 || cut ? real_TK : pos;   // virtual numbering continues through the tail
+      continue;
+    }
+    if (pos >= limit) {                                 // cut off inside an alignment step
+      x_gather[pos] = 0;
+      s_scatter[pos] = real_TK;
       continue;
     }
     int lo = 0, hi = E;
@@ -211,7 +235,7 @@ scatter_fill_kernel(const int* __restrict__ idx, const float* __restrict__ probs
     const int local = pos - s_efo[lo];
     if (local >= cnt) {
       x_gather[pos] = 0;
-      s_scatter[pos] = pad_mode == 0 ? real_TK : real_TK + (s_efo[lo] - s_base[lo]) + (local - cnt);
+      s_scatter[pos] = pad_mode == 0 || cut ? real_TK : real_TK + (s_efo[lo] - s_base[lo]) + (local - cnt);
     }
   }
   for (int i = real_TK + gtid; i < TKp_alloc; i += nthreads) scores[i] = 0.f;
@@ -285,6 +309,7 @@ int smoe_topk_metadata(const int32_t* idx, const float* probs, int64_t N, int64_
   if (K <= 0 || K > kMaxTopk || E <= 0 || E > 4096 || N < 0 || alignment <= 0) return SMOE_ERR_SHAPE;
   if (N * K >= (int64_t)1 << 31 || TKp_alloc >= (int64_t)1 << 31) return SMOE_ERR_SHAPE;
   if (!workspace || !efo || !counts) return SMOE_ERR_ARG;
+  TK_alloc = TK_alloc < 0 ? 0 : TK_alloc >= (int64_t)1 << 31 ? ((int64_t)1 << 31) - 1 : TK_alloc;
   const int units = (int)((N + 31) / 32);
   uint32_t* mask = (uint32_t*)workspace;
   int* unit_off = (int*)(mask + (size_t)(units + 1) * E);
@@ -293,8 +318,8 @@ int smoe_topk_metadata(const int32_t* idx, const float* probs, int64_t N, int64_
   const int ublocks = (units + kUnitsPerBlock - 1) / kUnitsPerBlock;
   if (ublocks > 0)
     unit_masks_kernel<<<ublocks, kRtThreads, 0, stream>>>(idx, (int)N, (int)K, (int)E, mask, unit_valid);
-  scan_kernel<<<(int)E + 1, kRtThreads, 0, stream>>>(mask, unit_valid, units, (int)E, (int)N, unit_off, counts,
-                                                     unit_base, naept);
+  scan_kernel<<<(int)E + 1, kRtThreads, 0, stream>>>(mask, unit_valid, units, (int)E, (int)N, (int)TK_alloc, unit_off,
+                                                     counts, unit_base, naept);
   // slots a row, rounded up: a unit of 32 rows is that many warps of the scatter
   const int kp = K <= 1 ? 1 : K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : 16;
   const int threads = kp > 8 ? 32 * kp : kRtThreads, units_per_block = threads / (32 * kp);

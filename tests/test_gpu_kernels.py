@@ -359,6 +359,23 @@ def test_topk_metadata_with_undersized_buffers_stays_in_bounds(ops):
     assert ((xg[:TKp] >= 0) & (xg[:TKp] < N)).all() and ((sr[:TK] >= 0) & (sr[:TK] < TKp)).all()
 
 
+
+@pytest.mark.parametrize("N,K,E,TK,TKp", [(512, 4, 8, 1024, 1024), (300, 4, 6, 1200, 1152), (300, 4, 6, 700, 2048), (40, 2, 4, 80, 200),
+                                          (64, 2, 4, 0, 0), (64, 2, 4, 10, 0), (64, 2, 4, 0, 512), (1000, 16, 40, 9000, 9984)])
+@pytest.mark.parametrize("lane_order,pad_mode", [(0, 0), (1, 1)])
+def test_topk_metadata_with_undersized_buffers_describes_what_fits(ops, N, K, E, TK, TKp, lane_order, pad_mode):
+    """naept, s_rev, s_scatter and the scores agree on the entries that are left, so no reader leaves its buffers."""
+    g = torch.Generator().manual_seed(N + TK)
+    idx = torch.stack([torch.randperm(E, generator=g)[:K] for _ in range(N)]).to(torch.int32)
+    idx[::5, 0] = -1
+    probs = torch.rand(N, K, generator=g)
+    ref = R.topk_metadata(idx, probs, E, 128, TK, TKp, lane_order=["expert", "slot"][lane_order],
+                          pad_mode=["sentinel", "virtual"][pad_mode])
+    got = ops.topk_metadata(idx.to(DEV), probs.to(DEV), E, 128, TK, TKp, lane_order=lane_order, pad_mode=pad_mode)
+    for k in MD_KEYS:
+        assert torch.equal(got[k].cpu(), ref[k]), k
+
+
 # ------------------------------------------------------------------ GEMMs
 def rand_fp8(shape, g, lo_exp=118, hi_exp=126):
     """Random e4m3 bytes (no NaN) and random ue8m0 scale bytes per 1x32 group."""

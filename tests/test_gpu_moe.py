@@ -237,6 +237,40 @@ def test_run_sonic_moe_masked_skewed_vs_oracles(sm, sizing):
     assert (sd.grad.cpu()[idx < 0] == 0).all()
 
 
+@pytest.mark.parametrize("one_call", [True, False])
+@pytest.mark.parametrize("short", [(0, 300), (5, 40), (7, 700), (range(8), 700)])
+def test_understated_token_counts_drop_entries_and_nothing_else(sm, monkeypatch, one_call, short):
+    """`tokens_per_expert` smaller than what the indices hold: the entries without room are left out of the pass, as if their
+    slots were masked, in the one-call path and step by step."""
+    import sonicmoe.functional as fn
+    T, H, I, E, K = 700, 256, 256, 8, 4
+    x, dy, w1, w2, _, _ = make_layer(T, H, I, E, K, 5)
+    idx, scores = masked_routing(T, E, K, E, 6)
+    counts = torch.bincount(idx[idx >= 0].long(), minlength=E)
+    at = torch.tensor(short[0] if isinstance(short[0], range) else [short[0]])
+    counts[at] = (counts[at] - short[1]).clamp(min=0)
+    TK, TKp = int(counts.sum()), sum(-(-c // 128) * 128 for c in counts.tolist())
+    md = R.topk_metadata(idx, scores, E, 128, TK, TKp)
+    kept = torch.zeros(T * K, dtype=torch.bool)
+    kept[md["score_src_idx"][:md["real_TK"]].long()] = True
+    assert int(kept.sum()) < int((idx >= 0).sum())
+    if not one_call:
+        monkeypatch.setattr(fn, "_ONE_CALL_BYTES", 0)
+
+    def run(idx, **kw):
+        leaves = [t.to(DEV).requires_grad_(True) for t in (x, scores, w1, w2)]
+        out = sm.run_sonic_moe(leaves[0], idx.to(DEV), leaves[1], K, E, leaves[2], leaves[3], fp8=True, **kw)
+        out.backward(dy.to(DEV))
+        torch.cuda.synchronize()
+        sm.ops.check_status(DEV)
+        return [out] + [t.grad for t in leaves]
+
+    got = run(idx, tokens_per_expert=counts.tolist())
+    want = run(torch.where(kept.view(T, K), idx, torch.full_like(idx, -1)))
+    for name, a, b in zip(("out", "dx", "ds", "dw1", "dw2"), got, want):
+        assert torch.equal(a, b), name
+
+
 def test_main_grad_accumulation_and_bit_exact_repeat(sm):
     T, H, I, E, K = 1024, 512, 256, 8, 4
     x, dy, w1, w2, _, _ = make_layer(T, H, I, E, K, 9)

@@ -1,6 +1,7 @@
 """The oracle's MoE restatements against each other and against autograd (CPU only).
 
 Config C1 of the benchmark set: T=256, H=256, I=128, E=8, K=2, seed 0."""
+import pytest
 import torch
 
 from oracle import moe as OM
@@ -85,3 +86,34 @@ def test_torch_baseline_module_matches_gold_on_its_own_routing():
     md = R.topk_metadata(idx, scores, 8, 1)
     gold = OM.moe_fp32(x, b.w1.detach(), b.w2.detach(), md)
     torch.testing.assert_close(out.detach(), gold["o"], rtol=1e-4, atol=1e-5)
+
+
+@pytest.mark.parametrize("lane_order", ["expert", "slot"])
+@pytest.mark.parametrize("N,K,E,TK,TKp", [(512, 4, 8, 1024, 1024), (300, 4, 6, 1200, 1152), (300, 4, 6, 700, 2048), (40, 2, 4, 80, 200),
+                                          (64, 2, 4, 0, 0), (64, 2, 4, 10, 0), (64, 2, 4, 0, 512)])
+def test_metadata_of_undersized_buffers_keeps_every_reader_in_bounds(lane_order, N, K, E, TK, TKp):
+    """What the readers of the metadata follow: quantizers and combine s_rev[naept[t] : naept[t+1]] and the scores there, score
+    gather scores[s_scatter[row]] of every row, column quantizers x_gather[row]."""
+    g = torch.Generator().manual_seed(N + TK)
+    idx = torch.stack([torch.randperm(E, generator=g)[:K] for _ in range(N)]).to(torch.int32)
+    idx[::5, 0] = -1
+    probs = torch.rand(N, K, generator=g)
+    full = R.topk_metadata(idx, probs, E, 128, lane_order=lane_order)
+    md = R.topk_metadata(idx, probs, E, 128, TK, TKp, lane_order=lane_order, pad_mode="virtual")
+    na, sr, ss, sc, src = (md[k].long() for k in ("naept", "s_reverse_scatter_idx", "s_scatter_idx", "topk_scores",
+                                                  "score_src_idx"))
+    n = int(na[-1])
+    assert n < full["real_TK"] and n <= min(TK, TKp) and (na[1:] >= na[:-1]).all() and na[0] == 0
+    assert int(md["efo"].max()) <= TKp // 128 * 128
+    assert len(sr) == TK and ((sr >= 0) & (sr < max(TKp, 1))).all() and len(set(sr[:n].tolist())) == n
+    assert len(md["topk_scores"]) == TKp and ((ss >= 0) & (ss < max(TKp, 1))).all()
+    assert (ss[sr[:n]] == torch.arange(n)).all() and int((ss < n).sum()) == n          # each other's inverse
+    assert (md["topk_scores"][n:] == 0).all() and (md["topk_scores"][:n] == probs.flatten()[src[:n]]).all()
+    tok = torch.repeat_interleave(torch.arange(N), na[1:] - na[:-1])
+    assert (src[:n] // K == tok).all() and (md["x_gather_idx"][sr[:n]] == tok).all()
+    # every kept entry lies where it lies with room for all, and the real rows of a segment come first
+    where = {int(s): int(p) for s, p in zip(full["score_src_idx"], full["s_reverse_scatter_idx"])}
+    assert all(where[int(s)] == int(p) for s, p in zip(src[:n], sr[:n]))
+    for a, b in zip(md["efo"][:-1].tolist(), md["efo"][1:].tolist()):
+        real = (ss[a:b] < n).int()
+        assert (real[1:] <= real[:-1]).all()
