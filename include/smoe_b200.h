@@ -426,6 +426,7 @@ typedef struct {
   void *saved, *scratch;       /* smoe_layer_bytes(args, 0); (args, 1) in the forward, (args, 2) in the backward */
   int32_t* status;
   int32_t* host_word;          /* pinned mirror of *status, posted at the end (not while capturing); may be null */
+  void* dx_ready;              /* backward: cudaEvent_t recorded when dx is complete, before the weight gradients; may be null */
 } smoe_layer_args;
 /* Bytes of an arena: which = 0 saved, 1 forward scratch, 2 backward scratch; -1 for sizes that are not taken. */
 int64_t smoe_layer_bytes(const smoe_layer_args* args, int which);

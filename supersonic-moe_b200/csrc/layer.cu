@@ -226,6 +226,7 @@ int smoe_layer_backward(const smoe_layer_args* args, void* stream) {
     SMOE_TRY(smoe_gemm_varlen_m_live(b.dz, b.dz_rsf, a.w1, a.w1_sf, sv.efo, sv.s_scatter, real_tk, b.dx_exp, R, H, 2 * I, E,
                                      a.status, stream));
     SMOE_TRY(smoe_combine(b.dx_exp, sv.s_rev, sv.naept, nullptr, a.out, a.T, H, stream));
+    if (a.dx_ready && cudaEventRecord((cudaEvent_t)a.dx_ready, (cudaStream_t)stream) != cudaSuccess) return SMOE_ERR_LAUNCH;
   }
   bool xc_rows = false;
   if (dw1) {

@@ -20,7 +20,7 @@ class LayerArgs(ctypes.Structure):
     _fields_ = ([(n, c_int64) for n in ("T", "H", "I", "E", "K", "TK_alloc", "TKp_alloc")]
                 + [(n, ctypes.c_int32) for n in ("lane_order", "pad_mode", "keep_z", "dw1_mode", "dw2_mode", "reserved")]
                 + [(n, c_void_p) for n in ("x", "dout", "idx", "probs", "w1", "w1_sf", "w2", "w2_sf", "out", "ds", "dw1",
-                                           "dw2", "counts", "saved", "scratch", "status", "host_word")])
+                                           "dw2", "counts", "saved", "scratch", "status", "host_word", "dx_ready")])
 
 
 DW_NONE, DW_ACCUMULATE, DW_STORE, DW_BF16 = 0, 1, 2, 3

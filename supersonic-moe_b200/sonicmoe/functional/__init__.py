@@ -344,12 +344,14 @@ _RESULT_READY: dict = {}
 
 
 def note_result_ready(t: torch.Tensor):
-    if t.is_cuda and not torch.cuda.is_current_stream_capturing():
-        if len(_RESULT_READY) >= 16:
-            _RESULT_READY.pop(next(iter(_RESULT_READY)))
-        ev = torch.cuda.Event()
-        ev.record()
-        _RESULT_READY[t.data_ptr()] = ev
+    """Record that `t` is complete; returns the event (None on the CPU and while a graph is captured)."""
+    if not t.is_cuda or torch.cuda.is_current_stream_capturing():
+        return None
+    if len(_RESULT_READY) >= 16:
+        _RESULT_READY.pop(next(iter(_RESULT_READY)))
+    ev = _RESULT_READY[t.data_ptr()] = torch.cuda.Event()
+    ev.record()
+    return ev
 
 
 def take_result_ready(t: torch.Tensor):
@@ -848,6 +850,7 @@ class _OneCallLayer(torch.autograd.Function):
         _lib.check(_lib.lib.smoe_layer_forward(args, ops._stream()), "layer_forward")
         if grad_mode:
             ctx.sizes = (args.T, args.H, args.I, args.E, args.K, args.TK_alloc, args.TKp_alloc)
+            ctx.x_is_leaf = x.is_leaf
             ctx.save_for_backward(x, w1, w2, saved)
         ctx.mark_non_differentiable(counts)
         return out, counts
@@ -878,6 +881,11 @@ class _OneCallLayer(torch.autograd.Function):
             dx = torch.empty_like(x)
             a.out = dx.data_ptr()
             _RESULT_READY.pop(a.out, None)       # an event noted for an earlier tensor at this address says nothing here
+            # dx of a leaf goes into .grad; any other has a reader in the graph, possibly an exchange on its own stream.  The
+            # event made here is recorded again by the call, between dx and the weight gradients.
+            ready = None if ctx.x_is_leaf else note_result_ready(dx)
+            if ready is not None:
+                a.dx_ready = ready.cuda_event
         if need_s:
             ds = torch.empty(T, a.K, dtype=torch.float32, device=dev)
             a.ds = ds.data_ptr()

@@ -126,6 +126,52 @@ def test_one_call_layer_gives_the_bits_of_the_step_by_step_path(sm, monkeypatch,
                 assert got.dtype == want.dtype and torch.equal(got, want), i
 
 
+@pytest.mark.parametrize("one_call", [True, False])
+def test_a_reader_of_dx_on_another_stream_need_not_wait_for_the_weight_gradients(sm, monkeypatch, one_call):
+    """Both paths note an event when dx is complete.  A reader that waits for that event alone sees all of dx, and the event
+    lies well before the end of the pass: the weight gradients follow it (64 experts of 2048 x 1024: they are most of it)."""
+    from sonicmoe.functional import take_result_ready
+    if not one_call:
+        monkeypatch.setattr(sm.functional, "_ONE_CALL_BYTES", 0)
+    T, H, I, E, K = 512, 2048, 1024, 64, 2
+    g = torch.Generator(device=DEV).manual_seed(3)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV).to(torch.bfloat16)
+    idx, scores = masked_routing(T, E, K, E, 4)
+    leaf, w1d, w2d = (t.requires_grad_(True) for t in (rand(T, H), rand(E, 2 * I, H) * 0.02, rand(E, H, I) * 0.02))
+    w1d.main_grad, w2d.main_grad = torch.zeros(E, 2 * I, H, device=DEV), torch.zeros(E, I, H, device=DEV)
+    side, seen, real = torch.cuda.Stream(), [], torch.cuda.Event
+
+    class Timed(real):
+        def __new__(cls, *a, **k):
+            return real.__new__(cls, enable_timing=True)
+
+    monkeypatch.setattr(torch.cuda, "Event", Timed)
+    for _ in range(2):                               # the first pass also makes the weights' FP8 copies
+        seen.clear()
+        rows = leaf * 1                              # not a leaf: its gradient has a reader in the graph
+
+        def reader(dx):
+            ready = take_result_ready(dx)
+            assert ready is not None
+            with torch.cuda.stream(side):
+                side.wait_event(ready)
+                seen.extend((dx.clone(), ready))
+            dx.record_stream(side)
+
+        rows.register_hook(reader)
+        start, end = Timed(), Timed()
+        out = sm.run_sonic_moe(rows, idx.to(DEV), scores.to(DEV), K, E, w1d, w2d, fp8=True)
+        grad = rand(T, H)
+        leaf.grad = None
+        torch.cuda.synchronize()
+        start.record()
+        out.backward(grad)
+        end.record()
+        torch.cuda.synchronize()
+    assert torch.equal(seen[0], leaf.grad)
+    assert start.elapsed_time(seen[1]) < 0.75 * start.elapsed_time(end)
+
+
 @pytest.mark.parametrize("T,H,I,E,K", [(1, 256, 128, 8, 2), (64, 384, 256, 64, 4), (300, 768, 384, 5, 3), (513, 512, 256, 3, 3)])
 def test_forward_without_a_graph_gives_the_same_bits(sm, T, H, I, E, K):
     """Under no_grad z is not written, pad rows are neither cleared nor stored, phantom tile halves not fetched: the output
