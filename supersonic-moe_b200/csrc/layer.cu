@@ -75,12 +75,12 @@ struct BwdScratch {
   int64_t parts;
   float *s, *dsp;
   uint8_t *dg, *dg_sf;              // dout, expert-sorted rows
-  uint8_t *dc, *dc_sf;              // dout, column-quantised
+  uint8_t *dc, *dc_sf;              // dout, column-quantised; null without dw2
   uint8_t *dz, *dz_rsf, *dz_csf, *dz_t;
   uint8_t *y1s, *y1s_sf;            // column-quantised: [rows, I], or [I, rows] when not fused
   uint8_t *dz_bf16, *y1s_bf16;
-  uint8_t* dx_exp;
-  uint8_t *xc, *xc_sf;
+  uint8_t* dx_exp;                  // null without dx
+  uint8_t *xc, *xc_sf;              // x, column-quantised; null without dw1
   size_t bytes;
   BwdScratch(const smoe_layer_args& a, void* arena) {
     Arena m(arena);
@@ -91,8 +91,11 @@ struct BwdScratch {
     dsp = m.take<float>(parts * R);
     dg = m.take(R * H);
     dg_sf = m.take(isa_bytes(R, H));
-    dc = m.take(R * H);
-    dc_sf = m.take(isa_bytes(H, R));
+    dc = dc_sf = dx_exp = xc = xc_sf = nullptr;
+    if (a.dw2_mode != SMOE_DW_NONE) {
+      dc = m.take(R * H);
+      dc_sf = m.take(isa_bytes(H, R));
+    }
     dz = m.take(R * 2 * I);
     dz_rsf = m.take(isa_bytes(R, 2 * I));
     dz_csf = m.take(isa_bytes(2 * I, R));
@@ -104,9 +107,11 @@ struct BwdScratch {
       dz_bf16 = m.take(R * 2 * I * 2);
       y1s_bf16 = m.take(R * I * 2);
     }
-    dx_exp = m.take(R * H * 2);
-    xc = m.take(R * H);
-    xc_sf = m.take(isa_bytes(H, R));
+    if (a.out) dx_exp = m.take(R * H * 2);
+    if (a.dw1_mode != SMOE_DW_NONE) {
+      xc = m.take(R * H);
+      xc_sf = m.take(isa_bytes(H, R));
+    }
     bytes = m.used;
   }
 };

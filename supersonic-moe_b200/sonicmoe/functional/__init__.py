@@ -798,9 +798,9 @@ class _DownProjection(torch.autograd.Function):
 # ----------------------------------------------------------------------------
 # small layers: the same launches from one native call per pass
 # ----------------------------------------------------------------------------
-# Bytes of scratch up to which a layer takes the one-call path (csrc/layer.cu).  All intermediates of a pass are alive at
-# once there, where the step-by-step path frees each after its last reader, so the peak grows by at most the bound.  It lies
-# where the kernels begin to outlast the host: a forward + backward of T=1024, H=3072, I=1536, E=K=8 (200 MB) is 0.53 ms of
+# Bytes of scratch up to which a layer takes the one-call path (csrc/layer.cu): the larger arena of forward and backward.  All
+# intermediates of a pass are alive at once there, where the step-by-step path frees each after its last reader, so the peak
+# grows by at most the bound.  It lies where the kernels begin to outlast the host: a forward + backward of T=1024, H=3072, I=1536, E=K=8 (200 MB) is 0.53 ms of
 # kernels and took 0.73 ms step by step (0.56 in one call), T=8192 is 2.7 ms of kernels for 0.72 ms of Python.
 _ONE_CALL_BYTES = 256 << 20
 
@@ -814,11 +814,17 @@ def _one_call_args(x, idx, w1, w2, E, K, TK, TKp, act, fp8_config):
         return None
     T, H = x.shape
     I = w2.shape[2]
-    if (T == 0 or E > 256 or H % 128 or I % 128 or TKp % 128 or tuple(w1.shape) != (E, 2 * I, H) or tuple(w2.shape) != (E, H, I)
-            or TKp * (5 * H + 4 * I if torch.is_grad_enabled() else 3 * H + I) > _ONE_CALL_BYTES):
+    if T == 0 or E > 256 or H % 128 or I % 128 or TKp % 128 or tuple(w1.shape) != (E, 2 * I, H) or tuple(w2.shape) != (E, H, I):
         return None
     a = _lib.LayerArgs(T, H, I, E, K, TK, TKp)
     a.x = x.data_ptr()
+    a.forward_bytes = scratch = _lib.lib.smoe_layer_bytes(a, 1)
+    if torch.is_grad_enabled():
+        a.out = a.x if x.requires_grad else None           # which gradients the backward will be asked for
+        a.dw1_mode, a.dw2_mode = int(w1.requires_grad), int(w2.requires_grad)
+        scratch = max(scratch, _lib.lib.smoe_layer_bytes(a, 2))
+    if not 0 <= scratch <= _ONE_CALL_BYTES:
+        return None
     a.status, a.host_word = ops.status_pointers(x.device)
     return a
 
@@ -842,7 +848,7 @@ class _OneCallLayer(torch.autograd.Function):
         counts = torch.empty(args.E, dtype=torch.int32, device=dev)
         args.lane_order, args.pad_mode, args.keep_z = lane_order, pad_mode, int(grad_mode)
         saved = _u8(_lib.lib.smoe_layer_bytes(args, 0), dev)
-        scratch = _u8(_lib.lib.smoe_layer_bytes(args, 1), dev)
+        scratch = _u8(args.forward_bytes, dev)
         args.idx, args.probs = idx.data_ptr(), probs.data_ptr()
         args.w1, args.w1_sf, args.w2, args.w2_sf = w1_q.data_ptr(), w1_sf.data_ptr(), w2_q.data_ptr(), w2_sf.data_ptr()
         args.out, args.counts, args.saved, args.scratch = (out.data_ptr(), counts.data_ptr(), saved.data_ptr(),

@@ -126,6 +126,33 @@ def test_one_call_layer_gives_the_bits_of_the_step_by_step_path(sm, monkeypatch,
                 assert got.dtype == want.dtype and torch.equal(got, want), i
 
 
+@pytest.mark.parametrize("wanted", ["all", "w2", "none"])
+@pytest.mark.parametrize("T,H,I,E,K", [(300, 896, 896, 4, 3), (300, 256, 512, 4, 3), (100, 384, 1408, 3, 2)])
+def test_one_call_scratch_stays_below_its_bound(sm, monkeypatch, T, H, I, E, K, wanted):
+    """The path is taken exactly where the larger of its two scratch arenas fits the bound: H or I off the multiples of 256
+    need more (bf16 dz and y1s), fewer gradients less."""
+    x, dy, w1, w2, _, _ = make_layer(T, H, I, E, K, 7)
+    idx, scores = masked_routing(T, E, K, E, 8)
+    arenas, real = [], sm.functional._u8
+    monkeypatch.setattr(sm.functional, "_u8", lambda n, dev: arenas.append(n) or real(n, dev))
+
+    def largest(limit):
+        """of the scratch arenas of a forward + backward, or None"""
+        monkeypatch.setattr(sm.functional, "_ONE_CALL_BYTES", limit)
+        arenas.clear()
+        leaves = [t.to(DEV).requires_grad_(wanted == "all") for t in (x, w1)] + [w2.to(DEV).requires_grad_(wanted != "none")]
+        out = sm.run_sonic_moe(leaves[0], idx.to(DEV), scores.to(DEV), K, E, leaves[1], leaves[2], fp8=True)
+        if wanted != "none":
+            out.backward(dy.to(DEV))
+        torch.cuda.synchronize()
+        sm.ops.check_status(DEV)
+        return max(arenas[1:]) if arenas else None         # the first one keeps z for the backward: both paths have it
+
+    with torch.set_grad_enabled(wanted != "none"):
+        need = largest(1 << 40)
+        assert largest(need) == need and largest(need - 1) is None
+
+
 @pytest.mark.parametrize("one_call", [True, False])
 def test_a_reader_of_dx_on_another_stream_need_not_wait_for_the_weight_gradients(sm, monkeypatch, one_call):
     """Both paths note an event when dx is complete.  A reader that waits for that event alone sees all of dx, and the event
