@@ -88,3 +88,26 @@ def test_gated_output_payload_wants_four_tensors():
         F.attach_preallocated_gated_outputs(sf, (1, 2, 3))
     assert F.attach_preallocated_gated_outputs(sf, (1, 2, 3, 4)) is sf
     assert getattr(sf, F._GATED_OUTPUT_PAYLOAD_ATTR) == (1, 2, 3, 4)
+
+
+@pytest.mark.parametrize("where", ["class", "subclass", "instance", "nowhere"])
+def test_a_replaced_switch_loss_is_the_one_called(monkeypatch, where):
+    """The auxiliary-loss kernels stand in for `MoE._compute_switch_loss` as this package defines it; another function under
+    that name - on the class itself too - is called with logits, probabilities and expert frequencies."""
+    import sonicmoe.moe as M
+    from sonicmoe.enums import ActivationType
+    logits, freq = torch.randn(5, 4), torch.arange(4, dtype=torch.int32)
+    monkeypatch.setattr(M, "moe_TC_softmax_topk_layer", lambda x, *a, **k: (x, logits, freq))
+    monkeypatch.setattr(M, "switch_loss", lambda *a: "kernels")
+
+    def other(self, logits, probs, expert_frequency):
+        assert torch.allclose(probs, torch.softmax(logits, -1)) and expert_frequency is freq
+        return "other"
+
+    cls = type("Sub", (M.MoE,), {"_compute_switch_loss": other}) if where == "subclass" else M.MoE
+    if where == "class":
+        monkeypatch.setattr(M.MoE, "_compute_switch_loss", other)
+    moe = cls(4, 2, 32, 32, ActivationType.SWIGLU, add_bias=False, std=0.02)
+    if where == "instance":
+        moe._compute_switch_loss = other.__get__(moe)
+    assert moe(torch.randn(5, 32))[1] == ("kernels" if where == "nowhere" else "other")
