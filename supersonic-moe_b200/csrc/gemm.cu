@@ -173,12 +173,12 @@ static bool use_gemm3(const GemmParams& p) {
   if (p.N % kBN3 != 0 || p.E > kMaxExperts2) return false;
   if (MODE == WGRAD && (p.rows % 256 != 0 || p.b_mn)) return false;
   if (MODE == PLAIN && p.b_mn) return false;      // a 192-byte MN-major slice is not a swizzle atom
-  // PLAIN: the 256-wide tile does as well or better nearly everywhere since the accumulator hand-back stopped stalling -
-  // N=3072, K=1536, E=8, 1 / 8 / 64 row tiles an expert 384-wide 19.3 / 43.8 / 245.5 us, 256-wide 20.0 / 41.4 / 237.8; E=32,
-  // one: 47.9 / 43.8; N=K=3072, E=8, 4 / 8: 41.7 / 68.4 against 38.7 / 64.8.  The wide one keeps long reductions over many
-  // rows, where its fewer operand bytes just show: N=K=3072, 64 row tiles: 429.0 against 430.8; N=K=6144, 8: 221.5 / 223.0.
-  if (MODE == PLAIN && g_force_bn == 0 && p.N % 256 == 0 && (p.K < 3072 || (int64_t)p.rows < (int64_t)p.E * 2048))
-    return false;
+  // PLAIN: wherever N is a multiple of both widths the 256-wide tile is taken, whatever the reduction length and the number of
+  // rows (p.rows is what the caller allocated, not what is routed).  Over N = 768 .. 6144, K = 1536 .. 6144, E = 2 / 8 / 32 and
+  // 1 .. 64 row tiles an expert, 166 of 192 points are faster with it, by 5 % in the median: N=K=3072, E=8, 8 / 16 / 32 / 64 row
+  // tiles 384-wide 76.7 / 112.8 / 209.9 / 425.9 us, 256-wide 72.7 / 112.6 / 204.7 / 418.8; N=K=6144, 8 / 64: 233.5 / 1810 against
+  // 230.3 / 1786.  The others are single counts at which the last wave fills better (N <= 1536, up to 10 %), no range.
+  if (MODE == PLAIN && g_force_bn == 0 && p.N % 256 == 0) return false;
   return true;
 }
 
