@@ -137,8 +137,7 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   if (pairs <= 0) return SMOE_OK;
   GemmParams q = p;
   q.dbg_stage_cut = g_stage_cut;
-  if (MODE == WGRAD && p.accumulate && !p.out_bf16)
-    q.stages_lent = (S::EPI_WARPS * 4096 + S::STAGE_BYTES - 1) / S::STAGE_BYTES;
+  if (MODE == WGRAD && p.accumulate && !p.out_bf16) q.stages_lent = S::LENT_STAGES;
   q.l2_prefetch = g_l2_prefetch >= 0 ? g_l2_prefetch : kDefaultL2Prefetch;
   kern<<<(unsigned)(2 * pairs), S::THREADS, S::TOTAL, stream>>>(ta, tb, tsa, tsb, om.c, om.c2, om.c3, q);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;

@@ -258,6 +258,13 @@ struct Gemm2Smem {
   static constexpr int TOTAL = STAGES * STAGE_BYTES + SF_BYTES + EPI_BYTES + AUX_BYTES + 1024;
   static_assert(TOTAL <= 227 * 1024, "shared memory budget");
   static_assert((3 * STAGES + 4 + 2 * SF_SLOTS) * 8 <= 496, "barrier storage");
+  // WGRAD into an existing f32 gradient: ring stages that hold 4 KB staging tiles (32 rows of 128 bytes, 128-byte swizzle) of
+  // the epilogue warps instead; the last ones of the ring, STAGES - LENT_STAGES on
+  static constexpr int LENT_TILE = 4096;
+  static constexpr int LENT_STAGES = (EPI_WARPS * LENT_TILE + STAGE_BYTES - 1) / STAGE_BYTES;
+  static_assert(STAGE_BYTES % 1024 == 0, "operand tiles and lent staging tiles start on swizzle atoms");
+  static_assert(LENT_STAGES * STAGE_BYTES >= EPI_WARPS * LENT_TILE, "every epilogue warp has a staging tile");
+  static_assert(MODE != WGRAD || STAGES - LENT_STAGES >= 4, "a ring is left (the timing experiments cut three stages more)");
   static constexpr int ACC_STAGES = (BN == 256) ? 1 : 2;  // TMEM: 512 columns
   static constexpr int SF_COLS = 4 + 4 * SFB_TILES;
   static constexpr int SF_COL0 = ACC_STAGES * BN;
@@ -774,8 +781,10 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
         }
       } else if (MODE == WGRAD) {
-        // Same scheme with f32 in 16-column pieces: 64-byte rows, SWIZZLE_64B, one 2 KB buffer; TMA reduce-add
-        // when accumulating into an existing gradient.
+        // Same scheme, the accumulator released before anything is stored; three forms of output: bf16 in 32-column pieces
+        // (64-byte rows, SWIZZLE_64B, the warp's 2 KB buffer), f32 added to an existing gradient in 32-column pieces
+        // (128-byte rows, SWIZZLE_128B, 4 KB tiles in the lent ring stages), f32 stored in 16-column pieces (64-byte rows,
+        // SWIZZLE_64B, 2 KB).
         constexpr int NC = COLS_PER_WARP / 32;
         uint32_t acc[NC][32];
 #pragma unroll
@@ -803,11 +812,11 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
         } else if (p.accumulate) {
           // Reduce-adds in whole 128-byte lines (32 columns), from 4 KB staging tiles in the ring stages lent for them; the
-          // L2 merges a 64-byte piece no cheaper than a line (E=128, M=768, N=2048: 400 -> 366 us; M=1536: 755 -> 729).
+          // L2 merges a 64-byte piece no cheaper than a line (E=128, M=768, N=2048: 400 -> 364 us; M=1536: 755 -> 726).
           // What bounds the rest is read-modify-write traffic in tile order: reading the old values with the epilogue's
           // own loads instead took 920 us, more staging tiles (two or three a warp) 760 and 834 us, fetching the tile
           // towards L2 ahead of time 800 us.
-          const uint32_t sb = smem_base + nst * S::STAGE_BYTES + (warp - 2) * 4096;
+          const uint32_t sb = smem_base + nst * S::STAGE_BYTES + (warp - 2) * S::LENT_TILE;
           const int crow = t.e * p.rows + t.m0 + q * 32;
 #pragma unroll
           for (int c = 0; c < NC; ++c) {

@@ -409,6 +409,12 @@ quant_cols_kernel(const void* __restrict__ src_, const uint8_t* __restrict__ src
   }
 }
 
+__device__ __forceinline__ uint32_t q_max_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+
 // ------------------------------------------------------------------ weights, both orientations
 // One [N, K] expert matrix per blockIdx.z, one 128x128 tile per block.  A tile of W is read ONCE and leaves twice:
 // quantised 1x32 along K in place (q, `row_isa` = ISA scales of the stacked (E*N, K) operand) and 1x32 along N with
@@ -421,12 +427,6 @@ quant_cols_kernel(const void* __restrict__ src_, const uint8_t* __restrict__ src
 // Measured at E=128, H=2048, I=768 (604 M weights, 2.45 GB, one launch per weight): 421 us = 5.8 TB/s, 0.89 of a plain
 // copy; one launch per expert for the transposed copy and a second read for the row copy took 3719 us (host-bound: 256
 // launches; their kernels alone 1345 us).
-__device__ __forceinline__ uint32_t q_max_bf16x2(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-
 constexpr int QW_TILE = 128, QW_PITCH = QW_TILE + 8;      // bf16 elements; 272 bytes: 16-byte aligned rows
 
 template <bool ROW, bool COL>
