@@ -219,6 +219,61 @@ def test_quant_iso32_bit_exact(ops, rows, cols):
     assert torch.equal(Q.unpack_isa(ci.cpu(), cols, rows), bs.t().repeat_interleave(32, dim=0))
 
 
+def test_quantizers_take_infinities_and_nan(ops):
+    """A NaN becomes an e4m3 NaN and does not count in its group's maximum; an infinity sets the largest scale and saturates,
+    its finite neighbours vanish: weights in both orientations, rows, columns left as rows, transposed, and from FP8."""
+    N = K = 256
+    x = adversarial_rows(N, K, 31)
+    x[10, 3], x[11, 40], x[12, 70] = float("inf"), float("-inf"), float("nan")
+    x[13, :32] = float("nan")                                       # a whole group of a row
+    x[64:96, 5] = float("nan")                                      # a whole group of a column
+    x[70, 9], x[71, 9], x[20, 33], x[20, 34] = float("nan"), float("inf"), float("nan"), float("inf")
+
+    def same(q, sc, ref, v, name):
+        """payload and scales of `v`: those of v without its NaNs, and NaN where it has one"""
+        rq, rs = ref(torch.where(torch.isnan(v), torch.zeros_like(v), v))
+        assert torch.equal(sc, rs), name
+        assert torch.equal(torch.where(torch.isnan(v), torch.full_like(q, 0x7F), rq), torch.where(torch.isnan(v), q & 0x7F, q)), name
+
+    xd = x.to(DEV)
+    q, ri, qt, ci = ops.quant_weight(torch.stack([xd, xd]))
+    for e in range(2):
+        same(q[e].cpu(), Q.unpack_isa(ri.cpu(), 2 * N, K)[e * N:(e + 1) * N], Q.row_quant, x, "weight")
+        same(qt[e].t().cpu(), Q.unpack_isa(ci.view(2, -1)[e].cpu(), K, N), Q.col_quant, x, "transposed weight")
+    q, raw, _ = ops.quant_rows(xd)
+    same(q.cpu(), raw.cpu(), Q.row_quant, x, "rows")
+    qt, ci = ops.quant_cols_t(xd, None, N)
+    same(qt.t().cpu(), Q.unpack_isa(ci.cpu(), K, N), Q.col_quant, x, "columns, transposed")
+    _, _, qc, ci = ops.quant_dual_gather(xd, torch.arange(N, dtype=torch.int32, device=DEV), N, with_rows=False)
+    same(qc.cpu(), Q.unpack_isa(ci.cpu(), K, N), Q.col_quant, x, "columns")
+    qt, ci = ops.requant_cols_t(q, raw, torch.arange(N, dtype=torch.int32, device=DEV), N)
+    same(qt.t().cpu(), Q.unpack_isa(ci.cpu(), K, N), Q.col_quant, Q.dequant_rows(q.cpu(), raw.cpu()).to(torch.bfloat16), "FP8 columns")
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("bad", ["masked", "inf", "nan", "nothing"])
+def test_switch_loss_of_infinite_and_nan_logits(ops, dt, bad):
+    """-inf logits (masked experts) cost nothing and get no gradient; a row without a softmax makes the loss and the gradients
+    NaN where the tensor expression has them."""
+    from sonicmoe.functional import switch_loss, switch_loss_expression
+    g = torch.Generator().manual_seed(1)
+    x0 = torch.randn(40, 70, generator=g)
+    freq = torch.randint(0, 9, (70,), generator=g, dtype=torch.int32).to(DEV)
+    if bad == "masked":
+        x0[:, 60:] = x0[3, 1:] = float("-inf")
+    else:
+        x0[7, 11 if bad != "nothing" else slice(None)] = {"inf": float("inf"), "nan": float("nan"), "nothing": float("-inf")}[bad]
+    got = []
+    for f in (switch_loss, switch_loss_expression):
+        x = x0.to(DEV, dt).requires_grad_(True)
+        loss = f(x, freq)
+        loss.backward()
+        got.append((loss.detach().float(), x.grad.float()))
+    for a, b in zip(*got):
+        assert torch.equal(torch.isnan(a), torch.isnan(b))
+        torch.testing.assert_close(a, b, rtol=2 ** -7 if dt == torch.bfloat16 else 1e-4, atol=1e-6, equal_nan=True)   # one rounding
+
+
 def test_combine_matches_oracle_and_repeats(ops):
     N, K, E, H = 512, 8, 16, 1024
     idx, probs = make_routing(N, K, E, 0.2, seed=2)

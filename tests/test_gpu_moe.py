@@ -126,6 +126,73 @@ def test_one_call_layer_gives_the_bits_of_the_step_by_step_path(sm, monkeypatch,
                 assert got.dtype == want.dtype and torch.equal(got, want), i
 
 
+@pytest.mark.parametrize("how", ["side_stream", "captured", "twice"])
+def test_one_call_layer_on_a_side_stream_under_capture_and_differentiated_twice(sm, monkeypatch, how):
+    """The one-call passes give the bits of the step-by-step ones on a stream that is not the default, replayed from a CUDA
+    graph on new inputs (main_grad added to by each replay), and in a second backward of a retained graph."""
+    T, H, I, E, K = 130, 256, 256, 6, 3
+    x, dy, w1, w2, _, _ = make_layer(T, H, I, E, K, 11)
+    idx, scores = masked_routing(T, E, K, E, 12)
+    x2, dy2 = x.flip(0).contiguous(), dy.flip(0).contiguous()
+
+    def leaves():
+        t = [v.to(DEV).requires_grad_(True) for v in (x, scores, w1, w2)]
+        t[2].main_grad, t[3].main_grad = torch.zeros(E, 2 * I, H, device=DEV), torch.zeros(E, I, H, device=DEV)
+        return t, idx.to(DEV), dy.to(DEV)
+
+    def step(t, idx, dy, **kw):
+        t[0].grad = t[1].grad = None
+        out = sm.run_sonic_moe(t[0], idx, t[1], K, E, t[2], t[3], fp8=True)
+        out.backward(dy, **kw)
+        return out
+
+    def results(t, out):
+        torch.cuda.synchronize()
+        sm.ops.check_status(DEV)
+        return [v.detach().clone() for v in (out, t[0].grad, t[1].grad, t[2].main_grad, t[3].main_grad)]
+
+    monkeypatch.setattr(sm.functional, "_ONE_CALL_BYTES", 0)
+    t, i, d = leaves()
+    if how == "captured":
+        step(t, i, d)
+        with torch.no_grad():
+            t[0].copy_(x2), d.copy_(dy2)
+    out = step(t, i, d)
+    if how == "twice":
+        out = step(t, i, d)
+        with torch.no_grad():
+            t[0].grad.mul_(2), t[1].grad.mul_(2)
+    want = results(t, out)
+
+    monkeypatch.setattr(sm.functional, "_ONE_CALL_BYTES", 1 << 40)
+    t, i, d = leaves()
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    if how == "side_stream":
+        with torch.cuda.stream(side):
+            out = step(t, i, d)
+    elif how == "twice":
+        out = step(t, i, d, retain_graph=True)
+        out.backward(d)
+    else:
+        with torch.cuda.stream(side):
+            step(t, i, d)                            # the weights' FP8 copies; and what a graph wants warmed up
+            t[2].main_grad.zero_(), t[3].main_grad.zero_()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            out = step(t, i, d)
+        graph.replay()
+        with torch.no_grad():
+            t[0].copy_(x2), d.copy_(dy2)
+        graph.replay()
+    for n, (a, b) in enumerate(zip(results(t, out), want)):
+        assert torch.equal(a, b), n
+    if how == "captured":
+        del out
+        graph.reset()
+
+
 @pytest.mark.parametrize("wanted", ["all", "w2", "none"])
 @pytest.mark.parametrize("T,H,I,E,K", [(300, 896, 896, 4, 3), (300, 256, 512, 4, 3), (100, 384, 1408, 3, 2)])
 def test_one_call_scratch_stays_below_its_bound(sm, monkeypatch, T, H, I, E, K, wanted):
@@ -200,9 +267,12 @@ def test_a_reader_of_dx_on_another_stream_need_not_wait_for_the_weight_gradients
 
 
 @pytest.mark.parametrize("T,H,I,E,K", [(1, 256, 128, 8, 2), (64, 384, 256, 64, 4), (300, 768, 384, 5, 3), (513, 512, 256, 3, 3)])
-def test_forward_without_a_graph_gives_the_same_bits(sm, T, H, I, E, K):
+@pytest.mark.parametrize("one_call", [True, False])
+def test_forward_without_a_graph_gives_the_same_bits(sm, monkeypatch, T, H, I, E, K, one_call):
     """Under no_grad z is not written, pad rows are neither cleared nor stored, phantom tile halves not fetched: the output
     is that of the training forward bit for bit, whatever the buffers held before (NaN here)."""
+    if not one_call:
+        monkeypatch.setattr(sm.functional, "_ONE_CALL_BYTES", 0)
     x, _, w1, w2, wr, _ = make_layer(T, H, I, E, K, T)
     moe = sm.MoE(E, K, H, I, sm.ActivationType.SWIGLU, add_bias=False, std=0.02).to(DEV).to(torch.bfloat16)
     with torch.no_grad():
@@ -211,15 +281,21 @@ def test_forward_without_a_graph_gives_the_same_bits(sm, T, H, I, E, K):
         moe.c_proj.weight.copy_(w2)
     xd = x.to(DEV)
     want, _ = moe(xd, use_fp8=True)
+    idx, scores = masked_routing(T, E, K, E, 9)
+    routed = (idx.to(DEV), scores.to(DEV), K, E, moe.c_fc.weight, moe.c_proj.weight)
+    want_routed = sm.run_sonic_moe(xd, *routed, fp8=True)
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     poison = [torch.full((n,), 255, dtype=torch.uint8, device=DEV) for n in (1 << 24, 1 << 23, 1 << 22, 1 << 20, 1 << 18)]
     del poison                                       # the allocator hands these bytes out again
     with torch.no_grad():
         got, _ = moe(xd, is_inference_mode=True, use_fp8=True)
+        place = torch.full_like(xd, float("nan"))
+        got_routed = sm.run_sonic_moe(xd, *routed, fp8=True, out=None if one_call else place)
     torch.cuda.synchronize()
     sm.ops.check_status(DEV)
-    assert torch.equal(got, want)
+    assert torch.equal(got, want) and torch.equal(got_routed, want_routed)
+    assert one_call or got_routed.data_ptr() == place.data_ptr()
 
 
 @pytest.mark.parametrize("T,H,I,E,K,seed", [(256, 256, 128, 8, 2, 0), (1024, 512, 256, 16, 4, 1),
