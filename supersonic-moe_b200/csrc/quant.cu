@@ -759,10 +759,9 @@ quant_dual_kernel(const uint4* __restrict__ x, const int* __restrict__ idx, cons
 }
 
 
-// The barrier-free form of the transposed column quantizer (every dim a GEMM takes; at dim = 3072 96 -> 85 us, see there).
-// Half a scale tile more, or buffers off the 16-byte boundary of its accesses, go to the kernel that stages 64 columns.
-static bool whole_tiles(int64_t dim, const void* src, const void* q, const void* isa) {
-  return dim % 128 == 0 && (((uintptr_t)src | (uintptr_t)q | (uintptr_t)isa) & 15) == 0;
+// What every column kernel accesses 16 bytes at a time, and its scales by the word
+static bool cols_aligned(const void* src, const void* q, const void* isa) {
+  return (((uintptr_t)src | (uintptr_t)q) & 15) == 0 && ((uintptr_t)isa & 3) == 0;
 }
 
 extern "C" {
@@ -840,7 +839,10 @@ int smoe_quant_cols_t(const void* src_bf16, const int32_t* idx, const int32_t* v
                       void* q_t, void* isa, void* stream) {
   if (rows < 0 || rows % 128 || dim <= 0 || dim % 64) return SMOE_ERR_SHAPE;
   if (rows == 0) return SMOE_OK;
-  if (whole_tiles(dim, src_bf16, q_t, isa)) {
+  if (!cols_aligned(src_bf16, q_t, isa)) return SMOE_ERR_ALIGN;
+  // whole scale tiles (every dim a GEMM takes): the form without barriers; half a tile more: 64 columns staged (dim = 3072:
+  // 85 against 96 us)
+  if (dim % 128 == 0) {
     quant_cols_t_kernel<false><<<dim3((unsigned)(rows / 128), (unsigned)((dim + 255) / 256)), 32 * QT_WARPS, 0,
                                  (cudaStream_t)stream>>>(src_bf16, nullptr, idx, valid_rows, rows, (int)dim, (uint8_t*)q_t,
                                                          (uint8_t*)isa);
@@ -857,7 +859,8 @@ int smoe_requant_cols_t(const void* src_fp8, const void* src_scales, const int32
   if (rows < 0 || rows % 128 || dim <= 0 || dim % 64) return SMOE_ERR_SHAPE;
   if (rows == 0) return SMOE_OK;      // nothing routed: not an error, and the (empty) buffers may be null
   if (!src_scales) return SMOE_ERR_ARG;
-  if (whole_tiles(dim, src_fp8, q_t, isa)) {
+  if (!cols_aligned(src_fp8, q_t, isa)) return SMOE_ERR_ALIGN;
+  if (dim % 128 == 0) {
     quant_cols_t_kernel<true><<<dim3((unsigned)(rows / 128), (unsigned)((dim + 255) / 256)), 32 * QT_WARPS, 0,
                                 (cudaStream_t)stream>>>(src_fp8, (const uint8_t*)src_scales, idx, valid_rows, rows, (int)dim,
                                                         (uint8_t*)q_t, (uint8_t*)isa);
@@ -874,6 +877,7 @@ int smoe_quant_iso32(const void* x_bf16, int64_t rows, int64_t cols, void* q, vo
                      void* stream) {
   if (rows < 0 || rows % 128 || cols <= 0 || cols % 128) return SMOE_ERR_SHAPE;
   if (rows == 0) return SMOE_OK;
+  if (!cols_aligned(x_bf16, q, col_isa) || ((uintptr_t)q_t & 15) || ((uintptr_t)row_isa & 1)) return SMOE_ERR_ALIGN;
   dim3 grid((unsigned)(rows / CT_ROWS), (unsigned)(cols / CT_COLS));
   quant_cols_kernel<true, false><<<grid, 256, 0, (cudaStream_t)stream>>>(x_bf16, nullptr, nullptr, rows, (int)cols,
                                                                          (uint8_t*)q_t, (uint8_t*)col_isa, (uint8_t*)q,

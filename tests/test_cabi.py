@@ -43,3 +43,14 @@ def test_host_side_argument_checks(built_library):
                                   None, None, None) == 1                            # top-k > 16
     assert lib.smoe_topk_metadata_workspace(64, 8) > 0
     assert lib.smoe_combine(None, None, None, None, None, 4, 12, None) == 1        # H % 8
+
+
+def test_column_quantizers_refuse_misaligned_buffers(built_library):
+    """Every column kernel moves 16 bytes at a time: a source or payload off that boundary is an error code, never a launch."""
+    from sonicmoe._lib import lib
+    for dim in (64, 128):
+        for src, q, isa in ((8, 16, 16), (16, 24, 16), (16, 16, 18)):
+            assert lib.smoe_quant_cols_t(src, None, None, 128, dim, q, isa, None) == 2
+            assert lib.smoe_requant_cols_t(src, 16, None, None, 128, dim, q, isa, None) == 2
+    assert lib.smoe_quant_iso32(8, 128, 128, 16, 16, None, 16, None) == 2
+    assert lib.smoe_quant_iso32(16, 128, 128, 16, 16, 8, 16, None) == 2
