@@ -343,15 +343,29 @@ def _after_accumulate(base):
 _RESULT_READY: dict = {}
 
 
-def note_result_ready(t: torch.Tensor):
-    """Record that `t` is complete; returns the event (None on the CPU and while a graph is captured)."""
+_RESULT_READY_MAX = 16
+
+
+def _result_event(t: torch.Tensor):
+    """The event that will say `t` is complete (None on the CPU and while a graph is captured), created but not yet recorded for
+    `t`.  An event nobody asked about - that of an earlier tensor at this address, or the oldest of many - is used again: making
+    and destroying one costs a small layer's backward 40 of 650 us."""
+    ev = _RESULT_READY.pop(t.data_ptr(), None)
     if not t.is_cuda or torch.cuda.is_current_stream_capturing():
         return None
-    if len(_RESULT_READY) >= 16:
-        _RESULT_READY.pop(next(iter(_RESULT_READY)))
-    ev = _RESULT_READY[t.data_ptr()] = torch.cuda.Event()
-    ev.record()
+    if ev is None and len(_RESULT_READY) >= _RESULT_READY_MAX:
+        ev = _RESULT_READY.pop(next(iter(_RESULT_READY)), None)
+    if ev is None or ev.device != t.device:
+        ev = torch.cuda.Event()
+        ev.record()
+    _RESULT_READY[t.data_ptr()] = ev
     return ev
+
+
+def note_result_ready(t: torch.Tensor):
+    ev = _result_event(t)
+    if ev is not None:
+        ev.record()
 
 
 def take_result_ready(t: torch.Tensor):
@@ -822,7 +836,8 @@ def _one_call_args(x, idx, w1, w2, E, K, TK, TKp, act, fp8_config):
     if torch.is_grad_enabled():
         a.out = a.x if x.requires_grad else None           # which gradients the backward will be asked for
         a.dw1_mode, a.dw2_mode = int(w1.requires_grad), int(w2.requires_grad)
-        scratch = max(scratch, _lib.lib.smoe_layer_bytes(a, 2))
+        a.backward_bytes = _lib.lib.smoe_layer_bytes(a, 2)
+        scratch = max(scratch, a.backward_bytes)
     if not 0 <= scratch <= _ONE_CALL_BYTES:
         return None
     a.status, a.host_word = ops.status_pointers(x.device)
@@ -856,7 +871,7 @@ class _OneCallLayer(torch.autograd.Function):
         _lib.check(_lib.lib.smoe_layer_forward(args, ops._stream()), "layer_forward")
         if grad_mode:
             ctx.sizes = (args.T, args.H, args.I, args.E, args.K, args.TK_alloc, args.TKp_alloc)
-            ctx.x_is_leaf = x.is_leaf
+            ctx.backward_bytes, ctx.x_is_leaf = args.backward_bytes, x.is_leaf
             ctx.save_for_backward(x, w1, w2, saved)
         ctx.mark_non_differentiable(counts)
         return out, counts
@@ -886,12 +901,13 @@ class _OneCallLayer(torch.autograd.Function):
             a.w1, a.w1_sf = w1t_q.data_ptr(), w1t_sf.data_ptr()
             dx = torch.empty_like(x)
             a.out = dx.data_ptr()
-            _RESULT_READY.pop(a.out, None)       # an event noted for an earlier tensor at this address says nothing here
             # dx of a leaf goes into .grad; any other has a reader in the graph, possibly an exchange on its own stream.  The
-            # event made here is recorded again by the call, between dx and the weight gradients.
-            ready = None if ctx.x_is_leaf else note_result_ready(dx)
-            if ready is not None:
-                a.dx_ready = ready.cuda_event
+            # call records the event between dx and the weight gradients.
+            if ctx.x_is_leaf:
+                _RESULT_READY.pop(a.out, None)   # an event noted for an earlier tensor at this address says nothing here
+            else:
+                ready = _result_event(dx)
+                a.dx_ready = None if ready is None else ready.cuda_event
         if need_s:
             ds = torch.empty(T, a.K, dtype=torch.float32, device=dev)
             a.ds = ds.data_ptr()
@@ -913,7 +929,7 @@ class _OneCallLayer(torch.autograd.Function):
                 bf16 = w1.dtype == torch.bfloat16 and _mn_wgrad_ok(E, 2 * I, H)
                 dw1 = torch.empty(E, 2 * I, H, dtype=torch.bfloat16 if bf16 else torch.float32, device=dev)
                 a.dw1_mode, a.dw1 = _lib.DW_BF16 if bf16 else _lib.DW_STORE, dw1.data_ptr()
-        scratch = _u8(_lib.lib.smoe_layer_bytes(a, 2), dev)
+        scratch = _u8(ctx.backward_bytes, dev)       # of every gradient that could be asked for: never less than this pass needs
         a.scratch = scratch.data_ptr()
         _lib.check(_lib.lib.smoe_layer_backward(a, ops._stream()), "layer_backward")
         if mg2 is not None:
