@@ -176,7 +176,9 @@ static bool use_gemm3(const GemmParams& p) {
   // rows (p.rows is what the caller allocated, not what is routed).  Over N = 768 .. 6144, K = 1536 .. 6144, E = 2 / 8 / 32 and
   // 1 .. 64 row tiles an expert, 166 of 192 points are faster with it, by 5 % in the median: N=K=3072, E=8, 8 / 16 / 32 / 64 row
   // tiles 384-wide 76.7 / 112.8 / 209.9 / 425.9 us, 256-wide 72.7 / 112.6 / 204.7 / 418.8; N=K=6144, 8 / 64: 233.5 / 1810 against
-  // 230.3 / 1786.  The others are single counts at which the last wave fills better (N <= 1536, up to 10 %), no range.
+  // 230.3 / 1786.  The others are single counts at which the last wave fills better (up to 10 %), no range.  Where N is a multiple
+  // of 384 only, the choice is between 384 and 192 columns, and the wide one stays for its long products: N=1920, K=3072, E=8, 1 /
+  // 8 / 16 / 64 row tiles 29.7 / 56.3 / 84.9 / 261.1 us against 29.7 / 54.1 / 89.0 / 305.0.
   if (MODE == PLAIN && g_force_bn == 0 && p.N % 256 == 0) return false;
   return true;
 }

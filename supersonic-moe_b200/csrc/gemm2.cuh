@@ -954,8 +954,9 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         // Issue slots of the epilogue warps bound the tile, not the MMAs: a profile counted 1500 instructions per warp and
         // 32-column chunk at 0.43 issued a cycle, 21 k cycles a tile for 9.2 k cycles of MMAs (H=3072).  So the f32
         // arithmetic runs on pairs, maxima and power-of-two scalings on bf16 pairs, the column scales travel through shared
-        // memory, and the wait for the staging tile comes as late as it can: 316 -> 296 us at T=8192, H=3072, I=1536,
-        // E=K=8, 1333 -> 1232 us at H=I=4096.  (Twelve epilogue warps of 64 columns instead of eight of 96: 309 us.)
+        // memory, and the wait for the staging tile comes as late as it can: 326 -> 309 us at T=8192, H=3072, I=1536,
+        // E=K=8, 59.8 -> 54.8 at T=1024, 1071 -> 1032 us at H=I=4096, in isolation on one box.  (Twelve epilogue warps of 64
+        // columns instead of eight of 96 cost 2 % more.)
         // a ragged last column tile (N not a multiple of BN): chunks at or beyond column N hold products with
         // rows of the next expert's weights (or TMA zero fill) and are skipped whole (N is a multiple of 32)
         if (t.valid && c_base < p.N && !(p.debug_skip_store & 2)) {

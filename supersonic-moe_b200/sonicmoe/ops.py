@@ -95,11 +95,11 @@ def check_status(device):
         _raise_status(device, s)
 
 
-# The layer reads the status word without ever waiting for the GPU: the end of a forward / backward launches a
-# one-thread kernel that stores the word into pinned host memory (a kernel store, not a memcpy: it cannot queue behind
-# bulk transfers on a copy engine); the next entry into the layer looks at that host word and raises if it is
+# The layer reads the status word without ever waiting for the GPU: at the end of a forward / backward a kernel (a
+# one-thread kernel of its own; in a one-call forward the combine) stores the word into pinned host memory (a kernel
+# store, not a memcpy: it cannot queue behind bulk transfers on a copy engine); the next entry into the layer looks at that host word and raises if it is
 # non-zero.  The word is sticky on the device, so a failure surfaces at the latest one call after the pass whose
-# post saw it, and a healthy run pays one tiny launch per pass and no synchronisation.
+# post saw it, and a healthy run pays at most one tiny launch per pass and no synchronisation.
 _posted = {}     # device index -> pinned int32[1] mirror of the device status word
 
 
