@@ -11,6 +11,7 @@
 //                         one more block scans valid[.] -> token-major bases, real_TK
 //   3. scatter_fill_kernel recomputes the padded offsets in shared memory, writes
 //                         every output, then fills pad rows and over-allocated tails
+// Small problems run the three steps in one kernel (metadata_cluster_kernel).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -109,31 +110,41 @@ scan_kernel(const uint32_t* __restrict__ mask, const int* __restrict__ unit_vali
   }
 }
 
-template <int KP>
-__global__ void __launch_bounds__(KP > 8 ? 32 * KP : 256)
-scatter_fill_kernel(const int* __restrict__ idx, const float* __restrict__ probs, int N, int K, int E, int alignment,
-                    int TK_alloc, int TKp_alloc, int lane_order, int pad_mode, const uint32_t* __restrict__ mask,
-                    const int* __restrict__ unit_off, const int* __restrict__ unit_base,
-                    const int* __restrict__ counts, int* __restrict__ efo_out, int* __restrict__ x_gather,
-                    int* __restrict__ s_scatter, int* __restrict__ s_rev, int* __restrict__ naept,
-                    float* __restrict__ scores, int* __restrict__ src_idx, int scatter_blocks) {
-  extern __shared__ int s_mem[];
-  int* s_efo = s_mem;              // [E+1] padded offsets
-  int* s_base = s_mem + (E + 1);   // [E+1] unpadded offsets
-  int* s_warp = s_base + (E + 1);  // [33]
-  const int lane = threadIdx.x & 31;
+// What the scatter and the fill write, and the sizes they go by
+struct TopkOut {
+  const int* idx;
+  const float* probs;
+  int N, K, E, alignment, TK_alloc, TKp_alloc, lane_order, pad_mode;
+  int *efo, *x_gather, *s_scatter, *s_rev, *naept;
+  float* scores;
+  int *src_idx, *counts;
+};
 
-  const int tot_p = block_excl_scan(
+// Offsets of the experts' segments, in shared memory, and what of the problem fits the buffers
+struct Layout {
+  int limit;       // expert-sorted positions at or beyond it are not published
+  int tot_p;       // padded rows
+  int real_TK;     // entries that are published, naept[N]
+  bool cut;
+};
+
+// s_efo / s_base [E+1]: padded and unpadded offsets from counts(e); the whole block takes part, `first`: this block writes efo
+// and, of a cut pass, naept[N]
+template <typename C>
+__device__ Layout block_layout(const TopkOut& o, C counts, int* s_efo, int* s_base, int* s_warp, bool first) {
+  Layout l;
+  const int E = o.E, alignment = o.alignment;
+  l.tot_p = block_excl_scan(
       E,
       [&](int e) {
-        const int c = counts[e];
+        const int c = counts(e);
         return c > 0 ? (c + alignment - 1) / alignment * alignment : 0;
       },
       [&](int e, int ex) { s_efo[e] = ex; }, s_warp);
   const int tot_u = block_excl_scan(
-      E, [&](int e) { return counts[e]; }, [&](int e, int ex) { s_base[e] = ex; }, s_warp);
+      E, [&](int e) { return counts(e); }, [&](int e, int ex) { s_base[e] = ex; }, s_warp);
   if (threadIdx.x == 0) {
-    s_efo[E] = tot_p;
+    s_efo[E] = l.tot_p;
     s_base[E] = tot_u;
   }
   __syncthreads();
@@ -143,90 +154,93 @@ scatter_fill_kernel(const int* __restrict__ idx, const float* __restrict__ probs
   // clamp(limit - s_efo[e]) rows, so the token-major base of a unit is the sum of what its experts keep of the units before -
   // and of what is left the first TK_alloc entries stay; the row of a later one becomes a pad row (it lies among the last rows
   // of its expert: token-major order is ascending there).  naept, s_rev, s_scatter and the scores then agree with each other.
-  const int limit = TKp_alloc / alignment * alignment;
-  if (blockIdx.x == 0)
-    for (int e = threadIdx.x; e <= E; e += blockDim.x) efo_out[e] = min(s_efo[e], limit);
-  const int real_TKp = tot_p;
-  const bool cut = tot_p > limit || tot_u > TK_alloc;
-  int real_TK = tot_u;              // entries that are published, naept[N]
-  if (cut) {
+  l.limit = o.TKp_alloc / alignment * alignment;
+  if (first)
+    for (int e = threadIdx.x; e <= E; e += blockDim.x) o.efo[e] = min(s_efo[e], l.limit);
+  l.cut = l.tot_p > l.limit || tot_u > o.TK_alloc;
+  l.real_TK = tot_u;
+  if (l.cut) {
     const int fit = block_excl_scan(
-        E, [&](int e) { return max(min(counts[e], limit - s_efo[e]), 0); }, [](int, int) {}, s_warp);
-    real_TK = min(fit, TK_alloc);
-    if (blockIdx.x == 0 && threadIdx.x == 0) naept[N] = real_TK;
+        E, [&](int e) { return max(min(counts(e), l.limit - s_efo[e]), 0); }, [](int, int) {}, s_warp);
+    l.real_TK = min(fit, o.TK_alloc);
+    if (first && threadIdx.x == 0) o.naept[o.N] = l.real_TK;
   }
+  return l;
+}
 
-  // ---- scatter: one thread per (row, slot) ----
-  // A unit of 32 rows is KP warps (KP: slots a row, rounded up to a power of two), slots fastest: the loads of indices and
-  // probabilities and the three token-major stores of a warp then fall into consecutive addresses, and a launch spreads over
-  // K times as many SMs as with one row a thread (16384 rows, K=8, E=128: 11.0 -> 6.0 us).
-  if ((int)blockIdx.x < scatter_blocks) {
-    constexpr int RPW = 32 / KP;                              // rows per warp
-    const int warp = threadIdx.x >> 5;
-    const int unit = blockIdx.x * ((int)blockDim.x / (32 * KP)) + warp / KP;
-    const int k = lane & (KP - 1), rw = lane / KP;            // slot; row within the warp
-    const int r = (warp % KP) * RPW + rw;                     // row within the unit
-    const int row = unit * 32 + r;
-    const bool in = row < N && k < K;
-    int e = in ? idx[(size_t)row * K + k] : -1;
-    if (e < 0 || e >= E) e = -1;
-    int pos = 0;
-    if (e >= 0) {
-      const uint32_t m = mask[(size_t)unit * E + e];
-      pos = s_efo[e] + unit_off[(size_t)unit * E + e] + __popc(m & ((1u << r) - 1u));
-      if (pos >= limit) e = -1;
-    }
-    const uint32_t ball = __ballot_sync(0xffffffffu, e >= 0);
-    if (lane == 0) s_warp[warp] = __popc(ball);
-    __syncthreads();
-    int tm_base = 0;
-    if (unit * 32 < N) {
-      if (!cut) tm_base = unit_base[unit];
-      else
-        for (int j = 0; j < E; ++j) tm_base += max(min(unit_off[(size_t)unit * E + j], limit - s_efo[j]), 0);
-    }
-    for (int w = warp - warp % KP; w < warp; ++w) tm_base += s_warp[w];
-    const int row_base = tm_base + __popc(ball & ((1u << (rw * KP)) - 1u));        // rw * KP <= 31
-    const int cap = cut ? real_TK : TK_alloc;
-    if (row < N && k == 0) naept[row] = min(row_base, cap);
-    int rank = 0;
-    if (lane_order == 0) {
+// ---- scatter: one thread per (row, slot) ----
+// A unit of 32 rows is KP warps (KP: slots a row, rounded up to a power of two), slots fastest: the loads of indices and
+// probabilities and the three token-major stores of a warp then fall into consecutive addresses, and a launch spreads over
+// K times as many SMs as with one row a thread (16384 rows, K=8, E=128: 11.0 -> 6.0 us).
+// mask(e) / off(e): rows of the unit that selected e, and e's rows in the units before; base(): entries before the unit.
+// Every thread of the block takes part, also for a unit beyond the last.
+template <int KP, typename M, typename F, typename B>
+__device__ __forceinline__ void scatter_unit(const TopkOut& o, const Layout& l, const int* s_efo, int* s_warp, int unit, M mask,
+                                             F off, B base) {
+  constexpr int RPW = 32 / KP;                              // rows per warp
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int k = lane & (KP - 1), rw = lane / KP;            // slot; row within the warp
+  const int r = (warp % KP) * RPW + rw;                     // row within the unit
+  const int row = unit * 32 + r;
+  const bool in = row < o.N && k < o.K;
+  int e = in ? o.idx[(size_t)row * o.K + k] : -1;
+  if (e < 0 || e >= o.E) e = -1;
+  int pos = 0;
+  if (e >= 0) {
+    pos = s_efo[e] + off(e) + __popc(mask(e) & ((1u << r) - 1u));
+    if (pos >= l.limit) e = -1;
+  }
+  const uint32_t ball = __ballot_sync(0xffffffffu, e >= 0);
+  if (lane == 0) s_warp[warp] = __popc(ball);
+  __syncthreads();
+  int tm_base = 0;
+  if (unit * 32 < o.N) {
+    if (!l.cut) tm_base = base();
+    else
+      for (int j = 0; j < o.E; ++j) tm_base += max(min(off(j), l.limit - s_efo[j]), 0);
+  }
+  for (int w = warp - warp % KP; w < warp; ++w) tm_base += s_warp[w];
+  const int row_base = tm_base + __popc(ball & ((1u << (rw * KP)) - 1u));        // rw * KP <= 31
+  const int cap = l.cut ? l.real_TK : o.TK_alloc;
+  if (row < o.N && k == 0) o.naept[row] = min(row_base, cap);
+  int rank = 0;
+  if (o.lane_order == 0) {
 #pragma unroll
-      for (int j = 0; j < KP; ++j) {
-        const int ej = __shfl_sync(0xffffffffu, e, rw * KP + j);
-        rank += (ej >= 0 && ej < e) ? 1 : 0;
-      }
-    } else {
-      rank = __popc(ball & ((1u << lane) - 1u)) - __popc(ball & ((1u << (rw * KP)) - 1u));
+    for (int j = 0; j < KP; ++j) {
+      const int ej = __shfl_sync(0xffffffffu, e, rw * KP + j);
+      rank += (ej >= 0 && ej < e) ? 1 : 0;
     }
-    if (e >= 0) {
-      const int tm = row_base + rank;
-      const bool kept = tm < cap;
-      x_gather[pos] = kept ? row : 0;
-      s_scatter[pos] = kept ? tm : real_TK;
-      if (kept) {
-        s_rev[tm] = pos;
-        src_idx[tm] = row * K + k;
-        if (tm < TKp_alloc) scores[tm] = probs[(size_t)row * K + k];
-      }
+  } else {
+    rank = __popc(ball & ((1u << lane) - 1u)) - __popc(ball & ((1u << (rw * KP)) - 1u));
+  }
+  if (e >= 0) {
+    const int tm = row_base + rank;
+    const bool kept = tm < cap;
+    o.x_gather[pos] = kept ? row : 0;
+    o.s_scatter[pos] = kept ? tm : l.real_TK;
+    if (kept) {
+      o.s_rev[tm] = pos;
+      o.src_idx[tm] = row * o.K + k;
+      if (tm < o.TKp_alloc) o.scores[tm] = o.probs[(size_t)row * o.K + k];
     }
   }
+}
 
-  // ---- pad rows and over-allocated tails ----
-  const int nthreads = gridDim.x * blockDim.x;
-  const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
-  for (int pos = gtid; pos < TKp_alloc; pos += nthreads) {
-    if (pos >= real_TKp) {
-      x_gather[pos] = 0;
-      s_scatter[pos] = pad_mode == 0 || cut ? real_TK : pos;   // virtual numbering continues through the tail
+// ---- pad rows and over-allocated tails ---- (thread gtid of nthreads)
+__device__ __forceinline__ void fill_pads(const TopkOut& o, const Layout& l, const int* s_efo, const int* s_base, int gtid,
+                                          int nthreads) {
+  for (int pos = gtid; pos < o.TKp_alloc; pos += nthreads) {
+    if (pos >= l.tot_p) {
+      o.x_gather[pos] = 0;
+      o.s_scatter[pos] = o.pad_mode == 0 || l.cut ? l.real_TK : pos;   // virtual numbering continues through the tail
       continue;
     }
-    if (pos >= limit) {                                 // cut off inside an alignment step
-      x_gather[pos] = 0;
-      s_scatter[pos] = real_TK;
+    if (pos >= l.limit) {                               // cut off inside an alignment step
+      o.x_gather[pos] = 0;
+      o.s_scatter[pos] = l.real_TK;
       continue;
     }
-    int lo = 0, hi = E;
+    int lo = 0, hi = o.E;
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
       if (s_efo[mid + 1] <= pos) lo = mid + 1; else hi = mid;
@@ -234,15 +248,138 @@ scatter_fill_kernel(const int* __restrict__ idx, const float* __restrict__ probs
     const int cnt = s_base[lo + 1] - s_base[lo];
     const int local = pos - s_efo[lo];
     if (local >= cnt) {
-      x_gather[pos] = 0;
-      s_scatter[pos] = pad_mode == 0 || cut ? real_TK : real_TK + (s_efo[lo] - s_base[lo]) + (local - cnt);
+      o.x_gather[pos] = 0;
+      o.s_scatter[pos] = o.pad_mode == 0 || l.cut ? l.real_TK : l.real_TK + (s_efo[lo] - s_base[lo]) + (local - cnt);
     }
   }
-  for (int i = real_TK + gtid; i < TKp_alloc; i += nthreads) scores[i] = 0.f;
-  for (int i = real_TK + gtid; i < TK_alloc; i += nthreads) {
-    s_rev[i] = 0;
-    src_idx[i] = 0;
+  for (int i = l.real_TK + gtid; i < o.TKp_alloc; i += nthreads) o.scores[i] = 0.f;
+  for (int i = l.real_TK + gtid; i < o.TK_alloc; i += nthreads) {
+    o.s_rev[i] = 0;
+    o.src_idx[i] = 0;
   }
+}
+
+template <int KP>
+__global__ void __launch_bounds__(KP > 8 ? 32 * KP : 256)
+scatter_fill_kernel(const TopkOut o, const uint32_t* __restrict__ mask, const int* __restrict__ unit_off,
+                    const int* __restrict__ unit_base, int scatter_blocks) {
+  extern __shared__ int s_mem[];
+  int* s_efo = s_mem;                // [E+1] padded offsets
+  int* s_base = s_mem + (o.E + 1);   // [E+1] unpadded offsets
+  int* s_warp = s_base + (o.E + 1);  // [33]
+  const int* counts = o.counts;
+  const Layout l = block_layout(o, [&](int e) { return counts[e]; }, s_efo, s_base, s_warp, blockIdx.x == 0);
+  if ((int)blockIdx.x < scatter_blocks) {
+    const int unit = blockIdx.x * ((int)blockDim.x / (32 * KP)) + (threadIdx.x >> 5) / KP;
+    scatter_unit<KP>(
+        o, l, s_efo, s_warp, unit, [&](int e) { return mask[(size_t)unit * o.E + e]; },
+        [&](int e) { return unit_off[(size_t)unit * o.E + e]; }, [&]() { return unit_base[unit]; });
+  }
+  fill_pads(o, l, s_efo, s_base, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+// ---------------------------------------------------------------------------
+// The same metadata from one cluster of CTAs, for problems small enough that three launches and the gaps between them cost more
+// than the work: masks and counts stay in shared memory, each CTA takes a run of units, and what the CTAs before it hold of an
+// expert is read out of their shared memory.  Between two events, launches included: 64 rows x 8 over 128 experts 17.4 -> 13.8
+// us, 1024 x 8 over 8 experts 18.5 -> 14.3; from 2048 x 8 on the scatter wants more than eight SMs (17.4 -> 19.4).
+constexpr int kMetaCluster = 8, kMetaThreads = 512;
+constexpr int kMetaEntries = 8192;                   // rows x slots up to which it is taken
+constexpr size_t kMetaSmem = 48 * 1024;
+
+__host__ __device__ inline size_t meta_cluster_smem(int units, int E) {
+  const int upc = (units + kMetaCluster - 1) / kMetaCluster;
+  return sizeof(int) * ((size_t)upc * E * 2 + upc + 1 + 3 * (size_t)E + 2 * (E + 1) + 33);
+}
+
+__device__ __forceinline__ int ld_cluster(const int* p, int rank) {
+  uint32_t a, v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return (int)v;
+}
+
+template <int KP>
+__global__ void __cluster_dims__(kMetaCluster, 1, 1) __launch_bounds__(kMetaThreads)
+metadata_cluster_kernel(const TopkOut o) {
+  extern __shared__ int s_mem[];
+  const int E = o.E, K = o.K, tid = threadIdx.x, rank = blockIdx.x;
+  const int units = (o.N + 31) / 32, upc = (units + kMetaCluster - 1) / kMetaCluster;
+  const int u0 = min(rank * upc, units), nu = min(upc, units - u0);
+  uint32_t* s_mask = reinterpret_cast<uint32_t*>(s_mem);     // [upc][E]
+  int* s_off = s_mem + (size_t)upc * E;                      // [upc][E] rows of e in this CTA's units before
+  int* s_valid = s_off + (size_t)upc * E;                    // [upc + 1] entries of a unit, then of the units before it
+  int* s_cnt = s_valid + upc + 1;                            // [E] rows of e in this CTA's units (read by the others)
+  int* s_tot = s_cnt + E;                                    // [E] rows of e
+  int* s_first = s_tot + E;                                  // [E] rows of e in the CTAs before
+  int* s_efo = s_first + E;
+  int* s_base = s_efo + (E + 1);
+  int* s_warp = s_base + (E + 1);
+
+  for (int i = tid; i < nu * E; i += kMetaThreads) s_mask[i] = 0u;
+  for (int i = tid; i <= upc; i += kMetaThreads) s_valid[i] = 0;
+  __syncthreads();
+  const int row0 = u0 * 32, n_in = max(min(o.N - row0, nu * 32), 0) * K;
+  for (int i = tid; i < n_in; i += kMetaThreads) {
+    const int e = o.idx[(size_t)row0 * K + i], r = i / K;
+    if (e >= 0 && e < E) {
+      atomicOr(&s_mask[(r >> 5) * E + e], 1u << (r & 31));
+      atomicAdd(&s_valid[r >> 5], 1);                        // whole numbers: the order does not matter
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < E; e += kMetaThreads) {
+    int run = 0;
+    for (int u = 0; u < nu; ++u) {
+      s_off[u * E + e] = run;
+      run += __popc(s_mask[u * E + e]);
+    }
+    s_cnt[e] = run;
+  }
+  if (tid == kMetaThreads - 1) {
+    int run = 0;
+    for (int u = 0; u <= upc; ++u) {
+      const int v = s_valid[u];
+      s_valid[u] = run;
+      run += v;
+    }
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  for (int e = tid; e < E; e += kMetaThreads) {
+    int v[kMetaCluster], tot = 0, before = 0;
+#pragma unroll
+    for (int q = 0; q < kMetaCluster; ++q) v[q] = ld_cluster(s_cnt + e, q);
+#pragma unroll
+    for (int q = 0; q < kMetaCluster; ++q) {
+      if (q < rank) before += v[q];
+      tot += v[q];
+    }
+    s_tot[e] = tot;
+    s_first[e] = before;
+    if (rank == 0) o.counts[e] = tot;
+  }
+  int entries = 0, all_entries = 0;                          // of the CTAs before, of all
+#pragma unroll
+  for (int q = 0; q < kMetaCluster; ++q) {
+    const int v = ld_cluster(s_valid + upc, q);
+    if (q < rank) entries += v;
+    all_entries += v;
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // this CTA has read the others' shared memory
+  if (rank == 0 && tid == 0) o.naept[o.N] = min(all_entries, o.TK_alloc);    // (a cut pass writes it again, below)
+  __syncthreads();
+  const Layout l = block_layout(o, [&](int e) { return s_tot[e]; }, s_efo, s_base, s_warp, rank == 0);
+  constexpr int UPB = kMetaThreads / (32 * KP);              // units of a pass over the block
+  for (int ub = 0; ub < nu; ub += UPB) {
+    const int lu = ub + (tid >> 5) / KP;
+    const int unit = lu < nu ? u0 + lu : units;              // `units`: no rows
+    scatter_unit<KP>(
+        o, l, s_efo, s_warp, unit, [&](int e) { return s_mask[lu * E + e]; },
+        [&](int e) { return s_first[e] + s_off[lu * E + e]; }, [&]() { return entries + s_valid[lu]; });
+    __syncthreads();                                         // s_warp is written again
+  }
+  fill_pads(o, l, s_efo, s_base, rank * kMetaThreads + tid, kMetaCluster * kMetaThreads);
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");        // nobody reads this CTA's shared memory any more
 }
 
 // ---------------------------------------------------------------------------
@@ -311,6 +448,19 @@ int smoe_topk_metadata(const int32_t* idx, const float* probs, int64_t N, int64_
   if (!workspace || !efo || !counts) return SMOE_ERR_ARG;
   TK_alloc = TK_alloc < 0 ? 0 : TK_alloc >= (int64_t)1 << 31 ? ((int64_t)1 << 31) - 1 : TK_alloc;
   const int units = (int)((N + 31) / 32);
+  TopkOut o{idx, probs, (int)N, (int)K, (int)E, (int)alignment, (int)TK_alloc, (int)TKp_alloc, lane_order, pad_mode, efo,
+            x_gather_idx, s_scatter_idx, s_reverse_scatter_idx, naept, topk_scores, score_src_idx, counts};
+  // slots a row, rounded up: a unit of 32 rows is that many warps of the scatter
+  const int kp = K <= 1 ? 1 : K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : 16;
+  if (N * K <= kMetaEntries && TKp_alloc <= 4 * kMetaEntries && meta_cluster_smem(units, (int)E) <= kMetaSmem) {
+    auto one = kp == 1   ? metadata_cluster_kernel<1>
+               : kp == 2 ? metadata_cluster_kernel<2>
+               : kp == 4 ? metadata_cluster_kernel<4>
+               : kp == 8 ? metadata_cluster_kernel<8>
+                         : metadata_cluster_kernel<16>;
+    one<<<kMetaCluster, kMetaThreads, meta_cluster_smem(units, (int)E), stream>>>(o);
+    return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  }
   uint32_t* mask = (uint32_t*)workspace;
   int* unit_off = (int*)(mask + (size_t)(units + 1) * E);
   int* unit_valid = unit_off + (size_t)(units + 1) * E;
@@ -320,8 +470,6 @@ int smoe_topk_metadata(const int32_t* idx, const float* probs, int64_t N, int64_
     unit_masks_kernel<<<ublocks, kRtThreads, 0, stream>>>(idx, (int)N, (int)K, (int)E, mask, unit_valid);
   scan_kernel<<<(int)E + 1, kRtThreads, 0, stream>>>(mask, unit_valid, units, (int)E, (int)N, (int)TK_alloc, unit_off,
                                                      counts, unit_base, naept);
-  // slots a row, rounded up: a unit of 32 rows is that many warps of the scatter
-  const int kp = K <= 1 ? 1 : K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : 16;
   const int threads = kp > 8 ? 32 * kp : kRtThreads, units_per_block = threads / (32 * kp);
   const int sblocks = (units + units_per_block - 1) / units_per_block;
   int fill_blocks = (int)((TKp_alloc + threads - 1) / threads);
@@ -334,10 +482,7 @@ int smoe_topk_metadata(const int32_t* idx, const float* probs, int64_t N, int64_
                       : kp == 4 ? scatter_fill_kernel<4>
                       : kp == 8 ? scatter_fill_kernel<8>
                                 : scatter_fill_kernel<16>;
-  scatter_fill<<<grid, threads, smem, stream>>>(
-      idx, probs, (int)N, (int)K, (int)E, (int)alignment, (int)TK_alloc, (int)TKp_alloc, lane_order, pad_mode, mask,
-      unit_off, unit_base, counts, efo, x_gather_idx, s_scatter_idx, s_reverse_scatter_idx, naept, topk_scores,
-      score_src_idx, sblocks);
+  scatter_fill<<<grid, threads, smem, stream>>>(o, mask, unit_off, unit_base, sblocks);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 

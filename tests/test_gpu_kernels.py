@@ -1056,3 +1056,19 @@ def test_gemm_wgrad_bf16_is_the_rounded_f32_product(ops, layout, M, N, tiles):
     ops.check_status(DEV)
     assert torch.equal(got, want.to(torch.bfloat16))
     assert all((got[e] == 0).all() for e in range(E) if tiles[e] == 0)
+
+
+# 8192 entries is where the single-cluster form ends; E = 1024 does not fit its shared memory, and one unit leaves seven of the
+# eight CTAs without rows
+@pytest.mark.parametrize("N,K,E", [(1024, 8, 128), (1025, 8, 128), (8192, 1, 8), (8193, 1, 8), (512, 16, 256), (513, 16, 16),
+                                   (2, 8, 8), (257, 5, 1024), (480, 8, 600)])
+@pytest.mark.parametrize("lane_order,pad_mode,short", [(0, 0, 0), (1, 1, 0), (0, 0, 1)])
+def test_topk_metadata_on_both_sides_of_the_one_cluster_form(ops, N, K, E, lane_order, pad_mode, short):
+    idx, probs = make_routing(N, K, E, 0.2, seed=N + E, skew=True)
+    real = int((idx >= 0).sum())
+    TK, TKp = (None, None) if not short else (real * 3 // 4, (real // 2 + 127) // 128 * 128)
+    got = ops.topk_metadata(idx.to(DEV), probs.to(DEV), E, 128, TK_alloc=TK, TKp_alloc=TKp, lane_order=lane_order, pad_mode=pad_mode)
+    ref = R.topk_metadata(idx, probs, E, 128, TK_alloc=got["TK_alloc"], TKp_alloc=got["TKp_alloc"],
+                          lane_order=["expert", "slot"][lane_order], pad_mode=["sentinel", "virtual"][pad_mode])
+    for k in MD_KEYS:
+        assert torch.equal(got[k].cpu(), ref[k]), k
