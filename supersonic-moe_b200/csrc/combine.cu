@@ -27,6 +27,8 @@ __device__ __forceinline__ uint32_t cvt_bf16x2(float lo, float hi) {
 // One block per token; a thread owns 8 consecutive columns (16-byte accesses).
 // Lanes of the token are added in ascending order.  Being the last kernel of a forward pass, it may also leave the status word
 // where the host looks for it (`host_word`, null: not): a kernel of its own for that one store costs a launch, 3 us and a gap.
+// ROWS: rows of a token whose loads are in flight together
+template <int ROWS>
 __global__ void __launch_bounds__(512)
 combine_kernel(const uint4* __restrict__ y, const int* __restrict__ s_rev, const int* __restrict__ naept,
                const float* __restrict__ scores, uint4* __restrict__ out, int H8, const int* __restrict__ status,
@@ -36,19 +38,22 @@ combine_kernel(const uint4* __restrict__ y, const int* __restrict__ s_rev, const
   const int beg = naept[t], end = naept[t + 1];
   for (int c = threadIdx.x; c < H8; c += blockDim.x) {
     float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    int j = beg;
-    for (; j + 4 <= end; j += 4) {
-      uint4 v[4];
-      float w[4];
+    for (int j = beg; j < end; j += ROWS) {
+      const int n = end - j;                 // rows of this batch that exist; the same for the whole block
+      uint4 v[ROWS];
+      float w[ROWS];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < ROWS; ++u) {
+        if (u >= n) break;
         v[u] = y[(int64_t)s_rev[j + u] * H8 + c];
         w[u] = scores ? scores[j + u] : 1.0f;
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) acc_bf16x8(v[u], w[u], a);
+      for (int u = 0; u < ROWS; ++u) {
+        if (u >= n) break;
+        acc_bf16x8(v[u], w[u], a);
+      }
     }
-    for (; j < end; ++j) acc_bf16x8(y[(int64_t)s_rev[j] * H8 + c], scores ? scores[j] : 1.0f, a);
     out[t * H8 + c] = make_uint4(cvt_bf16x2(a[0], a[1]), cvt_bf16x2(a[2], a[3]), cvt_bf16x2(a[4], a[5]),
                                  cvt_bf16x2(a[6], a[7]));
   }
@@ -300,8 +305,11 @@ int smoe_combine_post(const void* y_bf16, const int32_t* s_rev, const int32_t* n
   if (T == 0) return SMOE_OK;
   const int H8 = (int)(H / 8);
   const int threads = H8 >= 512 ? 512 : ((H8 + 31) / 32) * 32;
-  combine_kernel<<<(unsigned)T, threads, 0, (cudaStream_t)stream>>>((const uint4*)y_bf16, s_rev, naept, scores,
-                                                                    (uint4*)out_bf16, H8, status, pinned_host_word);
+  // A lone wave of blocks waits for its loads and asks for eight rows at once (64 tokens of 8 rows, H=2048: 11 us with four, 9
+  // with eight); with many blocks an SM the registers that takes cost more warps than it gains (T=8192, H=3072: 83 and 93 us)
+  auto kern = T <= 296 ? combine_kernel<8> : combine_kernel<4>;
+  kern<<<(unsigned)T, threads, 0, (cudaStream_t)stream>>>((const uint4*)y_bf16, s_rev, naept, scores, (uint4*)out_bf16, H8,
+                                                          status, pinned_host_word);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 

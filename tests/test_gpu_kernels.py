@@ -1072,3 +1072,23 @@ def test_topk_metadata_on_both_sides_of_the_one_cluster_form(ops, N, K, E, lane_
                           lane_order=["expert", "slot"][lane_order], pad_mode=["sentinel", "virtual"][pad_mode])
     for k in MD_KEYS:
         assert torch.equal(got[k].cpu(), ref[k]), k
+
+
+@pytest.mark.parametrize("T,K", [(1, 1), (7, 3), (296, 8), (297, 8), (300, 11)])
+def test_combine_batches_of_rows(ops, T, K):
+    """Four and eight rows of a token in flight, with remainders and tokens without rows: one fma chain in lane order."""
+    g = torch.Generator().manual_seed(T + K)
+    n = torch.randint(0, K + 1, (T,), generator=g)
+    naept = torch.zeros(T + 1, dtype=torch.int32)
+    naept[1:] = torch.cumsum(n, 0)
+    total, H = int(naept[-1]), 264
+    y = torch.randn(total + 1, H, generator=g).to(torch.bfloat16)
+    s_rev = torch.randperm(total + 1, generator=g)[:max(total, 1)].to(torch.int32)
+    scores = torch.rand(max(total, 1), generator=g)
+    for w in (scores, None):
+        got = ops.combine(y.to(DEV), s_rev.to(DEV), naept.to(DEV), None if w is None else w.to(DEV), T).cpu()
+        for t in range(T):
+            acc = torch.zeros(H, dtype=torch.float64)
+            for j in range(int(naept[t]), int(naept[t + 1])):      # fma: the product is exact, the sum rounded to f32
+                acc = (acc + (1.0 if w is None else float(w[j])) * y[int(s_rev[j])].double()).float().double()
+            assert torch.equal(got[t], acc.float().to(torch.bfloat16)), t
