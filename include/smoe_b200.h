@@ -279,6 +279,15 @@ int smoe_gemm_gated_infer(const void* x_sorted_fp8, const void* a_sf, const void
                           const int* s_scatter_idx, const int* real_tk, void* y1_fp8, void* y1_sf, int64_t rows, int64_t N,
                           int64_t K, int64_t E, int* status, void* stream);
 
+/* The two forward GEMMs made for few rows per expert (any counts are computed right).  The first counts[e] rows of expert e's segment are computed and written, the others may hold anything
+ * and stay as they are.  E <= 256; scales 16-byte aligned. */
+int smoe_gemm_gated_few(const void* x_sorted_fp8, const void* a_sf, const void* w1_fp8, const void* w1_sf, const int* efo,
+                        const int* counts, void* y1_fp8, void* y1_sf, int64_t rows, int64_t N, int64_t K, int64_t E,
+                        int* status, void* stream);
+int smoe_gemm_varlen_m_few(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,
+                           const int* counts, void* c_bf16, int64_t rows, int64_t N, int64_t K, int64_t E,
+                           int* status, void* stream);
+
 /* Backward of the activation: D = dout[a_idx] . W2T[e]^T (N = I, K = H) and, against the saved e4m3 z,
  * dz (bf16 [rows,2N]), y1s = s*y (bf16 [rows,N]) and per-column-tile partial sums of ds ([partials, rows] f32).
  * Replaces gemm_dgated (sonicmoe/quack_utils/sm100_funcs.py:824-885, _gated_epilogues.py:2772-3000). */

@@ -8,6 +8,7 @@
 #include "gemm.cuh"
 #include "gemm2.cuh"
 #include "gemm3.cuh"
+#include "gemm_few.cuh"
 #include "smoe_b200.h"
 #include "smoe_internal.h"
 
@@ -359,6 +360,33 @@ static int run(const void* a, int64_t a_rows, int64_t a_cols, const void* b, int
   return launch<128, M1>(ta, tb, p, max_tiles_128, stream);
 }
 
+// ---- few rows per expert: weights as the M operand -------------------------------------------------------------------
+template <int MODE>
+static int run_few(const void* x, const void* w, int64_t rows, const FewParams& p, cudaStream_t stream) {
+  using S = FewSmem;
+  static bool attr_set[kMaxDevices] = {};
+  auto kern = gemm_few_kernel<MODE>;
+  if (!ensure_smem_attr(kern, S::TOTAL, attr_set)) return SMOE_ERR_LAUNCH;
+  CUtensorMap tw, tx;
+  int rc = make_tmap_u8(&tw, w, (uint64_t)p.E * p.N, p.K, BK, BM);
+  if (!rc) rc = make_tmap_u8(&tx, x, rows, p.K, BK, 16);
+  if (rc) return rc;
+  const int64_t tiles = (rows / kFewNT) * (p.N / BM);      // an upper bound
+  const int grid = tiles < sm_count() ? (int)tiles : sm_count();
+  kern<<<grid, kFewThreads, S::TOTAL, stream>>>(tw, tx, p);
+  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+}
+
+static int check_few(const void* x, const void* w, const void* x_sf, const void* w_sf, const int* efo, const int* counts,
+                     int64_t rows, int64_t N, int64_t K, int64_t E) {
+  if (rows < 0 || rows % 128 || rows >= (int64_t)1 << 31 || N <= 0 || N % 128 || K <= 0 || K % 128 || E <= 0 ||
+      E > kMaxExperts2)
+    return SMOE_ERR_SHAPE;
+  if (rows > 0 && (!x || !w || !x_sf || !w_sf || !efo || !counts)) return SMOE_ERR_ARG;
+  if (((uintptr_t)x_sf | (uintptr_t)w_sf) & 15) return SMOE_ERR_ALIGN;
+  return SMOE_OK;
+}
+
 // A weight-gradient call over zero routed rows: the product is empty, so an accumulating call leaves c as it is and
 // an overwriting call stores zeros.
 static int wgrad_nothing_routed(float* c, int64_t M, int64_t N, int64_t E, int accumulate, cudaStream_t stream) {
@@ -450,6 +478,31 @@ int smoe_gemm_gated_infer(const void* x_sorted_fp8, const void* a_sf, const void
   p.y1_fp8 = (uint8_t*)y1_fp8; p.y1_sf = (uint8_t*)y1_sf; p.s_scatter = s_scatter_idx; p.real_tk = real_tk;
   p.status = status; p.debug_skip_store = g_skip_store;
   return run<GATED>(x_sorted_fp8, rows, K, w1_fp8, E * N, K, p, (int)((rows / 128) * (N / 128)), (cudaStream_t)stream);
+}
+
+int smoe_gemm_gated_few(const void* x_sorted_fp8, const void* a_sf, const void* w1_fp8, const void* w1_sf, const int* efo,
+                        const int* counts, void* y1_fp8, void* y1_sf, int64_t rows, int64_t N, int64_t K, int64_t E,
+                        int* status, void* stream) {
+  const int rc = check_few(x_sorted_fp8, w1_fp8, a_sf, w1_sf, efo, counts, rows, N, K, E);
+  if (rc) return rc;
+  if (N % 256) return SMOE_ERR_SHAPE;
+  if (rows == 0) return SMOE_OK;
+  if (!y1_fp8 || !y1_sf) return SMOE_ERR_ARG;
+  FewParams p{(int)N, (int)K, (int)E, efo, counts, (const uint8_t*)w1_sf, (const uint8_t*)a_sf, nullptr, (uint8_t*)y1_fp8,
+              (uint8_t*)y1_sf, status};
+  return run_few<GATED>(x_sorted_fp8, w1_fp8, rows, p, (cudaStream_t)stream);
+}
+
+int smoe_gemm_varlen_m_few(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,
+                           const int* counts, void* c_bf16, int64_t rows, int64_t N, int64_t K, int64_t E,
+                           int* status, void* stream) {
+  const int rc = check_few(a_fp8, b_fp8, a_sf, b_sf, efo, counts, rows, N, K, E);
+  if (rc) return rc;
+  if (rows == 0) return SMOE_OK;
+  if (!c_bf16) return SMOE_ERR_ARG;
+  FewParams p{(int)N, (int)K, (int)E, efo, counts, (const uint8_t*)b_sf, (const uint8_t*)a_sf, (__nv_bfloat16*)c_bf16,
+              nullptr, nullptr, status};
+  return run_few<PLAIN>(a_fp8, b_fp8, rows, p, (cudaStream_t)stream);
 }
 
 int64_t smoe_gemm_dgated_partials(int64_t N);

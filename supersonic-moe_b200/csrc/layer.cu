@@ -157,6 +157,13 @@ static int wgrad(const void* A, const void* A_sf, bool a_rows, const void* B, co
   return smoe_gemm_wgrad(A, A_sf, B, B_sf, efo, (float*)c, M, N, rows, E, acc, status, stream);
 }
 
+// Whether an inference call has so few rows per expert (of an even spread, and at most T: a token takes an expert once) that
+// reading the weights bounds its GEMMs.  Gated + plain GEMM, routed rows as M against weights as M, us:
+//   E=128 H=2048 I=768, K=8:  4 rows 147 / 115, 32 rows 152 / 133, 48 rows 152 / 150, 64 rows 152 / 215
+//   E=32 H=3072 I=1536, K=8:  8 rows 115 / 93, 40 rows 115 / 106, 50 rows 115 / 120
+//   E=K=8 H=I=4096:           1 row 100 / 84, 32 rows 100 / 91, 64 rows 101 / 105
+static bool few_rows(const smoe_layer_args& a) { return a.T <= 40 || a.T * a.K <= 40 * a.E; }
+
 }  // namespace smoe
 
 using namespace smoe;
@@ -181,14 +188,20 @@ int smoe_layer_forward(const smoe_layer_args* args, void* stream) {
                               sv.s_scatter, sv.s_rev, sv.naept, sv.scores, sv.src_idx, a.counts, sc.ws, stream));
   SMOE_TRY(smoe_quant_rows_scatter(a.x, a.T, H, sv.naept, sv.s_rev, a.keep_z ? sv.s_scatter : nullptr, rows, R, sc.xg,
                                    sc.xg_sf, stream));
-  if (a.keep_z)
-    SMOE_TRY(smoe_gemm_gated(sc.xg, R, nullptr, sc.xg_sf, a.w1, a.w1_sf, sv.efo, sv.z, sv.z_sc, sc.y1, sc.y1_sf, R, 2 * I, H,
-                             E, a.status, stream));
-  else
-    SMOE_TRY(smoe_gemm_gated_infer(sc.xg, sc.xg_sf, a.w1, a.w1_sf, sv.efo, sv.s_scatter, real_tk, sc.y1, sc.y1_sf, R, 2 * I,
-                                   H, E, a.status, stream));
-  SMOE_TRY(smoe_gemm_varlen_m_live(sc.y1, sc.y1_sf, a.w2, a.w2_sf, sv.efo, sv.s_scatter, real_tk, sc.y2, R, H, I, E, a.status,
-                                   stream));
+  if (!a.keep_z && few_rows(a)) {
+    SMOE_TRY(smoe_gemm_gated_few(sc.xg, sc.xg_sf, a.w1, a.w1_sf, sv.efo, a.counts, sc.y1, sc.y1_sf, R, 2 * I, H, E, a.status,
+                                 stream));
+    SMOE_TRY(smoe_gemm_varlen_m_few(sc.y1, sc.y1_sf, a.w2, a.w2_sf, sv.efo, a.counts, sc.y2, R, H, I, E, a.status, stream));
+  } else {
+    if (a.keep_z)
+      SMOE_TRY(smoe_gemm_gated(sc.xg, R, nullptr, sc.xg_sf, a.w1, a.w1_sf, sv.efo, sv.z, sv.z_sc, sc.y1, sc.y1_sf, R, 2 * I, H,
+                               E, a.status, stream));
+    else
+      SMOE_TRY(smoe_gemm_gated_infer(sc.xg, sc.xg_sf, a.w1, a.w1_sf, sv.efo, sv.s_scatter, real_tk, sc.y1, sc.y1_sf, R, 2 * I,
+                                     H, E, a.status, stream));
+    SMOE_TRY(smoe_gemm_varlen_m_live(sc.y1, sc.y1_sf, a.w2, a.w2_sf, sv.efo, sv.s_scatter, real_tk, sc.y2, R, H, I, E,
+                                     a.status, stream));
+  }
   int32_t* word;
   SMOE_TRY(host_word(a, stream, &word));
   return smoe_combine_post(sc.y2, sv.s_rev, sv.naept, sv.scores, a.out, a.T, H, a.status, word, stream);

@@ -54,6 +54,8 @@ SIGNATURES = {
     "smoe_gemm_varlen_m": (_I, [_P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _P, _P]),
     "smoe_gemm_varlen_m_live": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _P, _P]),
     "smoe_gemm_gated_infer": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _P, _P]),
+    "smoe_gemm_gated_few": (_I, [_P] * 8 + [_L] * 4 + [_P, _P]),
+    "smoe_gemm_varlen_m_few": (_I, [_P] * 7 + [_L] * 4 + [_P, _P]),
     "smoe_gemm_varlen_m_bt": (_I, [_P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _P, _P]),
     "smoe_transpose_u8": (_I, [_P, _L, _L, _L, _P, _P]),
     "smoe_gemm_gated": (_I, [_P, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _P, _P]),

@@ -1092,3 +1092,60 @@ def test_combine_batches_of_rows(ops, T, K):
             for j in range(int(naept[t]), int(naept[t + 1])):      # fma: the product is exact, the sum rounded to f32
                 acc = (acc + (1.0 if w is None else float(w[j])) * y[int(s_rev[j])].double()).float().double()
             assert torch.equal(got[t], acc.float().to(torch.bfloat16)), t
+
+
+@pytest.mark.parametrize("counts,H,I", [([4, 0, 1, 9], 256, 128), ([64, 65, 16, 17, 0, 128], 512, 256), ([0, 0, 300], 128, 384),
+                                        ([31] * 40, 1152, 128)])
+def test_forward_gemms_for_few_rows_match_the_general_kernels(ops, counts, H, I):
+    """Weights as the M operand against routed rows as the M operand: the live rows of both forward GEMMs, with anything in the
+    others (the general kernels read them too, and keep them apart)."""
+    from sonicmoe._lib import check, lib
+    g = torch.Generator().manual_seed(sum(counts))
+    E = len(counts)
+    efo = torch.zeros(E + 1, dtype=torch.int32)
+    efo[1:] = torch.cumsum(torch.tensor([-(-c // 128) * 128 for c in counts]), 0)
+    rows = int(efo[-1]) + 128
+    live = torch.cat([torch.arange(int(efo[e]), int(efo[e]) + c) for e, c in enumerate(counts)])
+    xq = torch.randint(0, 256, (rows, H), generator=g, dtype=torch.uint8)
+    xs = torch.randint(0, 256, (rows, H // 32), generator=g, dtype=torch.uint8)
+    lq, ls = rand_fp8((len(live), H), g)
+    xq[live], xs[live] = lq, ls
+    (w1, w1s), (w2, w2s) = rand_fp8((E, 2 * I, H), g), rand_fp8((E, H, I), g)
+    d = lambda t: t.contiguous().to(DEV)
+    xq, xsf, w1, w2 = d(xq), d(Q.pack_isa(xs, rows, H)), d(w1), d(w2)
+    w1sf = d(Q.pack_isa(w1s.reshape(E * 2 * I, H // 32), E * 2 * I, H))
+    w2sf = d(Q.pack_isa(w2s.reshape(E * H, I // 32), E * H, I))
+    efo_d, cnt, real = d(efo), d(torch.tensor(counts, dtype=torch.int32)), d(torch.tensor([len(live)], dtype=torch.int32))
+    s_scatter = torch.full((rows,), len(live), dtype=torch.int32)
+    s_scatter[live] = torch.arange(len(live), dtype=torch.int32)
+    s_scatter, st, P = d(s_scatter), torch.cuda.current_stream().cuda_stream, lambda t: t.data_ptr()
+    status = ops.status_word(DEV)
+    out = []
+    for few in (False, True):
+        y = torch.full((rows, I), 0xAA, dtype=torch.uint8, device=DEV)
+        ysf = torch.full((ops.isa_bytes(rows, I),), 0xAA, dtype=torch.uint8, device=DEV)
+        c = torch.full((rows, H), float("nan"), dtype=torch.bfloat16, device=DEV)
+        if few:
+            check(lib.smoe_gemm_gated_few(P(xq), P(xsf), P(w1), P(w1sf), P(efo_d), P(cnt), P(y), P(ysf), rows, 2 * I, H, E,
+                                          P(status), st), "gated_few")
+            check(lib.smoe_gemm_varlen_m_few(P(y), P(ysf), P(w2), P(w2sf), P(efo_d), P(cnt), P(c), rows, H, I, E, P(status),
+                                             st), "varlen_m_few")
+            dead = torch.ones(rows, dtype=torch.bool)
+            dead[live] = False
+            assert (y.cpu()[dead] == 0xAA).all() and torch.isnan(c.cpu()[dead]).all()        # left as they were
+        else:
+            check(lib.smoe_gemm_gated_infer(P(xq), P(xsf), P(w1), P(w1sf), P(efo_d), P(s_scatter), P(real), P(y), P(ysf), rows,
+                                            2 * I, H, E, P(status), st), "gated_infer")
+            check(lib.smoe_gemm_varlen_m_live(P(y), P(ysf), P(w2), P(w2sf), P(efo_d), P(s_scatter), P(real), P(c), rows, H, I,
+                                              E, P(status), st), "varlen_m_live")
+        torch.cuda.synchronize()
+        ops.check_status(DEV)
+        out.append((y.cpu()[live], Q.unpack_isa(ysf.cpu(), rows, I)[live], c.cpu()[live].float()))
+    (y0, s0, c0), (y1, s1, c1) = out
+    # the tensor core adds the products of a K step in an order of its own, so a value next to a rounding boundary may move
+    same = s0 == s1
+    assert (~same).float().mean() < 2e-3
+    assert (y0 != y1)[same.repeat_interleave(32, 1)].float().mean() < 2e-3
+    assert torch.isfinite(c1).all()
+    cos, rr = stats(c1, c0)
+    assert cos > 0.9999 and rr < 4e-3, (cos, rr)
