@@ -309,6 +309,12 @@ int smoe_gemm_dgated_fused(const void* dout_fp8, const void* a_sf, const void* w
                            const int32_t* efo, const void* z_fp8, const void* z_scales, const float* s, void* dz_q,
                            void* dz_row_sf, void* dz_col_sf, void* y1s_q, void* y1s_col_sf, float* ds_partial,
                            int64_t rows, int64_t N, int64_t K, int64_t E, int32_t* status, void* stream);
+/* The same, row p's score read as scores[s_scatter_idx[p]] (what smoe_gather_scores would put into s[p]). */
+int smoe_gemm_dgated_fused_scored(const void* dout_fp8, const void* a_sf, const void* w2t_fp8, const void* w2t_sf,
+                                  const int32_t* efo, const void* z_fp8, const void* z_scales, const float* scores,
+                                  const int32_t* s_scatter_idx, void* dz_q, void* dz_row_sf, void* dz_col_sf, void* y1s_q,
+                                  void* y1s_col_sf, float* ds_partial, int64_t rows, int64_t N, int64_t K, int64_t E,
+                                  int32_t* status, void* stream);
 int64_t smoe_gemm_dgated_fused_partials(int64_t N);
 
 /* The same with the A rows fetched by index inside the kernel: dout_fp8 is the un-gathered [T,K] e4m3 gradient, row p
@@ -395,6 +401,11 @@ int smoe_gather_scores(const float* scores, const int32_t* s_scatter_idx, int64_
  * sonicmoe/functional/__init__.py:2384 and the ds scatter of :2488-2500. */
 int smoe_ds_finalize(const float* ds_partial, int64_t partials, int64_t rows, const int32_t* s_rev, int64_t TK,
                      const int32_t* real_tk, float* ds_tm, const int32_t* src_idx, float* scatter_out, void* stream);
+/* The same sums in the layout of the top-k table: ds f32 [T,K], 0 where a slot has no entry.  naept and src_idx as
+ * smoe_topk_metadata leaves them. */
+int smoe_ds_slots(const float* ds_partial, int64_t partials, int64_t rows, const int32_t* s_rev, const int32_t* naept,
+                  const int32_t* src_idx, int64_t T, int64_t K, float* ds, void* stream);
+
 
 /* *pinned_host_word = *status, written by a one-thread kernel on `stream`: `status` is the device word the GEMM entry
  * points report failures in, `pinned_host_word` page-locked host memory the device can address (cudaHostAlloc /

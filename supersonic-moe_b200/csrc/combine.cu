@@ -82,6 +82,24 @@ __global__ void ds_finalize_kernel(const float* __restrict__ part, int partials,
   if (ds) ds[i] = a;
 }
 
+// The same sums, written to the token's slots: a thread per (token, slot) looks for its entry among the token's, so that slots
+// without one (masked) get their zero here and not from a memset before.
+__global__ void ds_slots_kernel(const float* __restrict__ part, int partials, int64_t rows, const int* __restrict__ s_rev,
+                                const int* __restrict__ naept, const int* __restrict__ src_idx, int64_t slots, int K,
+                                float* __restrict__ ds) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= slots) return;
+  const int64_t t = i / K;
+  float a = 0.f;
+  for (int j = naept[t], end = naept[t + 1]; j < end; ++j) {
+    if (src_idx[j] != (int)i) continue;
+    const int64_t p = s_rev[j];
+    for (int q = 0; q < partials; ++q) a += part[(int64_t)q * rows + p];
+    break;
+  }
+  ds[i] = a;
+}
+
 // One warp per row: K rounds of arg-max (lowest index wins ties), then softmax
 // over the K selected logits in fp32.  A NaN logit counts as -inf.  A row with
 // fewer than K finite logits still gets K distinct, in-range indices: once the
@@ -331,6 +349,16 @@ int smoe_ds_finalize(const float* ds_partial, int64_t partials, int64_t rows, co
   if (scatter_out && !src_idx) return SMOE_ERR_ARG;
   ds_finalize_kernel<<<(unsigned)((TK + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
       ds_partial, (int)partials, rows, s_rev, TK, real_tk, ds_tm, src_idx, scatter_out);
+  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+}
+
+int smoe_ds_slots(const float* ds_partial, int64_t partials, int64_t rows, const int32_t* s_rev, const int32_t* naept,
+                  const int32_t* src_idx, int64_t T, int64_t K, float* ds, void* stream) {
+  if (T < 0 || K <= 0 || partials < 0 || T * K >= (int64_t)1 << 31) return SMOE_ERR_SHAPE;
+  if (T == 0) return SMOE_OK;
+  if (!naept || !ds || (rows > 0 && (!ds_partial || !s_rev || !src_idx))) return SMOE_ERR_ARG;      // no rows: all slots 0
+  ds_slots_kernel<<<(unsigned)((T * K + 255) / 256), 256, 0, (cudaStream_t)stream>>>(ds_partial, (int)partials, rows, s_rev,
+                                                                                  naept, src_idx, T * K, (int)K, ds);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 

@@ -526,8 +526,8 @@ int smoe_gemm_dgated(const void* dout_fp8, int64_t T, const int* a_idx, const vo
 
 static int dgated_fused_impl(const void* dout_fp8, int64_t a_rows, const int* a_idx, const void* a_sf,
                              const void* w2t_fp8, const void* w2t_sf, const int* efo, const void* z_fp8,
-                             const void* z_scales, const float* s, void* dz_q, void* dz_row_sf, void* dz_col_sf,
-                             void* y1s_q, void* y1s_col_sf, float* ds_partial, int64_t rows, int64_t N, int64_t K,
+                             const void* z_scales, const float* s, const int* s_idx, void* dz_q, void* dz_row_sf,
+                             void* dz_col_sf, void* y1s_q, void* y1s_col_sf, float* ds_partial, int64_t rows, int64_t N, int64_t K,
                              int64_t E, int* status, void* stream) {
   if (rows < 0 || rows % 128 || N % 128 || K % 128 || E <= 0) return SMOE_ERR_SHAPE;
   if (rows == 0) return SMOE_OK;
@@ -536,7 +536,7 @@ static int dgated_fused_impl(const void* dout_fp8, int64_t a_rows, const int* a_
   p.efo = efo; p.a_idx = a_idx; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)w2t_sf;
   p.sfa_ktiles = (int)(K / 128); p.sfb_ktiles = (int)(K / 128);
   p.z_fp8 = (uint8_t*)const_cast<void*>(z_fp8); p.z_sc = (uint8_t*)const_cast<void*>(z_scales);
-  p.s = s; p.dz = dz_q; p.y1s = y1s_q; p.ds_partial = ds_partial; p.status = status;
+  p.s = s; p.s_scatter = s_idx; p.dz = dz_q; p.y1s = y1s_q; p.ds_partial = ds_partial; p.status = status;
   p.dz_row_sf = (uint8_t*)dz_row_sf; p.dz_col_sf = (uint8_t*)dz_col_sf; p.y1s_col_sf = (uint8_t*)y1s_col_sf;
   p.debug_skip_store = g_skip_store;
   return run<DGATEDQ>(dout_fp8, a_rows, K, w2t_fp8, E * N, K, p, (int)((rows / 128) * (N / 128)),
@@ -547,7 +547,7 @@ int smoe_gemm_dgated_fused(const void* dout_fp8, const void* a_sf, const void* w
                            const int* efo, const void* z_fp8, const void* z_scales, const float* s, void* dz_q,
                            void* dz_row_sf, void* dz_col_sf, void* y1s_q, void* y1s_col_sf, float* ds_partial,
                            int64_t rows, int64_t N, int64_t K, int64_t E, int* status, void* stream) {
-  return dgated_fused_impl(dout_fp8, rows, nullptr, a_sf, w2t_fp8, w2t_sf, efo, z_fp8, z_scales, s, dz_q, dz_row_sf,
+  return dgated_fused_impl(dout_fp8, rows, nullptr, a_sf, w2t_fp8, w2t_sf, efo, z_fp8, z_scales, s, nullptr, dz_q, dz_row_sf,
                            dz_col_sf, y1s_q, y1s_col_sf, ds_partial, rows, N, K, E, status, stream);
 }
 
@@ -557,8 +557,18 @@ int smoe_gemm_dgated_fused_gather(const void* dout_fp8, int64_t T, const int* a_
                                   void* y1s_q, void* y1s_col_sf, float* ds_partial, int64_t rows, int64_t N,
                                   int64_t K, int64_t E, int* status, void* stream) {
   if (rows > 0 && (T <= 0 || a_idx == nullptr)) return SMOE_ERR_ARG;
-  return dgated_fused_impl(dout_fp8, T, a_idx, a_sf, w2t_fp8, w2t_sf, efo, z_fp8, z_scales, s, dz_q, dz_row_sf,
+  return dgated_fused_impl(dout_fp8, T, a_idx, a_sf, w2t_fp8, w2t_sf, efo, z_fp8, z_scales, s, nullptr, dz_q, dz_row_sf,
                            dz_col_sf, y1s_q, y1s_col_sf, ds_partial, rows, N, K, E, status, stream);
+}
+
+int smoe_gemm_dgated_fused_scored(const void* dout_fp8, const void* a_sf, const void* w2t_fp8, const void* w2t_sf,
+                                  const int* efo, const void* z_fp8, const void* z_scales, const float* scores,
+                                  const int* s_scatter_idx, void* dz_q, void* dz_row_sf, void* dz_col_sf, void* y1s_q,
+                                  void* y1s_col_sf, float* ds_partial, int64_t rows, int64_t N, int64_t K, int64_t E,
+                                  int* status, void* stream) {
+  if (rows > 0 && s_scatter_idx == nullptr) return SMOE_ERR_ARG;
+  return dgated_fused_impl(dout_fp8, rows, nullptr, a_sf, w2t_fp8, w2t_sf, efo, z_fp8, z_scales, scores, s_scatter_idx, dz_q,
+                           dz_row_sf, dz_col_sf, y1s_q, y1s_col_sf, ds_partial, rows, N, K, E, status, stream);
 }
 
 int64_t smoe_gemm_dgated_fused_partials(int64_t N) {

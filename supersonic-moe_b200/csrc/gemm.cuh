@@ -58,7 +58,8 @@ struct GemmParams {
   uint8_t* y1s_col_sf;  // DGATEDQ out: ISA scales of y1s^T as a (N, TKp) operand (1x32 along TKp)
   int* status;          // device status word: 0 ok, else first failure code
   const int* s_scatter; // PLAIN / GATED, may be null: row r is padding where s_scatter[r] >= *real_tk; 32-row slabs of
-  const int* real_tk;   // nothing but padding are then not stored (the two-CTA kernels)
+  const int* real_tk;   // nothing but padding are then not stored (the two-CTA kernels).  DGATEDQ, if not null: row r's
+                        // score is s[s_scatter[r]]
   int stages_lent;      // two-CTA WGRAD into an existing f32 gradient: ring stages that hold its staging tiles instead
   int debug_skip_store; // timing experiments only: drain TMEM but skip the global stores
   int dbg_stage_cut;    // timing experiments only: use this many fewer ring stages

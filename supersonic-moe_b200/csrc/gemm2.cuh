@@ -726,7 +726,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
         for (int i = 0; i < 4; ++i) zb[i] = reinterpret_cast<const uint4*>(zrow)[i];
         sc = *reinterpret_cast<const uint16_t*>(p.z_sc + grow * (Nz / 32) + (2 * c_base) / 32);
-        s_row = p.s[grow];
+        s_row = p.s[p.s_scatter != nullptr ? p.s_scatter[grow] : (int)grow];
       }
       const bool live = (MODE == PLAIN || MODE == GATED) && slab_live(p, t, t.m0 + q * 32);
       if (lane == 0) ok = mbar_wait(bar_tfull + 8 * as, aphase);

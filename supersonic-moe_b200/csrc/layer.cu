@@ -87,7 +87,7 @@ struct BwdScratch {
     const int64_t R = a.TKp_alloc, H = a.H, I = a.I;
     fused = mn_ok(a.E, I, H);
     parts = fused ? smoe_gemm_dgated_fused_partials(I) : smoe_gemm_dgated_partials(I);
-    s = m.take<float>(R);
+    s = fused ? nullptr : m.take<float>(R);       // scores of expert-sorted rows (the fused kernel looks them up itself)
     dsp = m.take<float>(parts * R);
     dg = m.take(R * H);
     dg_sf = m.take(isa_bytes(R, H));
@@ -219,12 +219,12 @@ int smoe_layer_backward(const smoe_layer_args* args, void* stream) {
   // dout's column-quantised copy: transposed where dw2 joins the 256 x 384 kernel, else left as rows (13 us cheaper to make
   // at T=8192, H=3072, K=8; the 256 x 256 kernel reads either in the same time)
   const bool dc_rows = b.fused && (!wide_ok(E, I, H) || a.dw2_mode == SMOE_DW_BF16);
-  SMOE_TRY(smoe_gather_scores(sv.scores, sv.s_scatter, R, b.s, stream));
+  if (!b.fused) SMOE_TRY(smoe_gather_scores(sv.scores, sv.s_scatter, R, b.s, stream));
   SMOE_TRY(smoe_quant_rows_scatter(a.dout, a.T, H, sv.naept, sv.s_rev, sv.s_scatter, rows, R, b.dg, b.dg_sf, stream));
   if (b.fused && dw2) SMOE_TRY(column_operand(a.dout, sv, rows, R, H, dc_rows, b.dc, b.dc_sf, stream));
   if (b.fused) {
-    SMOE_TRY(smoe_gemm_dgated_fused(b.dg, b.dg_sf, a.w2, a.w2_sf, sv.efo, sv.z, sv.z_sc, b.s, b.dz, b.dz_rsf, b.dz_csf, b.y1s,
-                                    b.y1s_sf, b.dsp, R, I, H, E, a.status, stream));
+    SMOE_TRY(smoe_gemm_dgated_fused_scored(b.dg, b.dg_sf, a.w2, a.w2_sf, sv.efo, sv.z, sv.z_sc, sv.scores, sv.s_scatter, b.dz,
+                                           b.dz_rsf, b.dz_csf, b.y1s, b.y1s_sf, b.dsp, R, I, H, E, a.status, stream));
   } else {
     SMOE_TRY(smoe_gemm_dgated(b.dg, R, nullptr, b.dg_sf, a.w2, a.w2_sf, sv.efo, sv.z, sv.z_sc, b.s, b.dz_bf16, b.y1s_bf16,
                               b.dsp, nullptr, R, I, H, E, a.status, stream));
@@ -234,11 +234,7 @@ int smoe_layer_backward(const smoe_layer_args* args, void* stream) {
     }
     SMOE_TRY(smoe_quant_iso32(b.dz_bf16, R, 2 * I, b.dz, b.dz_rsf, b.dz_t, b.dz_csf, stream));
   }
-  if (a.ds) {
-    if (cudaMemsetAsync(a.ds, 0, (size_t)(a.T * a.K) * sizeof(float), (cudaStream_t)stream) != cudaSuccess)
-      return SMOE_ERR_LAUNCH;
-    SMOE_TRY(smoe_ds_finalize(b.dsp, b.parts, R, sv.s_rev, a.TK_alloc, real_tk, nullptr, sv.src_idx, a.ds, stream));
-  }
+  if (a.ds) SMOE_TRY(smoe_ds_slots(b.dsp, b.parts, R, sv.s_rev, sv.naept, sv.src_idx, a.T, a.K, a.ds, stream));
   // dx before the weight gradients
   if (a.out) {
     SMOE_TRY(smoe_gemm_varlen_m_live(b.dz, b.dz_rsf, a.w1, a.w1_sf, sv.efo, sv.s_scatter, real_tk, b.dx_exp, R, H, 2 * I, E,

@@ -62,6 +62,7 @@ SIGNATURES = {
     "smoe_gemm_dgated": (_I, [_P, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _P, _P]),
     "smoe_gemm_dgated_partials": (_L, [_L]),
     "smoe_gemm_dgated_fused": (_I, [_P] * 14 + [_L, _L, _L, _L, _P, _P]),
+    "smoe_gemm_dgated_fused_scored": (_I, [_P] * 15 + [_L, _L, _L, _L, _P, _P]),
     "smoe_gemm_dgated_fused_partials": (_L, [_L]),
     "smoe_gemm_dgated_fused_gather": (_I, [_P, _L, _P] + [_P] * 13 + [_L, _L, _L, _L, _P, _P]),
     "smoe_gemm_wgrad": (_I, [_P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _I, _P, _P]),
@@ -74,6 +75,7 @@ SIGNATURES = {
     "smoe_combine_post": (_I, [_P, _P, _P, _P, _P, _L, _L, _P, _P, _P]),
     "smoe_gather_scores": (_I, [_P, _P, _L, _P, _P]),
     "smoe_ds_finalize": (_I, [_P, _L, _L, _P, _L, _P, _P, _P, _P, _P]),
+    "smoe_ds_slots": (_I, [_P, _L, _L, _P, _P, _P, _L, _L, _P, _P]),
     "smoe_status_post": (_I, [_P, _P, _P]),
     "smoe_layer_bytes": (_L, [ctypes.POINTER(LayerArgs), _I]),
     "smoe_layer_forward": (_I, [ctypes.POINTER(LayerArgs), _P]),

@@ -1149,3 +1149,34 @@ def test_forward_gemms_for_few_rows_match_the_general_kernels(ops, counts, H, I)
     assert torch.isfinite(c1).all()
     cos, rr = stats(c1, c0)
     assert cos > 0.9999 and rr < 4e-3, (cos, rr)
+
+
+@pytest.mark.parametrize("T,K,E,I", [(200, 4, 6, 256), (33, 2, 5, 512)])
+def test_scores_and_ds_by_index_match_the_separate_kernels(ops, T, K, E, I):
+    """GemmDGated looking up a row's score itself against a gathered copy, and ds summed straight into the top-k table's slots
+    against the scatter over a cleared table: the same bits, masked slots zero."""
+    from sonicmoe._lib import check, lib
+    H = 256
+    idx, probs = make_routing(T, K, E, 0.3, seed=T)
+    md = ops.topk_metadata(idx.to(DEV), probs.to(DEV), E, 128)
+    R_, g = md["TKp_alloc"], torch.Generator().manual_seed(3)
+    n = int(md["efo"][-1])
+    (dq, ds_), (wq, ws) = rand_fp8((R_, H), g), rand_fp8((E, I, H), g)
+    zq, zs = rand_fp8((R_, 2 * I), g)
+    d = lambda t: t.contiguous().to(DEV)
+    a = (d(dq), d(Q.pack_isa(ds_, R_, H)), d(wq), d(Q.pack_isa(ws.reshape(E * I, H // 32), E * I, H)), md["efo"], d(zq), d(zs))
+    s = ops.gather_scores(md["topk_scores"], md["s_scatter_idx"])
+    want = ops.gemm_dgated_fused(*a, s, R_)
+    got = [torch.empty_like(t) for t in want]
+    P, st = lambda t: t.data_ptr(), torch.cuda.current_stream().cuda_stream
+    check(lib.smoe_gemm_dgated_fused_scored(*map(P, a), P(md["topk_scores"]), P(md["s_scatter_idx"]), *map(P, got), R_, I, H, E,
+                                            P(ops.status_word(DEV)), st), "dgated_fused_scored")
+    torch.cuda.synchronize()
+    ops.check_status(DEV)
+    assert torch.equal(got[0][:n], want[0][:n]) and torch.equal(got[3][:n], want[3][:n])
+    assert torch.equal(got[5][:, :n], want[5][:, :n])
+    ref = ops.ds_finalize(want[5], md["s_reverse_scatter_idx"], md["TK_alloc"], md["naept"][-1:], md["score_src_idx"], T * K)[1]
+    out = torch.full((T, K), float("nan"), device=DEV)
+    check(lib.smoe_ds_slots(P(want[5]), want[5].shape[0], R_, P(md["s_reverse_scatter_idx"]), P(md["naept"]),
+                            P(md["score_src_idx"]), T, K, P(out), st), "ds_slots")
+    assert torch.equal(out.flatten(), ref.flatten()) and (out.cpu()[idx < 0] == 0).all()
