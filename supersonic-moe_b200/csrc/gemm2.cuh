@@ -14,6 +14,15 @@ constexpr int kEpiWarps2 = 8;
 constexpr int kThreads2 = 32 * (2 + kEpiWarps2);
 constexpr int kMaxExperts2 = 256;   // expert offsets cached in shared memory by the two-CTA kernel
 constexpr int kDefaultL2Prefetch = 0;
+// Reduce-adds into a gradient that lies in HBM: the L2 fetches a line when the sum arrives, and the sums wait for that.  A warp
+// therefore asks for the old values of its next pieces (32 rows x 128 bytes) a little ahead.  Reduce-adds alone in tile order
+// (1.6 GB of gradient): 664 us, with the next one to four pieces prefetched 562, eight pieces 613; loading, adding and storing
+// instead 530, but no longer safe against a second writer.
+// A tile of few K tiles is bound by this traffic, one of many by its MMAs, which the prefetches then slow down.  dw1 + dw2 in
+// one launch, E=8 M=3072 + 1536 N=3072, by K tiles per expert, us: 8 210 -> 185, 16 246 -> 236, 20 270 -> 264, 24 294 -> 294,
+// 32 353 -> 359, 48 493 -> 507, 64 639 -> 656; E=128 M=1536 N=2048 of skewed load, dw1 935 -> 880; E=32, 8 K tiles 824 -> 671.
+constexpr int kReduceAhead = 2;          // pieces
+constexpr int kReduceAheadKTiles = 20;   // K tiles of a tile up to which it is done
 constexpr int kSfGroup2 = 4;        // K tiles whose scales travel in one TMA copy (box rows of the scale tensor maps)
 
 // ---- cluster helpers -------------------------------------------------------
@@ -729,6 +738,9 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         s_row = p.s[p.s_scatter != nullptr ? p.s_scatter[grow] : (int)grow];
       }
       const bool live = (MODE == PLAIN || MODE == GATED) && slab_live(p, t, t.m0 + q * 32);
+      const bool ahead = MODE == WGRAD && p.accumulate && t.nkt <= kReduceAheadKTiles;
+      if (ahead && lane == 0)                                    // the first pieces of the old gradient (see kReduceAhead)
+        for (int c = 0; c < kReduceAhead; ++c) tma_prefetch_l2_2d(&tmap_c, c_base + c * 32, t.e * p.rows + t.m0 + q * 32);
       if (lane == 0) ok = mbar_wait(bar_tfull + 8 * as, aphase);
       ok = __shfl_sync(0xffffffff, ok, 0);
       if (!ok) break;
@@ -813,14 +825,17 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         } else if (p.accumulate) {
           // Reduce-adds in whole 128-byte lines (32 columns), from 4 KB staging tiles in the ring stages lent for them; the
           // L2 merges a 64-byte piece no cheaper than a line (E=128, M=768, N=2048: 400 -> 364 us; M=1536: 755 -> 726).
-          // What bounds the rest is read-modify-write traffic in tile order: reading the old values with the epilogue's
-          // own loads instead took 920 us, more staging tiles (two or three a warp) 760 and 834 us, fetching the tile
-          // towards L2 ahead of time 800 us.
+          // What bounds the rest is read-modify-write traffic in tile order (see kReduceAhead): reading the old values with the
+          // epilogue's own loads took 920 us where this took 726, more staging tiles (two or three a warp) 760 and 834 us,
+          // fetching the whole tile towards L2 ahead of time 800 us.
           const uint32_t sb = smem_base + nst * S::STAGE_BYTES + (warp - 2) * S::LENT_TILE;
           const int crow = t.e * p.rows + t.m0 + q * 32;
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
-            if (lane == 0) bulk_wait_group_read<0>();
+            if (lane == 0) {
+              if (ahead && c + kReduceAhead < NC) tma_prefetch_l2_2d(&tmap_c, c_base + (c + kReduceAhead) * 32, crow);
+              bulk_wait_group_read<0>();
+            }
             __syncwarp();
             stage_f32_32(sb, lane, acc[c]);
             fence_proxy_async_smem();

@@ -64,6 +64,7 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                   const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
                   const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ SecondMaps second,
                   const GemmParams p) {
+  static_assert(kReduceAhead <= 3, "pieces fetched before the wait lie in the first half");
   static_assert(MODE == PLAIN || MODE == WGRAD, "the 384-wide tile exists for the plain and weight-gradient GEMMs");
   using S = Gemm3Smem<MODE>;
   constexpr int BN = kBN3, HN = kHN3;
@@ -471,6 +472,11 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
         }
       } else {  // WGRAD: f32, one half at a time (96 accumulator registers per half)
+        const CUtensorMap* dw_map = t.prob ? &second.c : &tmap_c;
+        const int dw_row = t.e * (t.prob ? p.rows2 : p.rows) + t.m0 + q * 32, dw_col = t.n0 + grp * CPW;
+        const bool ahead = p.accumulate && t.nkt <= kReduceAheadKTiles;
+        if (ahead && lane == 0)                                 // the first pieces of the old gradient (see kReduceAhead)
+          for (int c = 0; c < kReduceAhead; ++c) tma_prefetch_l2_2d(dw_map, dw_col + c * 32, dw_row);
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
           if (lane == 0) ok = mbar_wait(bar_tfull + 8 * h, aphase);
@@ -509,14 +515,17 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (p.accumulate) {                   // whole 128-byte lines, both staging buffers as one (see gemm2.cuh)
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-              if (lane == 0) bulk_wait_group_read<0>();
+              if (lane == 0) {
+                const int a = h * NC + c + kReduceAhead;          // piece number, three a half
+                if (ahead && a < 2 * NC) tma_prefetch_l2_2d(dw_map, dw_col + a / NC * HN + a % NC * 32, dw_row);
+                bulk_wait_group_read<0>();
+              }
               __syncwarp();
               stage_f32_32(stg, lane, acc[c]);
               fence_proxy_async_smem();
               __syncwarp();
               if (lane == 0) {
-                tma_reduce_add_2d(t.prob ? &second.c : &tmap_c, stg, t.n0 + h * HN + grp * CPW + c * 32,
-                                  t.e * (t.prob ? p.rows2 : p.rows) + t.m0 + q * 32);
+                tma_reduce_add_2d(dw_map, stg, dw_col + h * HN + c * 32, dw_row);
                 bulk_commit_group();
               }
             }
