@@ -18,6 +18,7 @@ Dataflow (one code path, MXFP8 1x32 ue8m0 everywhere a GEMM runs):
 """
 from __future__ import annotations
 
+import functools
 import os
 import weakref
 from contextlib import contextmanager
@@ -26,7 +27,7 @@ import torch
 import torch.nn.functional as F
 
 from .. import _lib, ops
-from ..config import get_active_config
+from ..config import SonicMoEConfig, get_active_config
 from ..enums import ActivationType, activation_code, require_swiglu
 
 # ----------------------------------------------------------------------------
@@ -145,9 +146,13 @@ def _base_of(w: torch.Tensor) -> torch.Tensor:
     return w._base if w._base is not None else w
 
 
+def _weight_key(w, kind):
+    return w.data_ptr(), w.shape, w.stride(), kind, w.get_device()
+
+
 def _weight_cache_get(w, base, kind):
     """(payload, scales) of a cached FP8 copy that is still current, else None."""
-    hit = _WEIGHT_CACHE.get((w.data_ptr(), tuple(w.shape), tuple(w.stride()), kind, w.device.index))
+    hit = _WEIGHT_CACHE.get(_weight_key(w, kind))
     # address + version are not enough: a freed weight's address is handed out again by the caching allocator,
     # with a fresh version counter that can coincide - the entry also remembers WHICH tensor it was made from
     if hit is not None and hit[0] == base._version and hit[3]() is base:
@@ -158,8 +163,7 @@ def _weight_cache_get(w, base, kind):
 def _weight_cache_put(w, base, kind, q, sf):
     if len(_WEIGHT_CACHE) >= _WEIGHT_CACHE_MAX:
         _WEIGHT_CACHE.pop(next(iter(_WEIGHT_CACHE)))
-    _WEIGHT_CACHE[(w.data_ptr(), tuple(w.shape), tuple(w.stride()), kind, w.device.index)] = (
-        base._version, q, sf, weakref.ref(base))
+    _WEIGHT_CACHE[_weight_key(w, kind)] = (base._version, q, sf, weakref.ref(base))
 
 
 def _bf16_weight(w):
@@ -251,13 +255,15 @@ def _gemm_plain(a_q, a_sf, b_q, b_sf, stored_kn, efo, s_scatter_idx=None, naept=
     return ops.gemm_varlen_m(a_q, a_sf, ops.transpose_u8(b_q), b_sf, efo)     # transient K-major copy
 
 
+_NO_CONFIG = SonicMoEConfig()        # every field unset: the environment decides, read at each call
+
+
 def _modes(fp8_config):
     """(iso32_weight, stagewise_memory) of this call: an explicit config wins, then the active one, then the
     environment."""
     cfg = fp8_config if fp8_config is not None else get_active_config()
     if cfg is None:
-        from ..config import SonicMoEConfig
-        cfg = SonicMoEConfig()
+        cfg = _NO_CONFIG
     return cfg.resolve_iso32_weight(), cfg.resolve_stagewise_memory()
 
 
@@ -313,7 +319,7 @@ def drop_weight_fp8(*weights: torch.Tensor):
     """Forget the cached FP8 copies (both orientations) of the given weights only."""
     for w in weights:
         for transposed in (False, True, "iso32"):
-            _WEIGHT_CACHE.pop((w.data_ptr(), tuple(w.shape), tuple(w.stride()), transposed, w.device.index), None)
+            _WEIGHT_CACHE.pop(_weight_key(w, transposed), None)
 
 
 # ----------------------------------------------------------------------------
@@ -819,6 +825,14 @@ class _DownProjection(torch.autograd.Function):
 _ONE_CALL_BYTES = 256 << 20
 
 
+@functools.lru_cache(maxsize=1024)
+def _layer_bytes(T, H, I, E, K, TK, TKp, keep_z, dx, dw1, dw2):
+    """smoe_layer_bytes of the three arenas (saved, forward, backward) for these sizes and wanted gradients."""
+    a = _lib.LayerArgs(T, H, I, E, K, TK, TKp)
+    a.keep_z, a.dw1_mode, a.dw2_mode, a.out = int(keep_z), int(dw1), int(dw2), 1 if dx else None
+    return tuple(_lib.lib.smoe_layer_bytes(a, which) for which in (0, 1, 2))
+
+
 def _one_call_args(x, idx, w1, w2, E, K, TK, TKp, act, fp8_config):
     """LayerArgs of a layer that the one-call path takes, else None."""
     cfg = fp8_config if fp8_config is not None else get_active_config()
@@ -830,16 +844,17 @@ def _one_call_args(x, idx, w1, w2, E, K, TK, TKp, act, fp8_config):
     I = w2.shape[2]
     if T == 0 or E > 256 or H % 128 or I % 128 or TKp % 128 or tuple(w1.shape) != (E, 2 * I, H) or tuple(w2.shape) != (E, H, I):
         return None
-    a = _lib.LayerArgs(T, H, I, E, K, TK, TKp)
-    a.x = x.data_ptr()
-    a.forward_bytes = scratch = _lib.lib.smoe_layer_bytes(a, 1)
-    if torch.is_grad_enabled():
-        a.out = a.x if x.requires_grad else None           # which gradients the backward will be asked for
-        a.dw1_mode, a.dw2_mode = int(w1.requires_grad), int(w2.requires_grad)
-        a.backward_bytes = _lib.lib.smoe_layer_bytes(a, 2)
-        scratch = max(scratch, a.backward_bytes)
+    dx = dw1 = dw2 = False
+    grad = torch.is_grad_enabled()
+    if grad:                                    # which gradients the backward will be asked for
+        dx, dw1, dw2 = x.requires_grad, w1.requires_grad, w2.requires_grad
+    saved, forward, backward = _layer_bytes(T, H, I, E, K, TK, TKp, grad, dx, dw1, dw2)
+    scratch = max(forward, backward) if grad else forward
     if not 0 <= scratch <= _ONE_CALL_BYTES:
         return None
+    a = _lib.LayerArgs(T, H, I, E, K, TK, TKp)
+    a.x = x.data_ptr()
+    a.saved_bytes, a.forward_bytes, a.backward_bytes = saved, forward, backward
     a.status, a.host_word = ops.status_pointers(x.device)
     return a
 
@@ -862,7 +877,7 @@ class _OneCallLayer(torch.autograd.Function):
         out = torch.empty_like(x)
         counts = torch.empty(args.E, dtype=torch.int32, device=dev)
         args.lane_order, args.pad_mode, args.keep_z = lane_order, pad_mode, int(grad_mode)
-        saved = _u8(_lib.lib.smoe_layer_bytes(args, 0), dev)
+        saved = _u8(args.saved_bytes, dev)
         scratch = _u8(args.forward_bytes, dev)
         args.idx, args.probs = idx.data_ptr(), probs.data_ptr()
         args.w1, args.w1_sf, args.w2, args.w2_sf = w1_q.data_ptr(), w1_sf.data_ptr(), w2_q.data_ptr(), w2_sf.data_ptr()

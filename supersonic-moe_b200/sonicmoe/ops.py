@@ -4,6 +4,8 @@ there is no CPU path.
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from ._lib import check, lib
@@ -68,7 +70,9 @@ def _timed(fn):
 def _dev_index(device) -> int:
     """Ordinal of a CUDA device given as a device, a string or an int; "cuda" without an ordinal means the current
     device (so that "cuda" and "cuda:0" name the same status word)."""
-    d = torch.device(device) if not isinstance(device, int) else torch.device("cuda", device)
+    if isinstance(device, int):
+        return device
+    d = device if isinstance(device, torch.device) else torch.device(device)
     if d.type != "cuda":
         raise RuntimeError("sonicmoe kernels need CUDA tensors (no CPU fallback)")
     return d.index if d.index is not None else torch.cuda.current_device()
@@ -100,7 +104,15 @@ def check_status(device):
 # store, not a memcpy: it cannot queue behind bulk transfers on a copy engine); the next entry into the layer looks at that host word and raises if it is
 # non-zero.  The word is sticky on the device, so a failure surfaces at the latest one call after the pass whose
 # post saw it, and a healthy run pays at most one tiny launch per pass and no synchronisation.
-_posted = {}     # device index -> pinned int32[1] mirror of the device status word
+_posted = {}     # device index -> (pinned int32[1] mirror of the device status word, a ctypes view of it, both addresses)
+
+
+def _mirror(key):
+    m = _posted.get(key)
+    if m is None:
+        host = torch.zeros(1, dtype=_I32).pin_memory()
+        m = _posted[key] = (host, ctypes.c_int32.from_address(host.data_ptr()), status_word(key).data_ptr(), host.data_ptr())
+    return m
 
 
 def post_status(device):
@@ -108,31 +120,25 @@ def post_status(device):
     is captured)."""
     if torch.device(device).type != "cuda" or torch.cuda.is_current_stream_capturing():
         return
-    key = _dev_index(device)
-    host = _posted.get(key)
-    if host is None:
-        host = _posted[key] = torch.zeros(1, dtype=_I32).pin_memory()
-    check(lib.smoe_status_post(_p(status_word(device)), host.data_ptr(), _stream()), "status_post")
+    m = _mirror(_dev_index(device))
+    check(lib.smoe_status_post(m[2], m[3], _stream()), "status_post")
 
 
 def status_pointers(device):
     """(device address of the status word, host address of its pinned mirror)."""
-    key = _dev_index(device)
-    host = _posted.get(key)
-    if host is None:
-        host = _posted[key] = torch.zeros(1, dtype=_I32).pin_memory()
-    return status_word(key).data_ptr(), host.data_ptr()
+    return _mirror(_dev_index(device))[2:]
 
 
 def poll_status(device):
     """Look at the host mirror of the status word; raise on a recorded failure.  Never waits."""
-    if torch.device(device).type != "cuda":
+    device = torch.device(device)
+    if device.type != "cuda":
         return
-    host = _posted.get(_dev_index(device))
-    if host is not None:
-        code = int(host[0])
+    m = _posted.get(_dev_index(device))
+    if m is not None:
+        code = m[1].value
         if code != 0:
-            host[0] = 0
+            m[1].value = 0
             _raise_status(device, code)
 
 
@@ -165,16 +171,23 @@ def topk_metadata(idx, probs, E, alignment=128, TK_alloc=None, TKp_alloc=None, l
         TK_alloc = N * min(K, E)
     if TKp_alloc is None:
         TKp_alloc = -(-TK_alloc // alignment) * alignment + E * alignment
-    dev = idx.device
-    e = lambda n, dt=_I32: torch.empty(max(int(n), 0), dtype=dt, device=dev)
-    out = dict(efo=e(E + 1), x_gather_idx=e(TKp_alloc), s_scatter_idx=e(TKp_alloc),
-               s_reverse_scatter_idx=e(TK_alloc), naept=e(N + 1), topk_scores=e(TKp_alloc, torch.float32),
-               score_src_idx=e(TK_alloc), counts=e(E))
-    ws = e(lib.smoe_topk_metadata_workspace(N, E), _U8)
-    check(lib.smoe_topk_metadata(_p(idx), _p(probs), N, K, E, alignment, TK_alloc, TKp_alloc, lane_order, pad_mode,
-                                 _p(out["efo"]), _p(out["x_gather_idx"]), _p(out["s_scatter_idx"]),
-                                 _p(out["s_reverse_scatter_idx"]), _p(out["naept"]), _p(out["topk_scores"]),
-                                 _p(out["score_src_idx"]), _p(out["counts"]), _p(ws), _stream()), "topk_metadata")
+    # six integer tables are pieces of one allocation (an allocation each costs the host more than the kernels run); x_gather,
+    # read 16 bytes at a time, comes first.  counts, which callers keep and may change, is a tensor of its own.
+    TK, TKp, dev = max(int(TK_alloc), 0), max(int(TKp_alloc), 0), idx.device
+    buf = torch.empty(2 * TKp + 2 * TK + E + N + 2, dtype=_I32, device=dev)
+    x_gather, s_scatter, s_rev, src_idx, efo, naept = buf.split((TKp, TKp, TK, TK, E + 1, N + 1))
+    counts = torch.empty(E, dtype=_I32, device=dev)
+    scores = torch.empty(TKp, dtype=torch.float32, device=dev)
+    ws = torch.empty(lib.smoe_topk_metadata_workspace(N, E), dtype=_U8, device=dev)
+    at = buf.data_ptr()
+    p_src = at + 4 * (2 * TKp + TK)
+    p_efo = p_src + 4 * TK
+    p_naept = p_efo + 4 * (E + 1)
+    check(lib.smoe_topk_metadata(idx.data_ptr(), probs.data_ptr(), N, K, E, alignment, TK_alloc, TKp_alloc, lane_order, pad_mode,
+                                 p_efo, at, at + 4 * TKp, at + 8 * TKp, p_naept, scores.data_ptr(), p_src, counts.data_ptr(), ws.data_ptr(),
+                                 _stream()), "topk_metadata")
+    out = dict(efo=efo, x_gather_idx=x_gather, s_scatter_idx=s_scatter, s_reverse_scatter_idx=s_rev, naept=naept,
+               topk_scores=scores, score_src_idx=src_idx, counts=counts)
     out["TK_alloc"], out["TKp_alloc"] = TK_alloc, TKp_alloc
     return out
 
