@@ -373,7 +373,19 @@ static int run_few(const void* x, const void* w, int64_t rows, const FewParams& 
   if (rc) return rc;
   const int64_t tiles = (rows / kFewNT) * (p.N / BM);      // an upper bound
   const int grid = tiles < sm_count() ? (int)tiles : sm_count();
-  kern<<<grid, kFewThreads, S::TOTAL, stream>>>(tw, tx, p);
+  // Launched so that it may begin while the kernel before it ends.  Kernels that let it (the scatter quantizer, which makes the
+  // up-projection's rows, and this kernel) write neither offsets, counts nor weights; after any other kernel it waits as usual.
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kFewThreads);
+  cfg.dynamicSmemBytes = S::TOTAL;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, tw, tx, p) != cudaSuccess) return SMOE_ERR_LAUNCH;
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 

@@ -77,6 +77,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return true;
 }
 
+// ---------------------------------------------------------------- kernels that follow one another
+// The next kernel of the stream may start once every block has said so (or ended); what it may then touch without waiting is
+// what was complete before this kernel began.  A no-op where the next kernel was launched without the attribute.
+__device__ __forceinline__ void next_kernel_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Until the kernel before has ended and its writes are visible; a no-op in a launch without the attribute
+__device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1) {
   asm volatile(

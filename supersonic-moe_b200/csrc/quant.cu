@@ -146,6 +146,8 @@ quant_rows_scatter_kernel(const uint4* __restrict__ x, int64_t T, int K, const i
                           const int* __restrict__ valid_rows, int64_t rows, uint4* __restrict__ q,
                           uint8_t* __restrict__ isa, int token_blocks) {
   extern __shared__ __align__(16) uint8_t s_rowbuf[];
+  // a GEMM launched to do so may fetch its weights meanwhile (gemm_few.cuh)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int k_tiles = K >> 7, k16 = K >> 4;
   if ((int)blockIdx.x < token_blocks) {

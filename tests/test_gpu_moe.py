@@ -298,6 +298,46 @@ def test_forward_without_a_graph_gives_the_same_bits(sm, monkeypatch, T, H, I, E
     assert one_call or got_routed.data_ptr() == place.data_ptr()
 
 
+@pytest.mark.parametrize("how", ["back_to_back", "side_stream", "captured"])
+def test_inference_on_few_tokens_in_sequence(sm, how):
+    """The GEMMs of a small inference call begin while the kernel before them ends: calls that follow one another on changing
+    inputs, with their buffers handed on from call to call, on another stream and from a CUDA graph, give the bits of the
+    training forward, which waits for everything."""
+    T, H, I, E, K, n = 24, 512, 256, 16, 4, 6
+    _, _, w1, w2, wr, _ = make_layer(T, H, I, E, K, 21)
+    moe = sm.MoE(E, K, H, I, sm.ActivationType.SWIGLU, add_bias=False, std=0.02).to(DEV).to(torch.bfloat16)
+    with torch.no_grad():
+        moe.router.weight.copy_(wr), moe.c_fc.weight.copy_(w1), moe.c_proj.weight.copy_(w2)
+    g = torch.Generator().manual_seed(5)
+    xs = [torch.randn(T, H, generator=g).to(torch.bfloat16).to(DEV) for _ in range(n)]
+    want = [moe(x, use_fp8=True)[0].detach() for x in xs]
+    torch.cuda.synchronize()
+    infer = lambda x: moe(x, is_inference_mode=True, use_fp8=True)[0]
+    with torch.no_grad():
+        if how == "captured":
+            static = xs[0].clone()
+            side = torch.cuda.Stream()
+            with torch.cuda.stream(side):
+                infer(static)
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                out = infer(infer(static) * 0 + static)
+            got = []
+            for x in xs:
+                static.copy_(x)
+                graph.replay()
+                got.append(out.clone())
+            del graph
+        else:
+            with torch.cuda.stream(torch.cuda.Stream() if how == "side_stream" else torch.cuda.current_stream()):
+                got = [infer(x) for x in xs for _ in range(3)][::3]
+    torch.cuda.synchronize()
+    sm.ops.check_status(DEV)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("T,H,I,E,K,seed", [(256, 256, 128, 8, 2, 0), (1024, 512, 256, 16, 4, 1),
                                              (512, 1024, 384, 8, 8, 2)])
 def test_moe_module_fwd_bwd_vs_fp32_oracle(sm, T, H, I, E, K, seed):
