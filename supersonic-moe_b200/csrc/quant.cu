@@ -628,12 +628,20 @@ __device__ __forceinline__ uint32_t qc_scales(uint4 (&v)[8], int sub) {
 // fastest.  T=8192, H=3072, K=E=8: 86.0 -> 71.7 us; T=16384, H=2048, K=8, E=128 (285 MB out): 125 -> 102 us, against a warp
 // per 32 x 256 slab, whose 255 registers left four warps an SM.
 constexpr int QC_TILES = 4;      // row tiles of a block, one after the other
+// Column tiles of a strip: a strip of all source rows is what the L2 has to hold while every expert's rows are gathered from it.
+// With all columns in one strip a source of 67 MB was read from HBM once per expert.  All columns / 16 / 8 / 4 tiles, us:
+// T=8192 H=4096 K=E=8 124 / 92 / 88 / 87, T=8192 H=3072 77 / 71 / 71 / 69, T=16384 H=2048 K=8 E=128, skewed, 109 / 108 / 96 / 96,
+// T=4096 H=3072 E=32 41 / 42 / 41 / 42.
+constexpr int QC_STRIP = 8;
 
 __global__ void __launch_bounds__(256, 4)
 quant_cols_rows_kernel(const void* __restrict__ src, const int* __restrict__ idx, const int* __restrict__ valid_rows,
                        int64_t rows, int dim, uint8_t* __restrict__ q, uint8_t* __restrict__ col_isa) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane >> 3;
-  const int ct = blockIdx.x % (dim >> 7), rt0 = blockIdx.x / (dim >> 7) * QC_TILES;
+  // strips of QC_STRIP column tiles, one after the other; within a strip column tiles fastest, then row tiles
+  const int groups = ((int)(rows >> 7) + QC_TILES - 1) / QC_TILES, strip = blockIdx.x / (QC_STRIP * groups);
+  const int width = min(QC_STRIP, (dim >> 7) - strip * QC_STRIP), in_strip = blockIdx.x - strip * QC_STRIP * groups;
+  const int ct = strip * QC_STRIP + in_strip % width, rt0 = in_strip / width * QC_TILES;
   const int grp = warp >> 1;                                          // 32-row group of the 128-row tile
   const int col = ct * 128 + (warp & 1) * 64 + (lane & 7) * 8;        // this lane's columns [col, col + 8)
   const int row0 = grp * 32 + sub * 8;                                // and rows of a tile [row0, row0 + 8)
