@@ -1180,3 +1180,18 @@ def test_scores_and_ds_by_index_match_the_separate_kernels(ops, T, K, E, I):
     check(lib.smoe_ds_slots(P(want[5]), want[5].shape[0], R_, P(md["s_reverse_scatter_idx"]), P(md["naept"]),
                             P(md["score_src_idx"]), T, K, P(out), st), "ds_slots")
     assert torch.equal(out.flatten(), ref.flatten()) and (out.cpu()[idx < 0] == 0).all()
+
+
+@pytest.mark.parametrize("T,dim,rows,valid", [(50, 1280, 640, 640), (200, 2048, 1152, 1056), (40, 1792, 128, 96)])
+def test_row_major_column_quantizer_walks_every_strip(ops, T, dim, rows, valid):
+    """More than one strip of 1024 columns, the last one narrower, with row groups that are not full: the bytes and scales of the
+    transposed form, and nothing beyond the valid rows."""
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, dim, generator=g).to(torch.bfloat16).to(DEV)
+    idx = torch.randint(0, T, (rows,), generator=g, dtype=torch.int32).to(DEV)
+    n = torch.tensor([valid], dtype=torch.int32, device=DEV)
+    _, _, q, sf = ops.quant_dual_gather(x, idx, rows, n, with_rows=False)
+    q_t, sf_t = ops.quant_cols_t(x, idx, rows)
+    assert torch.equal(q[:valid].t(), q_t[:, :valid])
+    a, b = Q.unpack_isa(sf.cpu(), dim, rows), Q.unpack_isa(sf_t.cpu(), dim, rows)
+    assert torch.equal(a[:, :valid // 32], b[:, :valid // 32])
