@@ -280,9 +280,7 @@ int smoe_gemm_gated_infer(const void* x_sorted_fp8, const void* a_sf, const void
                           int64_t K, int64_t E, int* status, void* stream);
 
 /* The two forward GEMMs made for few rows per expert (any counts are computed right).  The first counts[e] rows of expert
- * e's segment are computed and written, the others may hold anything and stay as they are.  E <= 256; scales 16-byte aligned.
- * Right after smoe_quant_rows_scatter or one of these two, efo, counts and weights may be read before that call's kernel has
- * ended (which writes none of them). */
+ * e's segment are computed and written, the others may hold anything and stay as they are.  E <= 256; scales 16-byte aligned. */
 int smoe_gemm_gated_few(const void* x_sorted_fp8, const void* a_sf, const void* w1_fp8, const void* w1_sf, const int* efo,
                         const int* counts, void* y1_fp8, void* y1_sf, int64_t rows, int64_t N, int64_t K, int64_t E,
                         int* status, void* stream);

@@ -361,8 +361,11 @@ static int run(const void* a, int64_t a_rows, int64_t a_cols, const void* b, int
 }
 
 // ---- few rows per expert: weights as the M operand -------------------------------------------------------------------
+// `early`: launched so that it may begin while the kernel before it in the stream ends.  It then reads offsets, counts and weights
+// before that kernel's writes have to be visible, whether or not that kernel says that it may be overtaken; so a caller may ask
+// for it only where the kernel before writes none of the three and itself began after they were complete.
 template <int MODE>
-static int run_few(const void* x, const void* w, int64_t rows, const FewParams& p, cudaStream_t stream) {
+static int run_few(const void* x, const void* w, int64_t rows, const FewParams& p, bool early, cudaStream_t stream) {
   using S = FewSmem;
   static bool attr_set[kMaxDevices] = {};
   auto kern = gemm_few_kernel<MODE>;
@@ -373,8 +376,6 @@ static int run_few(const void* x, const void* w, int64_t rows, const FewParams& 
   if (rc) return rc;
   const int64_t tiles = (rows / kFewNT) * (p.N / BM);      // an upper bound
   const int grid = tiles < sm_count() ? (int)tiles : sm_count();
-  // Launched so that it may begin while the kernel before it ends.  Kernels that let it (the scatter quantizer, which makes the
-  // up-projection's rows, and this kernel) write neither offsets, counts nor weights; after any other kernel it waits as usual.
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -384,7 +385,7 @@ static int run_few(const void* x, const void* w, int64_t rows, const FewParams& 
   cfg.dynamicSmemBytes = S::TOTAL;
   cfg.stream = stream;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   if (cudaLaunchKernelEx(&cfg, kern, tw, tx, p) != cudaSuccess) return SMOE_ERR_LAUNCH;
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
@@ -397,6 +398,31 @@ static int check_few(const void* x, const void* w, const void* x_sf, const void*
   if (rows > 0 && (!x || !w || !x_sf || !w_sf || !efo || !counts)) return SMOE_ERR_ARG;
   if (((uintptr_t)x_sf | (uintptr_t)w_sf) & 15) return SMOE_ERR_ALIGN;
   return SMOE_OK;
+}
+
+int gemm_gated_few(const void* x_sorted_fp8, const void* a_sf, const void* w1_fp8, const void* w1_sf, const int* efo,
+                   const int* counts, void* y1_fp8, void* y1_sf, int64_t rows, int64_t N, int64_t K, int64_t E, int* status,
+                   bool early, void* stream) {
+  const int rc = check_few(x_sorted_fp8, w1_fp8, a_sf, w1_sf, efo, counts, rows, N, K, E);
+  if (rc) return rc;
+  if (N % 256) return SMOE_ERR_SHAPE;
+  if (rows == 0) return SMOE_OK;
+  if (!y1_fp8 || !y1_sf) return SMOE_ERR_ARG;
+  FewParams p{(int)N, (int)K, (int)E, efo, counts, (const uint8_t*)w1_sf, (const uint8_t*)a_sf, nullptr, (uint8_t*)y1_fp8,
+              (uint8_t*)y1_sf, status};
+  return run_few<GATED>(x_sorted_fp8, w1_fp8, rows, p, early, (cudaStream_t)stream);
+}
+
+int gemm_varlen_m_few(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,
+                      const int* counts, void* c_bf16, int64_t rows, int64_t N, int64_t K, int64_t E, int* status, bool early,
+                      void* stream) {
+  const int rc = check_few(a_fp8, b_fp8, a_sf, b_sf, efo, counts, rows, N, K, E);
+  if (rc) return rc;
+  if (rows == 0) return SMOE_OK;
+  if (!c_bf16) return SMOE_ERR_ARG;
+  FewParams p{(int)N, (int)K, (int)E, efo, counts, (const uint8_t*)b_sf, (const uint8_t*)a_sf, (__nv_bfloat16*)c_bf16,
+              nullptr, nullptr, status};
+  return run_few<PLAIN>(a_fp8, b_fp8, rows, p, early, (cudaStream_t)stream);
 }
 
 // A weight-gradient call over zero routed rows: the product is empty, so an accumulating call leaves c as it is and
@@ -495,26 +521,13 @@ int smoe_gemm_gated_infer(const void* x_sorted_fp8, const void* a_sf, const void
 int smoe_gemm_gated_few(const void* x_sorted_fp8, const void* a_sf, const void* w1_fp8, const void* w1_sf, const int* efo,
                         const int* counts, void* y1_fp8, void* y1_sf, int64_t rows, int64_t N, int64_t K, int64_t E,
                         int* status, void* stream) {
-  const int rc = check_few(x_sorted_fp8, w1_fp8, a_sf, w1_sf, efo, counts, rows, N, K, E);
-  if (rc) return rc;
-  if (N % 256) return SMOE_ERR_SHAPE;
-  if (rows == 0) return SMOE_OK;
-  if (!y1_fp8 || !y1_sf) return SMOE_ERR_ARG;
-  FewParams p{(int)N, (int)K, (int)E, efo, counts, (const uint8_t*)w1_sf, (const uint8_t*)a_sf, nullptr, (uint8_t*)y1_fp8,
-              (uint8_t*)y1_sf, status};
-  return run_few<GATED>(x_sorted_fp8, w1_fp8, rows, p, (cudaStream_t)stream);
+  return gemm_gated_few(x_sorted_fp8, a_sf, w1_fp8, w1_sf, efo, counts, y1_fp8, y1_sf, rows, N, K, E, status, false, stream);
 }
 
 int smoe_gemm_varlen_m_few(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,
                            const int* counts, void* c_bf16, int64_t rows, int64_t N, int64_t K, int64_t E,
                            int* status, void* stream) {
-  const int rc = check_few(a_fp8, b_fp8, a_sf, b_sf, efo, counts, rows, N, K, E);
-  if (rc) return rc;
-  if (rows == 0) return SMOE_OK;
-  if (!c_bf16) return SMOE_ERR_ARG;
-  FewParams p{(int)N, (int)K, (int)E, efo, counts, (const uint8_t*)b_sf, (const uint8_t*)a_sf, (__nv_bfloat16*)c_bf16,
-              nullptr, nullptr, status};
-  return run_few<PLAIN>(a_fp8, b_fp8, rows, p, (cudaStream_t)stream);
+  return gemm_varlen_m_few(a_fp8, a_sf, b_fp8, b_sf, efo, counts, c_bf16, rows, N, K, E, status, false, stream);
 }
 
 int64_t smoe_gemm_dgated_partials(int64_t N);

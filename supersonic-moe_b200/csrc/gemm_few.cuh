@@ -10,8 +10,8 @@
 // an output row.  GATED: gate and up lie in neighbouring lanes, the 32 values that share a scale in two neighbouring warps.
 // Live rows only are computed and written: the first counts[e] of expert e's segment.
 //
-// The kernel may start before the one before it in the stream has ended (see run_few): until wait_for_kernel_before it touches
-// only offsets, counts and weights.  Its set-up and the weights of the first ring pass then lie under the end of the kernel
+// Where its caller allows it (see run_few) the kernel starts before the one before it in the stream has ended: until
+// wait_for_kernel_before it touches only offsets, counts and weights.  Its set-up and the weights of the first ring pass then lie under the end of the kernel
 // before: an inference call replayed from a graph, E=128 H=2048 I=768 64 tokens 130 -> 123 us, E=32 H=3072 I=1536 64 tokens
 // 115 -> 104, E=8 16 tokens 57 -> 51 (starting from 167, 139 and 76 with routed rows as M and the kernels around it as they were).
 #pragma once

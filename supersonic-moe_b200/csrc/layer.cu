@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include "smoe_b200.h"
+#include "smoe_internal.h"
 
 namespace smoe {
 
@@ -189,9 +190,12 @@ int smoe_layer_forward(const smoe_layer_args* args, void* stream) {
   SMOE_TRY(smoe_quant_rows_scatter(a.x, a.T, H, sv.naept, sv.s_rev, a.keep_z ? sv.s_scatter : nullptr, rows, R, sc.xg,
                                    sc.xg_sf, stream));
   if (!a.keep_z && few_rows(a)) {
-    SMOE_TRY(smoe_gemm_gated_few(sc.xg, sc.xg_sf, a.w1, a.w1_sf, sv.efo, a.counts, sc.y1, sc.y1_sf, R, 2 * I, H, E, a.status,
-                                 stream));
-    SMOE_TRY(smoe_gemm_varlen_m_few(sc.y1, sc.y1_sf, a.w2, a.w2_sf, sv.efo, a.counts, sc.y2, R, H, I, E, a.status, stream));
+    // Both may begin early: the quantizer, launched the ordinary way, began when offsets, counts and weights were complete, and
+    // neither it nor the up-projection writes any of them.  T > 0, so that the quantizer is there
+    const bool early = a.T > 0;
+    SMOE_TRY(gemm_gated_few(sc.xg, sc.xg_sf, a.w1, a.w1_sf, sv.efo, a.counts, sc.y1, sc.y1_sf, R, 2 * I, H, E, a.status, early,
+                            stream));
+    SMOE_TRY(gemm_varlen_m_few(sc.y1, sc.y1_sf, a.w2, a.w2_sf, sv.efo, a.counts, sc.y2, R, H, I, E, a.status, early, stream));
   } else {
     if (a.keep_z)
       SMOE_TRY(smoe_gemm_gated(sc.xg, R, nullptr, sc.xg_sf, a.w1, a.w1_sf, sv.efo, sv.z, sv.z_sc, sc.y1, sc.y1_sf, R, 2 * I, H,

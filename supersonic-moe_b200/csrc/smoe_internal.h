@@ -1,7 +1,9 @@
-/* Symbols the library exports for its own tests and timing experiments.  They are NOT part of the product ABI
- * (include/smoe_b200.h): process-global, unsynchronised, and able to switch stores off. */
+/* Calls between the library's own files and symbols it exports for its own tests and timing experiments.  None is part of the
+ * product ABI (include/smoe_b200.h); the exported ones are process-global, unsynchronised, and able to switch stores off. */
 #ifndef SMOE_INTERNAL_H_
 #define SMOE_INTERNAL_H_
+
+#include <stdint.h>
 
 #ifdef __cplusplus
 extern "C" {
@@ -24,5 +26,17 @@ int smoe_internal_gemm_trace(void* device_buffer);
 
 #ifdef __cplusplus
 }
+
+namespace smoe {
+// smoe_gemm_gated_few and smoe_gemm_varlen_m_few as a layer calls them.  `early`: the kernel may begin while the one before it in
+// the stream ends, and reads efo, counts and weights before that one's writes are visible: only for a caller that knows the
+// kernel before, that it writes none of the three, and that they were complete when it began.
+int gemm_gated_few(const void* x_sorted_fp8, const void* a_sf, const void* w1_fp8, const void* w1_sf, const int* efo,
+                   const int* counts, void* y1_fp8, void* y1_sf, int64_t rows, int64_t N, int64_t K, int64_t E, int* status,
+                   bool early, void* stream);
+int gemm_varlen_m_few(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,
+                      const int* counts, void* c_bf16, int64_t rows, int64_t N, int64_t K, int64_t E, int* status, bool early,
+                      void* stream);
+}  // namespace smoe
 #endif
 #endif /* SMOE_INTERNAL_H_ */
