@@ -449,7 +449,7 @@ typedef struct {
   void* dx_ready;              /* backward: cudaEvent_t recorded when dx is complete, before the weight gradients; may be null */
 } smoe_layer_args;
 /* Bytes of an arena: which = 0 saved, 1 forward scratch, 2 backward scratch; -1 for sizes that are not taken.  The last
- * depends on which gradients are asked for (out null or not, dw1_mode, dw2_mode). */
+ * depends on which gradients are asked for (out null or not, dw1_mode, dw2_mode).  Nothing but the arguments decides. */
 int64_t smoe_layer_bytes(const smoe_layer_args* args, int which);
 int smoe_layer_forward(const smoe_layer_args* args, void* stream);
 int smoe_layer_backward(const smoe_layer_args* args, void* stream);

@@ -597,7 +597,7 @@ int smoe_gemm_dgated_fused_scored(const void* dout_fp8, const void* a_sf, const 
 }
 
 int64_t smoe_gemm_dgated_fused_partials(int64_t N) {
-  const int bn = pick_bn2<DGATEDQ>(N);
+  const int bn = pick_bn2<DGATEDQ>(N) == 192 ? 192 : 128;      // (0 where the single-CTA kernels are forced, which have no such mode)
   return (bn == 192 ? Gemm2Smem<192, DGATEDQ>::COL_GROUPS : Gemm2Smem<128, DGATEDQ>::COL_GROUPS) * ((N + bn - 1) / bn);
 }
 

@@ -89,7 +89,9 @@ struct BwdScratch {
     fused = mn_ok(a.E, I, H);
     parts = fused ? smoe_gemm_dgated_fused_partials(I) : smoe_gemm_dgated_partials(I);
     s = fused ? nullptr : m.take<float>(R);       // scores of expert-sorted rows (the fused kernel looks them up itself)
-    dsp = m.take<float>(parts * R);
+    // room for the narrowest column tile, 128 columns in two groups, whatever tile is in use: the size follows from the arguments
+    // alone, and may be remembered by them
+    dsp = m.take<float>(2 * ((I + 127) / 128) * R);
     dg = m.take(R * H);
     dg_sf = m.take(isa_bytes(R, H));
     dc = dc_sf = dx_exp = xc = xc_sf = nullptr;

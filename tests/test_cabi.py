@@ -54,3 +54,21 @@ def test_column_quantizers_refuse_misaligned_buffers(built_library):
             assert lib.smoe_requant_cols_t(src, 16, None, None, 128, dim, q, isa, None) == 2
     assert lib.smoe_quant_iso32(8, 128, 128, 16, 16, None, 16, None) == 2
     assert lib.smoe_quant_iso32(16, 128, 128, 16, 16, 8, 16, None) == 2
+
+
+@pytest.mark.parametrize("H,I,E", [(256, 128, 8), (512, 768, 16), (3072, 1536, 8), (4096, 4096, 8), (1024, 1280, 37)])
+def test_arena_sizes_follow_from_the_arguments_alone(built_library, H, I, E):
+    """A caller may remember an arena's size by the problem: forcing another column tile between asking and running must not make
+    the layer need more than was asked for."""
+    from sonicmoe._lib import LayerArgs, lib
+    a = LayerArgs(512, H, I, E, 4, 2048, 2048 + E * 128)
+    a.keep_z, a.dw1_mode, a.dw2_mode, a.out = 1, 1, 1, 16
+    want = [lib.smoe_layer_bytes(a, which) for which in (0, 1, 2)]
+    assert min(want) > 0
+    for knobs in (128, 192, 256, 384, 128 | (1 << 17), 1 << 17):
+        lib.smoe_internal_gemm_knobs(knobs)
+        try:
+            got = [lib.smoe_layer_bytes(a, which) for which in (0, 1, 2)]
+        finally:
+            lib.smoe_internal_gemm_knobs(0)
+        assert got == want, knobs
