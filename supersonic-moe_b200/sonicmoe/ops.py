@@ -171,21 +171,19 @@ def topk_metadata(idx, probs, E, alignment=128, TK_alloc=None, TKp_alloc=None, l
         TK_alloc = N * min(K, E)
     if TKp_alloc is None:
         TKp_alloc = -(-TK_alloc // alignment) * alignment + E * alignment
-    # six integer tables are pieces of one allocation (an allocation each costs the host more than the kernels run); x_gather,
-    # read 16 bytes at a time, comes first.  counts, which callers keep and may change, is a tensor of its own.
-    TK, TKp, dev = max(int(TK_alloc), 0), max(int(TKp_alloc), 0), idx.device
-    buf = torch.empty(2 * TKp + 2 * TK + E + N + 2, dtype=_I32, device=dev)
-    x_gather, s_scatter, s_rev, src_idx, efo, naept = buf.split((TKp, TKp, TK, TK, E + 1, N + 1))
-    counts = torch.empty(E, dtype=_I32, device=dev)
-    scores = torch.empty(TKp, dtype=torch.float32, device=dev)
-    ws = torch.empty(lib.smoe_topk_metadata_workspace(N, E), dtype=_U8, device=dev)
-    at = buf.data_ptr()
-    p_src = at + 4 * (2 * TKp + TK)
-    p_efo = p_src + 4 * TK
-    p_naept = p_efo + 4 * (E + 1)
+    # A tensor each: callers keep some, write to some and save others for a backward.  16384 x 8 over 128 experts, us a call, bound
+    # by the host: a `torch.empty` each 30.8, `new_empty` 29.4; views of one tensor, which share a version counter and a lifetime
+    # and start anywhere, 27.1.
+    TK, TKp = max(int(TK_alloc), 0), max(int(TKp_alloc), 0)
+    x_gather = torch.empty(TKp, dtype=_I32, device=idx.device)
+    e = x_gather.new_empty
+    s_scatter, s_rev, src_idx, efo, naept, counts = e(TKp), e(TK), e(TK), e(E + 1), e(N + 1), e(E)
+    scores = e(TKp, dtype=torch.float32)
+    ws = e(lib.smoe_topk_metadata_workspace(N, E), dtype=_U8)
     check(lib.smoe_topk_metadata(idx.data_ptr(), probs.data_ptr(), N, K, E, alignment, TK_alloc, TKp_alloc, lane_order, pad_mode,
-                                 p_efo, at, at + 4 * TKp, at + 8 * TKp, p_naept, scores.data_ptr(), p_src, counts.data_ptr(), ws.data_ptr(),
-                                 _stream()), "topk_metadata")
+                                 efo.data_ptr(), x_gather.data_ptr(), s_scatter.data_ptr(), s_rev.data_ptr(), naept.data_ptr(),
+                                 scores.data_ptr(), src_idx.data_ptr(), counts.data_ptr(), ws.data_ptr(), _stream()),
+          "topk_metadata")
     out = dict(efo=efo, x_gather_idx=x_gather, s_scatter_idx=s_scatter, s_reverse_scatter_idx=s_rev, naept=naept,
                topk_scores=scores, score_src_idx=src_idx, counts=counts)
     out["TK_alloc"], out["TKp_alloc"] = TK_alloc, TKp_alloc

@@ -1195,3 +1195,27 @@ def test_row_major_column_quantizer_walks_every_strip(ops, T, dim, rows, valid):
     assert torch.equal(q[:valid].t(), q_t[:, :valid])
     a, b = Q.unpack_isa(sf.cpu(), dim, rows), Q.unpack_isa(sf_t.cpu(), dim, rows)
     assert torch.equal(a[:, :valid // 32], b[:, :valid // 32])
+
+
+@pytest.mark.parametrize("how", ["ops", "dispatched", "general"])
+def test_metadata_tables_are_tensors_of_their_own(ops, how):
+    """Each table has its own storage and version: one written in place between a forward and a backward leaves the others fit for
+    it, one kept keeps no other alive, and each starts where the allocator starts a tensor."""
+    import sonicmoe
+    from sonicmoe.ernie_compat import deepep_topk_to_sonic_metadata
+    N, K, E = 37, 3, 5
+    idx, probs = make_routing(N, K, E, 0.2, seed=4)
+    if how == "ops":
+        md = ops.topk_metadata(idx.to(DEV), probs.to(DEV), E, 1)
+        tables = [md[k] for k in MD_KEYS]
+    elif how == "dispatched":
+        tables = [t for t in deepep_topk_to_sonic_metadata(idx.to(DEV), probs.to(DEV), None, E) if isinstance(t, torch.Tensor)]
+    else:
+        tok, slot = (idx >= 0).nonzero(as_tuple=True)
+        tables = sonicmoe.functional.general_routing_router_metadata(probs[tok, slot].to(DEV), tok.to(torch.int32).to(DEV),
+                                                                     idx[tok, slot].to(DEV), N, E)
+    before = [t._version for t in tables]
+    for t in tables:
+        assert t.untyped_storage().nbytes() == t.numel() * t.element_size() and t.data_ptr() % 256 == 0
+    tables[1].add_(1)
+    assert [t._version - v for t, v in zip(tables, before)] == [0, 1] + [0] * (len(tables) - 2)
