@@ -71,3 +71,85 @@ def test_only_the_layer_lets_the_gemms_begin_early(ops):
               "varlen_m_few")
 
     assert early_starts(metadata_then_gemms) == 0
+
+
+def deq_inputs(shape, g):
+    """e4m3 values of N(0,1) and their 1x32 scales, as the quantizers make them."""
+    q, sc = Q.row_quant(torch.randn(shape, generator=g).reshape(-1, shape[-1]).to(torch.bfloat16))
+    return q.reshape(shape), sc.reshape(*shape[:-1], -1)
+
+
+def both_forms(ops, counts, H, I, seed, change=None):
+    """y1 payload, y1 scales and output rows of the live rows from the 256-row kernels and from the few-row ones.  `change` edits
+    (x, x scales, w1, w1 scales, w2, w2 scales) of the live rows before."""
+    from sonicmoe._lib import check, lib
+    g = torch.Generator().manual_seed(seed)
+    E = len(counts)
+    seg = [-(-c // 128) * 128 for c in counts]
+    efo = torch.zeros(E + 1, dtype=torch.int32)
+    efo[1:] = torch.cumsum(torch.tensor(seg), 0)
+    rows = int(efo[-1]) + 128
+    live = torch.cat([torch.arange(int(efo[e]), int(efo[e]) + min(c, seg[e])) for e, c in enumerate(counts)])
+    xq = torch.randint(0, 256, (rows, H), generator=g, dtype=torch.uint8)
+    xs = torch.randint(0, 256, (rows, H // 32), generator=g, dtype=torch.uint8)
+    (lq, ls), (w1, w1s), (w2, w2s) = deq_inputs((len(live), H), g), deq_inputs((E, 2 * I, H), g), deq_inputs((E, H, I), g)
+    if change is not None:
+        change(lq, ls, w1, w1s, w2, w2s)
+    xq[live], xs[live] = lq, ls
+    d = lambda t: t.contiguous().to(DEV)
+    xq, xsf, w1, w2 = d(xq), d(Q.pack_isa(xs, rows, H)), d(w1), d(w2)
+    w1sf = d(Q.pack_isa(w1s.reshape(E * 2 * I, H // 32), E * 2 * I, H))
+    w2sf = d(Q.pack_isa(w2s.reshape(E * H, I // 32), E * H, I))
+    s_scatter = torch.full((rows,), len(live), dtype=torch.int32)
+    s_scatter[live] = torch.arange(len(live), dtype=torch.int32)
+    efo, cnt, real, s_scatter = d(efo), *(d(torch.as_tensor(t, dtype=torch.int32)) for t in (counts, [len(live)], s_scatter))
+    P, st, status = lambda t: t.data_ptr(), torch.cuda.current_stream().cuda_stream, ops.status_word(DEV).data_ptr()
+    out = []
+    for few in (False, True):
+        y = torch.full((rows, I), 0xAA, dtype=torch.uint8, device=DEV)
+        ysf = torch.full((ops.isa_bytes(rows, I),), 0xAA, dtype=torch.uint8, device=DEV)
+        c = torch.full((rows, H), 7.0, dtype=torch.bfloat16, device=DEV)
+        if few:
+            check(lib.smoe_gemm_gated_few(P(xq), P(xsf), P(w1), P(w1sf), P(efo), P(cnt), P(y), P(ysf), rows, 2 * I, H, E, status,
+                                          st), "gated_few")
+            check(lib.smoe_gemm_varlen_m_few(P(y), P(ysf), P(w2), P(w2sf), P(efo), P(cnt), P(c), rows, H, I, E, status, st),
+                  "varlen_m_few")
+            dead = torch.ones(rows, dtype=torch.bool)
+            dead[live] = False
+            assert (y.cpu()[dead] == 0xAA).all() and (c.cpu()[dead] == 7.0).all()            # left as they were
+        else:
+            check(lib.smoe_gemm_gated_infer(P(xq), P(xsf), P(w1), P(w1sf), P(efo), P(s_scatter), P(real), P(y), P(ysf), rows,
+                                            2 * I, H, E, status, st), "gated_infer")
+            check(lib.smoe_gemm_varlen_m_live(P(y), P(ysf), P(w2), P(w2sf), P(efo), P(s_scatter), P(real), P(c), rows, H, I, E,
+                                              status, st), "varlen_m_live")
+        torch.cuda.synchronize()
+        ops.check_status(DEV)
+        out.append((y.cpu()[live], Q.unpack_isa(ysf.cpu(), rows, I)[live], c.cpu()[live].float()))
+    return out
+
+
+def assert_same_values(a, b):
+    """Both forms multiply the same operands; the tensor core may add the products of a K step in another order, which moves a
+    value next to a rounding boundary of e4m3 or bf16."""
+    (y0, s0, c0), (y1, s1, c1) = a, b
+    same = s0 == s1
+    assert (~same).float().mean() < 2e-3 and (y0 != y1)[same.repeat_interleave(32, 1)].float().mean() < 2e-3
+    assert torch.equal(torch.isnan(c0), torch.isnan(c1)) and torch.equal(torch.isinf(c0), torch.isinf(c1))
+    ok = torch.isfinite(c0)
+    assert float((c0[ok] - c1[ok]).norm()) <= 4e-3 * float(c0[ok].norm())
+
+
+def test_nan_and_overflow_leave_the_bytes_of_the_general_kernels(ops):
+    """A row of NaN, a NaN in one weight row of an expert, and a row that overflows f32: payload and scale bytes of the up-projection
+    included."""
+    def change(x, xs, w1, w1s, w2, w2s):
+        x[1, 5] = 0x7F                  # every output of row 1
+        w1[3, 6, 9] = 0x7F              # one gate column of expert 3, live rows 12 and 13
+        xs[4, :] = 0xFE                 # row 4 times 2^127
+        x[6] = 0                        # a row of zeros
+    a, b = both_forms(ops, [3, 0, 9, 2], 256, 128, 5, change)
+    assert_same_values(a, b)
+    (y0, s0, c0), (y1, s1, c1) = a, b
+    nan = (y0 & 0x7F) == 0x7F
+    assert nan[1].all() and nan[12:, 3].all() and not nan[0].any() and torch.equal(nan, (y1 & 0x7F) == 0x7F)
+    assert torch.equal(s0[[1, 4, 6]], s1[[1, 4, 6]]) and torch.isnan(c1[[1, 12, 13]]).all() and (c1[6] == 0).all()
