@@ -79,13 +79,14 @@ def deq_inputs(shape, g):
     return q.reshape(shape), sc.reshape(*shape[:-1], -1)
 
 
-def both_forms(ops, counts, H, I, seed, change=None):
+def both_forms(ops, counts, H, I, seed, change=None, segments=None):
     """y1 payload, y1 scales and output rows of the live rows from the 256-row kernels and from the few-row ones.  `change` edits
-    (x, x scales, w1, w1 scales, w2, w2 scales) of the live rows before."""
+    (x, x scales, w1, w1 scales, w2, w2 scales) of the live rows before; `segments`: rows an expert's segment has, where `counts`
+    asks for more."""
     from sonicmoe._lib import check, lib
     g = torch.Generator().manual_seed(seed)
     E = len(counts)
-    seg = [-(-c // 128) * 128 for c in counts]
+    seg = segments or [-(-c // 128) * 128 for c in counts]
     efo = torch.zeros(E + 1, dtype=torch.int32)
     efo[1:] = torch.cumsum(torch.tensor(seg), 0)
     rows = int(efo[-1]) + 128
@@ -153,3 +154,15 @@ def test_nan_and_overflow_leave_the_bytes_of_the_general_kernels(ops):
     nan = (y0 & 0x7F) == 0x7F
     assert nan[1].all() and nan[12:, 3].all() and not nan[0].any() and torch.equal(nan, (y1 & 0x7F) == 0x7F)
     assert torch.equal(s0[[1, 4, 6]], s1[[1, 4, 6]]) and torch.isnan(c1[[1, 12, 13]]).all() and (c1[6] == 0).all()
+
+
+@pytest.mark.parametrize("last", [0, 3, 65])
+def test_all_256_experts(ops, last):
+    counts = [0] * 256
+    counts[0], counts[100], counts[254], counts[255] = 1, 17, 2, last
+    assert_same_values(*both_forms(ops, counts, 128, 128, 6 + last))
+
+
+def test_counts_beyond_a_segment_that_was_cut(ops):
+    """Metadata made into too small buffers leaves the experts' whole counts beside offsets that are cut."""
+    assert_same_values(*both_forms(ops, [140, 70, 500, 9], 256, 128, 7, segments=[128, 128, 256, 0]))
