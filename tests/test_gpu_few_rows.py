@@ -166,3 +166,39 @@ def test_all_256_experts(ops, last):
 def test_counts_beyond_a_segment_that_was_cut(ops):
     """Metadata made into too small buffers leaves the experts' whole counts beside offsets that are cut."""
     assert_same_values(*both_forms(ops, [140, 70, 500, 9], 256, 128, 7, segments=[128, 128, 256, 0]))
+
+
+@pytest.mark.parametrize("T,K,E,H,I,few", [
+    (40, 8, 8, 256, 128, True), (41, 8, 8, 256, 128, False), (64, 5, 8, 256, 128, True), (64, 6, 8, 256, 128, False),
+    (65, 1, 8, 256, 128, True), (80, 1, 8, 256, 128, True), (81, 1, 8, 256, 128, False),             # ten rows on average
+    (640, 8, 128, 256, 128, False), (5120, 1, 128, 256, 128, False),                                 # forty
+    (192, 1, 64, 6144, 128, True), (193, 1, 64, 6144, 128, False),                                   # one slot: 3 and 4 x 48 tiles
+    (128, 4, 64, 6144, 128, True), (129, 4, 64, 6144, 128, False), (128, 5, 64, 128, 3072, False)])  # all slots
+def test_which_inference_calls_take_the_few_row_gemms(ops, T, K, E, H, I, few):
+    """The few-row GEMMs are the only launches of a layer call that may begin early."""
+    from sonicmoe._lib import check, lib
+    a, keep = layer_args(ops, T, H, I, E, K)
+    n = early_starts(lambda: check(lib.smoe_layer_forward(a, torch.cuda.current_stream().cuda_stream), "layer"))
+    assert n == (2 if few else 0)
+
+
+@pytest.mark.parametrize("T,K,E,busy", [(200, 1, 64, 150), (200, 2, 64, 200), (64, 3, 16, 64), (620, 1, 64, 620)])
+def test_inference_with_busy_experts(ops, T, K, E, busy):
+    """An expert of up to ten row tiles among idle ones: the output of the training forward, which takes the other kernels."""
+    import sonicmoe
+    H, I = 256, 128
+    g = torch.Generator().manual_seed(T + K)
+    logits = torch.rand(T, E, generator=g)
+    logits[:busy, 3] = 2.0
+    idx = logits.topk(K).indices
+    assert not (idx.sort(1).values.diff(dim=1) == 0).any()               # a row's experts are distinct
+    idx, scores = idx.to(torch.int32).to(DEV), torch.rand(T, K, generator=g).to(DEV)
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16).to(DEV)
+    w1 = (torch.randn(E, 2 * I, H, generator=g) * 0.05).to(torch.bfloat16).to(DEV).requires_grad_(True)
+    w2 = (torch.randn(E, H, I, generator=g) * 0.05).to(torch.bfloat16).to(DEV).requires_grad_(True)
+    want = sonicmoe.run_sonic_moe(x, idx, scores, K, E, w1, w2, fp8=True).detach()
+    with torch.no_grad():
+        got = sonicmoe.run_sonic_moe(x, idx, scores, K, E, w1, w2, fp8=True)
+    torch.cuda.synchronize()
+    ops.check_status(DEV)
+    assert float((got.float() - want.float()).norm()) <= 4e-3 * float(want.float().norm())
