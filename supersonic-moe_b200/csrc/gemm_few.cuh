@@ -39,8 +39,7 @@ struct FewSmem {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES + SF_BYTES;
   static constexpr int AMAX_BYTES = 2 * 4 * 16 * 4;             // GATED: [buffer][warp][column]
   static constexpr int AUX_BYTES = 512 + AMAX_BYTES + 3 * (kMaxExperts2 + 1) * 4 + 4;
-  static constexpr int STAGES_RAW = (227 * 1024 - 1024 - AUX_BYTES) / STAGE_BYTES;
-  static constexpr int STAGES = STAGES_RAW > 12 ? 12 : STAGES_RAW;
+  static constexpr int STAGES = (227 * 1024 - 1024 - AUX_BYTES) / STAGE_BYTES;           // 8
   static constexpr int TOTAL = STAGES * STAGE_BYTES + AUX_BYTES + 1024;
   static constexpr int SF_COL0 = 2 * NT;                        // two accumulators
   static constexpr int SF_COLS = 8;

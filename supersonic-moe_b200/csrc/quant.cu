@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ptx.cuh"
 #include "smoe_b200.h"
 
 namespace smoe {
@@ -110,7 +111,6 @@ __device__ __forceinline__ void bulk_store(void* dst, const void* src_smem, uint
 __device__ __forceinline__ void bulk_store_wait() {
   asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
 }
-__device__ __forceinline__ void fence_smem_to_bulk() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Clears the pad rows (s_scatter[row] >= real_tk) of an expert-sorted e4m3 buffer and their scales; warp w0 of nwarps.  Eight
 // lanes look at a row each, so that a warp waits for one load per eight rows (and not for one per row); more than eight rows
@@ -147,7 +147,7 @@ quant_rows_scatter_kernel(const uint4* __restrict__ x, int64_t T, int K, const i
                           uint8_t* __restrict__ isa, int token_blocks) {
   extern __shared__ __align__(16) uint8_t s_rowbuf[];
   // a GEMM launched to do so may fetch its weights meanwhile (gemm_few.cuh)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  next_kernel_may_start();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int k_tiles = K >> 7, k16 = K >> 4;
   if ((int)blockIdx.x < token_blocks) {
@@ -191,7 +191,7 @@ quant_rows_scatter_kernel(const uint4* __restrict__ x, int64_t T, int K, const i
         }
       }
     }
-    fence_smem_to_bulk();
+    fence_proxy_async_smem();
     __syncwarp();
     for (int j0 = beg; j0 < end; j0 += 32) {
       if (j0 > beg) pos = j0 + lane < end ? s_rev[j0 + lane] : 0;
