@@ -68,12 +68,8 @@ static int make_tmap_dw(CUtensorMap* m, const GemmParams& p, void* c, uint64_t r
 }
 
 static int g_force_bn = 0;
-static int g_skip_store = 0;
 static int g_force_v1 = 0;
 static int g_force_gather4 = 0;     // A rows by index: TMA gather4 instead of the cp.async load warps
-static int g_stage_cut = 0;
-static int g_l2_prefetch = -1;     // -1: the kernel's default
-static void* g_trace = nullptr;    // timing experiment: per-tile stamps of the MMA issuer (256 x 384 kernel)
 
 // Per-device state: the SM count and the "large dynamic shared memory" function attribute belong to a device,
 // not to the process, so both are kept per device ordinal.
@@ -137,9 +133,7 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   if (max_pair_tiles < pairs) pairs = max_pair_tiles;
   if (pairs <= 0) return SMOE_OK;
   GemmParams q = p;
-  q.dbg_stage_cut = g_stage_cut;
   if (MODE == WGRAD && p.accumulate && !p.out_bf16) q.stages_lent = S::LENT_STAGES;
-  q.l2_prefetch = g_l2_prefetch >= 0 ? g_l2_prefetch : kDefaultL2Prefetch;
   kern<<<(unsigned)(2 * pairs), S::THREADS, S::TOTAL, stream>>>(ta, tb, tsa, tsb, om.c, om.c2, om.c3, q);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
@@ -156,12 +150,8 @@ static int launch3(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   int64_t pairs = sm_count() / 2;
   if (max_pair_tiles < pairs) pairs = max_pair_tiles;
   if (pairs <= 0) return SMOE_OK;
-  GemmParams q = p;
-  q.dbg_stage_cut = g_stage_cut > 2 ? 2 : g_stage_cut;      // the head / tail schedule holds two stages
-  q.l2_prefetch = g_l2_prefetch;                            // this kernel reads it as "length of the head / tail", -1 = default
-  q.trace = reinterpret_cast<long long*>(g_trace);
   SecondMaps none{};
-  kern<<<(unsigned)(2 * pairs), S::THREADS, S::TOTAL, stream>>>(ta, tb, tsa, tsb, tc, second ? *second : none, q);
+  kern<<<(unsigned)(2 * pairs), S::THREADS, S::TOTAL, stream>>>(ta, tb, tsa, tsb, tc, second ? *second : none, p);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 
@@ -439,19 +429,10 @@ using namespace smoe;
 
 extern "C" {
 
-int smoe_internal_gemm_trace(void* device_buffer) {
-  g_trace = device_buffer;
-  return SMOE_OK;
-}
-
-int smoe_internal_gemm_knobs(int bn) {
-  g_force_bn = bn & 0xFFFF;
-  g_skip_store = ((bn >> 16) & 1) | (((bn >> 18) & 1) << 1);   // bit 16: no stores; bit 18: no epilogue (fused dgated)
-  g_force_v1 = (bn >> 17) & 1;
-  g_skip_store |= ((bn >> 19) & 0x1F) << 2;    // bits 19..23 -> timing-experiment bits 2..6 of GemmParams::debug_skip_store
-  g_force_gather4 = (bn >> 31) & 1;            // bit 31: indexed A rows through TMA gather4
-  g_stage_cut = (bn >> 24) & 3;                // bits 24..25: ring stages to leave unused
-  g_l2_prefetch = ((bn >> 26) & 0x1F) - 1;     // bits 26..30: L2 prefetch distance + 1 (0 = kernel default)
+int smoe_internal_gemm_knobs(int bits) {
+  g_force_bn = bits & 0xFFFF;
+  g_force_v1 = (bits >> 17) & 1;
+  g_force_gather4 = (bits >> 31) & 1;
   return SMOE_OK;
 }
 
@@ -466,7 +447,7 @@ int smoe_gemm_varlen_m_live(const void* a_fp8, const void* a_sf, const void* b_f
   p.efo = efo; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)b_sf;
   p.sfa_ktiles = (int)(K / 128); p.sfb_ktiles = (int)(K / 128);
   p.s_scatter = s_scatter_idx; p.real_tk = real_tk;
-  p.c = c_bf16; p.status = status; p.debug_skip_store = g_skip_store;
+  p.c = c_bf16; p.status = status;
   return run<PLAIN>(a_fp8, rows, K, b_fp8, E * N, K, p, (int)((rows / 128) * (N / 128)), (cudaStream_t)stream);
 }
 
@@ -483,7 +464,7 @@ int smoe_gemm_varlen_m_bt(const void* a_fp8, const void* a_sf, const void* b_kn_
   p.rows = (int)rows; p.N = (int)N; p.K = (int)K; p.E = (int)E;
   p.efo = efo; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)b_sf;
   p.sfa_ktiles = (int)(K / 128); p.sfb_ktiles = (int)(K / 128);
-  p.c = c_bf16; p.status = status; p.debug_skip_store = g_skip_store;
+  p.c = c_bf16; p.status = status;
   p.b_mn = 1;                                      // B of expert e = rows [e*K, (e+1)*K) of an [E*K, N] matrix
   return run<PLAIN>(a_fp8, rows, K, b_kn_fp8, E * K, N, p, (int)((rows / 128) * (N / 128)), (cudaStream_t)stream);
 }
@@ -499,7 +480,7 @@ int smoe_gemm_gated(const void* x_fp8, int64_t T, const int* a_idx, const void* 
   p.efo = efo; p.a_idx = a_idx; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)w1_sf;
   p.sfa_ktiles = (int)(K / 128); p.sfb_ktiles = (int)(K / 128);
   p.z_fp8 = (uint8_t*)z_fp8; p.z_sc = (uint8_t*)z_scales; p.y1_fp8 = (uint8_t*)y1_fp8; p.y1_sf = (uint8_t*)y1_sf;
-  p.status = status; p.debug_skip_store = g_skip_store;
+  p.status = status;
   return run<GATED>(x_fp8, T, K, w1_fp8, E * N, K, p, (int)((rows / 128) * (N / 128)), (cudaStream_t)stream);
 }
 
@@ -514,7 +495,7 @@ int smoe_gemm_gated_infer(const void* x_sorted_fp8, const void* a_sf, const void
   p.efo = efo; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)w1_sf;
   p.sfa_ktiles = (int)(K / 128); p.sfb_ktiles = (int)(K / 128);
   p.y1_fp8 = (uint8_t*)y1_fp8; p.y1_sf = (uint8_t*)y1_sf; p.s_scatter = s_scatter_idx; p.real_tk = real_tk;
-  p.status = status; p.debug_skip_store = g_skip_store;
+  p.status = status;
   return run<GATED>(x_sorted_fp8, rows, K, w1_fp8, E * N, K, p, (int)((rows / 128) * (N / 128)), (cudaStream_t)stream);
 }
 
@@ -563,7 +544,6 @@ static int dgated_fused_impl(const void* dout_fp8, int64_t a_rows, const int* a_
   p.z_fp8 = (uint8_t*)const_cast<void*>(z_fp8); p.z_sc = (uint8_t*)const_cast<void*>(z_scales);
   p.s = s; p.s_scatter = s_idx; p.dz = dz_q; p.y1s = y1s_q; p.ds_partial = ds_partial; p.status = status;
   p.dz_row_sf = (uint8_t*)dz_row_sf; p.dz_col_sf = (uint8_t*)dz_col_sf; p.y1s_col_sf = (uint8_t*)y1s_col_sf;
-  p.debug_skip_store = g_skip_store;
   return run<DGATEDQ>(dout_fp8, a_rows, K, w2t_fp8, E * N, K, p, (int)((rows / 128) * (N / 128)),
                       (cudaStream_t)stream);
 }
@@ -615,7 +595,7 @@ int smoe_gemm_wgrad(const void* a_t_fp8, const void* a_sf, const void* b_t_fp8, 
   p.rows = (int)M; p.N = (int)N; p.K = (int)TKp; p.E = (int)E;
   p.efo = efo; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)b_sf;
   p.sfa_ktiles = (int)(TKp / 128); p.sfb_ktiles = (int)(TKp / 128);
-  p.c = c; p.accumulate = accumulate; p.status = status; p.debug_skip_store = g_skip_store;
+  p.c = c; p.accumulate = accumulate; p.status = status;
   return run<WGRAD>(a_t_fp8, M, TKp, b_t_fp8, N, TKp, p, (int)(E * (M / 128) * (N / 128)), (cudaStream_t)stream);
 }
 
@@ -628,7 +608,7 @@ int smoe_gemm_wgrad_mn(const void* a_fp8, const void* a_sf, const void* b_fp8, c
   p.rows = (int)M; p.N = (int)N; p.K = (int)TKp; p.E = (int)E;
   p.efo = efo; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)b_sf;
   p.sfa_ktiles = (int)(TKp / 128); p.sfb_ktiles = (int)(TKp / 128);
-  p.c = c; p.accumulate = accumulate; p.status = status; p.debug_skip_store = g_skip_store;
+  p.c = c; p.accumulate = accumulate; p.status = status;
   p.a_mn = layout & 1; p.b_mn = (layout >> 1) & 1;
   return run<WGRAD>(a_fp8, p.a_mn ? TKp : M, p.a_mn ? M : TKp, b_fp8, p.b_mn ? TKp : N, p.b_mn ? N : TKp, p,
                     (int)(E * (M / 128) * (N / 128)), (cudaStream_t)stream);
@@ -647,7 +627,7 @@ int smoe_gemm_wgrad_bf16(const void* a_fp8, const void* a_sf, const void* b_fp8,
   p.rows = (int)M; p.N = (int)N; p.K = (int)TKp; p.E = (int)E;
   p.efo = efo; p.sfa = (const uint8_t*)a_sf; p.sfb = (const uint8_t*)b_sf;
   p.sfa_ktiles = (int)(TKp / 128); p.sfb_ktiles = (int)(TKp / 128);
-  p.c = c_bf16; p.out_bf16 = 1; p.status = status; p.debug_skip_store = g_skip_store;
+  p.c = c_bf16; p.out_bf16 = 1; p.status = status;
   p.a_mn = layout & 1; p.b_mn = (layout >> 1) & 1;
   return run<WGRAD>(a_fp8, p.a_mn ? TKp : M, p.a_mn ? M : TKp, b_fp8, p.b_mn ? TKp : N, p.b_mn ? N : TKp, p,
                     (int)(E * (M / 128) * (N / 128)), (cudaStream_t)stream);
@@ -670,7 +650,7 @@ int smoe_gemm_wgrad_mn_pair(const void* a1_fp8, const void* a1_sf, const void* b
   p.rows = (int)M1; p.rows2 = (int)M2; p.N = (int)N; p.K = (int)TKp; p.E = (int)E;
   p.efo = efo; p.sfa = (const uint8_t*)a1_sf; p.sfb = (const uint8_t*)b1_sf;
   p.sfa_ktiles = (int)(TKp / 128); p.sfb_ktiles = (int)(TKp / 128);
-  p.c = c1; p.c2 = c2; p.accumulate = accumulate; p.status = status; p.debug_skip_store = g_skip_store;
+  p.c = c1; p.c2 = c2; p.accumulate = accumulate; p.status = status;
   p.a_mn = a_rows_major_tk ? 1 : 0;
   return run3_wgrad_pair(a1_fp8, b1_fp8, p, a2_fp8, b2_fp8, (const uint8_t*)a2_sf, (const uint8_t*)b2_sf, TKp,
                          (cudaStream_t)stream);

@@ -39,7 +39,6 @@ struct GemmParams {
   int sfb_ktiles;
   // outputs / epilogue operands
   void* c;              // PLAIN: bf16 [rows,N]; WGRAD: f32 [E,rows,N]
-  long long* trace;     // timing experiment (256x384 kernel): per-tile stamps of the MMA issuer, else null
   int rows2;            // WGRAD, 256x384 kernel: output rows per expert of a SECOND product run by the same launch
   void* c2;             //   (same N, K range and operand layouts; own A, B, scales and f32 [E,rows2,N] output); 0: none
   int accumulate;       // WGRAD: add into c instead of overwriting
@@ -61,9 +60,6 @@ struct GemmParams {
   const int* real_tk;   // nothing but padding are then not stored (the two-CTA kernels).  DGATEDQ, if not null: row r's
                         // score is s[s_scatter[r]]
   int stages_lent;      // two-CTA WGRAD into an existing f32 gradient: ring stages that hold its staging tiles instead
-  int debug_skip_store; // timing experiments only: drain TMEM but skip the global stores
-  int dbg_stage_cut;    // timing experiments only: use this many fewer ring stages
-  int l2_prefetch;      // K tiles ahead of the shared-memory ring at which operand tiles are prefetched into L2 (0 = off)
 };
 
 template <int BN>
@@ -325,7 +321,7 @@ gemm_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             v.y = pack_bf16x2(__uint_as_float(r[8 * i + 2]), __uint_as_float(r[8 * i + 3]));
             v.z = pack_bf16x2(__uint_as_float(r[8 * i + 4]), __uint_as_float(r[8 * i + 5]));
             v.w = pack_bf16x2(__uint_as_float(r[8 * i + 6]), __uint_as_float(r[8 * i + 7]));
-            if (!p.debug_skip_store || v.x == 0x12345678u) dst[c * 4 + i] = v;
+            dst[c * 4 + i] = v;
           }
         }
       } else if (MODE == WGRAD) {

@@ -13,7 +13,6 @@ namespace smoe {
 constexpr int kEpiWarps2 = 8;
 constexpr int kThreads2 = 32 * (2 + kEpiWarps2);
 constexpr int kMaxExperts2 = 256;   // expert offsets cached in shared memory by the two-CTA kernel
-constexpr int kDefaultL2Prefetch = 0;
 // Reduce-adds into a gradient that lies in HBM: the L2 fetches a line when the sum arrives, and the sums wait for that.  A warp
 // therefore asks for the old values of its next pieces (32 rows x 128 bytes) a little ahead.  Reduce-adds alone in tile order
 // (1.6 GB of gradient): 664 us, with the next one to four pieces prefetched 562, eight pieces 613; loading, adding and storing
@@ -433,7 +432,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const uint32_t sf_base = smem_u32(sfring);
   const int n_col_tiles = (p.N + BN - 1) / BN;
   const int n_total = (MODE == WGRAD) ? p.E * (p.rows / (2 * BM)) * n_col_tiles : s_pairs[p.E] * n_col_tiles;
-  const int nst = S::STAGES - p.dbg_stage_cut - p.stages_lent;       // ring stages in use
+  const int nst = S::STAGES - p.stages_lent;       // ring stages in use
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
@@ -449,8 +448,6 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    const bool dbg_noload = (p.debug_skip_store & 4) != 0;   // timing experiment: operands fetched for one ring pass only
-    int dbg_filled = 0;
     for (int tile = pair_id; tile < n_total_u && ok; tile += n_pairs_grid) {
       const PairTile tl = pair_tile<BN, MODE>(tile, rank, p, s_efo, s_pairs);
       const int nkt = __shfl_sync(0xffffffffu, tl.nkt, 0);
@@ -479,28 +476,16 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         const uint32_t full = full0 + 8 * stage;
         const uint32_t a_dst = smem_base + stage * S::STAGE_BYTES;
         const uint32_t b_dst = a_dst + S::A_BYTES;
-        if (!CPG && dbg_noload && dbg_filled >= nst) {
-          if (rank == 0 && elect_one()) mbar_arrive(bar_full + 8 * stage);
-        } else {
-          ++dbg_filled;
-          if (elect_one()) {
-            if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, tx_bytes);
-            if (a_mn) tma_load_2d_pair(a_dst, &tmap_a, full, m0, kt * BK);
-            else if (!GATHER && !CPG && load_a) tma_load_2d_pair(a_dst, &tmap_a, full, kt * BK, a_row);
-            if (b_mn) tma_load_2d_pair(b_dst, &tmap_b, full, b_row, b_k0 + kt * BK);
-            else tma_load_2d_pair(b_dst, &tmap_b, full, kt * BK, b_row);
-            const int kp = kt + p.l2_prefetch;
-            if (p.l2_prefetch > 0 && kp < kt0 + nkt) {
-              if (a_mn) tma_prefetch_l2_2d(&tmap_a, m0, kp * BK);
-              else if (!GATHER && !CPG) tma_prefetch_l2_2d(&tmap_a, kp * BK, a_row);
-              if (b_mn) tma_prefetch_l2_2d(&tmap_b, b_row, b_k0 + kp * BK);
-              else tma_prefetch_l2_2d(&tmap_b, kp * BK, b_row);
-            }
-          }
-          if (GATHER) {
-            __syncwarp();
-            tma_gather4_pair(a_dst + lane * 4 * BK, &tmap_a, full, kt * BK, rows4.x, rows4.y, rows4.z, rows4.w);
-          }
+        if (elect_one()) {
+          if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, tx_bytes);
+          if (a_mn) tma_load_2d_pair(a_dst, &tmap_a, full, m0, kt * BK);
+          else if (!GATHER && !CPG && load_a) tma_load_2d_pair(a_dst, &tmap_a, full, kt * BK, a_row);
+          if (b_mn) tma_load_2d_pair(b_dst, &tmap_b, full, b_row, b_k0 + kt * BK);
+          else tma_load_2d_pair(b_dst, &tmap_b, full, kt * BK, b_row);
+        }
+        if (GATHER) {
+          __syncwarp();
+          tma_gather4_pair(a_dst + lane * 4 * BK, &tmap_a, full, kt * BK, rows4.x, rows4.y, rows4.z, rows4.w);
         }
         if (++stage == nst) { stage = 0; phase ^= 1; }
       }
@@ -529,7 +514,6 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const uint32_t b_lo0 = (((smem_base + S::A_BYTES) & 0x3FFFF) >> 4) | ((b_mn ? (uint32_t)(S::B_BYTES >> 4) : 1u) << 16);
       const uint32_t sf_lo0 = (sf_base & 0x3FFFF) >> 4;
       const int n_total_u = __shfl_sync(0xffffffffu, n_total, 0);
-      const bool skip_sf_cp = (p.debug_skip_store & 16) != 0;
       int stage = 0, as = 0, sfs = 0;
       uint32_t phase = 0, aphase = 0, sfphase = 0;
       bool ok = true;
@@ -559,12 +543,10 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           const uint32_t sfb_t = sfa_t + 4;
           const bool sf_done = (kg == S::SF_GROUP - 1 || k == nkt - 1);      // last use of this scale slot
           if (elect_one()) {
-            if (!skip_sf_cp) {
-              tc_cp_sf_pair_lo(sfa_t, sf_lo, sf_hi);
+            tc_cp_sf_pair_lo(sfa_t, sf_lo, sf_hi);
 #pragma unroll
-              for (int j = 0; j < S::SFB_TILES; ++j)
-                tc_cp_sf_pair_lo(sfb_t + 4 * j, sf_lo + ((S::SF_GROUP * 512 * (1 + j)) >> 4), sf_hi);
-            }
+            for (int j = 0; j < S::SFB_TILES; ++j)
+              tc_cp_sf_pair_lo(sfb_t + 4 * j, sf_lo + ((S::SF_GROUP * 512 * (1 + j)) >> 4), sf_hi);
 #pragma unroll
             for (int kb = 0; kb < BK / 32; ++kb)
               mma_mxf8_pair_lo(d_tmem, a_lo + a_step * kb, b_lo + b_step * kb, desc_hi, idesc_kb[kb], sfa_t,
@@ -748,9 +730,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + as * BN + half * COLS_PER_WARP;
 
       bool released = false;
-      if (p.debug_skip_store & 8) {
-        // timing experiment: the accumulator is handed back untouched
-      } else if (MODE == PLAIN) {
+      if (MODE == PLAIN) {
         // Drain the whole row segment into registers (bf16-packed), hand the accumulator back to the
         // MMA warp, then stage and store.  32 columns of bf16 = 64-byte rows, SWIZZLE_64B, 2 x 2 KB.
         constexpr int NC = COLS_PER_WARP / 32;
@@ -948,17 +928,15 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
           fence_proxy_async_smem();
           __syncwarp();
-          if (!(p.debug_skip_store & 1)) {
-            if (lane == 0) {
-              if (p.z_fp8 != nullptr) tma_store_2d(&tmap_c, stg, zc, t.m0 + q * 32);     // z e4m3 [rows, 2I]
-              tma_store_2d(&tmap_c2, stg + 2048, zc / 2, t.m0 + q * 32);     // y1 e4m3 [rows, I]
-              bulk_commit_group();
-            }
-            if (p.z_fp8 != nullptr) *reinterpret_cast<uint16_t*>(p.z_sc + grow * (Nz / 32) + zc / 32) = (uint16_t)zs;
-            const int g = zc / 64;
-            p.y1_sf[((grow / 128) * (size_t)(Ny / 128) + g / 4) * 512 + (grow % 32) * 16 + ((grow % 128) / 32) * 4 +
-                    (g % 4)] = (uint8_t)e;
+          if (lane == 0) {
+            if (p.z_fp8 != nullptr) tma_store_2d(&tmap_c, stg, zc, t.m0 + q * 32);     // z e4m3 [rows, 2I]
+            tma_store_2d(&tmap_c2, stg + 2048, zc / 2, t.m0 + q * 32);     // y1 e4m3 [rows, I]
+            bulk_commit_group();
           }
+          if (p.z_fp8 != nullptr) *reinterpret_cast<uint16_t*>(p.z_sc + grow * (Nz / 32) + zc / 32) = (uint16_t)zs;
+          const int g = zc / 64;
+          p.y1_sf[((grow / 128) * (size_t)(Ny / 128) + g / 4) * 512 + (grow % 32) * 16 + ((grow % 128) / 32) * 4 +
+                  (g % 4)] = (uint8_t)e;
         }
       } else if (MODE == DGATEDQ) {
         // D columns [c_base, c_base + BN/2) in chunks of 32.  Per chunk dz (64 columns) and y1s (32 columns)
@@ -974,7 +952,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         // columns instead of eight of 96 cost 2 % more.)
         // a ragged last column tile (N not a multiple of BN): chunks at or beyond column N hold products with
         // rows of the next expert's weights (or TMA zero fill) and are skipped whole (N is a multiple of 32)
-        if (t.valid && c_base < p.N && !(p.debug_skip_store & 2)) {
+        if (t.valid && c_base < p.N) {
           const int Nz = 2 * p.N;
           const float s = s_row;
           const int row_grp = (t.m0 + q * 32) >> 5;      // 32-row group index along TKp
@@ -1087,7 +1065,6 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                            wy[4 * j + 2], wy[4 * j + 3]);
             fence_proxy_async_smem();
             __syncwarp();
-            if (p.debug_skip_store & 1) continue;
             if (lane == 0) {
               tma_store_2d(&tmap_c, stg, 2 * dcol, t.m0 + q * 32);          // dz e4m3 [TKp, 2I]
               tma_store_2d(&tmap_c2, stg + 2048, dcol, t.m0 + q * 32);      // y1s e4m3 [TKp, I]

@@ -126,7 +126,7 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int n_total = (MODE == WGRAD) ? p.E * ((p.rows + p.rows2) / (2 * BM)) * n_col_tiles
                                       : s_pairs[p.E] * n_col_tiles;
   const bool a_mn = MODE == WGRAD && p.a_mn;
-  const int nst = S::STAGES - p.dbg_stage_cut;      // timing experiment: a shallower ring (0 in product use)
+  constexpr int nst = S::STAGES;
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs): warp-uniform loops, one
@@ -137,8 +137,6 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
     const uint32_t full0 = map_to_cta(bar_full, 0);
     const int n_total_u = __shfl_sync(0xffffffffu, n_total, 0);
-    const bool dbg_noload = (p.debug_skip_store & 4) != 0;   // timing experiment: operands fetched for one ring pass only
-    int dbg_filled = 0;
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -166,17 +164,12 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         const uint32_t full = full0 + 8 * stage;
         const uint32_t a_dst = smem_base + stage * S::STAGE_BYTES;
         const uint32_t b_dst = a_dst + S::A_BYTES;
-        if (dbg_noload && dbg_filled >= nst) {
-          if (rank == 0 && elect_one()) mbar_arrive(bar_full + 8 * stage);
-        } else {
-          ++dbg_filled;
-          if (elect_one()) {
-            if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, tx_bytes);
-            if (a_mn) tma_load_2d_pair(a_dst, ta, full, m0, kt * BK);
-            else if (!(phantom && rank == 1)) tma_load_2d_pair(a_dst, ta, full, kt * BK, a_row);
-            tma_load_2d_pair(b_dst, tb, full, kt * BK, b_row);
-            tma_load_2d_pair(b_dst + S::BH_BYTES, tb, full, kt * BK, b_row + HN);
-          }
+        if (elect_one()) {
+          if (rank == 0) mbar_expect_tx(bar_full + 8 * stage, tx_bytes);
+          if (a_mn) tma_load_2d_pair(a_dst, ta, full, m0, kt * BK);
+          else if (!(phantom && rank == 1)) tma_load_2d_pair(a_dst, ta, full, kt * BK, a_row);
+          tma_load_2d_pair(b_dst, tb, full, kt * BK, b_row);
+          tma_load_2d_pair(b_dst + S::BH_BYTES, tb, full, kt * BK, b_row + HN);
         }
         if (++stage == nst) { stage = 0; phase ^= 1; }
       }
@@ -199,9 +192,6 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       int stage = 0, sfs = 0;
       uint32_t phase = 0, aphase = 0, sfphase = 0;
       bool ok = true;
-      // K tiles issued half-by-half at both ends of a tile (a timing experiment may shorten it)
-      const int JJ = (p.l2_prefetch >= 0 && p.l2_prefetch < kHeadTail3) ? p.l2_prefetch : kHeadTail3;
-
       // MMAs of K tile number k (of its tile) held in ring stage st, into accumulator half h
       auto issue_half = [&](int st, int k, int h) {
         const uint32_t a_lo = a_lo0 + st * (S::STAGE_BYTES >> 4);
@@ -214,15 +204,11 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                            (k | kb) != 0);
       };
 
-      long long* trace = (pair_id == 0) ? p.trace : nullptr;      // timing experiment, null in product use
-      int trace_n = 0;
       for (int tile = pair_id; tile < n_total_u && ok; tile += n_pairs_grid) {
         const PairTile t = pair_tile<BN, MODE>(tile, 0, p, s_efo, s_pairs);
         const int nkt = __shfl_sync(0xffffffffu, t.nkt, 0);
         if (nkt == 0) continue;
-        const long long tr0 = trace ? clock64() : 0;
-        long long tr_full = 0, tr_sf = 0, tr_acc1 = 0, tr_first = 0;
-        const int J = nkt >= 2 * JJ ? JJ : 0;
+        const int J = nkt >= 2 * kHeadTail3 ? kHeadTail3 : 0;      // K tiles issued half-by-half at both ends of a tile
         int held0 = 0, held1 = 0;             // ring stages of the K tiles whose half-1 MMAs are still to come
         static_assert(kHeadTail3 == 2, "held0 / held1");
         ok = __all_sync(0xffffffffu, mbar_wait(bar_tempty, aphase ^ 1));
@@ -232,36 +218,25 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (!ok) break;
         }
         tc_fence_after();
-        const long long tr1 = trace ? clock64() : 0;
         for (int k = 0; k < nkt; ++k) {
           // first touch of K tile k: its operands and scales have landed; scales go to TMEM; half 0 always,
           // half 1 too unless the K tile belongs to the head or the tail of the tile
           const int kg = k & (S::SF_GROUP - 1);
           if (kg == 0) {
-            const long long c0 = trace ? clock64() : 0;
             ok = __all_sync(0xffffffffu, mbar_wait(bar_sffull + 8 * sfs, sfphase));
             if (!ok) break;
-            if (trace) tr_sf += clock64() - c0;
           }
-          const long long c1 = trace ? clock64() : 0;
           ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * stage, phase));
           if (!ok) break;
-          if (trace) {
-            const long long d = clock64() - c1;
-            tr_full += d;
-            if (k == 0) tr_first = d;
-          }
           const bool both = (k >= J && k < nkt - J);
           const bool sf_done = (kg == S::SF_GROUP - 1 || k == nkt - 1);
           const uint32_t sf_lo = sf_lo0 + ((sfs * S::SF_SLOT_BYTES + kg * 512) >> 4);
           const uint32_t sfa_t = tmem_base + S::SF_COL0 + stage * S::SF_COLS;
           if (elect_one()) {
-            if (!(p.debug_skip_store & 16)) {
-              tc_cp_sf_pair_lo(sfa_t, sf_lo, sf_hi);
+            tc_cp_sf_pair_lo(sfa_t, sf_lo, sf_hi);
 #pragma unroll
-              for (int j = 0; j < S::SFB_TILES; ++j)
-                tc_cp_sf_pair_lo(sfa_t + 4 + 4 * j, sf_lo + ((S::SF_GROUP * 512 * (1 + j)) >> 4), sf_hi);
-            }
+            for (int j = 0; j < S::SFB_TILES; ++j)
+              tc_cp_sf_pair_lo(sfa_t + 4 + 4 * j, sf_lo + ((S::SF_GROUP * 512 * (1 + j)) >> 4), sf_hi);
             if (sf_done) tc_commit_pair(bar_sfempty + 8 * sfs, 3);   // the copies above were the slot's last readers
             issue_half(stage, k, 0);
             if (both) {
@@ -279,11 +254,9 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           // end of the head / of the tail: the half-1 MMAs of the K tiles held back
           const bool head_end = (J > 0 && k == J - 1), tail_end = (J > 0 && k == nkt - 1);
           if (head_end) {
-            const long long c2 = trace ? clock64() : 0;
             ok = __all_sync(0xffffffffu, mbar_wait(bar_tempty + 8, aphase ^ 1));
             if (!ok) break;
             tc_fence_after();
-            if (trace) tr_acc1 = clock64() - c2;
           }
           if (head_end || tail_end) {
             if (elect_one()) {
@@ -303,20 +276,6 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (J == 0) tc_commit_pair(bar_tfull, 3);
           tc_commit_pair(bar_tfull + 8, 3);
         }
-        if (trace) {
-          // how long the tensor pipe still works on what has been issued: wait for this tile's last commit here
-          const long long c3 = clock64();
-          long long drain0 = 0;
-          if (J > 0) { mbar_wait(bar_tfull, aphase); drain0 = clock64() - c3; }
-          mbar_wait(bar_tfull + 8, aphase);
-          const long long drain = clock64() - c3;
-          if (trace_n < 256 && lane == 0) {
-            long long* r = trace + 8 * trace_n;
-            r[0] = tr0; r[1] = tr1; r[2] = tr_full; r[3] = tr_sf; r[4] = tr_acc1; r[5] = c3; r[6] = drain0;
-            r[7] = nkt | (drain << 16);
-          }
-        }
-        ++trace_n;
         aphase ^= 1;
       }
       if (!ok && lane == 0) { *s_abort = 1; atomicCAS(p.status, 0, 202); }
@@ -381,14 +340,9 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     uint32_t aphase = 0;
     int buf = 0;
     bool ok = true;
-    // timing experiment: the first epilogue warp of the leader CTA of pair 0 stamps its side of the hand-over
-    long long* etrace = (p.trace != nullptr && pair_id == 0 && rank == 0 && warp == S::LEAD_WARPS && lane == 0)
-                            ? p.trace + 8 * 256 : nullptr;
-    int etrace_n = 0;
     for (int tile = pair_id; tile < n_total && ok; tile += n_pairs_grid) {
       const PairTile t = pair_tile<BN, MODE>(tile, rank, p, s_efo, s_pairs);
       const size_t grow = (size_t)t.m0 + row_in_tile;
-      long long es[6] = {0, 0, 0, 0, 0, 0};
       if (t.nkt == 0) {
         if (MODE == WGRAD && p.out_bf16) {
           uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.c) +
@@ -412,44 +366,28 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         uint32_t pk[2][NC][16];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          if (etrace && h == 0) es[0] = clock64();
           if (lane == 0) ok = mbar_wait(bar_tfull + 8 * h, aphase);
           ok = __shfl_sync(0xffffffff, ok, 0);
           if (!ok) break;
-          if (etrace && h == 0) es[1] = clock64();
           tc_fence_after();
-          if (!(p.debug_skip_store & 8)) {
-            // all of this warp's columns of the half in one go (one wait), the accumulator is handed back before
-            // the conversion: the drain is what the next tile's MMAs wait for
-            const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + h * HN + grp * CPW;
-            uint32_t r[NC][32];
+          // all of this warp's columns of the half in one go (one wait), the accumulator is handed back before
+          // the conversion: the drain is what the next tile's MMAs wait for
+          const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + h * HN + grp * CPW;
+          uint32_t r[NC][32];
 #pragma unroll
-            for (int c = 0; c < NC; ++c) tmem_ld32(t_row + c * 32, r[c]);
-            if (etrace && h == 0) es[3] = clock64();            // (experiment: loads issued)
-            tmem_ld_wait();
-            if (etrace && h == 0) es[4] = clock64();            // (experiment: loads complete)
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster_relaxed(tempty0 + 8 * h);
-            if (etrace && h == 0) es[2] = clock64();
+          for (int c = 0; c < NC; ++c) tmem_ld32(t_row + c * 32, r[c]);
+          tmem_ld_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_relaxed(tempty0 + 8 * h);
 #pragma unroll
-            for (int c = 0; c < NC; ++c)
+          for (int c = 0; c < NC; ++c)
 #pragma unroll
-              for (int i = 0; i < 16; ++i)
-                pk[h][c][i] = pack_bf16x2(__uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1]));
-          } else {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster_relaxed(tempty0 + 8 * h);
-          }
+            for (int i = 0; i < 16; ++i)
+              pk[h][c][i] = pack_bf16x2(__uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1]));
         }
         if (!ok) break;
-        if (etrace && etrace_n < 256) {
-#pragma unroll
-          for (int i = 0; i < 6; ++i) etrace[8 * etrace_n + i] = es[i];
-        }
-        ++etrace_n;
-        if (live && !(p.debug_skip_store & 8)) {
+        if (live) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
 #pragma unroll
@@ -484,17 +422,13 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (!ok) break;
           tc_fence_after();
           uint32_t acc[NC][32];
-          const bool drain = !(p.debug_skip_store & 8);
-          if (drain) {
-            const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + h * HN + grp * CPW;
+          const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + h * HN + grp * CPW;
 #pragma unroll
-            for (int c = 0; c < NC; ++c) tmem_ld32(t_row + c * 32, acc[c]);
-            tmem_ld_wait();
-          }
+          for (int c = 0; c < NC; ++c) tmem_ld32(t_row + c * 32, acc[c]);
+          tmem_ld_wait();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster_relaxed(tempty0 + 8 * h);
-          if (!drain) continue;
           if (p.out_bf16) {
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
