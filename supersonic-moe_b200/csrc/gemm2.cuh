@@ -19,7 +19,8 @@ constexpr int kMaxExperts2 = 256;   // expert offsets cached in shared memory by
 // instead 530, but no longer safe against a second writer.
 // A tile of few K tiles is bound by this traffic, one of many by its MMAs, which the prefetches then slow down.  dw1 + dw2 in
 // one launch, E=8 M=3072 + 1536 N=3072, by K tiles per expert, us: 8 210 -> 185, 16 246 -> 236, 20 270 -> 264, 24 294 -> 294,
-// 32 353 -> 359, 48 493 -> 507, 64 639 -> 656; E=128 M=1536 N=2048 of skewed load, dw1 935 -> 880; E=32, 8 K tiles 824 -> 671.
+// 32 353 -> 359, 48 493 -> 507, 64 639 -> 656; E=32, 8 K tiles 824 -> 671; dw1 alone, E=128 M=1536 N=2048, 131072 rows: even load,
+// 8 K tiles, 730 -> 576, Zipf(1.2), most experts one K tile, 801 -> 771; E=8 M=N=6144, 3 K tiles, 572 -> 461.
 constexpr int kReduceAhead = 2;          // pieces
 constexpr int kReduceAheadKTiles = 20;   // K tiles of a tile up to which it is done
 constexpr int kSfGroup2 = 4;        // K tiles whose scales travel in one TMA copy (box rows of the scale tensor maps)

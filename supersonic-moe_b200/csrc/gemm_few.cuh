@@ -283,7 +283,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
           float* am = s_amax + buf * 64;
           if (lane < 16) am[q * 16 + lane] = mine;
           asm volatile("bar.sync %0, 64;" ::"r"(1 + (q >> 1)) : "memory");
-          // of column lane & 15; a group of nothing but NaN has the scale of zeros, as in the other kernels, whose maxima begin at 0
+          // of column lane & 15; a group of nothing but NaN has the scale of zeros, as in the other kernels (maxima from 0 on)
           const int e = e8m0_of(fmaxf(fmaxf(mine, am[(q ^ 1) * 16 + (lane & 15)]), 0.f));
           const float qs_mine = qscale_of(e);
           buf ^= 1;           // the other buffer next: this one is written again only after one more barrier

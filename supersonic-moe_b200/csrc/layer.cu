@@ -170,7 +170,8 @@ static int wgrad(const void* A, const void* A_sf, bool a_rows, const void* B, co
 //   More: a busy expert's weights are fetched once per 64 rows where the other form needs one pass per 256.  Few rows on average
 //   and a bound on what one slot, and all K, put on the same experts keep that small.  Whole forward, replayed from a graph, cold
 //   L2, general / this, us (even load; Zipf(1.2), mean of three; all tokens on the same K experts), admitted | beyond the rule:
-//     E=128 H=2048 I=768 K=8   T=160  168 / 139, 102 / 95, 49 / 52  |  T=320  168 / 146, 117 / 120, 57 / 78;  640  174 / 162, 141 / 178, 65 / 121
+//     E=128 H=2048 I=768 K=8   T=160  168 / 139, 102 / 95, 49 / 52  |  T=320  168 / 146, 117 / 120, 57 / 78
+//                                                                      T=640  174 / 162, 141 / 178, 65 / 121
 //     E=128 H=2048 I=768 K=1   T=576  168 / 139, 60 / 51, 43 / 37   |  T=5120  186 / 170, 98 / 154, 72 / 131
 //     E=256 H=2048 I=768 K=4   T=320  303 / 238, 89 / 85, 47 / 55   |  T=576  303 / 238, 95 / 104, 53 / 70
 //     E=128 H=4096 I=1536 K=4  T=160  509 / 407, 168 / 162, 66 / 84 |  T=256  520 / 420, 183 / 194, 63 / 106
