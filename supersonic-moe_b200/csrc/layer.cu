@@ -175,7 +175,7 @@ static int wgrad(const void* A, const void* A_sf, bool a_rows, const void* B, co
 //     E=128 H=2048 I=768 K=1   T=576  168 / 139, 60 / 51, 43 / 37   |  T=5120  186 / 170, 98 / 154, 72 / 131
 //     E=256 H=2048 I=768 K=4   T=320  303 / 238, 89 / 85, 47 / 55   |  T=576  303 / 238, 95 / 104, 53 / 70
 //     E=128 H=4096 I=1536 K=4  T=160  509 / 407, 168 / 162, 66 / 84 |  T=256  520 / 420, 183 / 194, 63 / 106
-//   Over the 208 points measured that the rule admits (9 layer sizes, 8 to 256 experts, K = 1 to 8) an even load gains 6 to 47 %
+//   Over the 208 points measured that the rule admits (10 layer sizes, 8 to 256 experts, K = 1 to 8) an even load gains 6 to 47 %
 //   (median 24), one slot of every token on one expert 0 to 43 (20), a Zipf load 19 in the median and loses at most 6 (one draw of
 //   three, 125 / 133); all K slots of all tokens on the same experts, as identical tokens have it, gains 12 in the median and loses
 //   at worst a quarter of calls as short as those above.

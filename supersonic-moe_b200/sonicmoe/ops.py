@@ -172,14 +172,13 @@ def topk_metadata(idx, probs, E, alignment=128, TK_alloc=None, TKp_alloc=None, l
     if TKp_alloc is None:
         TKp_alloc = -(-TK_alloc // alignment) * alignment + E * alignment
     # A tensor each: callers keep some, write to some and save others for a backward.  16384 x 8 over 128 experts, us a call, bound
-    # by the host: a `torch.empty` each 30.8, `new_empty` 29.4; views of one tensor, which share a version counter and a lifetime
-    # and start anywhere, 27.1.
-    TK, TKp = max(int(TK_alloc), 0), max(int(TKp_alloc), 0)
-    x_gather = torch.empty(TKp, dtype=_I32, device=idx.device)
-    e = x_gather.new_empty
-    s_scatter, s_rev, src_idx, efo, naept, counts = e(TKp), e(TK), e(TK), e(E + 1), e(N + 1), e(E)
+    # by the host: a `torch.empty` each 30.8, `new_empty` of the indices 28.7; views of one tensor, which share a version counter and
+    # a lifetime and start anywhere, 27.1.  (The method of a subclass of Tensor would return that subclass.)
+    TK, TKp = max(TK_alloc, 0), max(TKp_alloc, 0)
+    e = (idx if type(idx) is torch.Tensor else torch.empty(0, dtype=_I32, device=idx.device)).new_empty
+    x_gather, s_scatter, s_rev, src_idx, efo, naept, counts = e(TKp), e(TKp), e(TK), e(TK), e(E + 1), e(N + 1), e(E)
     scores = e(TKp, dtype=torch.float32)
-    ws = e(lib.smoe_topk_metadata_workspace(N, E), dtype=_U8)
+    ws = e(lib.smoe_topk_metadata_workspace(N, E) // 4)
     check(lib.smoe_topk_metadata(idx.data_ptr(), probs.data_ptr(), N, K, E, alignment, TK_alloc, TKp_alloc, lane_order, pad_mode,
                                  efo.data_ptr(), x_gather.data_ptr(), s_scatter.data_ptr(), s_rev.data_ptr(), naept.data_ptr(),
                                  scores.data_ptr(), src_idx.data_ptr(), counts.data_ptr(), ws.data_ptr(), _stream()),
