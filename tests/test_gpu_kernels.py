@@ -1016,6 +1016,33 @@ def test_two_weight_gradients_in_one_launch_give_the_bits_of_two_launches(ops):
                 assert bool((o1[1] == 0).all()) and bool((o2[1] == 0).all())      # the empty expert
 
 
+@pytest.mark.parametrize("order", ["rows", "columns", "mixed"])
+def test_quantizers_on_every_finite_bf16_value(ops, order):
+    """All bf16 bit patterns (both zeros and the subnormals among them; infinities and NaN are zero here), bit for bit:
+    neighbours in magnitude together in a row group or in a column group, so that every exponent and mantissa is a group's
+    maximum, or mixed, so that small values meet large scales."""
+    bits = torch.arange(65536, dtype=torch.int32).to(torch.int16)
+    v = bits.view(torch.bfloat16)
+    v = torch.where(torch.isfinite(v), v, torch.zeros_like(v))
+    v = v[torch.argsort(v.float().abs(), stable=True)]
+    if order == "mixed":
+        x = v[torch.randperm(65536, generator=torch.Generator().manual_seed(1))].view(512, 128)
+    else:
+        x = v.view(512, 128) if order == "rows" else v.view(128, 16, 32).permute(1, 2, 0).reshape(512, 128)
+    x = x.contiguous()
+    xd = x.to(DEV)
+    rq, rs = Q.row_quant(x)
+    cq, cs = Q.col_quant(x)
+    q, ri, q_t, ci = ops.quant_weight(xd[None])
+    assert torch.equal(q[0].cpu(), rq) and torch.equal(Q.unpack_isa(ri.cpu(), 512, 128), rs)
+    assert torch.equal(q_t[0].t().cpu(), cq) and torch.equal(Q.unpack_isa(ci.cpu(), 128, 512), cs)
+    q_t, ci = ops.quant_cols_t(xd, None, 512)
+    assert torch.equal(q_t.t().cpu(), cq) and torch.equal(Q.unpack_isa(ci.cpu(), 128, 512), cs)
+    x2 = torch.cat([xd, xd], 1).contiguous()                            # the row-major form wants multiples of 256 columns
+    _, _, qc, ci = ops.quant_dual_gather(x2, None, 512, with_rows=False)
+    assert torch.equal(qc.cpu(), torch.cat([cq, cq], 1)) and torch.equal(Q.unpack_isa(ci.cpu(), 256, 512), torch.cat([cs, cs]))
+
+
 @pytest.mark.parametrize("E,N,K", [(1, 128, 128), (3, 256, 128), (2, 384, 512), (5, 128, 640)])
 def test_quant_weight_both_orientations_from_one_read(ops, E, N, K):
     """Bytes and scales of the row quantizer over W and over W^T, in one pass or one orientation at a time."""
