@@ -82,20 +82,38 @@ __global__ void ds_finalize_kernel(const float* __restrict__ part, int partials,
   if (ds) ds[i] = a;
 }
 
-// The same sums, written to the token's slots: a thread per (token, slot) looks for its entry among the token's, so that slots
-// without one (masked) get their zero here and not from a memset before.
-__global__ void ds_slots_kernel(const float* __restrict__ part, int partials, int64_t rows, const int* __restrict__ s_rev,
-                                const int* __restrict__ naept, const int* __restrict__ src_idx, int64_t slots, int K,
-                                float* __restrict__ ds) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// The same sums, written to the token's slots.  A block takes 64 slots of the table: it first puts the entries of their tokens down at
+// the slots they came from, so that a slot finds its entry with one look (or none: masked, zero) and every store is in order.
+// Bound by latency (a few hundred bytes a thread in a chain of loads), so blocks are small and a thread's partial sums are loaded
+// eight at a time, added in order.  Against a thread searching its token's entries, in blocks of 256, T=1024, K=8, 16 partials:
+// 20.5 -> 10.3 us between events, from a cold L2.
+constexpr int kDsSlots = 64;
+
+__global__ void __launch_bounds__(kDsSlots)
+ds_slots_kernel(const float* __restrict__ part, int partials, int64_t rows, const int* __restrict__ s_rev,
+                const int* __restrict__ naept, const int* __restrict__ src_idx, int64_t slots, int K, float* __restrict__ ds) {
+  __shared__ int s_entry[kDsSlots];
+  const int64_t i0 = blockIdx.x * (int64_t)kDsSlots, i = i0 + threadIdx.x;
+  s_entry[threadIdx.x] = -1;
+  __syncthreads();
+  const int64_t t0 = i0 / K, t1 = (min(i0 + kDsSlots, slots) - 1) / K;
+  for (int j = naept[t0] + threadIdx.x, end = naept[t1 + 1]; j < end; j += kDsSlots) {
+    const int64_t at = src_idx[j] - i0;
+    if (at >= 0 && at < kDsSlots) s_entry[at] = j;
+  }
+  __syncthreads();
   if (i >= slots) return;
-  const int64_t t = i / K;
   float a = 0.f;
-  for (int j = naept[t], end = naept[t + 1]; j < end; ++j) {
-    if (src_idx[j] != (int)i) continue;
-    const int64_t p = s_rev[j];
-    for (int q = 0; q < partials; ++q) a += part[(int64_t)q * rows + p];
-    break;
+  const int j = s_entry[threadIdx.x];
+  if (j >= 0) {
+    const float* p = part + s_rev[j];
+    for (int q0 = 0; q0 < partials; q0 += 8) {
+      float v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = q0 + q < partials ? p[(int64_t)(q0 + q) * rows] : 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) if (q0 + q < partials) a += v[q];
+    }
   }
   ds[i] = a;
 }
@@ -357,8 +375,8 @@ int smoe_ds_slots(const float* ds_partial, int64_t partials, int64_t rows, const
   if (T < 0 || K <= 0 || partials < 0 || T * K >= (int64_t)1 << 31) return SMOE_ERR_SHAPE;
   if (T == 0) return SMOE_OK;
   if (!naept || !ds || (rows > 0 && (!ds_partial || !s_rev || !src_idx))) return SMOE_ERR_ARG;      // no rows: all slots 0
-  ds_slots_kernel<<<(unsigned)((T * K + 255) / 256), 256, 0, (cudaStream_t)stream>>>(ds_partial, (int)partials, rows, s_rev,
-                                                                                  naept, src_idx, T * K, (int)K, ds);
+  ds_slots_kernel<<<(unsigned)((T * K + kDsSlots - 1) / kDsSlots), kDsSlots, 0, (cudaStream_t)stream>>>(
+      ds_partial, (int)partials, rows, s_rev, naept, src_idx, T * K, (int)K, ds);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 

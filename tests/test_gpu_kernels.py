@@ -1178,7 +1178,7 @@ def test_forward_gemms_for_few_rows_match_the_general_kernels(ops, counts, H, I)
     assert cos > 0.9999 and rr < 4e-3, (cos, rr)
 
 
-@pytest.mark.parametrize("T,K,E,I", [(200, 4, 6, 256), (33, 2, 5, 512)])
+@pytest.mark.parametrize("T,K,E,I", [(200, 4, 6, 256), (33, 2, 5, 512), (77, 5, 7, 256)])
 def test_scores_and_ds_by_index_match_the_separate_kernels(ops, T, K, E, I):
     """GemmDGated looking up a row's score itself against a gathered copy, and ds summed straight into the top-k table's slots
     against the scatter over a cleared table: the same bits, masked slots zero."""
