@@ -119,7 +119,8 @@ static int pick_bn(int64_t N) {
 
 // ---- two-CTA kernel -----------------------------------------------------------
 struct OutMaps {
-  CUtensorMap c, c2, c3;
+  CUtensorMap c, c2;
+  CUtensorMap bh;       // B in boxes of half a tile's rows (half tiles of the 256-column kernel)
 };
 
 template <int BN, int MODE, bool CPG = false>
@@ -130,11 +131,12 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   auto kern = gemm2_mxf8_kernel<BN, MODE, CPG>;
   if (!ensure_smem_attr(kern, S::TOTAL, attr_set)) return SMOE_ERR_LAUNCH;
   int64_t pairs = sm_count() / 2;
-  if (max_pair_tiles < pairs) pairs = max_pair_tiles;
+  const int64_t units = S::HALVES && !p.b_mn ? 2 * max_pair_tiles : max_pair_tiles;
+  if (units < pairs) pairs = units;
   if (pairs <= 0) return SMOE_OK;
   GemmParams q = p;
   if (MODE == WGRAD && p.accumulate && !p.out_bf16) q.stages_lent = S::LENT_STAGES;
-  kern<<<(unsigned)(2 * pairs), S::THREADS, S::TOTAL, stream>>>(ta, tb, tsa, tsb, om.c, om.c2, om.c3, q);
+  kern<<<(unsigned)(2 * pairs), S::THREADS, S::TOTAL, stream>>>(ta, tb, tsa, tsb, om.c, om.c2, om.bh, q);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 
@@ -252,12 +254,14 @@ static int pick_bn2(int64_t N) {
 
 template <int MODE>
 static int run2(const void* a, int64_t a_rows, int64_t a_cols, const void* b, int64_t b_rows, int64_t b_cols,
-                GemmParams& p, const OutMaps& om, int bn, int64_t sfa_tiles, int64_t sfb_tiles, cudaStream_t stream) {
+                GemmParams& p, OutMaps& om, int bn, int64_t sfa_tiles, int64_t sfb_tiles, cudaStream_t stream) {
   CUtensorMap ta, tb, tsa, tsb;
   const bool gather = p.a_idx != nullptr;
   int rc = make_tmap_u8(&ta, a, a_rows, a_cols, BK, gather ? 1 : BM);
   if (rc) return rc;
   rc = make_tmap_u8(&tb, b, b_rows, b_cols, BK, bn / 2);
+  om.bh = tb;
+  if (!rc && bn == 256 && (MODE == PLAIN || MODE == GATED) && !p.b_mn) rc = make_tmap_u8(&om.bh, b, b_rows, b_cols, BK, bn / 4);
   if (rc) return rc;
   rc = make_tmap(&tsa, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, p.sfa, sfa_tiles, 128, 128, kSfGroup2,
                  CU_TENSOR_MAP_SWIZZLE_NONE);
@@ -331,7 +335,6 @@ static int run(const void* a, int64_t a_rows, int64_t a_cols, const void* b, int
           rc = make_tmap(&om.c, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.z_fp8, p.rows, p.N, 64, 32, CU_TENSOR_MAP_SWIZZLE_64B);
       }
       if (rc) return rc;
-      om.c3 = om.c;
       return run2<MODE>(a, a_rows, a_cols, b, b_rows, b_cols, p, om, bn2, sfa_tiles, sfb_tiles, stream);
     }
   }

@@ -275,6 +275,7 @@ struct Gemm2Smem {
   static_assert(LENT_STAGES * STAGE_BYTES >= EPI_WARPS * LENT_TILE, "every epilogue warp has a staging tile");
   static_assert(MODE != WGRAD || STAGES - LENT_STAGES >= 4, "a ring is left (the timing experiments cut three stages more)");
   static constexpr int ACC_STAGES = (BN == 256) ? 1 : 2;  // TMEM: 512 columns
+  static constexpr bool HALVES = BN == 256 && (MODE == PLAIN || MODE == GATED);    // half tiles at the end of a launch
   static constexpr int SF_COLS = 4 + 4 * SFB_TILES;
   static constexpr int SF_COL0 = ACC_STAGES * BN;
   static_assert(SF_COL0 + STAGES * SF_COLS <= 512, "TMEM budget");
@@ -291,6 +292,7 @@ struct PairTile {
   int kt0, nkt; // K-tile range
   int valid;    // 0: this CTA's half lies beyond its expert's rows - compute, store nothing
   int prob;     // WGRAD with two products in one launch: which one this tile belongs to
+  int cols;     // columns (BN, or half of them at the end of a launch: see `tile_of`)
 };
 
 // varlen-M: experts own ceil(n_e / 2) row pairs; s_pairs = exclusive prefix of that.
@@ -298,6 +300,7 @@ template <int BN, int MODE>
 __device__ __forceinline__ PairTile pair_tile(int tile, int rank, const GemmParams& p, const int* s_efo,
                                               const int* s_pairs) {
   PairTile t;
+  t.cols = BN;
   const int n_tiles = (p.N + BN - 1) / BN;     // DGATEDQ may run a ragged last column tile
   t.prob = 0;
   if (MODE == WGRAD) {
@@ -372,7 +375,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((Gemm2Smem<BN, MODE,
 gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
                   const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_c2,
-                  const __grid_constant__ CUtensorMap tmap_c3, const GemmParams p) {
+                  const __grid_constant__ CUtensorMap tmap_bh, const GemmParams p) {
   using S = Gemm2Smem<BN, MODE, CPG>;
   const bool GATHER = !CPG && p.a_idx != nullptr;   // rows of A fetched by index with TMA gather4 vs. a plain tile
   extern __shared__ uint8_t smem_raw[];
@@ -383,6 +386,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   uint64_t* bars = reinterpret_cast<uint64_t*>(aux);     // full[S], empty[S], tfull[2], tempty[2], sffull[2], sfempty[2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux + 496);
   volatile int* s_abort = reinterpret_cast<volatile int*>(aux + 500);
+  volatile int* s_tiles = reinterpret_cast<volatile int*>(aux + 504);    // number of whole tiles, number of tiles of either kind
   int* s_efo = reinterpret_cast<int*>(aux + 512);
   int* s_pairs = s_efo + (kMaxExperts2 + 1);
 
@@ -401,7 +405,23 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   for (int i = threadIdx.x; i <= p.E; i += blockDim.x) s_efo[i] = p.efo[i];
   __syncthreads();
-  if (warp == 2) prefix_row_pairs(s_efo, s_pairs, p.E, lane);
+  if (warp == 2) {
+    prefix_row_pairs(s_efo, s_pairs, p.E, lane);
+    __syncwarp();
+    if (lane == 0) {
+      const int n_col_tiles = (p.N + BN - 1) / BN;
+      const int n_total = (MODE == WGRAD) ? p.E * (p.rows / (2 * BM)) * n_col_tiles : s_pairs[p.E] * n_col_tiles;
+      // A last wave of few tiles keeps the other CTA pairs waiting for a whole tile.  Where there are at most half as many left
+      // as pairs, each is done as two tiles of half the columns (B K-major: the halves have a tensor map of their own).
+      // us, H=3072, I=1536, E=8, up-projection / down-projection / dx: 1024 rows an expert (384 tiles, 14 left) 81.3 / 47.1 / 70.8 ->
+      // 78.1 / 45.4 / 69.9, 2048 rows (28 left) 146.4 / 81.7 / 132.2 -> 144.1 / 80.3 / 131.2, 128 rows 37.8 / 22.9 / 33.1 -> 35.0 /
+      // 20.9 / 31.1; H=6144, I=3072, 384 rows (14 left) 161.4 / 84.3 / 141.7 -> 156.1 / 82.0 / 138.4.  With more left than that no
+      // pair would have less to do.
+      const int left = S::HALVES && !p.b_mn ? n_total % n_pairs_grid : 0;
+      s_tiles[0] = 2 * left <= n_pairs_grid ? n_total - left : n_total;
+      s_tiles[1] = 2 * n_total - s_tiles[0];
+    }
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::STAGES; ++s) {
       mbar_init(bar_full + 8 * s, S::FULL_ARRIVALS);   // leader's: its producer arms it, both CTAs' copies credit it
@@ -431,9 +451,17 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t sf_base = smem_u32(sfring);
-  const int n_col_tiles = (p.N + BN - 1) / BN;
-  const int n_total = (MODE == WGRAD) ? p.E * (p.rows / (2 * BM)) * n_col_tiles : s_pairs[p.E] * n_col_tiles;
   const int nst = S::STAGES - p.stages_lent;       // ring stages in use
+  auto tile_of = [&](int u, int r) {
+    const int n_full = S::HALVES ? s_tiles[0] : 0;
+    const bool half = S::HALVES && u >= n_full;
+    PairTile t = pair_tile<BN, MODE>(half ? n_full + ((u - n_full) >> 1) : u, r, p, s_efo, s_pairs);
+    if (half) {
+      t.cols = BN / 2;
+      t.n0 += ((u - n_full) & 1) * (BN / 2);
+    }
+    return t;
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
@@ -441,16 +469,17 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // per-lane state (four row indices each).
     if (lane == 0) {
       prefetch_tmap(&tmap_a); prefetch_tmap(&tmap_b);
+      if (S::HALVES && s_tiles[1] > s_tiles[0]) prefetch_tmap(&tmap_bh);
     }
     const uint32_t full0 = map_to_cta(bar_full, 0);      // the leader's full barriers
-    const int n_total_u = __shfl_sync(0xffffffffu, n_total, 0);
+    const int n_work_u = __shfl_sync(0xffffffffu, s_tiles[1], 0);
     // MN-major operands: both of a weight gradient, or the B of a PLAIN product whose weights lie [E, K, N]
     const bool a_mn = MODE == WGRAD && p.a_mn, b_mn = (MODE == WGRAD || MODE == PLAIN) && p.b_mn;
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int tile = pair_id; tile < n_total_u && ok; tile += n_pairs_grid) {
-      const PairTile tl = pair_tile<BN, MODE>(tile, rank, p, s_efo, s_pairs);
+    for (int tile = pair_id; tile < n_work_u && ok; tile += n_pairs_grid) {
+      const PairTile tl = tile_of(tile, rank);
       const int nkt = __shfl_sync(0xffffffffu, tl.nkt, 0);
       if (nkt == 0) continue;
       const int kt0 = __shfl_sync(0xffffffffu, tl.kt0, 0);
@@ -461,15 +490,17 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       int4 rows4 = make_int4(0, 0, 0, 0);
       if (GATHER && valid) rows4 = *reinterpret_cast<const int4*>(p.a_idx + m0 + 4 * lane);
       const int b_base = (MODE == WGRAD) ? n0 : te * p.N + n0;
+      const int cols = S::HALVES ? __shfl_sync(0xffffffffu, tl.cols, 0) : BN;
+      const CUtensorMap* tb = cols == BN ? &tmap_b : &tmap_bh;
       const bool b_mn_plain = MODE == PLAIN && b_mn;       // B of expert te = rows [te*K, (te+1)*K) of an [E*K, N] matrix
-      const int b_row = (b_mn_plain ? n0 : b_base) + rank * (BN / 2);
+      const int b_row = (b_mn_plain ? n0 : b_base) + rank * (cols / 2);
       const int b_k0 = b_mn_plain ? te * p.K : 0;
       const int a_row = valid ? m0 : 0;
       // an expert with an odd number of row tiles: the pair's second half is a phantom, whose A rows need not be
       // fetched (whatever its ring slots hold only reaches accumulator rows that nobody stores)
       const bool phantom = MODE != WGRAD && !GATHER && !CPG &&
                            __shfl_sync(0xffffffffu, m0 + (rank ? 0 : BM) >= s_efo[te + 1], 0);
-      const uint32_t tx_bytes = S::TX_BYTES - (phantom ? S::A_BYTES : 0);
+      const uint32_t tx_bytes = S::TX_BYTES - (phantom ? S::A_BYTES : 0) - (cols == BN ? 0 : S::B_BYTES);
       const bool load_a = !(phantom && rank == 1);
       for (int kt = kt0; kt < kt0 + nkt; ++kt) {
         ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * stage, phase ^ 1));
@@ -482,7 +513,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (a_mn) tma_load_2d_pair(a_dst, &tmap_a, full, m0, kt * BK);
           else if (!GATHER && !CPG && load_a) tma_load_2d_pair(a_dst, &tmap_a, full, kt * BK, a_row);
           if (b_mn) tma_load_2d_pair(b_dst, &tmap_b, full, b_row, b_k0 + kt * BK);
-          else tma_load_2d_pair(b_dst, &tmap_b, full, kt * BK, b_row);
+          else tma_load_2d_pair(b_dst, tb, full, kt * BK, b_row);
         }
         if (GATHER) {
           __syncwarp();
@@ -514,15 +545,17 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const uint32_t a_lo0 = ((smem_base & 0x3FFFF) >> 4) | ((a_mn ? (uint32_t)(S::A_BYTES >> 4) : 1u) << 16);
       const uint32_t b_lo0 = (((smem_base + S::A_BYTES) & 0x3FFFF) >> 4) | ((b_mn ? (uint32_t)(S::B_BYTES >> 4) : 1u) << 16);
       const uint32_t sf_lo0 = (sf_base & 0x3FFFF) >> 4;
-      const int n_total_u = __shfl_sync(0xffffffffu, n_total, 0);
+      const int n_work_u = __shfl_sync(0xffffffffu, s_tiles[1], 0);
       int stage = 0, as = 0, sfs = 0;
       uint32_t phase = 0, aphase = 0, sfphase = 0;
       bool ok = true;
-      for (int tile = pair_id; tile < n_total_u && ok; tile += n_pairs_grid) {
-        const PairTile t = pair_tile<BN, MODE>(tile, 0, p, s_efo, s_pairs);
+      for (int tile = pair_id; tile < n_work_u && ok; tile += n_pairs_grid) {
+        const PairTile t = tile_of(tile, 0);
         const int nkt = __shfl_sync(0xffffffffu, t.nkt, 0);
         if (nkt == 0) continue;
         const int n0 = __shfl_sync(0xffffffffu, t.n0, 0);
+        // N field of the instruction descriptor: columns / 8
+        const uint32_t n_less = S::HALVES && __shfl_sync(0xffffffffu, t.cols, 0) != BN ? (uint32_t)(BN / 16) << 17 : 0u;
         ok = __all_sync(0xffffffffu, mbar_wait(bar_tempty + 8 * as, aphase ^ 1));
         if (!ok) break;
         tc_fence_after();
@@ -550,7 +583,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               tc_cp_sf_pair_lo(sfb_t + 4 * j, sf_lo + ((S::SF_GROUP * 512 * (1 + j)) >> 4), sf_hi);
 #pragma unroll
             for (int kb = 0; kb < BK / 32; ++kb)
-              mma_mxf8_pair_lo(d_tmem, a_lo + a_step * kb, b_lo + b_step * kb, desc_hi, idesc_kb[kb], sfa_t,
+              mma_mxf8_pair_lo(d_tmem, a_lo + a_step * kb, b_lo + b_step * kb, desc_hi, idesc_kb[kb] - n_less, sfa_t,
                                sfb_t + sfb_shift, (k | kb) != 0);
             tc_commit_pair(bar_empty + 8 * stage, 3);
             if (sf_done) tc_commit_pair(bar_sfempty + 8 * sfs, 3);
@@ -576,13 +609,13 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // the warps run ahead as far as the ring has free stages.
     const int gw = warp - (2 + S::EPI_WARPS);           // rows [32 gw, 32 gw + 32) of the tile
     const int sub = lane >> 3, ch = lane & 7;
-    const int n_total_u = __shfl_sync(0xffffffffu, n_total, 0);
+    const int n_work_u = __shfl_sync(0xffffffffu, s_tiles[1], 0);
     const uint8_t* xq = reinterpret_cast<const uint8_t*>(p.a_src);
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int tile = pair_id; tile < n_total_u && ok; tile += n_pairs_grid) {
-      const PairTile tl = pair_tile<BN, MODE>(tile, rank, p, s_efo, s_pairs);
+    for (int tile = pair_id; tile < n_work_u && ok; tile += n_pairs_grid) {
+      const PairTile tl = tile_of(tile, rank);
       const int nkt = __shfl_sync(0xffffffffu, tl.nkt, 0);
       if (nkt == 0) continue;
       const int valid = __shfl_sync(0xffffffffu, tl.valid, 0);
@@ -621,10 +654,10 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // fence and the remote arrival of one stage overlap those of the others (a single thread walking the stages in
     // order forwarded one K tile per ~0.8 us and throttled the whole kernel).
     const uint32_t full0 = map_to_cta(bar_full, 0);
-    const int n_total_u = __shfl_sync(0xffffffffu, n_total, 0);
+    const int n_work_u = __shfl_sync(0xffffffffu, s_tiles[1], 0);
     int total_kt = 0;                                     // K tiles this CTA pair will run
-    for (int tile = pair_id; tile < n_total_u; tile += n_pairs_grid) {
-      const PairTile tl = pair_tile<BN, MODE>(tile, rank, p, s_efo, s_pairs);
+    for (int tile = pair_id; tile < n_work_u; tile += n_pairs_grid) {
+      const PairTile tl = tile_of(tile, rank);
       total_kt += __shfl_sync(0xffffffffu, tl.nkt, 0);
     }
     bool ok = true;
@@ -644,12 +677,12 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // ------------------------------------------------------------ scale producer (both CTAs)
     if (lane == 0) { prefetch_tmap(&tmap_sfa); prefetch_tmap(&tmap_sfb); }
     const uint32_t sffull0 = map_to_cta(bar_sffull, 0);
-    const int n_total_u = __shfl_sync(0xffffffffu, n_total, 0);
+    const int n_work_u = __shfl_sync(0xffffffffu, s_tiles[1], 0);
     int sfs = 0;
     uint32_t sfphase = 0;
     bool ok = true;
-    for (int tile = pair_id; tile < n_total_u && ok; tile += n_pairs_grid) {
-      const PairTile tl = pair_tile<BN, MODE>(tile, rank, p, s_efo, s_pairs);
+    for (int tile = pair_id; tile < n_work_u && ok; tile += n_pairs_grid) {
+      const PairTile tl = tile_of(tile, rank);
       const int nkt = __shfl_sync(0xffffffffu, tl.nkt, 0);
       if (nkt == 0) continue;
       const int kt0 = __shfl_sync(0xffffffffu, tl.kt0, 0);
@@ -691,10 +724,11 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     int as = 0;
     uint32_t aphase = 0;
     bool ok = true;
-    for (int tile = pair_id; tile < n_total && ok; tile += n_pairs_grid) {
-      const PairTile t = pair_tile<BN, MODE>(tile, rank, p, s_efo, s_pairs);
+    for (int tile = pair_id; tile < s_tiles[1] && ok; tile += n_pairs_grid) {
+      const PairTile t = tile_of(tile, rank);
       const size_t grow = (size_t)t.m0 + row_in_tile;
-      const int c_base = t.n0 + half * COLS_PER_WARP;
+      const int warp_cols = S::HALVES ? t.cols / 2 : COLS_PER_WARP;     // this warp's columns
+      const int c_base = t.n0 + half * warp_cols;
       if (t.nkt == 0) {
         if (MODE == WGRAD && p.out_bf16) {
           uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.c) +
@@ -728,7 +762,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       ok = __shfl_sync(0xffffffff, ok, 0);
       if (!ok) break;
       tc_fence_after();
-      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + as * BN + half * COLS_PER_WARP;
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + as * BN + half * warp_cols;
 
       bool released = false;
       if (MODE == PLAIN) {
@@ -737,7 +771,9 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         constexpr int NC = COLS_PER_WARP / 32;
         uint32_t pk[NC][16];
 #pragma unroll
-        for (int c = 0; c < NC; c += 2) {      // two TMEM loads in flight per wait: the drain is what the MMA waits for
+        for (int c = 0; c < NC; c += 2) {
+          if (c * 32 >= warp_cols) break;
+          // two TMEM loads in flight per wait: the drain is what the MMA waits for
           uint32_t r0[32], r1[32];
           tmem_ld32(t_row + c * 32, r0);
           if (c + 1 < NC) tmem_ld32(t_row + (c + 1) * 32, r1);
@@ -757,6 +793,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         released = true;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
+          if (c * 32 >= warp_cols) break;
           const uint32_t sb = stg;                 // one 2 KB staging buffer per warp
           if (lane == 0) bulk_wait_group_read<0>();
           __syncwarp();
@@ -853,18 +890,18 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         constexpr int CHUNKS = BN / 64, PER = (CHUNKS + S::COL_GROUPS - 1) / S::COL_GROUPS;
         constexpr bool DRAIN = (S::ACC_STAGES == 1);
         const int Nz = p.N, Ny = p.N / 2;
-        const int ch0 = half * PER;
-        const int nch = min(PER, CHUNKS - ch0);
-        const uint32_t t_tile = tmem_base + ((uint32_t)(q * 32) << 16) + as * BN;
+        const int z0 = t.n0 + half * (S::HALVES ? warp_cols : PER * 64);      // this warp's first z column
+        const int nch = S::HALVES ? warp_cols / 64 : min(PER, CHUNKS - half * PER);
+        const uint32_t t_z = tmem_base + ((uint32_t)(q * 32) << 16) + as * BN + (z0 - t.n0);
         uint32_t acc[DRAIN ? PER * 2 * 32 : 32];
         if (DRAIN) {
           static_assert(!DRAIN || PER * 2 * 32 == 128, "the single-accumulator tile is 256 wide: 128 columns per warp");
           if constexpr (!CPG) {
-            tmem_ld128(t_tile + ch0 * 64, reinterpret_cast<uint32_t(&)[128]>(acc));
+            tmem_ld128(t_z, reinterpret_cast<uint32_t(&)[128]>(acc));
           } else {      // sixteen warps per CTA leave 128 registers a thread: no room for one 128-register load
 #pragma unroll
             for (int c = 0; c < PER * 2; ++c)
-              tmem_ld32(t_tile + ch0 * 64 + c * 32, reinterpret_cast<uint32_t(&)[32]>(acc[DRAIN ? c * 32 : 0]));
+              tmem_ld32(t_z + c * 32, reinterpret_cast<uint32_t(&)[32]>(acc[DRAIN ? c * 32 : 0]));
           }
           tmem_ld_wait();
           tc_fence_before();
@@ -875,7 +912,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
         for (int ci = 0; ci < PER; ++ci) {
           if (ci >= nch || !live) break;
-          const int zc = t.n0 + (ch0 + ci) * 64;           // first z column of the chunk
+          const int zc = z0 + ci * 64;                     // first z column of the chunk
           float y[32];
           uint32_t zs = 0;
           // staging: z 32 rows x 64 B (64B swizzle) at stg, y1 32 rows x 32 B (32B swizzle) at stg + 2048
@@ -885,7 +922,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           for (int h = 0; h < 2; ++h) {
             uint32_t rl[32];
             if (!DRAIN) {
-              tmem_ld32(t_tile + (ch0 + ci) * 64 + h * 32, rl);
+              tmem_ld32(t_z + ci * 64 + h * 32, rl);
               tmem_ld_wait();
             }
             const uint32_t* r = DRAIN ? &acc[DRAIN ? (ci * 2 + h) * 32 : 0] : rl;

@@ -1063,6 +1063,39 @@ def test_quant_weight_both_orientations_from_one_read(ops, E, N, K):
     assert none_q is None and none_i is None and torch.equal(only_qt, q_t) and torch.equal(only_ci, ci)
 
 
+@pytest.mark.parametrize("tiles,N", [([41, 33], 512), ([1] * 37, 768), ([111], 512), ([1, 0, 2, 1], 256), ([73, 3], 512)])
+def test_gemms_whose_last_wave_is_done_in_half_tiles(ops, tiles, N):
+    """76, 111, 112, 3 and 78 tiles of 256 columns on 74 CTA pairs: 2, 37 (the most), 38 (one too many), 3 and 4 left; odd row
+    tiles among them.  The down-projection against a matmul, the up-projection against the kernel with 128 columns, whose sums
+    may differ by the order within an instruction."""
+    from sonicmoe._lib import lib
+    K, E = 256, len(tiles)
+    g = torch.Generator().manual_seed(sum(tiles) + N)
+    efo = make_efo(tiles)
+    rows = int(efo[-1])
+    (a_q, a_sc), (b_q, b_sc) = rand_fp8((rows, K), g), rand_fp8((E, N, K), g)
+    a_d, b_d, efo_d = a_q.to(DEV), b_q.to(DEV), efo.to(DEV)
+    a_sf = Q.pack_isa(a_sc, rows, K).to(DEV)
+    b_sf = Q.pack_isa(b_sc.reshape(E * N, K // 32), E * N, K).to(DEV)
+    c = ops.gemm_varlen_m(a_d, a_sf, b_d, b_sf, efo_d)
+    got = ops.gemm_gated(a_d, None, a_sf, b_d, b_sf, efo_d, rows)
+    lib.smoe_internal_gemm_knobs(128)
+    try:
+        ref = ops.gemm_gated(a_d, None, a_sf, b_d, b_sf, efo_d, rows)
+        torch.cuda.synchronize()
+    finally:
+        lib.smoe_internal_gemm_knobs(0)
+    ops.check_status(DEV)
+    A, B = deq(a_q, a_sc).to(DEV), deq(b_q, b_sc).to(DEV)
+    for e in range(E):
+        r0, r1 = int(efo[e]), int(efo[e + 1])
+        if r1 > r0:
+            cos, rr = stats(c[r0:r1], A[r0:r1] @ B[e].T)
+            assert cos > 0.99999 and rr < 4e-3, (e, cos, rr)
+    for x, y in zip(got, ref):
+        assert (x != y).float().mean() < 2e-3
+
+
 @pytest.mark.parametrize("layout", [0, 1, 2, 3])
 @pytest.mark.parametrize("M,N,tiles", [(256, 256, [1, 0, 2, 1]), (512, 768, [3, 2, 0, 0, 4, 1, 1, 2]), (256, 384 * 4, [9, 0, 5])])
 def test_gemm_wgrad_bf16_is_the_rounded_f32_product(ops, layout, M, N, tiles):
