@@ -40,9 +40,11 @@ struct Gemm3Smem {
   static constexpr int EPI_BUFS = 2;                            // staging buffers per warp, used in turn
   static constexpr int EPI_BYTES_PER_WARP = EPI_BUFS * 2048;    // bf16 32x32 or f32 32x16 per buffer
   static constexpr int EPI_BYTES = EPI_WARPS * EPI_BYTES_PER_WARP;
+  static constexpr int SINK_BYTES = MODE == WGRAD ? kReducePiece : 0;      // where pieces of the old gradient land
   static constexpr int AUX_BYTES = 512 + 2 * (kMaxExperts2 + 1) * 4 + 8;
   static constexpr int STAGES = 4;
-  static constexpr int TOTAL = STAGES * STAGE_BYTES + SF_BYTES + EPI_BYTES + AUX_BYTES + 1024;
+  static constexpr int TOTAL = STAGES * STAGE_BYTES + SF_BYTES + EPI_BYTES + SINK_BYTES + AUX_BYTES + 1024;
+  static_assert((2 * STAGES + 4 + 2 * SF_SLOTS + kReduceLoads * EPI_WARPS) * 8 <= 496, "barrier storage");
   static_assert(TOTAL <= 227 * 1024, "shared memory budget");
   static constexpr int SF_COLS = 4 + 4 * SFB_TILES;             // TMEM columns of one stage's scales
   static constexpr int SF_COL0 = kBN3;
@@ -72,12 +74,14 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sfring = smem + S::STAGES * S::STAGE_BYTES;
   uint8_t* epi = sfring + S::SF_BYTES;
-  uint8_t* aux = epi + S::EPI_BYTES;
+  uint8_t* sink = epi + S::EPI_BYTES;
+  uint8_t* aux = sink + S::SINK_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(aux);     // full[S], empty[S], tfull[2], tempty[2], sffull[2], sfempty[2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux + 496);
   volatile int* s_abort = reinterpret_cast<volatile int*>(aux + 500);
   int* s_efo = reinterpret_cast<int*>(aux + 512);
   int* s_pairs = s_efo + (kMaxExperts2 + 1);
+  volatile int* s_loads_old = s_pairs + (kMaxExperts2 + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -90,10 +94,14 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const uint32_t bar_tempty = bar_tfull + 8 * 2;
   const uint32_t bar_sffull = bar_tempty + 8 * 2;
   const uint32_t bar_sfempty = bar_sffull + 8 * S::SF_SLOTS;
+  const uint32_t bar_old = bar_sfempty + 8 * S::SF_SLOTS;  // pieces of the old gradient, kReduceLoads a warp
 
   for (int i = threadIdx.x; i <= p.E; i += blockDim.x) s_efo[i] = p.efo[i];
   __syncthreads();
-  if (warp == 2) prefix_row_pairs(s_efo, s_pairs, p.E, lane);
+  if (warp == 2) {
+    prefix_row_pairs(s_efo, s_pairs, p.E, lane);
+    if (MODE == WGRAD) *s_loads_old = loads_old(s_efo, p.E, lane);
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::STAGES; ++s) {
       mbar_init(bar_full + 8 * s, 1);        // leader's: its own producer arms it; both CTAs' copies credit it
@@ -107,6 +115,8 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       mbar_init(bar_sffull + 8 * s, 1);
       mbar_init(bar_sfempty + 8 * s, 1);
     }
+    if (MODE == WGRAD)
+      for (int s = 0; s < kReduceLoads * S::EPI_WARPS; ++s) mbar_init(bar_old + 8 * s, 1);
     *s_abort = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -340,6 +350,7 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     uint32_t aphase = 0;
     int buf = 0;
     bool ok = true;
+    OldPieces old{bar_old + 8 * kReduceLoads * (warp - S::LEAD_WARPS), smem_u32(sink)};
     for (int tile = pair_id; tile < n_total && ok; tile += n_pairs_grid) {
       const PairTile t = pair_tile<BN, MODE>(tile, rank, p, s_efo, s_pairs);
       const size_t grow = (size_t)t.m0 + row_in_tile;
@@ -412,9 +423,14 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       } else {  // WGRAD: f32, one half at a time (96 accumulator registers per half)
         const CUtensorMap* dw_map = t.prob ? &second.c : &tmap_c;
         const int dw_row = t.e * (t.prob ? p.rows2 : p.rows) + t.m0 + q * 32, dw_col = t.n0 + grp * CPW;
-        const bool ahead = p.accumulate && t.nkt <= kReduceAheadKTiles;
-        if (ahead && lane == 0)                                 // the first pieces of the old gradient (see kReduceAhead)
-          for (int c = 0; c < kReduceAhead; ++c) tma_prefetch_l2_2d(dw_map, dw_col + c * 32, dw_row);
+        const bool load_old = p.accumulate && t.nkt <= kReduceLoadKTiles && *s_loads_old;
+        const bool ahead = p.accumulate && !load_old && t.nkt <= kReduceAheadKTiles;
+        if (lane == 0) {                                        // the first pieces of the old gradient
+          if (load_old)
+            for (int c = 0; c < kReduceLoads; ++c) old.ask(dw_map, dw_col + c * 32, dw_row);
+          else if (ahead)
+            for (int c = 0; c < kReduceAhead; ++c) tma_prefetch_l2_2d(dw_map, dw_col + c * 32, dw_row);
+        }
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
           if (lane == 0) ok = mbar_wait(bar_tfull + 8 * h, aphase);
@@ -450,8 +466,14 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
               if (lane == 0) {
-                const int a = h * NC + c + kReduceAhead;          // piece number, three a half
-                if (ahead && a < 2 * NC) tma_prefetch_l2_2d(dw_map, dw_col + a / NC * HN + a % NC * 32, dw_row);
+                const int a = h * NC + c + (load_old ? kReduceLoads : kReduceAhead);      // piece number, three a half
+                const int acol = dw_col + a / NC * HN + a % NC * 32;
+                if (load_old) {
+                  ok &= old.await();
+                  if (a < 2 * NC) old.ask(dw_map, acol, dw_row);
+                } else if (ahead && a < 2 * NC) {
+                  tma_prefetch_l2_2d(dw_map, acol, dw_row);
+                }
                 bulk_wait_group_read<0>();
               }
               __syncwarp();
@@ -463,6 +485,8 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 bulk_commit_group();
               }
             }
+            ok = __shfl_sync(0xffffffff, ok, 0);
+            if (!ok) break;
             continue;
           }
 #pragma unroll
