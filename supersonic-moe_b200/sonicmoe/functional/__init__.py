@@ -663,10 +663,9 @@ class _DownProjection(torch.autograd.Function):
         w2_q, w2_sf, _ = _weight_operand(w2, False, link.get("iso32", False))
         y2 = ops.gemm_varlen_m(y1_q, y1_sf, w2_q, w2_sf, efo, s_scatter_idx, naept)
         del y1_q, y1_sf
-        o = ops.combine(y2, s_rev, naept, topk_scores, int(T), out=link.pop("out_buf", None))
+        o = ops.combine(y2, s_rev, naept, topk_scores, int(T), out=link.pop("out_buf", None), post=True)
         del y2
         _log_stage_memory(link.get("stagewise", False), "forward: after down-projection")
-        ops.post_status(o.device)
         ctx.link = link
         ctx.T = int(T)
         ctx.grad_handle = fp8_combine_grad_handle

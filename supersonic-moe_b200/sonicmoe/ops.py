@@ -100,7 +100,7 @@ def check_status(device):
 
 
 # The layer reads the status word without ever waiting for the GPU: at the end of a forward / backward a kernel (a
-# one-thread kernel of its own; in a one-call forward the combine) stores the word into pinned host memory (a kernel
+# one-thread kernel of its own; in a forward the combine) stores the word into pinned host memory (a kernel
 # store, not a memcpy: it cannot queue behind bulk transfers on a copy engine); the next entry into the layer looks at that host word and raises if it is
 # non-zero.  The word is sticky on the device, so a failure surfaces at the latest one call after the pass whose
 # post saw it, and a healthy run pays at most one tiny launch per pass and no synchronisation.
@@ -691,16 +691,22 @@ def glu_bwd(D, z_q, z_sc, s, act):
 
 # ---------------------------------------------------------------- token side
 @_timed
-def combine(y, s_rev, naept, scores, T, out=None):
+def combine(y, s_rev, naept, scores, T, out=None, post=False):
     """out[t] = sum over the token's lanes of scores * y[row] (bf16, fp32 accumulate); `out` places the result in a
-    caller-owned bf16 [T,H] buffer (e.g. memory that peer GPUs read)."""
+    caller-owned bf16 [T,H] buffer (e.g. memory that peer GPUs read).  `post`: as `post_status`, by the same kernel."""
     _cuda(y, s_rev, naept, scores)
     H = y.shape[1]
     if out is None:
         out = torch.empty(T, H, dtype=torch.bfloat16, device=y.device)
     elif out.dtype != torch.bfloat16 or tuple(out.shape) != (T, H) or not out.is_contiguous() or not out.is_cuda:
         raise ValueError(f"combine: out must be contiguous CUDA bf16 [{T},{H}]")
+    if post and T > 0 and not torch.cuda.is_current_stream_capturing():
+        status, host_word = status_pointers(y.device)
+        check(lib.smoe_combine_post(_p(y), _p(s_rev), _p(naept), _p(scores), _p(out), T, H, status, host_word, _stream()), "combine")
+        return out
     check(lib.smoe_combine(_p(y), _p(s_rev), _p(naept), _p(scores), _p(out), T, H, _stream()), "combine")
+    if post:
+        post_status(y.device)
     return out
 
 
