@@ -165,14 +165,16 @@ static bool use_gemm3(const GemmParams& p) {
   if (p.N % kBN3 != 0 || p.E > kMaxExperts2) return false;
   if (MODE == WGRAD && (p.rows % 256 != 0 || p.b_mn)) return false;
   if (MODE == PLAIN && p.b_mn) return false;      // a 192-byte MN-major slice is not a swizzle atom
-  // PLAIN: wherever N is a multiple of both widths the 256-wide tile is taken, whatever the reduction length and the number of
-  // rows (p.rows is what the caller allocated, not what is routed).  Over N = 768 .. 6144, K = 1536 .. 6144, E = 2 / 8 / 32 and
-  // 1 .. 64 row tiles an expert, 166 of 192 points are faster with it, by 5 % in the median: N=K=3072, E=8, 8 / 16 / 32 / 64 row
-  // tiles 384-wide 76.7 / 112.8 / 209.9 / 425.9 us, 256-wide 72.7 / 112.6 / 204.7 / 418.8; N=K=6144, 8 / 64: 233.5 / 1810 against
-  // 230.3 / 1786.  The others are single counts at which the last wave fills better (up to 10 %), no range.  Where N is a multiple
-  // of 384 only, the choice is between 384 and 192 columns, and the wide one stays for its long products: N=1920, K=3072, E=8, 1 /
-  // 8 / 16 / 64 row tiles 29.7 / 56.3 / 84.9 / 261.1 us against 29.7 / 54.1 / 89.0 / 305.0.
-  if (MODE == PLAIN && g_force_bn == 0 && p.N % 256 == 0) return false;
+  // PLAIN, N a multiple of both widths: the wide tile fetches a sixth fewer operand bytes per MMA, which under the power cap is
+  // time, but its waves are half as long again and its accumulators are handed over in two parts.  It is taken for reductions of
+  // 1536 and more and twelve row tiles an expert and more (as allocated, padding included).  Operands quantised from normal values,
+  // 256-wide / 384-wide, us, 16 and 64 row tiles an expert: N=3072 K=1536 E=8 69.0 / 66.0, 261.8 / 253.5; N=K=3072 120.7 / 114.8, 524.5 /
+  // 509.7; N=6144 K=3072 252.9 / 244.7, 861.7 / 842.2; E=32, 16 row tiles: 292.6 / 280.5, 549.9 / 541.2, 1182 / 1154; over N = 768 to
+  // 6144, 33 of 36 points are faster, by 2.9 % in the median, the others lose 2 % at most.  K = 768 loses 3 to 5 % (N=3072, E=8, 64 row tiles: 147.6 /
+  // 155.2).  At 8 row tiles it is the number of waves (N=K=3072, E=8 69.9 / 71.9, E=32 285.0 / 281.2), at 1 to 4 too (0.67 to 1.35).
+  // Where N is a multiple of 384 only, the choice is between 384 and 192 columns, and the wide one stays for its long products:
+  // N=1920, K=3072, E=8, 1 / 8 / 16 / 64 row tiles 29.7 / 56.3 / 84.9 / 261.1 us against 29.7 / 54.1 / 89.0 / 305.0.
+  if (MODE == PLAIN && g_force_bn == 0 && p.N % 256 == 0) return p.K >= 1536 && p.rows >= 12 * BM * p.E;
   return true;
 }
 
