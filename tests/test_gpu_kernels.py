@@ -1096,6 +1096,25 @@ def test_gemms_whose_last_wave_is_done_in_half_tiles(ops, tiles, N):
         assert (x != y).float().mean() < 2e-3
 
 
+@pytest.mark.parametrize("tiles,K", [([13, 11], 1536), ([12, 11], 1536), ([24, 0], 1408)])
+def test_plain_gemm_either_side_of_the_wide_tile(ops, tiles, K):
+    """N a multiple of 256 and of 384: twelve row tiles an expert and a reduction of 1536, one row tile less, one K tile less."""
+    N, E = 768, len(tiles)
+    g = torch.Generator().manual_seed(sum(tiles) + K)
+    efo = make_efo(tiles)
+    rows = int(efo[-1])
+    (a_q, a_sc), (b_q, b_sc) = rand_fp8((rows, K), g), rand_fp8((E, N, K), g)
+    c = ops.gemm_varlen_m(a_q.to(DEV), Q.pack_isa(a_sc, rows, K).to(DEV), b_q.to(DEV),
+                          Q.pack_isa(b_sc.reshape(E * N, K // 32), E * N, K).to(DEV), efo.to(DEV))
+    ops.check_status(DEV)
+    A, B = deq(a_q, a_sc).to(DEV), deq(b_q, b_sc).to(DEV)
+    for e in range(E):
+        r0, r1 = int(efo[e]), int(efo[e + 1])
+        if r1 > r0:
+            cos, rr = stats(c[r0:r1], A[r0:r1] @ B[e].T)
+            assert cos > 0.99999 and rr < 4e-3, (e, cos, rr)
+
+
 @pytest.mark.parametrize("layout", [0, 1, 2, 3])
 @pytest.mark.parametrize("M,N,tiles", [(256, 256, [1, 0, 2, 1]), (512, 768, [3, 2, 0, 0, 4, 1, 1, 2]), (256, 384 * 4, [9, 0, 5])])
 def test_gemm_wgrad_bf16_is_the_rounded_f32_product(ops, layout, M, N, tiles):
