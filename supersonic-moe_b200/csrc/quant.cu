@@ -687,9 +687,17 @@ quant_cols_rows_kernel(const void* __restrict__ src, const int* __restrict__ idx
   }
   __syncthreads();
   const int rt = rt0 + warp;
-  if (warp < QC_TILES && rt < rt_end && (int64_t)rt * 128 < n_valid)
-    reinterpret_cast<uint4*>(col_isa + ((size_t)ct * (size_t)(rows >> 7) + rt) * 512)[lane] =
-        reinterpret_cast<const uint4*>(s_isa)[threadIdx.x];
+  const int64_t left = n_valid - (int64_t)rt * 128;                   // rows of the warp's tile, if it has any
+  if (warp >= QC_TILES || rt >= rt_end || left <= 0) return;
+  const uint8_t* from = s_isa + threadIdx.x * 16;
+  uint8_t* to = col_isa + ((size_t)ct * (size_t)(rows >> 7) + rt) * 512 + lane * 16;
+  if (left > 96) {
+    *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(from);
+  } else {                                                            // a tile that is not full: byte g of a word is row group g's
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i)
+      if ((i & 3) * 32 < left) to[i] = from[i];
+  }
 }
 
 // q [dim, rows]: the reduction dimension contiguous.  A warp walks the four 32-row groups of a 128-row tile, gathers the bytes

@@ -1276,6 +1276,27 @@ def test_row_major_column_quantizer_walks_every_strip(ops, T, dim, rows, valid):
     assert torch.equal(a[:, :valid // 32], b[:, :valid // 32])
 
 
+@pytest.mark.parametrize("valid", [32, 96, 128, 160, 1056, 1152])
+def test_row_major_column_quantizer_leaves_what_is_beyond_the_valid_rows(ops, valid):
+    """A last tile of one, two or three row groups, and a whole one: payload and scale bytes of the groups at or beyond the valid
+    rows are those the buffers held before."""
+    from sonicmoe._lib import lib
+    T, dim, rows = 500, 256, 1280
+    g = torch.Generator().manual_seed(valid)
+    x = torch.randn(T, dim, generator=g).to(torch.bfloat16)
+    idx = torch.randint(0, T, (rows,), generator=g, dtype=torch.int32)
+    n = torch.tensor([valid], dtype=torch.int32, device=DEV)
+    q = torch.full((rows, dim), 0xA5, dtype=torch.uint8, device=DEV)
+    sf = torch.full((rows * dim // 32,), 0xA5, dtype=torch.uint8, device=DEV)
+    xd, idx_d = x.to(DEV), idx.to(DEV)
+    assert lib.smoe_quant_dual_gather(xd.data_ptr(), idx_d.data_ptr(), n.data_ptr(), rows, dim, None, None, q.data_ptr(),
+                                      sf.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    want_q, want_s = Q.col_quant(x[idx.long()][:valid])
+    got_s = Q.unpack_isa(sf.cpu(), dim, rows)
+    assert torch.equal(q[:valid].cpu(), want_q) and torch.equal(got_s[:, :valid // 32], want_s)
+    assert bool((q[valid:] == 0xA5).all()) and bool((got_s[:, valid // 32:] == 0xA5).all())
+
+
 @pytest.mark.parametrize("how", ["ops", "dispatched", "general"])
 def test_metadata_tables_are_tensors_of_their_own(ops, how):
     """Each table has its own storage and version: one written in place between a forward and a backward leaves the others fit for
