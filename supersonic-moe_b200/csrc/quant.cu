@@ -691,9 +691,9 @@ quant_cols_rows_kernel(const void* __restrict__ src, const int* __restrict__ idx
   if (warp >= QC_TILES || rt >= rt_end || left <= 0) return;
   const uint8_t* from = s_isa + threadIdx.x * 16;
   uint8_t* to = col_isa + ((size_t)ct * (size_t)(rows >> 7) + rt) * 512 + lane * 16;
-  if (left > 96) {
+  if (left > 96 && ((uintptr_t)col_isa & 15) == 0) {
     *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(from);
-  } else {                                                            // a tile that is not full: byte g of a word is row group g's
+  } else {       // a tile that is not full (byte g of a word is row group g's), or scales that start anywhere: byte by byte
 #pragma unroll 1
     for (int i = 0; i < 16; ++i)
       if ((i & 3) * 32 < left) to[i] = from[i];

@@ -1297,6 +1297,27 @@ def test_row_major_column_quantizer_leaves_what_is_beyond_the_valid_rows(ops, va
     assert bool((q[valid:] == 0xA5).all()) and bool((got_s[:, valid // 32:] == 0xA5).all())
 
 
+@pytest.mark.parametrize("off", [1, 4, 8])
+def test_row_major_column_quantizer_takes_scales_that_start_anywhere(ops, off):
+    """`col_isa` has no alignment condition: the same bytes at any address, whole tiles and one that is not full."""
+    from sonicmoe._lib import lib
+    T, dim, rows, valid = 300, 256, 768, 672
+    g = torch.Generator().manual_seed(off)
+    x = torch.randn(T, dim, generator=g).to(torch.bfloat16).to(DEV)
+    idx = torch.randint(0, T, (rows,), generator=g, dtype=torch.int32).to(DEV)
+    n = torch.tensor([valid], dtype=torch.int32, device=DEV)
+    got = []
+    for at in (0, off):
+        q = torch.zeros(rows, dim, dtype=torch.uint8, device=DEV)
+        sf = torch.full((rows * dim // 32 + 16,), 0xA5, dtype=torch.uint8, device=DEV)
+        assert sf.data_ptr() % 16 == 0
+        assert lib.smoe_quant_dual_gather(x.data_ptr(), idx.data_ptr(), n.data_ptr(), rows, dim, None, None, q.data_ptr(),
+                                          sf.data_ptr() + at, torch.cuda.current_stream().cuda_stream) == 0
+        assert bool((sf[:at] == 0xA5).all()) and bool((sf[at + rows * dim // 32:] == 0xA5).all())
+        got.append((q, sf[at:at + rows * dim // 32]))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize("how", ["ops", "dispatched", "general"])
 def test_metadata_tables_are_tensors_of_their_own(ops, how):
     """Each table has its own storage and version: one written in place between a forward and a backward leaves the others fit for
