@@ -165,16 +165,17 @@ static bool use_gemm3(const GemmParams& p) {
   if (p.N % kBN3 != 0 || p.E > kMaxExperts2) return false;
   if (MODE == WGRAD && (p.rows % 256 != 0 || p.b_mn)) return false;
   if (MODE == PLAIN && p.b_mn) return false;      // a 192-byte MN-major slice is not a swizzle atom
-  // PLAIN, N a multiple of both widths: the wide tile fetches a sixth fewer operand bytes per MMA, which under the power cap is
-  // time, but its waves are half as long again and its accumulators are handed over in two parts.  It is taken for reductions of
-  // 1536 and more and twelve row tiles an expert and more (as allocated, padding included).  Operands quantised from normal values,
-  // 256-wide / 384-wide, us, 16 and 64 row tiles an expert: N=3072 K=1536 E=8 69.0 / 66.0, 261.8 / 253.5; N=K=3072 120.7 / 114.8, 524.5 /
-  // 509.7; N=6144 K=3072 252.9 / 244.7, 861.7 / 842.2; E=32, 16 row tiles: 292.6 / 280.5, 549.9 / 541.2, 1182 / 1154; over N = 768 to
-  // 6144, 33 of 36 points are faster, by 2.9 % in the median, the others lose 2 % at most.  K = 768 loses 3 to 5 % (N=3072, E=8, 64 row tiles: 147.6 /
-  // 155.2).  At 8 row tiles it is the number of waves (N=K=3072, E=8 69.9 / 71.9, E=32 285.0 / 281.2), at 1 to 4 too (0.67 to 1.35).
-  // Where N is a multiple of 384 only, the choice is between 384 and 192 columns, and the wide one stays for its long products:
-  // N=1920, K=3072, E=8, 1 / 8 / 16 / 64 row tiles 29.7 / 56.3 / 84.9 / 261.1 us against 29.7 / 54.1 / 89.0 / 305.0.
-  if (MODE == PLAIN && g_force_bn == 0 && p.N % 256 == 0) return p.K >= 1536 && p.rows >= 12 * BM * p.E;
+  // PLAIN: wherever N is a multiple of both widths the 256-wide tile is taken, whatever the reduction length and the number of
+  // rows.  Which one is faster depends on the rows that are routed, by the number of waves at few row tiles an expert and, at many,
+  // because the wide tile fetches a sixth fewer operand bytes per MMA; and the host does not know them: p.rows is what the caller
+  // allocated, six times as much for one of eight ranks.  Operands quantised from normal values, E=8, 256-wide / 384-wide, us, by routed
+  // row tiles an expert, N=6144 K=3072: 2 49.2 / 50.2, 4 68.6 / 72.7, 6 89.1 / 97.3, 8 113.7 / 109.6, 10 134 / 136, 12 161 / 163, 16 215 /
+  // 208, 24 327 / 317; N=K=6144: 4 121.9 / 126.0, 6 164.9 / 183.3, 8 220 / 214, 12 328 / 334, 24 674 / 661; N=3072 K=1536: 16 85.0 / 84.0,
+  // 64 234.5 / 227.3; N=K=3072: 16 133.7 / 126.0, 24 179 / 179, 64 447.5 / 434.2.  (A training step of 64 full row tiles would be 1.1 % faster
+  // with the wide tile, these ranks' GEMMs up to 10 % slower.)  Where N is a multiple of 384 only, the choice is between 384 and 192
+  // columns, and the wide one stays for its long products: N=1920, K=3072, E=8, 1 / 8 / 16 / 64 row tiles 29.7 / 56.3 / 84.9 / 261.1 us
+  // against 29.7 / 54.1 / 89.0 / 305.0.
+  if (MODE == PLAIN && g_force_bn == 0 && p.N % 256 == 0) return false;
   return true;
 }
 
@@ -439,6 +440,12 @@ int smoe_internal_gemm_knobs(int bits) {
   g_force_v1 = (bits >> 17) & 1;
   g_force_gather4 = (bits >> 31) & 1;
   return SMOE_OK;
+}
+
+int smoe_internal_plain_tile(int64_t rows, int64_t N, int64_t K, int64_t E) {
+  GemmParams p{};
+  p.rows = (int)rows; p.N = (int)N; p.K = (int)K; p.E = (int)E;
+  return use_gemm3<PLAIN>(p) ? kBN3 : pick_bn2<PLAIN>(N);
 }
 
 int smoe_gemm_varlen_m_live(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,

@@ -5,9 +5,9 @@
 // tensor clocks instead of 32 KB for 512 - 17 % fewer operand bytes per MMA than the 256 x 256 tile - with no
 // multicast load anywhere (each CTA fetches its own rows of A and of both B halves with plain tiled TMA copies).
 // When it was written that bought 7-9 % on the plain and weight-gradient GEMMs; since the accumulator hand-back no
-// longer stalls (relaxed arrival, see the epilogue) the 256 x 256 kernel runs the activation-gradient GEMM in the
-// same time where reductions are short or rows are few (`use_gemm3` in gemm.cu has the rule).  This kernel is also the one
-// that runs the two weight gradients of a layer in a single launch.
+// longer stalls (relaxed arrival, see the epilogue) either kernel is the faster one for the plain GEMM, by up to 6 and 11 %,
+// as the routed rows have it, and this one stays where N is a multiple of 384 only (`use_gemm3` in gemm.cu has the rule
+// and the figures).  It is also the one that runs the two weight gradients of a layer in a single launch.
 //
 // The two accumulators also hide the accumulator hand-over between tiles: the last J K tiles of a tile are issued
 // half 0 first, so the epilogue drains accumulator 0 under the half-1 MMAs of those K tiles, and the next tile

@@ -1,5 +1,5 @@
-/* Calls between the library's own files, and a symbol it exports for its own tests.  None is part of the product ABI
- * (include/smoe_b200.h); the exported one is process-global and unsynchronised. */
+/* Calls between the library's own files, and two symbols it exports for its own tests.  None is part of the product ABI
+ * (include/smoe_b200.h); the knobs are process-global and unsynchronised. */
 #ifndef SMOE_INTERNAL_H_
 #define SMOE_INTERNAL_H_
 
@@ -13,6 +13,9 @@ extern "C" {
  * automatic); bit 17: force the single-CTA kernel; bit 31: indexed A rows through TMA gather4 instead of the cp.async load warps.
  * 0 restores the defaults. */
 int smoe_internal_gemm_knobs(int bits);
+
+/* Column tile of smoe_gemm_varlen_m on these sizes (rows: as allocated); 0: the single-CTA kernel. */
+int smoe_internal_plain_tile(int64_t rows, int64_t N, int64_t K, int64_t E);
 
 #ifdef __cplusplus
 }

@@ -56,6 +56,15 @@ def test_column_quantizers_refuse_misaligned_buffers(built_library):
     assert lib.smoe_quant_iso32(16, 128, 128, 16, 16, 8, 16, None) == 2
 
 
+@pytest.mark.parametrize("N,tile", [(768, 256), (3072, 256), (6144, 256), (512, 256), (1920, 384), (576, 192), (640, 128)])
+def test_column_tile_of_the_plain_gemm_does_not_depend_on_the_allocation(built_library, N, tile):
+    """A table with masked slots is sized for all of them: rows that are allocated say nothing about rows that are routed."""
+    from sonicmoe._lib import lib
+    for E in (1, 8, 64):
+        for K in (128, 1536, 6144):
+            assert {lib.smoe_internal_plain_tile(128 * E * t, N, K, E) for t in (1, 2, 12, 24, 64)} == {tile}
+
+
 @pytest.mark.parametrize("H,I,E", [(256, 128, 8), (512, 768, 16), (3072, 1536, 8), (4096, 4096, 8), (1024, 1280, 37)])
 def test_arena_sizes_follow_from_the_arguments_alone(built_library, H, I, E):
     """A caller may remember an arena's size by the problem: forcing another column tile between asking and running must not make

@@ -1098,14 +1098,24 @@ def test_gemms_whose_last_wave_is_done_in_half_tiles(ops, tiles, N):
 
 @pytest.mark.parametrize("tiles,K", [([13, 11], 1536), ([12, 11], 1536), ([24, 0], 1408)])
 def test_plain_gemm_either_side_of_the_wide_tile(ops, tiles, K):
-    """N a multiple of 256 and of 384: twelve row tiles an expert and a reduction of 1536, one row tile less, one K tile less."""
+    """N a multiple of 256 and of 384: the 256-wide kernel (the default), the 384-wide one and the 128-wide one, odd row tiles and an
+    empty expert among them, give the same bits, those of a matmul rounded once."""
+    from sonicmoe._lib import lib
     N, E = 768, len(tiles)
     g = torch.Generator().manual_seed(sum(tiles) + K)
     efo = make_efo(tiles)
     rows = int(efo[-1])
     (a_q, a_sc), (b_q, b_sc) = rand_fp8((rows, K), g), rand_fp8((E, N, K), g)
-    c = ops.gemm_varlen_m(a_q.to(DEV), Q.pack_isa(a_sc, rows, K).to(DEV), b_q.to(DEV),
-                          Q.pack_isa(b_sc.reshape(E * N, K // 32), E * N, K).to(DEV), efo.to(DEV))
+    args = (a_q.to(DEV), Q.pack_isa(a_sc, rows, K).to(DEV), b_q.to(DEV), Q.pack_isa(b_sc.reshape(E * N, K // 32), E * N, K).to(DEV),
+            efo.to(DEV))
+    c = ops.gemm_varlen_m(*args)
+    for width in (128, 256, 384):
+        lib.smoe_internal_gemm_knobs(width)
+        try:
+            assert lib.smoe_internal_plain_tile(rows, N, K, E) == width
+            assert torch.equal(ops.gemm_varlen_m(*args), c), width
+        finally:
+            lib.smoe_internal_gemm_knobs(0)
     ops.check_status(DEV)
     A, B = deq(a_q, a_sc).to(DEV), deq(b_q, b_sc).to(DEV)
     for e in range(E):
