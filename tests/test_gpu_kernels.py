@@ -735,6 +735,43 @@ def test_wgrad_accumulation_is_one_f32_addition(ops, bn, M, N, layout):
     assert torch.equal(out, old + fresh)
 
 
+@pytest.mark.parametrize("busy", [16, 17, 21])
+@pytest.mark.parametrize("width", [128, 192, 256, 384, "pair"])
+def test_wgrad_accumulation_over_several_tiles_of_a_cta_pair(ops, width, busy):
+    """More tiles than CTA pairs, experts on both sides of every rule about the old gradient: five K tiles an expert in the mean (16) or
+    just more (17, 21), tiles of five and six K tiles, of twenty at most and of more.  A pair of CTAs goes from tiles that load
+    old pieces to tiles that prefetch them or neither and back; the sums are old + product, to the bit, in every form."""
+    from sonicmoe._lib import lib
+    tiles = [5, 6, 0, 1, 9, 2, 5, 0, 3, 6, 1, busy, 4, 5, 2, 5]
+    assert (sum(tiles) <= 5 * sum(t > 0 for t in tiles)) == (busy == 16)
+    g = torch.Generator().manual_seed(busy)
+    E, N, TKp = len(tiles), 768, 128 * sum(tiles)
+    efo = make_efo(tiles).to(DEV)
+
+    def operand(n):
+        q, sc = rand_fp8((n, TKp), g)
+        return q.to(DEV), Q.pack_isa(sc, n, TKp).to(DEV)
+
+    ops_a = [operand(M) for M in ((1024, 512) if width == "pair" else (1024,))]
+    ops_b = [operand(N) for _ in ops_a]
+    old = [torch.randn(E, a.shape[0], N, generator=g).to(DEV) for a, _ in ops_a]
+    out, fresh = [t.clone() for t in old], [torch.full_like(t, 7.0) for t in old]
+    lib.smoe_internal_gemm_knobs(0 if width == "pair" else width)
+    try:
+        for dst, acc in ((out, True), (fresh, False)):
+            if width == "pair":
+                ops.gemm_wgrad_pair(*ops_a[0], *ops_b[0], dst[0], *ops_a[1], *ops_b[1], dst[1], efo, acc, False)
+            else:
+                ops.gemm_wgrad(*ops_a[0], *ops_b[0], efo, dst[0], accumulate=acc)
+        torch.cuda.synchronize()
+        ops.check_status(DEV)
+    finally:
+        lib.smoe_internal_gemm_knobs(0)
+    for o, f, was in zip(out, fresh, old):
+        assert torch.equal(o, was + f)
+        assert bool((f[2] == 0).all()) and bool((f[11] != 0).any())
+
+
 @pytest.mark.parametrize("layout", [1, 2, 3])
 @pytest.mark.parametrize("M,N,tiles", [(256, 256, [1, 0, 2, 1]), (512, 768, [3, 2, 0, 0, 4, 1, 1, 2]), (768, 256, [2, 1, 3])])
 def test_gemm_wgrad_mn_major_operands(ops, layout, M, N, tiles):
@@ -1066,34 +1103,45 @@ def test_quant_weight_both_orientations_from_one_read(ops, E, N, K):
 @pytest.mark.parametrize("tiles,N", [([41, 33], 512), ([1] * 37, 768), ([111], 512), ([1, 0, 2, 1], 256), ([73, 3], 512)])
 def test_gemms_whose_last_wave_is_done_in_half_tiles(ops, tiles, N):
     """76, 111, 112, 3 and 78 tiles of 256 columns on 74 CTA pairs: 2, 37 (the most), 38 (one too many), 3 and 4 left; odd row
-    tiles among them.  The down-projection against a matmul, the up-projection against the kernel with 128 columns, whose sums
-    may differ by the order within an instruction."""
+    tiles among them.  The down-projection against a matmul; both projections, rows of A as they lie or by index, z kept or not,
+    against the kernel with 128 columns, bit for bit."""
     from sonicmoe._lib import lib
     K, E = 256, len(tiles)
     g = torch.Generator().manual_seed(sum(tiles) + N)
     efo = make_efo(tiles)
     rows = int(efo[-1])
     (a_q, a_sc), (b_q, b_sc) = rand_fp8((rows, K), g), rand_fp8((E, N, K), g)
-    a_d, b_d, efo_d = a_q.to(DEV), b_q.to(DEV), efo.to(DEV)
+    at = torch.randperm(rows, generator=g)                        # row r of A' is row at[r] of x
+    x_q = torch.empty_like(a_q)
+    x_q[at] = a_q
+    a_d, x_d, b_d, at_d, efo_d = a_q.to(DEV), x_q.to(DEV), b_q.to(DEV), at.to(torch.int32).to(DEV), efo.to(DEV)
     a_sf = Q.pack_isa(a_sc, rows, K).to(DEV)
     b_sf = Q.pack_isa(b_sc.reshape(E * N, K // 32), E * N, K).to(DEV)
-    c = ops.gemm_varlen_m(a_d, a_sf, b_d, b_sf, efo_d)
-    got = ops.gemm_gated(a_d, None, a_sf, b_d, b_sf, efo_d, rows)
+    live, naept = torch.arange(rows, dtype=torch.int32, device=DEV), torch.tensor([rows], dtype=torch.int32, device=DEV)
+
+    def forms():
+        out = [ops.gemm_varlen_m(a_d, a_sf, b_d, b_sf, efo_d), *ops.gemm_gated(a_d, None, a_sf, b_d, b_sf, efo_d, rows),
+               *ops.gemm_gated(x_d, at_d, a_sf, b_d, b_sf, efo_d, rows),
+               *ops.gemm_gated_infer(a_d, a_sf, b_d, b_sf, efo_d, live, naept)]
+        torch.cuda.synchronize()
+        ops.check_status(DEV)
+        return out
+
+    got = forms()
     lib.smoe_internal_gemm_knobs(128)
     try:
-        ref = ops.gemm_gated(a_d, None, a_sf, b_d, b_sf, efo_d, rows)
-        torch.cuda.synchronize()
+        ref = forms()
     finally:
         lib.smoe_internal_gemm_knobs(0)
-    ops.check_status(DEV)
+    for i, (x, y) in enumerate(zip(got, ref)):
+        assert torch.equal(x, y), i
+    assert all(torch.equal(x, y) for x, y in zip(got[1:5] + got[3:5], got[5:9] + got[9:11]))
     A, B = deq(a_q, a_sc).to(DEV), deq(b_q, b_sc).to(DEV)
     for e in range(E):
         r0, r1 = int(efo[e]), int(efo[e + 1])
         if r1 > r0:
-            cos, rr = stats(c[r0:r1], A[r0:r1] @ B[e].T)
+            cos, rr = stats(got[0][r0:r1], A[r0:r1] @ B[e].T)
             assert cos > 0.99999 and rr < 4e-3, (e, cos, rr)
-    for x, y in zip(got, ref):
-        assert (x != y).float().mean() < 2e-3
 
 
 @pytest.mark.parametrize("tiles,K", [([13, 11], 1536), ([12, 11], 1536), ([24, 0], 1408)])
@@ -1269,6 +1317,28 @@ def test_scores_and_ds_by_index_match_the_separate_kernels(ops, T, K, E, I):
     check(lib.smoe_ds_slots(P(want[5]), want[5].shape[0], R_, P(md["s_reverse_scatter_idx"]), P(md["naept"]),
                             P(md["score_src_idx"]), T, K, P(out), st), "ds_slots")
     assert torch.equal(out.flatten(), ref.flatten()) and (out.cpu()[idx < 0] == 0).all()
+
+
+@pytest.mark.parametrize("parts", [1, 7, 8, 9, 16, 17, 25])
+def test_ds_slots_add_their_partials_in_order(ops, parts):
+    """Partial sums around whole batches of eight, added one after the other from 0, to the bit; K does not divide a block's slots."""
+    from sonicmoe._lib import check, lib
+    T, K, E = 77, 5, 7
+    idx, probs = make_routing(T, K, E, 0.3, seed=parts)
+    md = ops.topk_metadata(idx.to(DEV), probs.to(DEV), E, 128)
+    R_, n = md["TKp_alloc"], int(md["naept"][-1])
+    part = torch.randn(parts, R_, generator=torch.Generator().manual_seed(parts))
+    part_d, out = part.to(DEV), torch.full((T, K), float("nan"), device=DEV)
+    P = lambda t: t.data_ptr()
+    check(lib.smoe_ds_slots(P(part_d), parts, R_, P(md["s_reverse_scatter_idx"]), P(md["naept"]), P(md["score_src_idx"]), T, K, P(out),
+                            torch.cuda.current_stream().cuda_stream), "ds_slots")
+    mine = part[:, md["s_reverse_scatter_idx"].cpu().long()[:n]]
+    acc = torch.zeros(n)
+    for q in range(parts):
+        acc = acc + mine[q]
+    want = torch.zeros(T * K)
+    want[md["score_src_idx"].cpu().long()[:n]] = acc
+    assert n == int((idx >= 0).sum()) and torch.equal(out.cpu().flatten(), want)
 
 
 @pytest.mark.parametrize("T,dim,rows,valid", [(50, 1280, 640, 640), (200, 2048, 1152, 1056), (40, 1792, 128, 96)])
