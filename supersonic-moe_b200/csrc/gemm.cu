@@ -448,6 +448,10 @@ int smoe_internal_plain_tile(int64_t rows, int64_t N, int64_t K, int64_t E) {
   return use_gemm3<PLAIN>(p) ? kBN3 : pick_bn2<PLAIN>(N);
 }
 
+int smoe_internal_reduce_loads(int k_tiles, int busy, int E, int tiles, int pairs) {
+  return reduce_loads(k_tiles, busy, E, tiles, pairs) ? 1 : 0;
+}
+
 int smoe_gemm_varlen_m_live(const void* a_fp8, const void* a_sf, const void* b_fp8, const void* b_sf, const int* efo,
                             const int* s_scatter_idx, const int* real_tk, void* c_bf16, int64_t rows, int64_t N, int64_t K,
                             int64_t E, int* status, void* stream) {

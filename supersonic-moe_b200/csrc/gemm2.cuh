@@ -23,20 +23,6 @@ constexpr int kMaxExperts2 = 256;   // expert offsets cached in shared memory by
 // 8 K tiles, 730 -> 576, Zipf(1.2), most experts one K tile, 801 -> 771; E=8 M=N=6144, 3 K tiles, 572 -> 461.
 constexpr int kReduceAhead = 2;          // pieces
 constexpr int kReduceAheadKTiles = 20;   // K tiles of a tile up to which it is done
-// With a few K tiles a tile all SMs together ask for more than HBM gives, and what it gives then drops from 6.4 TB/s (read and
-// written) to 5.4: deeper prefetches change nothing, two thirds of the SMs would run at the full rate (dw1, E=128 M=1536 N=2048, 4 K
-// tiles, us by CTA pairs: 74 653, 62 615, 50 521, 44 587; so would all of them, held back by a timer), but how many that takes
-// depends on the clocks.  So up to kReduceLoadKTiles K tiles a warp has its pieces loaded into shared memory, where nobody reads
-// them, and adds to a piece only once it has arrived: never more than two of its pieces are on their way.  us, prefetched -> loaded:
-// dw1 E=128 M=1536 N=2048, 1 / 2 / 3 / 4 / 5 K tiles 590 / 618 / 638 / 663 / 690 -> 524 / 543 / 552 / 567 / 646 (at the rate of a copy
-// 508 to 545); dw1 + dw2 in one launch, E=8 M=6144 + 3072 N=6144, 1 to 5: 700 / 707 / 727 / 748 / 764 -> 619 / 629 / 641 / 649 / 663,
-// N=3072, 179 / 177 / - / 182 / 186 -> 161 / 163 / - / 170 / 173.  At 6 K tiles either is the better one for some sizes (694 -> 663, 458 ->
-// 491, 475 -> 506), from 7 on the MMAs do the pacing (8: 442 -> 521).  One piece on its way: 581 / 571 / 599 / 639, three 579 / - / - /
-// 621, four as many as prefetches: no gain; pieces asked for under the tile before 573 / - / - / 660.
-constexpr int kReduceLoadKTiles = 5;
-constexpr int kReduceLoadMean = 5;      // and K tiles an expert with rows has in the mean
-constexpr int kReduceLoads = 2;
-constexpr int kReducePiece = 4096;       // bytes of a piece
 constexpr int kSfGroup2 = 4;        // K tiles whose scales travel in one TMA copy (box rows of the scale tensor maps)
 
 // ---- cluster helpers -------------------------------------------------------
@@ -243,22 +229,6 @@ __device__ __forceinline__ float warp_max_abs(float x) {
   return r;
 }
 
-// Pieces of an existing gradient on their way into the L2 (see kReduceLoadKTiles); one lane of an epilogue warp
-struct OldPieces {
-  uint32_t bars;                   // kReduceLoads barriers of this warp
-  uint32_t sink;                   // where the bytes land: any warp's may overwrite any other's
-  uint32_t asked = 0, seen = 0;
-  __device__ void ask(const void* tmap, int c0, int c1) {
-    const uint32_t bar = bars + 8 * (asked++ % kReduceLoads);
-    mbar_expect_tx(bar, kReducePiece);
-    tma_load_2d(sink, tmap, bar, c0, c1);
-  }
-  __device__ bool await() {
-    const uint32_t n = seen++;
-    return mbar_wait(bars + 8 * (n % kReduceLoads), (n / kReduceLoads) & 1);
-  }
-};
-
 // CPG: the rows of A are gathered by index inside the kernel with cp.async (four extra load warps per CTA) instead of
 // arriving as TMA tiles of a pre-gathered copy.
 template <int BN, int MODE, bool CPG = false>
@@ -296,15 +266,14 @@ struct Gemm2Smem {
   static constexpr int SF_BYTES = SF_SLOTS * SF_SLOT_BYTES;
   static constexpr int TOTAL = STAGES * STAGE_BYTES + SF_BYTES + EPI_BYTES + AUX_BYTES + 1024;
   static_assert(TOTAL <= 227 * 1024, "shared memory budget");
-  static_assert((3 * STAGES + 4 + 2 * SF_SLOTS + kReduceLoads * EPI_WARPS) * 8 <= 496, "barrier storage");
-  static_assert(MODE != WGRAD || EPI_BYTES >= kReducePiece, "old pieces land where nothing is staged");
+  static_assert((3 * STAGES + 4 + 2 * SF_SLOTS) * 8 <= 496, "barrier storage");
   // WGRAD into an existing f32 gradient: ring stages that hold 4 KB staging tiles (32 rows of 128 bytes, 128-byte swizzle) of
   // the epilogue warps instead; the last ones of the ring, STAGES - LENT_STAGES on
   static constexpr int LENT_TILE = 4096;
   static constexpr int LENT_STAGES = (EPI_WARPS * LENT_TILE + STAGE_BYTES - 1) / STAGE_BYTES;
   static_assert(STAGE_BYTES % 1024 == 0, "operand tiles and lent staging tiles start on swizzle atoms");
   static_assert(LENT_STAGES * STAGE_BYTES >= EPI_WARPS * LENT_TILE, "every epilogue warp has a staging tile");
-  static_assert(MODE != WGRAD || STAGES - LENT_STAGES >= 4, "a ring is left (the timing experiments cut three stages more)");
+  static_assert(MODE != WGRAD || STAGES - LENT_STAGES >= 4, "a ring is left");
   static constexpr int ACC_STAGES = (BN == 256) ? 1 : 2;  // TMEM: 512 columns
   static constexpr bool HALVES = BN == 256 && (MODE == PLAIN || MODE == GATED);    // half tiles at the end of a launch
   static constexpr int SF_COLS = 4 + 4 * SFB_TILES;
@@ -394,17 +363,6 @@ __device__ __forceinline__ void prefix_row_pairs(const int* s_efo, int* s_pairs,
   if (lane == 31 && E == 32 * PER) s_pairs[E] = run;
 }
 
-// Whether a launch loads the pieces of the old gradient (see kReduceLoadKTiles): where its experts have few K tiles on the average.
-// Among many tiles of busy experts, which leave HBM idle, prefetches are the better form for the others too.  Zipf loads, dw1 / dw2,
-// us, prefetched -> loaded: H=2048 I=768 E=128 K=8, 2048 tokens (2 K tiles in the mean) 519 / 271 -> 472 / 252, 4096 (3) 584 / 310 ->
-// 544 / 281, 6144 (4) 632 / 346 -> 597 / 308, 8192 (5) 678 / 374 -> 650 / 364; 16384 (9), not taken, 776 / 437 -> 806 / 448.
-// All lanes of a warp.
-__device__ __forceinline__ int loads_old(const int* s_efo, int E, int lane) {
-  int busy = 0;
-  for (int e = lane; e < E; e += 32) busy += s_efo[e + 1] > s_efo[e];
-  return s_efo[E] / BK <= kReduceLoadMean * (int)__reduce_add_sync(0xffffffffu, busy);
-}
-
 // Whether a warp's 32 rows starting at `row` hold anything to store.  The padding of an expert's segment lies at its end,
 // so a slab whose first row is padding is all padding.  A decode step of 64 tokens over 128 experts has four real rows in
 // each 128-row tile: three of a tile's four slabs are left out.
@@ -431,7 +389,6 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   volatile int* s_tiles = reinterpret_cast<volatile int*>(aux + 504);    // number of whole tiles, number of tiles of either kind
   int* s_efo = reinterpret_cast<int*>(aux + 512);
   int* s_pairs = s_efo + (kMaxExperts2 + 1);
-  volatile int* s_loads_old = s_pairs + (kMaxExperts2 + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -445,13 +402,11 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const uint32_t bar_sffull = bar_tempty + 8 * 2;
   const uint32_t bar_sfempty = bar_sffull + 8 * S::SF_SLOTS;
   const uint32_t bar_landed = bar_sfempty + 8 * S::SF_SLOTS;    // CPG: this CTA's gathered rows of a stage are in place
-  const uint32_t bar_old = bar_landed + 8 * S::STAGES;          // WGRAD: pieces of the old gradient, kReduceLoads a warp
 
   for (int i = threadIdx.x; i <= p.E; i += blockDim.x) s_efo[i] = p.efo[i];
   __syncthreads();
   if (warp == 2) {
     prefix_row_pairs(s_efo, s_pairs, p.E, lane);
-    if (MODE == WGRAD) *s_loads_old = loads_old(s_efo, p.E, lane);
     __syncwarp();
     if (lane == 0) {
       const int n_col_tiles = (p.N + BN - 1) / BN;
@@ -481,8 +436,6 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       mbar_init(bar_sffull + 8 * s, 1);                  // leader's: armed by its producer, credited by both CTAs
       mbar_init(bar_sfempty + 8 * s, 1);                 // commit arrival, in each CTA
     }
-    if (MODE == WGRAD)
-      for (int s = 0; s < kReduceLoads * S::EPI_WARPS; ++s) mbar_init(bar_old + 8 * s, 1);
     *s_abort = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -771,7 +724,6 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     int as = 0;
     uint32_t aphase = 0;
     bool ok = true;
-    OldPieces old{bar_old + 8 * kReduceLoads * (warp - 2), smem_u32(epi)};
     for (int tile = pair_id; tile < s_tiles[1] && ok; tile += n_pairs_grid) {
       const PairTile t = tile_of(tile, rank);
       const size_t grow = (size_t)t.m0 + row_in_tile;
@@ -803,15 +755,9 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         s_row = p.s[p.s_scatter != nullptr ? p.s_scatter[grow] : (int)grow];
       }
       const bool live = (MODE == PLAIN || MODE == GATED) && slab_live(p, t, t.m0 + q * 32);
-      const bool load_old = MODE == WGRAD && p.accumulate && t.nkt <= kReduceLoadKTiles && *s_loads_old;
-      const bool ahead = MODE == WGRAD && p.accumulate && !load_old && t.nkt <= kReduceAheadKTiles;
-      if (MODE == WGRAD && lane == 0 && (load_old || ahead)) {   // the first pieces of the old gradient
-        const int crow = t.e * p.rows + t.m0 + q * 32;
-        if (load_old)
-          for (int c = 0; c < kReduceLoads; ++c) old.ask(&tmap_c, c_base + c * 32, crow);
-        else
-          for (int c = 0; c < kReduceAhead; ++c) tma_prefetch_l2_2d(&tmap_c, c_base + c * 32, crow);
-      }
+      const bool ahead = MODE == WGRAD && p.accumulate && t.nkt <= kReduceAheadKTiles;
+      if (ahead && lane == 0)                                    // the first pieces of the old gradient (see kReduceAhead)
+        for (int c = 0; c < kReduceAhead; ++c) tma_prefetch_l2_2d(&tmap_c, c_base + c * 32, t.e * p.rows + t.m0 + q * 32);
       if (lane == 0) ok = mbar_wait(bar_tfull + 8 * as, aphase);
       ok = __shfl_sync(0xffffffff, ok, 0);
       if (!ok) break;
@@ -905,12 +851,7 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
             if (lane == 0) {
-              if (load_old) {
-                ok &= old.await();
-                if (c + kReduceLoads < NC) old.ask(&tmap_c, c_base + (c + kReduceLoads) * 32, crow);
-              } else if (ahead && c + kReduceAhead < NC) {
-                tma_prefetch_l2_2d(&tmap_c, c_base + (c + kReduceAhead) * 32, crow);
-              }
+              if (ahead && c + kReduceAhead < NC) tma_prefetch_l2_2d(&tmap_c, c_base + (c + kReduceAhead) * 32, crow);
               bulk_wait_group_read<0>();
             }
             __syncwarp();
@@ -922,8 +863,6 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               bulk_commit_group();
             }
           }
-          ok = __shfl_sync(0xffffffff, ok, 0);
-          if (!ok) break;
         } else
 #pragma unroll
         for (int c = 0; c < 2 * NC; ++c) {

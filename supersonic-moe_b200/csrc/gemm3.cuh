@@ -24,6 +24,49 @@ constexpr int kBN3 = 384;          // tile width
 constexpr int kHN3 = 192;          // width of one accumulator
 constexpr int kHeadTail3 = 2;      // K tiles issued half-by-half at both ends of a tile
 
+// Reduce-adds of this kernel into a gradient that lies in HBM.  With a few K tiles a tile all SMs together ask for more than HBM
+// gives, and what it gives then drops from 6.4 TB/s (read and written) to 5.4: deeper prefetches (kReduceAhead) change nothing, two
+// thirds of the SMs would run at the full rate, but how many that takes depends on the clocks.  So a warp has its pieces loaded into
+// shared memory, where nobody reads them, and adds to a piece only once it has arrived: never more than two of its pieces are on
+// their way.  That costs wherever HBM is not what everybody waits for, so it is done for tiles of at most kReduceLoadKTiles K
+// tiles in a launch (`reduce_loads`) that has few K tiles an expert in the mean, where every expert has rows, and many tiles a CTA
+// pair.  Loaded over prefetched, E=8 to 128, 1 to 5 K tiles an expert, even, Zipf and single busy experts, from a cold L2, at full
+// clocks and behind three large GEMMs, which take the clock down:
+//   24 tiles a CTA pair and more, every expert with rows   0.87 to 0.96 and 0.79 to 0.99
+//   15 to 24 tiles                                         0.90 to 1.01 and 0.90 to 1.05
+//   3 to 15 tiles                                          0.92 to 1.05 and 0.93 to 1.11
+//   half the experts without rows, seven eighths           0.90 to 1.11 and 0.92 to 1.18, 1.05 to 1.22 and 1.07 to 1.26
+// us: dw1 + dw2, E=8 M=6144 + 3072 N=6144, 1 / 2 / 3 / 4 / 5 K tiles 700 / 707 / 727 / 748 / 764 -> 619 / 629 / 641 / 649 / 663.  At 6
+// K tiles either is the better one for some sizes, from 7 on the MMAs do the pacing; 9 in the mean and a Zipf load lose 3 %.  One, three
+// or four pieces on their way instead of two: no gain.  The 256-column kernel, with 24 tiles and more and every expert with rows, takes
+// 0.83 to 1.01 at full clocks and 0.89 to 1.14 behind large GEMMs, so it prefetches.
+constexpr int kReduceLoadKTiles = 5;
+constexpr int kReduceLoadMean = 5;
+constexpr int kReduceLoadTiles = 24;     // a CTA pair
+constexpr int kReduceLoads = 2;
+constexpr int kReducePiece = 4096;       // bytes of a piece
+
+// k_tiles: of all experts; busy: experts with rows, of E; tiles: of the launch, for `pairs` CTA pairs
+__host__ __device__ inline bool reduce_loads(int k_tiles, int busy, int E, int tiles, int pairs) {
+  return k_tiles <= kReduceLoadMean * E && busy == E && tiles >= kReduceLoadTiles * pairs;
+}
+
+// Pieces of an existing gradient on their way into the L2; one lane of an epilogue warp
+struct OldPieces {
+  uint32_t bars;                   // kReduceLoads barriers of this warp
+  uint32_t sink;                   // where the bytes land: any warp's may overwrite any other's
+  uint32_t asked = 0, seen = 0;
+  __device__ void ask(const void* tmap, int c0, int c1) {
+    const uint32_t bar = bars + 8 * (asked++ % kReduceLoads);
+    mbar_expect_tx(bar, kReducePiece);
+    tma_load_2d(sink, tmap, bar, c0, c1);
+  }
+  __device__ bool await() {
+    const uint32_t n = seen++;
+    return mbar_wait(bars + 8 * (n % kReduceLoads), (n / kReduceLoads) & 1);
+  }
+};
+
 template <int MODE>
 struct Gemm3Smem {
   static constexpr int A_BYTES = BM * BK;                       // this CTA's 128 rows of A
@@ -100,7 +143,12 @@ gemm3_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   __syncthreads();
   if (warp == 2) {
     prefix_row_pairs(s_efo, s_pairs, p.E, lane);
-    if (MODE == WGRAD) *s_loads_old = loads_old(s_efo, p.E, lane);
+    if (MODE == WGRAD) {
+      int busy = 0;
+      for (int e = lane; e < p.E; e += 32) busy += s_efo[e + 1] > s_efo[e];
+      busy = (int)__reduce_add_sync(0xffffffffu, busy);
+      *s_loads_old = reduce_loads(s_efo[p.E] / BK, busy, p.E, p.E * ((p.rows + p.rows2) / (2 * BM)) * (p.N / BN), n_pairs_grid);
+    }
   }
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::STAGES; ++s) {

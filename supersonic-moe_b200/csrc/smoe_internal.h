@@ -1,4 +1,4 @@
-/* Calls between the library's own files, and two symbols it exports for its own tests.  None is part of the product ABI
+/* Calls between the library's own files, and three symbols it exports for its own tests.  None is part of the product ABI
  * (include/smoe_b200.h); the knobs are process-global and unsynchronised. */
 #ifndef SMOE_INTERNAL_H_
 #define SMOE_INTERNAL_H_
@@ -16,6 +16,10 @@ int smoe_internal_gemm_knobs(int bits);
 
 /* Column tile of smoe_gemm_varlen_m on these sizes (rows: as allocated); 0: the single-CTA kernel. */
 int smoe_internal_plain_tile(int64_t rows, int64_t N, int64_t K, int64_t E);
+
+/* 1 where a weight-gradient launch of the 384-column kernel loads the old gradient ahead of its sums: k_tiles of all experts, busy
+ * experts of E, output tiles on so many CTA pairs. */
+int smoe_internal_reduce_loads(int k_tiles, int busy, int E, int tiles, int pairs);
 
 #ifdef __cplusplus
 }

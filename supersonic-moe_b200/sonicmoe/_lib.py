@@ -92,6 +92,8 @@ SIGNATURES = {
 # exported for the library's own tests only (csrc/smoe_internal.h); not product ABI
 INTERNAL_SIGNATURES = {
     "smoe_internal_gemm_knobs": (_I, [_I]),
+    "smoe_internal_plain_tile": (_I, [_L, _L, _L, _L]),
+    "smoe_internal_reduce_loads": (_I, [_I, _I, _I, _I, _I]),
 }
 
 ERRORS = {1: "SMOE_ERR_SHAPE", 2: "SMOE_ERR_ALIGN", 3: "SMOE_ERR_DRIVER", 4: "SMOE_ERR_TMAP", 5: "SMOE_ERR_LAUNCH",

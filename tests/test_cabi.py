@@ -65,6 +65,16 @@ def test_column_tile_of_the_plain_gemm_does_not_depend_on_the_allocation(built_l
             assert {lib.smoe_internal_plain_tile(128 * E * t, N, K, E) for t in (1, 2, 12, 24, 64)} == {tile}
 
 
+@pytest.mark.parametrize("k_tiles,busy,E,tiles,loads", [
+    (740, 148, 148, 1776, 1), (741, 148, 148, 1776, 0), (740, 148, 148, 1775, 0), (700, 147, 148, 1776, 0),
+    (8, 8, 8, 1152, 0), (16, 16, 16, 128, 0), (96, 32, 256, 12288, 0), (28, 8, 8, 4608, 1), (0, 0, 8, 4608, 0)])
+def test_old_gradients_are_loaded_ahead_only_where_hbm_is_what_every_sum_waits_for(built_library, k_tiles, busy, E, tiles, loads):
+    """Five K tiles an expert, every expert with rows and 24 tiles for each of 74 CTA pairs, and one less or more of each; launches
+    of few tiles and of mostly idle experts, which the loads would hold up."""
+    from sonicmoe._lib import lib
+    assert lib.smoe_internal_reduce_loads(k_tiles, busy, E, tiles, 74) == loads
+
+
 @pytest.mark.parametrize("H,I,E", [(256, 128, 8), (512, 768, 16), (3072, 1536, 8), (4096, 4096, 8), (1024, 1280, 37)])
 def test_arena_sizes_follow_from_the_arguments_alone(built_library, H, I, E):
     """A caller may remember an arena's size by the problem: forcing another column tile between asking and running must not make

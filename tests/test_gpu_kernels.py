@@ -738,12 +738,10 @@ def test_wgrad_accumulation_is_one_f32_addition(ops, bn, M, N, layout):
 @pytest.mark.parametrize("busy", [16, 17, 21])
 @pytest.mark.parametrize("width", [128, 192, 256, 384, "pair"])
 def test_wgrad_accumulation_over_several_tiles_of_a_cta_pair(ops, width, busy):
-    """More tiles than CTA pairs, experts on both sides of every rule about the old gradient: five K tiles an expert in the mean (16) or
-    just more (17, 21), tiles of five and six K tiles, of twenty at most and of more.  A pair of CTAs goes from tiles that load
-    old pieces to tiles that prefetch them or neither and back; the sums are old + product, to the bit, in every form."""
+    """More tiles than CTA pairs, tiles of no K tile, of twenty at most and of more: a pair of CTAs goes from tiles that prefetch old
+    pieces to tiles that do not and back; the sums are old + product, to the bit, in every form."""
     from sonicmoe._lib import lib
     tiles = [5, 6, 0, 1, 9, 2, 5, 0, 3, 6, 1, busy, 4, 5, 2, 5]
-    assert (sum(tiles) <= 5 * sum(t > 0 for t in tiles)) == (busy == 16)
     g = torch.Generator().manual_seed(busy)
     E, N, TKp = len(tiles), 768, 128 * sum(tiles)
     efo = make_efo(tiles).to(DEV)
@@ -770,6 +768,43 @@ def test_wgrad_accumulation_over_several_tiles_of_a_cta_pair(ops, width, busy):
     for o, f, was in zip(out, fresh, old):
         assert torch.equal(o, was + f)
         assert bool((f[2] == 0).all()) and bool((f[11] != 0).any())
+
+
+@pytest.mark.parametrize("form", ["pair", "single"])
+@pytest.mark.parametrize("case", ["loads", "few tiles", "idle expert", "long"])
+def test_wgrad_accumulation_where_old_pieces_are_loaded(ops, form, case):
+    """The smallest launch whose old gradients are loaded ahead of the sums, and one expert less, one idle and a K tile an expert too many.
+    Tiles of five, of six and of more K tiles follow one another in a CTA pair; the sums are old + product, to the bit."""
+    from sonicmoe._lib import lib
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    E, N = 2 * pairs - (case == "few tiles"), 1152                      # 12 tiles an expert
+    Ms = (512, 512) if form == "pair" else (1024,)
+    tiles = [(1, 5, 2, 6, 1, 1, 5, 9, 3, 1, 2)[e % 11] for e in range(E)]
+    tiles[0] = 2 - 2 * (case == "idle expert")
+    if case == "long":
+        tiles[E // 2] += 5 * E + 1 - sum(tiles)
+    assert lib.smoe_internal_reduce_loads(sum(tiles), sum(t > 0 for t in tiles), E, 12 * E, pairs) == (case == "loads")
+    TKp, efo = 128 * sum(tiles), make_efo(tiles).to(DEV)
+    g = torch.Generator(DEV).manual_seed(E + len(Ms))
+
+    def operand(n):                                                     # any scale bytes will do, in whatever order
+        q = torch.randint(0, 256, (n, TKp), generator=g, dtype=torch.uint8, device=DEV)
+        return torch.where((q & 0x7F) == 0x7F, q & 0xF0, q), torch.randint(118, 127, (n * TKp // 32,), generator=g, dtype=torch.uint8,
+                                                                           device=DEV)
+
+    ops_a, ops_b = [operand(M) for M in Ms], [operand(N) for _ in Ms]
+    old = [torch.randn(E, M, N, generator=g, device=DEV) for M in Ms]
+    out, fresh = [t.clone() for t in old], [torch.full_like(t, 7.0) for t in old]
+    for dst, acc in ((out, True), (fresh, False)):
+        if form == "pair":
+            ops.gemm_wgrad_pair(*ops_a[0], *ops_b[0], dst[0], *ops_a[1], *ops_b[1], dst[1], efo, acc, False)
+        else:
+            ops.gemm_wgrad(*ops_a[0], *ops_b[0], efo, dst[0], accumulate=acc)
+    torch.cuda.synchronize()
+    ops.check_status(DEV)
+    for o, f, was in zip(out, fresh, old):
+        assert torch.equal(o, was + f) and bool((f[1] != 0).any())
+        assert bool((f[0] == 0).all()) == (case == "idle expert")
 
 
 @pytest.mark.parametrize("layout", [1, 2, 3])
