@@ -86,7 +86,8 @@ __global__ void ds_finalize_kernel(const float* __restrict__ part, int partials,
 // the slots they came from, so that a slot finds its entry with one look (or none: masked, zero) and every store is in order.
 // Bound by latency (a few hundred bytes a thread in a chain of loads), so blocks are small and a thread's partial sums are loaded
 // eight at a time, added in order.  Against a thread searching its token's entries, in blocks of 256, T=1024, K=8, 16 partials:
-// 20.5 -> 10.3 us between events, from a cold L2.
+// 20.5 -> 10.3 us between events, from a cold L2; T=8192 K=8, 12 partials 18.5 -> 10.2; K=1, where nothing was searched, the same up
+// to T=8192 and one to two us more from T=16384 on.
 constexpr int kDsSlots = 64;
 
 __global__ void __launch_bounds__(kDsSlots)

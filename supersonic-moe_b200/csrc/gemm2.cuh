@@ -415,8 +415,10 @@ gemm2_mxf8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       // as pairs, each is done as two tiles of half the columns (B K-major: the halves have a tensor map of their own).
       // us, H=3072, I=1536, E=8, up-projection / down-projection / dx: 1024 rows an expert (384 tiles, 14 left) 81.3 / 47.1 / 70.8 ->
       // 78.1 / 45.4 / 69.9, 2048 rows (28 left) 146.4 / 81.7 / 132.2 -> 144.1 / 80.3 / 131.2, 128 rows 37.8 / 22.9 / 33.1 -> 35.0 /
-      // 20.9 / 31.1; H=6144, I=3072, 384 rows (14 left) 161.4 / 84.3 / 141.7 -> 156.1 / 82.0 / 138.4.  With more left than that no
-      // pair would have less to do.
+      // 20.9 / 31.1; H=6144, I=3072, 384 rows (14 left) 161.4 / 84.3 / 141.7 -> 156.1 / 82.0 / 138.4.  Over seven layer sizes, E=8 to
+      // 128, one to twelve row tiles an expert, with halves over without: less than one wave 0.83 to 0.97, one to two 0.92 to 1.00,
+      // to eleven 0.97 to 0.99, beyond 0.99 to 1.00; launches that have none 1.002 in the median.  With more left than that no pair
+      // would have less to do.
       const int left = S::HALVES && !p.b_mn ? n_total % n_pairs_grid : 0;
       s_tiles[0] = 2 * left <= n_pairs_grid ? n_total - left : n_total;
       s_tiles[1] = 2 * n_total - s_tiles[0];

@@ -60,7 +60,7 @@ __device__ __forceinline__ uint32_t q_e8m0x2(uint32_t m) {
   asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(e), "r"(0x00080008u));
   return r - 0x00080008u;
 }
-// and their scales, 2^(127 - e) as bf16 (e <= 248: NaN)
+// and their scales, 2^(127 - e) as bf16; e <= 247, the exponent of infinity: every maximum starts from 0 and drops NaN
 __device__ __forceinline__ uint32_t q_scalex2(uint32_t e2) { return (0x00FE00FEu - e2) << 7; }
 // A bf16 pair times a pair of powers of two, in f32: exact, one instruction a value where unpacking and multiplying take two, and
 // on another pipe than the conversions; adding -0 keeps the sign of a zero
